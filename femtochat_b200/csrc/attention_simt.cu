@@ -217,6 +217,6 @@ template <> int attention_fwd<bf16>(const AttnArgs& a, cudaStream_t s) {
   return attention_fwd_simt<bf16>(a, s);
 }
 template <> int attention_bwd<bf16>(const AttnArgs& a, cudaStream_t s) {
-  if (attention_tc_supported(a)) return attention_bwd_tc(a, s);
+  if (attention_bwd_tc_supported(a)) return attention_bwd_tc(a, s);
   return attention_bwd_simt<bf16>(a, s);
 }

@@ -41,6 +41,11 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&h);
 }
 
+// What rounding (lo, hi) to the packed pair `h` left over, rounded in turn: together they hold 16 bits of each.
+__device__ __forceinline__ uint32_t rest_bf16(float lo, float hi, uint32_t h) {
+  return pack_bf16(lo - __uint_as_float(h << 16), hi - __uint_as_float(h & 0xffff0000u));
+}
+
 // Optional cycle accounting of the roles of the persistent forward kernels (compiled in with -DFEMTO_ATTN_CYCLES,
 // printed by the launcher when FEMTO_ATTN_PROF is set in the environment): consecutive laps of clock64(), summed per
 // role in CTA 0.  In a normal build every member is empty.
@@ -338,6 +343,11 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 // item's O out of tensor memory.
 constexpr int PF_SMEM = TILE_BYTES * 6 + 1024 + 256 + 3 * NS * 128 * 4;
 
+// RAGGED: T is not a multiple of the tile.  Tensor maps have one dimension per batch column, so the rows past a column's end
+// arrive as zeros and are clipped on the way out; causality masks them for every query of the column.  These lengths used to
+// take the SIMT kernel, which keeps P in fp32, so here P is the sum of two bf16 numbers: its high part lies over the first half
+// of S, its low part over the second, and P V is two products.  5 x 1000 tokens, 6 heads, causal: 2980 -> 25.6 us; 1500 tokens, 10 heads: 2230 -> 20.9 us.
+
 __device__ __forceinline__ void pf_item(const AttnArgs& a, int item, int nqt, int& qt, int& h, int& b) {
   // heavy (late) query tiles first; within a query tile all heads and batch rows cost about the same
   const int hb = a.H * a.B;
@@ -347,6 +357,7 @@ __device__ __forceinline__ void pf_item(const AttnArgs& a, int item, int nqt, in
   b = rem / a.H;
 }
 
+template <bool RAGGED>
 __global__ void __launch_bounds__(FWD_THREADS, 1)
 attn_fwd_persistent_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                            const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO, const FwdParams p,
@@ -374,7 +385,7 @@ attn_fwd_persistent_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid
 
   const AttnArgs& a = p.a;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nqt = a.T / BQ;
+  const int nqt = (a.T + BQ - 1) / BQ;
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2; i++) {
@@ -411,8 +422,15 @@ attn_fwd_persistent_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid
       int jlo = max(0, q0 - a.window_left) / BKV;
       if (a.doc_start) {
         // key tiles that lie before the earliest document start of these 128 queries are fully masked
-        const int4 v = *reinterpret_cast<const int4*>(a.doc_start + row0 + q0 + lane * 4);
-        const int mn = __reduce_min_sync(0xffffffffu, min(min(v.x, v.y), min(v.z, v.w)));
+        int v;
+        if constexpr (RAGGED) {
+          v = a.T;
+          for (int e = 0; e < 4; e++) v = min(v, a.doc_start[row0 + min(q0 + e * 32 + lane, a.T - 1)]);
+        } else {
+          const int4 v4 = *reinterpret_cast<const int4*>(a.doc_start + row0 + q0 + lane * 4);
+          v = min(min(v4.x, v4.y), min(v4.z, v4.w));
+        }
+        const int mn = __reduce_min_sync(0xffffffffu, v);
         jlo = max(jlo, mn / BKV);
       }
       const int ntile = jhi - jlo + 1;
@@ -422,20 +440,20 @@ attn_fwd_persistent_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid
         if (ok) {
           item_jlo[qs] = jlo;
           mbar_expect_tx(&q_full[qs], TILE_BYTES);   // the arrive publishes item_jlo to the roles that wait on q_full
-          tma_load_2d(sQ + qs * TILE_BYTES, &tmQ, &q_full[qs], p.q_col0 + h * HD, (int)(row0 + q0));
-          tma_load_2d(sQ + qs * TILE_BYTES + TILE_BYTES / 2, &tmQ, &q_full[qs], p.q_col0 + h * HD + 64, (int)(row0 + q0));
+          tma_load_3d(sQ + qs * TILE_BYTES, &tmQ, &q_full[qs], p.q_col0 + h * HD, q0, b);
+          tma_load_3d(sQ + qs * TILE_BYTES + TILE_BYTES / 2, &tmQ, &q_full[qs], p.q_col0 + h * HD + 64, q0, b);
           for (int i = 0; i < ntile; i++, tc++) {
             const int st = tc & 1;
             const uint32_t ph2 = ((tc - 2) >> 1) & 1;   // phase of tile tc-2, the previous user of this stage
-            const int krow = (int)(row0 + (jlo + i) * BKV);
+            const int krow = (jlo + i) * BKV;
             if (tc >= 2 && !mbar_wait(&s_full[st], ph2, abort_flag, a.status)) { ok = false; break; }
             mbar_expect_tx(&k_full[st], TILE_BYTES);
-            tma_load_2d(sK + st * TILE_BYTES, &tmK, &k_full[st], p.k_col0 + kvh * HD, krow);
-            tma_load_2d(sK + st * TILE_BYTES + TILE_BYTES / 2, &tmK, &k_full[st], p.k_col0 + kvh * HD + 64, krow);
+            tma_load_3d(sK + st * TILE_BYTES, &tmK, &k_full[st], p.k_col0 + kvh * HD, krow, b);
+            tma_load_3d(sK + st * TILE_BYTES + TILE_BYTES / 2, &tmK, &k_full[st], p.k_col0 + kvh * HD + 64, krow, b);
             if (tc >= 2 && !mbar_wait(&pv_done[st], ph2, abort_flag, a.status)) { ok = false; break; }
             mbar_expect_tx(&v_full[st], TILE_BYTES);
-            tma_load_2d(sV + st * TILE_BYTES, &tmV, &v_full[st], p.v_col0 + kvh * HD, krow);
-            tma_load_2d(sV + st * TILE_BYTES + TILE_BYTES / 2, &tmV, &v_full[st], p.v_col0 + kvh * HD + 64, krow);
+            tma_load_3d(sV + st * TILE_BYTES, &tmV, &v_full[st], p.v_col0 + kvh * HD, krow, b);
+            tma_load_3d(sV + st * TILE_BYTES + TILE_BYTES / 2, &tmV, &v_full[st], p.v_col0 + kvh * HD + 64, krow, b);
           }
         }
       }
@@ -505,6 +523,11 @@ attn_fwd_persistent_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid
 #pragma unroll
           for (int k = 0; k < BKV / 16; k++)
             mma_ts(tO, tS[st] + k * 8, smem_desc_sw128(v_addr + k * 2048, TILE_BYTES / 2, 1024), idesc_o, (i > 0 || k > 0) ? 1u : 0u);
+          if constexpr (RAGGED) {
+#pragma unroll
+            for (int k = 0; k < BKV / 16; k++)
+              mma_ts(tO, tS[st] + 64 + k * 8, smem_desc_sw128(v_addr + k * 2048, TILE_BYTES / 2, 1024), idesc_o, 1u);
+          }
           tc_commit(&pv_done[st]);
           cy.lap(1);
         }
@@ -539,7 +562,7 @@ attn_fwd_persistent_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid
       // it goes back to the producer once the store has read it.
       if (ok && lane == 0 && n >= 1) { bulk_wait_read<0>(); mbar_arrive(&q_free[(n - 1) & 1]); }
       int lo = max(0, q - a.window_left);
-      if (a.doc_start) lo = max(lo, a.doc_start[row0 + q]);
+      if (a.doc_start) lo = max(lo, a.doc_start[row0 + (RAGGED ? min(q, a.T - 1) : q)]);
       float m_used = -INFINITY, l = 0.f;
       for (int i = 0; i < ntile; i++, tc++) {
         const int st = tc & 1;
@@ -604,7 +627,7 @@ attn_fwd_persistent_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid
         float sm[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
         for (int u = 0; u < CW / 32; u++) {
-          uint32_t pk[16];
+          uint32_t pk[16], pl[16];
 #pragma unroll
           for (int j = 0; j < 16; j += 2) {
             const float p0 = fast_exp2(fmaf(x[u * 32 + 2 * j], c, -mm)), p1 = fast_exp2(fmaf(x[u * 32 + 2 * j + 1], c, -mm));
@@ -612,8 +635,10 @@ attn_fwd_persistent_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid
             sm[0] += p0; sm[1] += p1; sm[2] += p2; sm[3] += p3;
             pk[j] = pack_bf16(p0, p1);
             pk[j + 1] = pack_bf16(p2, p3);
+            if constexpr (RAGGED) { pl[j] = rest_bf16(p0, p1, pk[j]); pl[j + 1] = rest_bf16(p2, p3, pk[j + 1]); }
           }
           tmem_st16(tS[st] + lane_off + hs * (CW / 2) + u * 16, pk);
+          if constexpr (RAGGED) tmem_st16(tS[st] + lane_off + 64 + hs * (CW / 2) + u * 16, pl);
         }
         l += (sm[0] + sm[1]) + (sm[2] + sm[3]);
         cy.lap(4);
@@ -658,11 +683,11 @@ attn_fwd_persistent_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid
         }
         fence_proxy_async();
         __syncwarp();
-        if (lane == 0) {
-          tma_store_3d(&tmO, stage, h * HD + hs * CW, (int)(row0 + q0 + quad * 32), 0);
+        if (lane == 0 && (!RAGGED || q0 + quad * 32 < a.T)) {
+          tma_store_3d(&tmO, stage, h * HD + hs * CW, q0 + quad * 32, b);
           bulk_commit();
         }
-        if (hs == 0) {
+        if (hs == 0 && (!RAGGED || q < a.T)) {
           const long long si = ((long long)b * a.H + h) * a.T + q;
           const float ln2 = 0.6931471805599453f;
           if (a.lse) a.lse[si] = (m_used + log2f(l)) * ln2;
@@ -1119,7 +1144,7 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 
 bool attention_tc_supported(const AttnArgs& a) {
   if (a.hd != HD) return false;
-  if (a.T % BQ != 0 || a.T > 8192) return false;  // the dK/dV kernel lists at most 64 query tiles
+  if (a.T > 8192) return false;  // the dK/dV kernel lists at most 64 query tiles
   if ((a.q_stride & 7) || (a.kv_stride & 7) || (a.o_stride & 7)) return false;
   if (!aligned16(a.Q) || !aligned16(a.K) || !aligned16(a.V) || !aligned16(a.O)) return false;
   if (a.H % a.Hkv != 0) return false;
@@ -1161,10 +1186,7 @@ static void cycles_report(const char*, const char*, int, int) {}
 int attention_fwd_tc(const AttnArgs& a, cudaStream_t s) {
   if (!attention_tc_supported(a)) return femto_fail(FEMTO_ERR_UNSUPPORTED, "attention_fwd_tc: unsupported shape");
   const long long N = (long long)a.B * a.T;
-  CUtensorMap tmQ, tmK, tmV;
-  FEMTO_TRY(make_tmap_2d_bf16(&tmQ, a.Q, (uint64_t)a.H * HD, N, a.q_stride, 64, BQ));
-  FEMTO_TRY(make_tmap_2d_bf16(&tmK, a.K, (uint64_t)a.Hkv * HD, N, a.kv_stride, 64, BKV));
-  FEMTO_TRY(make_tmap_2d_bf16(&tmV, a.V, (uint64_t)a.Hkv * HD, N, a.kv_stride, 64, BKV));
+  const bool ragged = a.T % BQ != 0;
   FwdParams p;
   p.a = a;
   p.q_col0 = 0; p.k_col0 = 0; p.v_col0 = 0;
@@ -1172,7 +1194,8 @@ int attention_fwd_tc(const AttnArgs& a, cudaStream_t s) {
   const int dev = PerDevice::current();
   if (dev < 0 || !attr.done[dev]) {
     CUDA_TRY(cudaFuncSetAttribute(attn_fwd_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FWD_SMEM));
-    CUDA_TRY(cudaFuncSetAttribute(attn_fwd_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PF_SMEM));
+    CUDA_TRY(cudaFuncSetAttribute(attn_fwd_persistent_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, PF_SMEM));
+    CUDA_TRY(cudaFuncSetAttribute(attn_fwd_persistent_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PF_SMEM));
     CUDA_TRY(cudaFuncSetAttribute(attn_fwd_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PP_SMEM));
     if (dev >= 0) attr.done[dev] = true;
   }
@@ -1180,7 +1203,27 @@ int attention_fwd_tc(const AttnArgs& a, cudaStream_t s) {
   // 3 = persistent, two query tiles in ping-pong (measured slower so far); default 2 = persistent, one query tile at a time
   static int variant = -1;
   if (variant < 0) { const char* e = getenv("FEMTO_ATTN_FWD"); variant = (e && e[0] >= '1' && e[0] <= '3') ? e[0] - '0' : 2; }
-  // the persistent kernels assume every query tile is full and starts on a 16-byte boundary of the document starts
+  if (variant == 2 || ragged) {   // the older kernels assume that every query tile is full
+    const int nitems = (a.T + BQ - 1) / BQ * a.H * a.B;
+    const int grid = std::min(nitems, device_sm_count());
+    CUtensorMap tmQ, tmK, tmV, tmO;   // (columns, rows of one batch column, batch); O for one 64-column x 32-row box per softmax warp
+    const auto map = [&](CUtensorMap* m, const void* x, int heads, long long ld, int rows) {
+      return make_tmap_3d_bf16_sw(m, x, (uint64_t)heads * HD, a.T, a.B, ld, (uint64_t)a.T * ld, 64, rows, 3);
+    };
+    FEMTO_TRY(map(&tmQ, a.Q, a.H, a.q_stride, BQ));
+    FEMTO_TRY(map(&tmK, a.K, a.Hkv, a.kv_stride, BKV));
+    FEMTO_TRY(map(&tmV, a.V, a.Hkv, a.kv_stride, BKV));
+    FEMTO_TRY(map(&tmO, a.O, a.H, a.o_stride, 32));
+    if (ragged) attn_fwd_persistent_kernel<true><<<grid, FWD_THREADS, PF_SMEM, s>>>(tmQ, tmK, tmV, tmO, p, nitems, cycles_buffer());
+    else attn_fwd_persistent_kernel<false><<<grid, FWD_THREADS, PF_SMEM, s>>>(tmQ, tmK, tmV, tmO, p, nitems, cycles_buffer());
+    KERNEL_CHECK();
+    cycles_report("S issuer, P V issuer: waiting / issuing", "softmax (keys 0-63, 64-127): wait S / load+max / barrier / rescale / exp / arrive / item end", 1, 2);
+    return 0;
+  }
+  CUtensorMap tmQ, tmK, tmV;
+  FEMTO_TRY(make_tmap_2d_bf16(&tmQ, a.Q, (uint64_t)a.H * HD, N, a.q_stride, 64, BQ));
+  FEMTO_TRY(make_tmap_2d_bf16(&tmK, a.K, (uint64_t)a.Hkv * HD, N, a.kv_stride, 64, BKV));
+  FEMTO_TRY(make_tmap_2d_bf16(&tmV, a.V, (uint64_t)a.Hkv * HD, N, a.kv_stride, 64, BKV));
   if (variant == 3) {
     const int G = a.H / a.Hkv;
     const bool gqa = (G % 2) == 0;
@@ -1189,13 +1232,6 @@ int attention_fwd_tc(const AttnArgs& a, cudaStream_t s) {
     const int grid = std::min(nitems, device_sm_count());
     attn_fwd_pair_kernel<<<grid, FWD_THREADS, PP_SMEM, s>>>(tmQ, tmK, tmV, p, nitems, gqa ? 1 : 0, cycles_buffer());
     cycles_report("issuer: waiting / issuing", "softmax A, B: wait S / pass 1 / - / rescale / pass 2 / arrive / item end", 1, 1);
-  } else if (variant == 2) {
-    const int nitems = (a.T / BQ) * a.H * a.B;
-    const int grid = std::min(nitems, device_sm_count());
-    CUtensorMap tmO;   // O as [rows][H * 128] for 64-column x 32-row swizzled boxes (one per softmax warp)
-    FEMTO_TRY(make_tmap_3d_bf16_sw(&tmO, a.O, (uint64_t)a.H * HD, N, 1, a.o_stride, 0, 64, 32, 3));
-    attn_fwd_persistent_kernel<<<grid, FWD_THREADS, PF_SMEM, s>>>(tmQ, tmK, tmV, tmO, p, nitems, cycles_buffer());
-    cycles_report("S issuer, P V issuer: waiting / issuing", "softmax (keys 0-63, 64-127): wait S / load+max / barrier / rescale / exp / arrive / item end", 1, 2);
   } else {
     dim3 grid(a.T / BQ, a.H, a.B);
     attn_fwd_tc_kernel<<<grid, FWD_THREADS, FWD_SMEM, s>>>(tmQ, tmK, tmV, p);

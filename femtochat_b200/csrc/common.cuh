@@ -209,6 +209,7 @@ struct AttnArgs {
 template <typename T> int attention_fwd_simt(const AttnArgs& a, cudaStream_t s);
 template <typename T> int attention_bwd_simt(const AttnArgs& a, cudaStream_t s);
 bool attention_tc_supported(const AttnArgs& a);
+bool attention_bwd_tc_supported(const AttnArgs& a);
 int attention_fwd_tc(const AttnArgs& a, cudaStream_t s);
 int attention_bwd_tc(const AttnArgs& a, cudaStream_t s);
 size_t attention_bwd_tc_ws_bytes(int B, int T, int H, int hd);

@@ -109,6 +109,47 @@ def test_attention_forward_and_reverse(dtype, B, T, H, Hkv, hd, left, docs):
         assert rel <= (1e-2 if dtype == _lib.BF16 else 1e-5), rel
 
 
+@pytest.mark.parametrize("B,T,H,Hkv,left,docs", [
+    (2, 1, 2, 1, 1, False), (3, 5, 2, 2, 5, True), (2, 127, 2, 1, 127, False), (2, 129, 4, 2, 40, True), (3, 255, 2, 2, 255, True),
+    (2, 257, 6, 2, 100, False), (1, 1000, 10, 5, 300, True), (2, 1153, 2, 1, 2000, False)])
+def test_attention_of_ragged_lengths(B, T, H, Hkv, left, docs):
+    """Lengths that are no multiple of the 128-row tiles, several columns, on the tensor cores with P and dS in two bf16 parts: O is off
+    by its own rounding (2^-9 of it) and 2^-14 of the largest, the gradients by their rounding and that of the O they are computed from
+    (2^-9 each, rms below 4e-3); nothing past a column's end is read or written; accumulate adds."""
+    Q, K, V, dO, ds = _attn_inputs(_lib.BF16, B, T, H, Hkv, 128, seed=T, docs=docs)
+    Qd, Kd, Vd, dOd = (x.double() for x in (Q, K, V, dO))
+    docs64 = ds.long() if ds is not None else None
+    O_ref, l_ref, m_ref = fo.flash_attention_forward(Qd, Kd, Vd, (left, 0), docs64)
+    refs = fo.flash_attention_backward(dOd, Qd, Kd, Vd, O_ref, l_ref, m_ref, (left, 0), docs64)
+    dev = [x.cuda() for x in (Q, K, V, dO)]
+    dsd = ds.cuda() if ds is not None else None
+    guard = 64 * 1024                      # after each result: must stay as it is
+    held = [torch.full((x.numel() + guard,), 7.0, dtype=torch.bfloat16, device="cuda") for x in (Q, Q, K, V)]
+    O, dQ, dK, dV = (h[:x.numel()].view(x.shape) for h, x in zip(held, (Q, Q, K, V)))
+    lse = torch.zeros(B, H, T, device="cuda")
+    L = _lib.lib()
+    _lib.check(L.femto_attention_fwd(_lib.BF16, _lib.ptr(O), None, None, _lib.ptr(lse), _lib.ptr(dev[0]), _lib.ptr(dev[1]), _lib.ptr(dev[2]),
+                                     B, T, H, Hkv, 128, left, _lib.ptr(dsd), None))
+
+    def reverse(accumulate):
+        _lib.check(L.femto_attention_bwd(_lib.BF16, _lib.ptr(dQ), _lib.ptr(dK), _lib.ptr(dV), _lib.ptr(dev[3]), _lib.ptr(dev[0]), _lib.ptr(dev[1]),
+                                         _lib.ptr(dev[2]), _lib.ptr(O), _lib.ptr(lse), None, None, B, T, H, Hkv, 128, left, _lib.ptr(dsd), accumulate, None))
+        torch.cuda.synchronize()
+
+    reverse(0)
+    off = (O.double().cpu() - O_ref).abs()
+    assert (off <= O_ref.abs() * 2.0 ** -8 + O_ref.abs().max() * 2.0 ** -14).all()
+    assert (lse.double().cpu() - (m_ref + torch.log(l_ref))).abs().max() <= 1e-4
+    first = [x.clone() for x in (dQ, dK, dV)]
+    for got, ref in zip(first, refs):
+        assert (got.double().cpu() - ref).norm() <= 4e-3 * ref.norm() + 1e-2 * (ref.norm() == 0)
+    reverse(1)
+    for got, one in zip((dQ, dK, dV), first):
+        assert (got.float() - 2 * one.float()).norm() <= 4e-3 * 2 * one.float().norm() + 1e-6
+    for h, x in zip(held, (Q, Q, K, V)):
+        assert (h[x.numel():] == 7.0).all()
+
+
 def test_attention_at_benchmark_shape_geometric_documents():
     """The benchmark's attention shape: T=2048, 10 query / 5 kv heads, head_dim 128, short window 1024, documents of
     geometric(512) length (B=1 so that the fp64 naive reference stays small)."""
