@@ -175,6 +175,7 @@ void carve(femto_handle* h, Bump& b) {
     if (h->lp[i].ve) b.take(l.sh_ve, es * Vp * kv); else l.sh_ve = nullptr;
   }
   { char* end = nullptr; b.take(end, 0); h->weights_end = end; }
+  b.take(h->cast_jobs, sizeof(CastJob) * (2 + 7 * (size_t)h->L));
   b.take(h->tok0, 4 * N); b.take(h->tgt0, 4 * N); b.take(h->pos, 4 * N); b.take(h->doc_start, 4 * N);
   b.take(h->raw_tok, 4 * N); b.take(h->raw_tgt, 4 * N); b.take(h->raw_pos, 4 * N);
   b.take(h->xe, es * N * d); b.take(h->x0, es * N * d); b.take(h->xm, es * N * d); b.take(h->xnf, es * N * d);
@@ -203,6 +204,31 @@ void carve(femto_handle* h, Bump& b) {
   b.take(h->gemm_ws2, h->gemm_ws_bytes);
   h->attn_ws_bytes = std::max(sizeof(float) * N * h->H * 2, attention_bwd_tc_ws_bytes(h->maxB, h->T, h->H, h->hd));
   b.take(h->attn_ws, h->attn_ws_bytes);
+}
+
+// Where each tensor of Theta goes in the compute type; Q, K, V of a block lie side by side in one [d][d + 2 kv] matrix.
+int cast_table(femto_handle* h) {
+  std::vector<CastJob> jobs;
+  const long long d = h->d, kv = h->kv, dq = h->dq, Vp = h->Vp;
+  const int es = h->bf ? 2 : 4;
+  h->cast_blocks = 0;
+  auto add = [&](long long src, void* dst, long long rows, long long cols, long long ldd) {
+    jobs.push_back({src, rows * cols, cols, ldd, dst, h->cast_blocks, cols % 8 == 0 && ldd % 8 == 0 && aligned16(dst)});
+    h->cast_blocks += cdiv(rows * cols, CAST_BLOCK);
+  };
+  add(h->off_wte, h->sh_wte, Vp, d, d);
+  add(h->off_lm, h->sh_lm, Vp, d, d);
+  for (int i = 0; i < h->L; i++) {
+    const LayerP& p = h->lp[i];
+    const LayerBuf& l = h->lb[i];
+    char* qkv = reinterpret_cast<char*>(l.sh_wqkv);
+    add(p.wq, qkv, d, d, dq); add(p.wk, qkv + d * es, d, kv, dq); add(p.wv, qkv + (d + kv) * es, d, kv, dq);
+    add(p.wo, l.sh_wo, d, d, d); add(p.fc, l.sh_fc, d, 4 * d, 4 * d); add(p.proj, l.sh_proj, 4 * d, d, d);
+    if (p.ve) add(p.ve_table, l.sh_ve, Vp, kv, kv);
+  }
+  h->n_cast_jobs = (int)jobs.size();
+  CUDA_TRY(cudaMemcpy(h->cast_jobs, jobs.data(), sizeof(CastJob) * jobs.size(), cudaMemcpyHostToDevice));
+  return 0;
 }
 
 __global__ void k_rope_tables(float* sin_t, float* cos_t, int n, int half, int hd) {
@@ -236,6 +262,7 @@ int model_alloc(femto_handle* h) {
   real.base = h->arena;
   carve(h, real);
   CUDA_TRY(cudaMemset(h->status, 0, 256));
+  FEMTO_TRY(cast_table(h));
   const int half = h->hd / 2, n = h->cfg.max_document_tokens;
   k_rope_tables<<<cdiv((long long)n * half, 256), 256>>>(h->sin_t, h->cos_t, n, half, h->hd);
   KERNEL_CHECK();
@@ -266,25 +293,11 @@ void model_free(femto_handle* h) {
   h->arena = nullptr;
 }
 
-template <typename T> static int refresh_t(femto_handle* h, const float* theta, cudaStream_t s) {
-  const long long d = h->d, Vp = h->Vp, kv = h->kv;
-  FEMTO_TRY(Stream<T>::cast_from_f32(theta + h->off_wte, (T*)h->sh_wte, Vp * d, s));
-  FEMTO_TRY(Stream<T>::cast_from_f32(theta + h->off_lm, (T*)h->sh_lm, Vp * d, s));
-  for (int i = 0; i < h->L; i++) {
-    const LayerP& p = h->lp[i];
-    LayerBuf& l = h->lb[i];
-    FEMTO_TRY(Stream<T>::pack_qkv(theta + p.wq, theta + p.wk, theta + p.wv, (T*)l.sh_wqkv, h->d, h->kv, s));
-    FEMTO_TRY(Stream<T>::cast_from_f32(theta + p.wo, (T*)l.sh_wo, d * d, s));
-    FEMTO_TRY(Stream<T>::cast_from_f32(theta + p.fc, (T*)l.sh_fc, 4 * d * d, s));
-    FEMTO_TRY(Stream<T>::cast_from_f32(theta + p.proj, (T*)l.sh_proj, 4 * d * d, s));
-    if (p.ve) FEMTO_TRY(Stream<T>::cast_from_f32(theta + p.ve_table, (T*)l.sh_ve, Vp * kv, s));
-  }
+int model_refresh(femto_handle* h, const float* theta, cudaStream_t s) {
+  FEMTO_TRY(h->bf ? Stream<bf16>::cast_all(theta, h->cast_jobs, h->n_cast_jobs, h->cast_blocks, s)
+                  : Stream<float>::cast_all(theta, h->cast_jobs, h->n_cast_jobs, h->cast_blocks, s));
   h->weights_valid = true;
   return 0;
-}
-
-int model_refresh(femto_handle* h, const float* theta, cudaStream_t s) {
-  return h->bf ? refresh_t<bf16>(h, theta, s) : refresh_t<float>(h, theta, s);
 }
 
 // ---- forward / reverse schedule --------------------------------------------------------------------

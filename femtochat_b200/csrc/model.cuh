@@ -40,6 +40,8 @@ struct femto_handle {
   void *sh_wte = nullptr, *sh_lm = nullptr;
   char *weights_begin = nullptr, *weights_end = nullptr;   // the contiguous range holding every compute-type weight
   bool weights_valid = false;
+  struct CastJob* cast_jobs = nullptr;   // device table of model_refresh
+  int n_cast_jobs = 0, cast_blocks = 0;
   int *tok0 = nullptr, *tgt0 = nullptr, *pos = nullptr, *doc_start = nullptr, *raw_tok = nullptr, *raw_tgt = nullptr,
       *raw_pos = nullptr;
   void *xe = nullptr, *x0 = nullptr, *xm = nullptr, *xnf = nullptr;

@@ -772,23 +772,41 @@ __global__ void __launch_bounds__(256) k_xent_rows(const float* __restrict__ log
   }
 }
 
-template <typename T> __global__ void k_cast(const float* __restrict__ src, T* __restrict__ dst, long long n) {
-  pdl_trigger();
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    dst[i] = from_f<T>(src[i]);
-}
 // dst [D][D+2kv] <- wq [D][D] | wk [D][kv] | wv [D][kv]
+// The compute-type copy of every weight in one launch: blocks of CAST_BLOCK elements, each of one job of the table.  Bound by HBM (4 bytes
+// in, 2 out per weight); one launch per tensor with one element per thread and step reached 3.7 TB/s, this 7.0 (d20: 1.55 -> 0.81 ms).
 template <typename T>
-__global__ void k_pack_qkv(const float* __restrict__ wq, const float* __restrict__ wk, const float* __restrict__ wv,
-                           T* __restrict__ dst, int D, int kv) {
+__global__ void __launch_bounds__(256) k_cast_all(const float* __restrict__ theta, const CastJob* __restrict__ jobs, int n_jobs) {
   pdl_trigger();
-  const int W = D + 2 * kv;
-  const long long n = (long long)D * W;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    int r = (int)(i / W), c = (int)(i % W);
-    float v = c < D ? wq[(long long)r * D + c] : (c < D + kv ? wk[(long long)r * kv + (c - D)] : wv[(long long)r * kv + (c - D - kv)]);
-    dst[i] = from_f<T>(v);
+  int lo = 0, hi = n_jobs - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (jobs[mid].first_block <= (int)blockIdx.x) lo = mid; else hi = mid - 1;
   }
+  const CastJob j = jobs[lo];
+  const float* src = theta + j.src;
+  T* dst = reinterpret_cast<T*>(j.dst);
+  const long long i0 = (long long)((int)blockIdx.x - j.first_block) * CAST_BLOCK;
+  constexpr int V = 8, STEPS = CAST_BLOCK / (256 * V);
+  if (j.vec && (reinterpret_cast<uintptr_t>(src) & 7) == 0) {       // Theta's tensors start at even offsets
+    float2 f[STEPS][V / 2];
+#pragma unroll
+    for (int e = 0; e < STEPS; e++) {
+      const long long i = i0 + (e * 256 + threadIdx.x) * V;
+      if (i < j.n)
+#pragma unroll
+        for (int k = 0; k < V / 2; k++) f[e][k] = __ldcs(reinterpret_cast<const float2*>(src + i) + k);
+    }
+#pragma unroll
+    for (int e = 0; e < STEPS; e++) {
+      const long long i = i0 + (e * 256 + threadIdx.x) * V;
+      if (i >= j.n) break;
+      const float v[V] = {f[e][0].x, f[e][0].y, f[e][1].x, f[e][1].y, f[e][2].x, f[e][2].y, f[e][3].x, f[e][3].y};
+      store8<T>(dst + (j.ldd == j.cols ? i : i / j.cols * j.ldd + i % j.cols), v);
+    }
+    return;
+  }
+  for (long long i = i0 + threadIdx.x; i < i0 + CAST_BLOCK && i < j.n; i += 256) dst[i / j.cols * j.ldd + i % j.cols] = from_f<T>(src[i]);
 }
 
 __global__ void __launch_bounds__(1024) k_sum_rows(const float* __restrict__ rows, int n, float* out,
@@ -1048,17 +1066,8 @@ int Stream<T>::xent_rows(const float* logits, long long ldl, const int* tgt0, in
   KERNEL_CHECK();
   return 0;
 }
-template <typename T> int Stream<T>::cast_from_f32(const float* src, T* dst, long long n, cudaStream_t s) {
-  int nb = (int)std::min<long long>(cdiv(n, 256), 148 * 32);
-  k_cast<T><<<nb, 256, 0, s>>>(src, dst, n);
-  KERNEL_CHECK();
-  return 0;
-}
-template <typename T>
-int Stream<T>::pack_qkv(const float* wq, const float* wk, const float* wv, T* dst, int D, int kv, cudaStream_t s) {
-  long long n = (long long)D * (D + 2 * kv);
-  int nb = (int)std::min<long long>(cdiv(n, 256), 148 * 32);
-  k_pack_qkv<T><<<nb, 256, 0, s>>>(wq, wk, wv, dst, D, kv);
+template <typename T> int Stream<T>::cast_all(const float* theta, const CastJob* jobs, int n_jobs, int blocks, cudaStream_t s) {
+  k_cast_all<T><<<blocks, 256, 0, s>>>(theta, jobs, n_jobs);
   KERNEL_CHECK();
   return 0;
 }

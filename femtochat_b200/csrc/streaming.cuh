@@ -3,6 +3,15 @@
 #pragma once
 #include "common.cuh"
 
+// One tensor of Theta on its way into the compute type: dst[i / cols * ldd + i % cols] = theta[src + i], i < n.
+struct CastJob {
+  long long src, n, cols, ldd;
+  void* dst;
+  int first_block;     // the job's blocks of CAST_BLOCK elements follow those of the job before
+  int vec;             // rows, pitch and dst are whole groups of 8
+};
+constexpr int CAST_BLOCK = 8192;
+
 template <typename T> struct Stream {
   static int prep_tokens(const int* tokens, const int* targets, const int* positions, int B, int Tlen,
                          int index_base, int vocab, int maxdoc, int* tok0, int* tgt0, int* pos, int* doc_start,
@@ -40,8 +49,7 @@ template <typename T> struct Stream {
   static int xent_rows(const float* logits, long long ldl, const int* tgt0, int n, int V, float w,
                        const float* w_dev, T* dlogit,
                        long long lddl, float* loss_rows, cudaStream_t s);
-  static int cast_from_f32(const float* src, T* dst, long long n, cudaStream_t s);
-  static int pack_qkv(const float* wq, const float* wk, const float* wv, T* dst, int D, int kv, cudaStream_t s);
+  static int cast_all(const float* theta, const CastJob* jobs, int n_jobs, int blocks, cudaStream_t s);
 };
 
 int sum_rows_to_scalar(const float* rows, int n, float* out, const int* tgt0, int* n_valid_out, float scale_by_valid,
