@@ -329,7 +329,9 @@ static int step_t(femto_handle* h, const float* theta, float* delta, const int* 
   const float eps = h->eps;
   const bool mean = reduction == FEMTO_REDUCTION_MEAN;
   // with a side stream the GEMMs give up one ring stage (32 KB), so that streaming kernels of the other stream fit beside them
-  auto GA = [&]() { GemmArgs g; g.ws = h->gemm_ws; g.ws_bytes = h->gemm_ws_bytes; g.status = h->status; g.ring = (backward && side) ? 5 : 0; return g; };
+  auto GA = [&]() { GemmArgs g; g.ws = h->gemm_ws; g.ws_bytes = h->gemm_ws_bytes; g.status = h->status; g.ring = (backward && side) ? 5 : 0; g.any_size = true; return g; };
+  // (any_size: fewer rows than a tile still are faster on the tensor cores than in the SIMT kernel, whose blocks walk K alone:
+  // 24 rows of d12 175 us a product, 17.4 us so)
   // Y[N][out] = X[N][in] * W[in][out]
   auto lin_fwd = [&](const void* X, int in, const void* W, int out, void* Y, int ldy, int epi, const void* aux) {
     GemmArgs g = GA();
