@@ -350,6 +350,14 @@ static int decode_t(femto_kv_cache* c, const float* theta, const int* tokens, co
   const int d = h->d, dq = h->dq, kv = h->kv, H = h->H, Hkv = h->Hkv, hd = h->hd, L = h->L;
   const float eps = h->eps;
   const int t = c->len;   // row of the new token in every column's cache
+  if (sizeof(T) == 2 && B <= c->step.columns) {
+    DecodeStepArgs a = {};
+    a.theta = theta; a.xe_prev = (bf16*)c->xe_prev; a.tok0 = c->tok0; a.pos = c->pos; a.doc_start = c->doc_start; a.lastpos = c->lastpos;
+    a.logits = logits_out; a.B = B; a.t = t; a.maxT = c->maxT;
+    FEMTO_TRY(decode_step_run(h, c->step, a, tokens, positions, s));
+    c->len = t + 1;
+    return 0;
+  }
   k_decode_prep<<<cdiv(B, 128), 128, 0, s>>>(tokens, positions, B, h->cfg.index_base, h->V, h->cfg.max_document_tokens, t, c->tok0,
                                              c->pos, c->doc_start, c->lastpos, h->status);
   KERNEL_CHECK();
@@ -408,7 +416,9 @@ extern "C" int32_t femto_kv_cache_create(femto_handle* h, int32_t max_batch, int
   const size_t widest = std::max<size_t>({(size_t)cdiv(h->d, KCH) * RM * (size_t)h->Vp, (size_t)cdiv(4 * h->d, KCH) * RM * (size_t)h->d,
                                           (size_t)cdiv(h->d, KCH) * RM * (size_t)std::max(4 * h->d, h->dq)});
   c->part_floats = std::max(widest, (size_t)max_batch * h->H * MAX_SPLITS * (h->hd + 2));
-  const size_t total = 2 * per_layer * h->L + 2 * al(es * (size_t)max_batch * h->d) + 4 * al(4 * (size_t)max_batch) + al(4 * c->part_floats);
+  decode_step_plan(h, max_batch, c->step);
+  const size_t total = 2 * per_layer * h->L + 2 * al(es * (size_t)max_batch * h->d) + 4 * al(4 * (size_t)max_batch) + al(4 * c->part_floats) +
+                       (c->step.columns ? decode_step_bytes(h, c->step) : 0);
   cudaError_t e = cudaMalloc(&c->mem, total);
   if (e != cudaSuccess) {
     delete c;
@@ -423,7 +433,11 @@ extern "C" int32_t femto_kv_cache_create(femto_handle* h, int32_t max_batch, int
   c->pos = (int*)p; p += al(4 * (size_t)max_batch);
   c->doc_start = (int*)p; p += al(4 * (size_t)max_batch);
   c->lastpos = (int*)p; p += al(4 * (size_t)max_batch);
-  c->part = (float*)p;
+  c->part = (float*)p; p += al(4 * c->part_floats);
+  if (c->step.columns) {
+    decode_step_carve(h, p, c->step);
+    if (const int r = decode_step_setup(h, c->step, c->K, c->V)) { cudaFree(c->mem); delete c; return r; }
+  }
   *out = c;
   return 0;
 }

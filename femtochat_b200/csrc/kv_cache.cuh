@@ -4,6 +4,7 @@
 #pragma once
 #include <vector>
 
+#include "decode_step.cuh"
 #include "model.cuh"
 
 struct LayerState {
@@ -27,6 +28,7 @@ struct femto_kv_cache {
   int *tok0 = nullptr, *pos = nullptr, *doc_start = nullptr, *lastpos = nullptr;   // GPT: [maxB]
   float* part = nullptr;                      // split-key partials of the decode attention / split-K of the products
   size_t part_floats = 0;
+  DecodeStepState step;                       // GPT: what the resident decode kernel needs
   std::vector<LayerState> state;              // layer-listing decoders
   void* kv_exp = nullptr;                     // their attention layers: keys and values of one column expanded from the latents
 };

@@ -424,6 +424,35 @@ def test_kv_cache_decode_matches_full_context_recompute(cfgkw, ctype, doc_mask, 
         c.close()
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("B,H,G,L,doc_mask", [(1, 4, 2, 2, True), (3, 8, 1, 3, False), (8, 3, 3, 2, True), (9, 2, 1, 5, False), (16, 6, 2, 2, True), (17, 2, 2, 2, False)])
+def test_decode_step_of_bf16_columns_matches_the_oracle(B, H, G, L, doc_mask):
+    """The resident decode kernel at its edges: one column, a full and a begun second tile of eight, the most it takes and
+    one more (the chain of kernels); 1, 2, 3 and 8 query heads a key head; more keys than one range; a padded vocabulary.
+    Tolerance as for the cache test above: bf16 rounding through the blocks, relative to the largest logit."""
+    kw = dict(sequence_len=210, max_document_tokens=512, vocab_size=1000, n_layer=L, n_head=H, n_kv_head=G, n_embed=128 * H, window_pattern="SL")
+    cfg, ocfg = fb.GPTConfig(**kw), fo.GPTConfig(**kw)
+    lay, olay = fb.parameter_layout(cfg), fo.parameter_layout(ocfg)
+    th = torch.zeros(lay.nparams)
+    fo.initialize(th, ocfg, olay, 17, all_nonzero=True)
+    T, Tp = 210, 201
+    tok = torch.randint(1, 1001, (B, T), generator=torch.Generator().manual_seed(B), dtype=torch.int32)
+    pos = torch.arange(T, dtype=torch.int32)[None, :].repeat(B, 1)
+    pos[B // 2, 150:] -= 150
+    cache_o = {}
+    fo.Model(ocfg, fo.StepOptions(eps=fo.EPS_BF16, short_window=70, doc_mask=doc_mask)).forward(th, tok, tok, pos, cache=cache_o)
+    z_ref = cache_o["z"].float().reshape(B, T, 1000)
+    model = fb.GPT(fb.Params(th.cuda()), cfg, lay, compute_type="bfloat16", short_window=70, doc_mask=doc_mask)
+    st = model.state(B)
+    kc = fb.KVCache(st, B, T)
+    fb.prefill(model, kc, tok[:, :Tp], pos[:, :Tp])
+    for t in range(Tp, T):
+        z = fb.decode_step(model, kc, tok[:, t], pos[:, t]).cpu()
+        assert (z - z_ref[:, t]).abs().max() <= 2.5e-2 * float(z_ref.abs().max()), t
+    assert st.status_word() == 0
+    kc.close()
+
+
 def test_generate_with_cache_equals_generate_by_recompute():
     """`generate` (src/generation.jl:26-56): greedy decoding (temperature 0) through the cache gives the tokens of
     the reference's recompute-everything loop; with sampling the same generator state gives the same tokens."""
