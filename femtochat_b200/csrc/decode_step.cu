@@ -5,12 +5,17 @@
 // weight stream only when its predecessor had finished.  Here one block per multiprocessor stays for the whole step.  One warp of
 // it copies the weights of the block's share of ALL products of the step by TMA into a ring in shared memory and knows nothing of
 // the rest, so the stream runs on while the chain of dependent phases - norm + QKV, attention, output projection, norm + MLP up,
-// MLP down - passes from block to block through counters in global memory.  A token: d12, one column 1150 -> 328 us; d20, eight columns of 540 tokens 2600 -> 1136 us.
-// (Copies issued by the eight computing warps
-// themselves, cp.async, held up their loads of activations: 400 us a token, d12.)
+// MLP down - passes from block to block.  (Copies issued by the eight computing warps themselves, cp.async, held up their loads of
+// activations: 400 us a token, d12.)
+//
+// What a phase leaves goes to global memory as words of 8 bytes, 4 of data and 4 that name the launch and the layer; who needs it
+// reads until the name is right.  A store and a load carry a value across, where data, a fence, a counter and a poll (the
+// first form of this kernel) took 2 us a phase and 328 us a token of d12, 1136 us of eight columns of d20.  No buffer is
+// written again before its readers of the layer before are done, since every phase needs all of the one before it.
+// Measured a token, chain of launches -> now: d12, one column 1150 -> 210 us; d20, eight columns of 540 tokens 2600 -> 970 us.
 //
 // Shares: an item is 64 output columns times d rows of a matrix, so that QKV, wo and fc have N / 64 items and proj four times
-// d / 64 (its four partial sums are added by whoever reads them, in order).  Items go round the blocks without a restart
+// d / 64 (its four partial sums are added, in order, by the block that has the first).  Items go round the blocks without a restart
 // from product to product, which balances the stream.  The rows of X are the 8-column operand of mma.m16n8k16, the
 // weights its 16-row operand: a lane takes 8 columns of the four rows of W that are its own in the fragment, and byte
 // permutations make the (k, k+1) pairs.  RMS norms have no weights here, so the reciprocal root multiplies the product.
@@ -23,17 +28,32 @@
 namespace {
 
 constexpr int THREADS = 256, WARPS = 8, SLOT = 128 * 64 * 2,      // computing threads; a slot of the ring: 128 rows of 64 columns
-              HD = 128, MAX_SPLITS = 32, COUNTER_STRIDE = 16;   // counters 64 bytes apart
+              HD = 128, MAX_SPLITS = 32;
 constexpr int RED_PITCH = 66;      // floats per fragment register pair of a warp's sums; 66: a column's eight land in eight banks
-constexpr long long SPIN_LIMIT = 1 << 20;
+constexpr int SPIN_LIMIT = 1 << 20;
 
 __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t s) {
   uint32_t r;
   asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(s));
   return r;
 }
-// What other blocks wrote is read past L1
-__device__ __forceinline__ float4 ld4(const float* p) { return __ldcg(reinterpret_cast<const float4*>(p)); }
+// Words that carry their name: two of them a load, straight from L2
+__device__ __forceinline__ uint4 named_load2(const uint2* p) {
+  uint4 v;
+  asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint2 named_load(const uint2* p) {
+  uint2 v;
+  asm volatile("ld.volatile.global.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void named_store(uint2* p, uint32_t data, uint32_t name) {
+  asm volatile("st.volatile.global.v2.u32 [%0], {%1, %2};" ::"l"(p), "r"(data), "r"(name) : "memory");
+}
+__device__ __forceinline__ void named_store(uint2* p, float data, uint32_t name) { named_store(p, __float_as_uint(data), name); }
+__device__ __forceinline__ float lo_f(uint32_t p) { return __uint_as_float(p << 16); }
+__device__ __forceinline__ float hi_f(uint32_t p) { return __uint_as_float(p & 0xffff0000u); }
 __device__ __forceinline__ uint32_t pack2(float a, float b) {
   __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<uint32_t*>(&h);
@@ -46,12 +66,13 @@ __device__ __forceinline__ void put4(bf16* row, int col, uint32_t lo, uint32_t h
   w[0] = lo; w[2] = hi;
 }
 
-// ---- the new token of every column: its id and position, normalised embedding and smear; counters to zero -------------
+// ---- the new token of every column: its id and position, normalised embedding and smear, and the first block's mixed stream ----
+// launches[0] counts the launches so far, launches[1] is this one's number for the blocks of the step.
 __global__ void __launch_bounds__(THREADS) k_step_begin(const DecodeStepArgs a, const int* tokens, const int* positions, int base, int vocab,
                                                         int maxdoc) {
   const int b = blockIdx.x, tid = threadIdx.x;
-  if (b == 0)
-    for (int i = tid; i < a.n_counters; i += THREADS) a.counters[i * COUNTER_STRIDE] = 0;
+  const uint32_t launch = a.launches[0] + 1, name = launch * (a.L + 1) + 1;
+  if (b == 0 && tid == 0) a.launches[1] = launch;
   int tk = tokens[b] - base;
   bool bad = tk < 0 || tk >= vocab;
   tk = min(max(tk, 0), vocab - 1);
@@ -84,16 +105,26 @@ __global__ void __launch_bounds__(THREADS) k_step_begin(const DecodeStepArgs a, 
   pre = warp_sum(pre);
   const float gate = a.theta[a.off_lam_s] * (1.f / (1.f + expf(-pre)));
   bf16* prev = a.xe_prev + (long long)b * a.d;
-  for (int c = tid; c < a.d; c += THREADS) {
-    const bf16 e = __float2bfloat16_rn(__bfloat162float(src[c]) * inv);
-    a.x0[(long long)b * a.d + c] = __bfloat162float(e) + gate * __bfloat162float(prev[c]);
-    prev[c] = e;
+  const float mix = a.theta[a.blocks[0].lam_b] + a.theta[a.blocks[0].lam_x0];
+  for (int c = 2 * tid; c < a.d; c += 2 * THREADS) {
+    float x[2];
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+      const bf16 e = __float2bfloat16_rn(__bfloat162float(src[c + i]) * inv);
+      x[i] = __bfloat162float(e) + gate * __bfloat162float(prev[c + i]);
+      prev[c + i] = e;
+      const long long at = (long long)b * a.d + c + i;
+      a.x0[at] = x[i];
+      x[i] *= mix;
+      named_store(a.xm + at, x[i], name);
+    }
+    named_store(a.xn + ((long long)b * a.d + c) / 2, pack2(x[0], x[1]), name);
   }
 }
 
 // ---- the step ----------------------------------------------------------------------------------------------------------
 template <int NT, int GMAX, int RING>
-__global__ void __launch_bounds__(THREADS + 32, 1) k_decode_step(const DecodeStepArgs a) {
+__global__ void __launch_bounds__(THREADS + 128, 1) k_decode_step(const DecodeStepArgs a) {
   extern __shared__ __align__(1024) unsigned char smem[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, c = lane & 3, cta = blockIdx.x, grid = gridDim.x;
   const int d = a.d, B = a.B, xp = d + 16;        // 16: the eight rows of an 8-byte fragment load fall into different banks
@@ -102,6 +133,7 @@ __global__ void __launch_bounds__(THREADS + 32, 1) k_decode_step(const DecodeSte
   float* red = reinterpret_cast<float*>(X + 8 * NT * xp);
   const DecodeBlock* blocks = reinterpret_cast<const DecodeBlock*>(reinterpret_cast<unsigned char*>(red) + a.red_bytes);
   __shared__ float ssp[8 * NT][33], inv_s[8 * NT], qs[GMAX][HD], kvs[2][HD];
+  const uint32_t launch = a.launches[1];
   __shared__ int given_up;
   __shared__ uint64_t full[RING], empty[RING];
   const int steps = d >> 7, np = 4 * a.L + 1;
@@ -114,14 +146,14 @@ __global__ void __launch_bounds__(THREADS + 32, 1) k_decode_step(const DecodeSte
     const int j = cta - before % grid;
     return j < 0 ? j + grid : j;
   };
-  auto blocks_of = [&](int p) { return min(items_of(p), grid); };
   {
     const uint32_t* src = reinterpret_cast<const uint32_t*>(a.blocks);
     uint32_t* dst = const_cast<uint32_t*>(reinterpret_cast<const uint32_t*>(blocks));
-    for (int i = tid; i < a.L * (int)sizeof(DecodeBlock) / 4; i += THREADS + 32) dst[i] = src[i];
+    for (int i = tid; i < a.L * (int)sizeof(DecodeBlock) / 4; i += THREADS + 128) dst[i] = src[i];
   }
-  for (int i = tid; i < 8 * NT * xp / 2; i += THREADS + 32) reinterpret_cast<uint32_t*>(X)[i] = 0;   // rows from B on stay zero
+  for (int i = tid; i < 8 * NT * xp / 2; i += THREADS + 128) reinterpret_cast<uint32_t*>(X)[i] = 0;   // rows from B on stay zero
   if (tid == 0) {
+    if (cta == 0) a.launches[0] = launch;
     given_up = 0;
     for (int i = 0; i < RING; i++) { sm100::mbar_init(&full[i], 1); sm100::mbar_init(&empty[i], WARPS); }
     sm100::fence_barrier_init();
@@ -129,8 +161,10 @@ __global__ void __launch_bounds__(THREADS + 32, 1) k_decode_step(const DecodeSte
   __syncthreads();
 
   // ---- the stream of weights ----
-  if (warp == WARPS) {
-    if (lane) return;
+  // (a warpgroup for it, which gives its registers to the computing ones: 4 x 24 + 8 x 240 = 12 x 168 a lane)
+  if (warp >= WARPS) {
+    sm100::reg_dealloc<24>();
+    if (warp > WARPS || lane) return;
     int n = 0, slot = 0, turn = 0;
     for (int p = 0; p < np; p++) {
       const int tiles = (p & 3) == 3 ? d >> 6 : 1 << 30;
@@ -150,32 +184,32 @@ __global__ void __launch_bounds__(THREADS + 32, 1) k_decode_step(const DecodeSte
       for (uint32_t k = 0; k < sm100::WAIT_LIMIT && !sm100::mbar_try_wait(&full[i % RING], (i / RING) & 1); k++) {}
     return;
   }
+  sm100::reg_alloc<240>();
   int slot = 0;
   uint32_t parity = 0;
 
-  // A wait ends when `n` blocks have arrived, or, with an error in the status word, after about a second.
-  auto wait = [&](int counter, int n) {
-    if (tid == 0 && !*(volatile int*)&given_up) {
-      const unsigned int* p = a.counters + counter * COUNTER_STRIDE;
-      for (long long spin = 0;; spin++) {
-        unsigned int v;
-        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-        if (v >= (unsigned int)n) break;
-        if (spin >= SPIN_LIMIT) { atomicOr(a.status, ST_WAIT_TIMEOUT); given_up = 1; break; }
-      }
-    }
-    compute_sync();
-  };
-  auto arrive = [&](int counter) {
-    compute_sync();
-    if (tid == 0) {
-      __threadfence();
-      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.counters + counter * COUNTER_STRIDE) : "memory");
+  // Reads until done() says that every word has its name, or, with an error in the status word, for about a second.
+  auto until = [&](auto&& done) {
+    for (int spin = 0; !done(); spin++) {
+      if (spin < SPIN_LIMIT && ((spin & 63) != 63 || !*(volatile int*)&given_up)) continue;
+      if (spin >= SPIN_LIMIT) { atomicOr(a.status, ST_WAIT_TIMEOUT); *(volatile int*)&given_up = 1; }
+      break;
     }
   };
-  // One item: sums of this warp's steps over the ring, then over the warps in order; out(b, column, sum).
-  auto product = [&](int tile, bool normed, auto&& out) {
-    float acc[4][NT][4] = {};
+  auto word = [&](const uint2* p, uint32_t name) {
+    uint2 v;
+    until([&] { v = named_load(p); return v.y == name; });
+    return __uint_as_float(v.x);
+  };
+  // One item: sums of this warp's steps over the ring, then over the warps in order; out(b, column, sum, what before(b, column) gave).
+  // A warp has 32 neighbouring columns of one row at a time.
+  auto product = [&](int tile, bool normed, auto&& before, auto&& out) {
+    float acc[4][NT][4] = {}, aux[2 * NT];
+#pragma unroll
+    for (int k = 0; k < 2 * NT; k++) {
+      const int o = tid + k * THREADS;
+      aux[k] = o < 64 * B ? before(o >> 6, tile * 64 + (o & 63)) : 0.f;
+    }
     const bf16* xr = X + g * xp + warp * 16 + 4 * c;
     // this lane's rows 2 c, 2 c + 1, 2 c + 8, 2 c + 9 of the warp's 16, 16-byte unit g of each where the 128-byte swizzle put it
     const unsigned char* wl = ring + (warp * 16 + 2 * c) * 128;
@@ -229,96 +263,105 @@ __global__ void __launch_bounds__(THREADS + 32, 1) k_decode_step(const DecodeSte
       inv_s[tid] = 1.f / sqrtf(ss / d + a.eps);
     }
     compute_sync();
-    for (int o = tid; o < 64 * B; o += THREADS) {
-      const int b = o >> 6, n = o & 63;
+#pragma unroll
+    for (int k = 0; k < 2 * NT; k++) {
+      const int o = tid + k * THREADS, b = o >> 6, n = o & 63;
+      if (o >= 64 * B) break;
       const float* p = red + ((n & 7) * NT + (b >> 3)) * RED_PITCH + (n >> 3) * 8 + (b & 7);
       float v = 0.f;
 #pragma unroll
       for (int w = 0; w < WARPS; w++) v += p[w * 8 * NT * RED_PITCH];
-      out(b, tile * 64 + n, normed ? v * inv_s[b] : v);
+      out(b, tile * 64 + n, normed ? v * inv_s[b] : v, aux[k]);
     }
     compute_sync();
   };
-  // Rows of X from value(b, column) (four at a time), with the sums of squares of every 128 columns.  The loads of several
-  // pieces are in flight together: they are latency, 0.8 us a piece if each waits for the one before.
-  auto rows_of = [&](auto&& value, auto&& done) {
-    constexpr int U = 4;
+  auto nothing = [](int, int) { return 0.f; };
+  // two neighbouring columns of a row (neighbouring lanes) as one word of bf16
+  auto store_pair = [&](uint2* row, int col, float v, uint32_t name) {
+    const float w = __shfl_xor_sync(0xffffffffu, v, 1);
+    if (!(lane & 1)) named_store(row + (col >> 1), pack2(v, w), name);
+  };
+  // Rows of X: d columns of every row of `src` (pairs; `pitch` words a row), with the sums of squares of every 128 columns.
+  // All loads of a thread are in flight together (10: eight rows of 1280).
+  auto rows_of = [&](const uint2* src, int pitch, uint32_t name, bool squares) {
+    constexpr int U = 10;
     for (int q0 = warp; q0 < B * steps; q0 += WARPS * U) {
-      float4 v[U];
+      uint4 v[U];
+      until([&] {
+        bool ok = true;
 #pragma unroll
-      for (int u = 0; u < U; u++) {
-        const int q = q0 + u * WARPS;
-        if (q < B * steps) v[u] = value(q / steps, q % steps * 128 + lane * 4);
-      }
+        for (int u = 0; u < U; u++) {
+          const int q = q0 + u * WARPS;
+          if (q >= B * steps) break;
+          v[u] = named_load2(src + (long long)(q / steps) * pitch + q % steps * 64 + lane * 2);
+          ok &= v[u].y == name && v[u].w == name;
+        }
+        return ok;
+      });
 #pragma unroll
       for (int u = 0; u < U; u++) {
         const int q = q0 + u * WARPS;
         if (q >= B * steps) break;
-        const int b = q / steps, k = q % steps, col = k * 128 + lane * 4;
-        const float4 x = done(b, col, v[u]);
-        put4(X + b * xp, col, pack2(x.x, x.y), pack2(x.z, x.w));
-        const float ss = warp_sum(x.x * x.x + x.y * x.y + x.z * x.z + x.w * x.w);
+        const int b = q / steps, k = q % steps;
+        put4(X + b * xp, k * 128 + lane * 4, v[u].x, v[u].z);
+        if (!squares) continue;
+        const float x = lo_f(v[u].x), y = hi_f(v[u].x), z = lo_f(v[u].z), w = hi_f(v[u].z), ss = warp_sum(x * x + y * y + z * z + w * w);
         if (lane == 0) ssp[b][k] = ss;
       }
     }
     compute_sync();
   };
-  // the residual stream after a block: what the attention left, plus the four partial sums of its MLP
   const long long Bd = (long long)B * d;
-  auto stream = [&](int b, int col) {
-    const long long at = (long long)b * d + col;
-    float4 v = ld4(a.xa + at);
-#pragma unroll
-    for (int s = 0; s < 4; s++) { const float4 p = ld4(a.part + s * Bd + at); v.x += p.x; v.y += p.y; v.z += p.z; v.w += p.w; }
-    return v;
-  };
   const int G = a.H / a.Hkv, n_attn = B * a.Hkv * a.splits;
 
   for (int l = 0; l < a.L; l++) {
     const DecodeBlock& blk = blocks[l];
-    // ---- mix, norm, QKV ----
+    const uint32_t name = launch * (a.L + 1) + l + 1;
+    // ---- norm, QKV ----
     if (int j = first_item(4 * l); j < items.x) {
-      const float lb = a.theta[blk.lam_b], l0 = a.theta[blk.lam_x0];
-      if (l > 0) wait(5 * l - 1, blocks_of(4 * l - 1));
-      const bool writer = j == 0;
-      if (l == 0)      // the stream is the embedding
-        rows_of([&](int b, int col) { return ld4(a.x0 + (long long)b * d + col); },
-                [&](int b, int col, float4 x) {
-                  const float4 m = make_float4(lb * x.x + l0 * x.x, lb * x.y + l0 * x.y, lb * x.z + l0 * x.z, lb * x.w + l0 * x.w);
-                  if (writer) *reinterpret_cast<float4*>(a.xm + (long long)b * d + col) = m;
-                  return m;
-                });
-      else
-        rows_of([&](int b, int col) {
-                  const float4 e = ld4(a.x0 + (long long)b * d + col), x = stream(b, col);
-                  return make_float4(lb * x.x + l0 * e.x, lb * x.y + l0 * e.y, lb * x.z + l0 * e.z, lb * x.w + l0 * e.w);
-                },
-                [&](int b, int col, float4 m) {
-                  const long long at = (long long)b * d + col;
-                  if (writer) {
-                    *reinterpret_cast<float4*>(a.xm + at) = m;
-                    if (l == a.backout + 1) *reinterpret_cast<float4*>(a.xb + at) = stream(b, col);
-                  }
-                  return m;
-                });
+      rows_of(a.xn, d / 2, name, true);
+      const bool first = j == 0;
       for (; j < items.x; j += grid)
-        product(j, true, [&](int b, int col, float v) { a.qkv[(long long)b * a.dq + col] = v; });
-      if (writer && tid < B) a.inv[tid] = inv_s[tid];
-      arrive(5 * l);
+        product(j, true, nothing, [&](int b, int col, float v, float) { named_store(a.qkv + (long long)b * a.dq + col, v, name); });
+      if (first)       // the first sixteen of the normalised row, for the gate of the value embeddings
+        for (int i = tid; i < 16 * B; i += THREADS) {
+          const int b = i >> 4, k = i & 15, w = (k & 4) + ((k >> 3) & 1) + (k & 2);
+          named_store(a.h16 + i, __bfloat162float(X[b * xp + 2 * w + (k & 1)]) * inv_s[b], name);
+        }
+      compute_sync();
     }
     // ---- attention: one item is a column's key head and a range of its keys ----
     int j = first_item(4 * l) - items.x % grid;
     if (j < 0) j += grid;
-    bool any = false;
     for (; j < n_attn; j += grid) {
       const int sp = j % a.splits, kvh = j / a.splits % a.Hkv, b = j / a.splits / a.Hkv;
       int lo = max(0, a.t - blk.window);
       if (a.docs) lo = max(lo, a.doc_start[b]);
       const int nk = a.t - lo, per = (nk + a.splits - 1) / a.splits;       // cached keys; the new one goes with the last range
-      const int k0 = min(a.t, lo + sp * per), k1 = min(a.t, k0 + per);
+      const int k0 = min(a.t, lo + sp * per), n_old = min(a.t, k0 + per) - k0;
       const bool last = sp == a.splits - 1;
       bf16* Kb = blk.K + (long long)b * a.maxT * a.kv + (long long)kvh * HD;
       bf16* Vb = blk.V + (long long)b * a.maxT * a.kv + (long long)kvh * HD;
+      // half a warp takes every sixteenth key, U at a time; a lane has eight channels.  What does not depend on the projections -
+      // rotation, value embedding, cached keys and values - is on its way before they are waited for.
+      const int hl = lane & 15, str = warp * 2 + (lane >> 4);
+      constexpr int U = GMAX > 2 ? 2 : 4;
+      uint4 kr[U], vr[U];
+      auto cached = [&](int at) {
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+          kr[u] = vr[u] = make_uint4(0, 0, 0, 0);
+          const long long k = at + 16 * u + str;
+          if (k < n_old) {
+            kr[u] = *reinterpret_cast<const uint4*>(Kb + (k0 + k) * a.kv + hl * 8);
+            vr[u] = *reinterpret_cast<const uint4*>(Vb + (k0 + k) * a.kv + hl * 8);
+          }
+        }
+      };
+      for (int i = tid + 64 * U; i < n_old * 4; i += THREADS) {
+        const bf16* r = (i & 2 ? Vb : Kb) + (long long)(k0 + (i >> 2)) * a.kv + (i & 1) * 64;
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(r));
+      }
       const long long rot = (long long)a.pos[b] * (HD / 2) + 2 * lane;
       const float2 cs = *reinterpret_cast<const float2*>(a.cos_t + rot), sn = *reinterpret_cast<const float2*>(a.sin_t + rot);
       uint2 ve = make_uint2(0, 0);
@@ -327,53 +370,46 @@ __global__ void __launch_bounds__(THREADS + 32, 1) k_decode_step(const DecodeSte
         ve = *reinterpret_cast<const uint2*>(blk.ve + (long long)a.tok0[b] * a.kv + (long long)kvh * HD + 4 * lane);
         if (lane < 12) wg = a.theta[blk.ve_gate + lane * a.Hkv + kvh];
       }
-      if (!any) {
-        for (int i = tid; i < (k1 - k0) * 4; i += THREADS) {      // the cached rows are on their way while the projections finish
-          const bf16* r = (i & 2 ? Vb : Kb) + (long long)(k0 + (i >> 2)) * a.kv + (i & 1) * 64;
-          asm volatile("prefetch.global.L2 [%0];" ::"l"(r));
-        }
-        wait(5 * l, blocks_of(4 * l));
-      }
-      any = true;
+      cached(0);
       // queries, and with the last range the new key and value: one warp a vector
       for (int v = warp; v < G + (last ? 2 : 0); v += WARPS) {
         const int col = v < G ? (kvh * G + v) * HD : d + (v - G) * a.kv + kvh * HD;
-        const float* src = a.qkv + (long long)b * a.dq + col;
-        if (v < G + 1) {        // channels 2 lane, 2 lane + 1 and their partners 64 further
-          const float2 x1 = __ldcg(reinterpret_cast<const float2*>(src + 2 * lane)), x2 = __ldcg(reinterpret_cast<const float2*>(src + 64 + 2 * lane));
+        const uint2* src = a.qkv + (long long)b * a.dq + col;
+        uint4 p, q;
+        const int at = v <= G ? 2 * lane : 4 * lane;
+        until([&] {
+          p = named_load2(src + at); q = named_load2(src + at + (v <= G ? 64 : 2));
+          return p.y == name && p.w == name && q.y == name && q.w == name;
+        });
+        float4 x = make_float4(__uint_as_float(p.x), __uint_as_float(p.z), __uint_as_float(q.x), __uint_as_float(q.z));
+        if (v <= G) {        // channels 2 lane, 2 lane + 1 and their partners 64 further
           const float c0 = round_to<bf16>(cs.x), c1 = round_to<bf16>(cs.y), s0 = round_to<bf16>(sn.x), s1 = round_to<bf16>(sn.y);
-          const float y0 = x1.x * c0 + x2.x * s0, y1 = x1.y * c1 + x2.y * s1, z0 = -x1.x * s0 + x2.x * c0, z1 = -x1.y * s1 + x2.y * c1;
+          const float y0 = x.x * c0 + x.z * s0, y1 = x.y * c1 + x.w * s1, z0 = -x.x * s0 + x.z * c0, z1 = -x.y * s1 + x.w * c1;
           const float r = 1.2f / sqrtf(warp_sum(y0 * y0 + y1 * y1 + z0 * z0 + z1 * z1) / HD + a.eps);
           if (v < G) {
             const float f = r * rsqrtf((float)HD);
             *reinterpret_cast<float2*>(&qs[v][2 * lane]) = make_float2(y0 * f, y1 * f);
             *reinterpret_cast<float2*>(&qs[v][64 + 2 * lane]) = make_float2(z0 * f, z1 * f);
           } else {
-            const uint32_t p = pack2(y0 * r, y1 * r), q = pack2(z0 * r, z1 * r);
+            const uint32_t lo2 = pack2(y0 * r, y1 * r), hi2 = pack2(z0 * r, z1 * r);
             bf16* dst = Kb + (long long)a.t * a.kv;
-            *reinterpret_cast<uint32_t*>(dst + 2 * lane) = p;
-            *reinterpret_cast<uint32_t*>(dst + 64 + 2 * lane) = q;
-            kvs[0][2 * lane] = __uint_as_float(p << 16); kvs[0][2 * lane + 1] = __uint_as_float(p & 0xffff0000u);
-            kvs[0][64 + 2 * lane] = __uint_as_float(q << 16); kvs[0][65 + 2 * lane] = __uint_as_float(q & 0xffff0000u);
+            *reinterpret_cast<uint32_t*>(dst + 2 * lane) = lo2;
+            *reinterpret_cast<uint32_t*>(dst + 64 + 2 * lane) = hi2;
+            kvs[0][2 * lane] = lo_f(lo2); kvs[0][2 * lane + 1] = hi_f(lo2);
+            kvs[0][64 + 2 * lane] = lo_f(hi2); kvs[0][65 + 2 * lane] = hi_f(hi2);
           }
         } else {
-          float4 x = ld4(src + 4 * lane);
           if (blk.ve) {
-            const float pre = warp_sum(lane < 12 ? __ldcg(a.xm + (long long)b * d + lane) * __ldcg(a.inv + b) * wg : 0.f);
+            const float pre = warp_sum(lane < 12 ? word(a.h16 + b * 16 + lane, name) * wg : 0.f);
             const float gate = 3.f / (1.f + expf(-pre));
-            x.x += gate * __uint_as_float(ve.x << 16); x.y += gate * __uint_as_float(ve.x & 0xffff0000u);
-            x.z += gate * __uint_as_float(ve.y << 16); x.w += gate * __uint_as_float(ve.y & 0xffff0000u);
+            x.x += gate * lo_f(ve.x); x.y += gate * hi_f(ve.x); x.z += gate * lo_f(ve.y); x.w += gate * hi_f(ve.y);
           }
-          const uint32_t p = pack2(x.x, x.y), q = pack2(x.z, x.w);
-          *reinterpret_cast<uint2*>(Vb + (long long)a.t * a.kv + 4 * lane) = make_uint2(p, q);
-          kvs[1][4 * lane] = __uint_as_float(p << 16); kvs[1][4 * lane + 1] = __uint_as_float(p & 0xffff0000u);
-          kvs[1][4 * lane + 2] = __uint_as_float(q << 16); kvs[1][4 * lane + 3] = __uint_as_float(q & 0xffff0000u);
+          const uint32_t lo2 = pack2(x.x, x.y), hi2 = pack2(x.z, x.w);
+          *reinterpret_cast<uint2*>(Vb + (long long)a.t * a.kv + 4 * lane) = make_uint2(lo2, hi2);
+          kvs[1][4 * lane] = lo_f(lo2); kvs[1][4 * lane + 1] = hi_f(lo2); kvs[1][4 * lane + 2] = lo_f(hi2); kvs[1][4 * lane + 3] = hi_f(hi2);
         }
       }
       compute_sync();
-      // half a warp takes every sixteenth key, four at a time; a lane has eight channels
-      const int hl = lane & 15, str = warp * 2 + (lane >> 4);
-      constexpr int U = GMAX > 2 ? 2 : 4;
       constexpr int QR = GMAX > 2 ? 1 : GMAX;      // many heads: their queries stay in shared memory
       float q[QR][8], o[GMAX][8] = {}, m[GMAX], lsum[GMAX] = {};
 #pragma unroll
@@ -383,22 +419,26 @@ __global__ void __launch_bounds__(THREADS + 32, 1) k_decode_step(const DecodeSte
 #pragma unroll
         for (int e = 0; e < 8; e++) q[h][e] = h < G ? qs[h][hl * 8 + e] : 0.f;
       }
-      const int rounds = k1 - k0 + (last ? 1 : 0);
-      for (int base = 0; base < rounds; base += 16 * U) {
+      const int n_keys = n_old + (last ? 1 : 0);
+      for (int base = 0; base < n_keys; base += 16 * U) {
         float kf[U][8], vf[U][8];
         bool ok[U];
 #pragma unroll
         for (int u = 0; u < U; u++) {
           const int k = base + 16 * u + str;
-          ok[u] = k < rounds;
-          if (k < k1 - k0) {
-            load_vec<bf16, 8>(Kb + (long long)(k0 + k) * a.kv + hl * 8, kf[u]);
-            load_vec<bf16, 8>(Vb + (long long)(k0 + k) * a.kv + hl * 8, vf[u]);
-          } else {
+          ok[u] = k < n_keys;
+          const uint32_t pk[4] = {kr[u].x, kr[u].y, kr[u].z, kr[u].w}, pv[4] = {vr[u].x, vr[u].y, vr[u].z, vr[u].w};
 #pragma unroll
-            for (int e = 0; e < 8; e++) { kf[u][e] = ok[u] ? kvs[0][hl * 8 + e] : 0.f; vf[u][e] = ok[u] ? kvs[1][hl * 8 + e] : 0.f; }
+          for (int e = 0; e < 8; e++) {
+            kf[u][e] = e & 1 ? hi_f(pk[e >> 1]) : lo_f(pk[e >> 1]);
+            vf[u][e] = e & 1 ? hi_f(pv[e >> 1]) : lo_f(pv[e >> 1]);
+          }
+          if (k == n_old && last) {
+#pragma unroll
+            for (int e = 0; e < 8; e++) { kf[u][e] = kvs[0][hl * 8 + e]; vf[u][e] = kvs[1][hl * 8 + e]; }
           }
         }
+        if (base + 16 * U < n_old) cached(base + 16 * U);
 #pragma unroll
         for (int h = 0; h < GMAX; h++) {
           if (h >= G) break;
@@ -408,10 +448,14 @@ __global__ void __launch_bounds__(THREADS + 32, 1) k_decode_step(const DecodeSte
             s[u] = 0.f;
 #pragma unroll
             for (int e = 0; e < 8; e++) s[u] = fmaf(GMAX > 2 ? qs[h][hl * 8 + e] : q[h < QR ? h : 0][e], kf[u][e], s[u]);
-#pragma unroll
-            for (int x = 8; x > 0; x >>= 1) s[u] += __shfl_xor_sync(0xffffffffu, s[u], x);
-            if (ok[u]) mn = fmaxf(mn, s[u]);
           }
+#pragma unroll
+          for (int x = 8; x > 0; x >>= 1)
+#pragma unroll
+            for (int u = 0; u < U; u++) s[u] += __shfl_xor_sync(0xffffffffu, s[u], x);
+#pragma unroll
+          for (int u = 0; u < U; u++)
+            if (ok[u]) mn = fmaxf(mn, s[u]);
           if (mn == -INFINITY) continue;      // no key yet (the shuffles above were for both halves)
           const float corr = __expf(m[h] - mn);          // 0 for the first keys
           lsum[h] *= corr;
@@ -445,111 +489,114 @@ __global__ void __launch_bounds__(THREADS + 32, 1) k_decode_step(const DecodeSte
         if (lane == 0) { r[HD] = mn; r[HD + 1] = L; }
       }
       compute_sync();
+      // and the ranges, in order, by the block that has the first (several ranges: an item a block, so nobody it waits for waits for it)
       for (int i = tid; i < G * HD; i += THREADS) {
         const int h = i / HD, ch = i % HD;
         float M = -INFINITY, L = 0.f, v = 0.f;
+#pragma unroll
         for (int w = 0; w < WARPS; w++) M = fmaxf(M, red[(w * GMAX + h) * (HD + 4) + HD]);
+#pragma unroll
         for (int w = 0; w < WARPS; w++) {
           const float* r = red + (w * GMAX + h) * (HD + 4);
           const float f = r[HD] == -INFINITY ? 0.f : __expf(r[HD] - M);
           L += r[HD + 1] * f; v += r[ch] * f;
         }
-        const long long at = ((long long)b * a.H + kvh * G + h) * a.splits + sp;
-        a.att[at * HD + ch] = v;
-        if (ch == 0) a.att_ml[at] = make_float2(M, L);
+        const long long head = (long long)b * a.H + kvh * G + h;
+        uint2* part = a.att_part + head * MAX_SPLITS * (HD + 2);
+        if (sp > 0) {
+          part += sp * (HD + 2);
+          named_store(part + 2 + ch, v, name);
+          if (ch < 2) named_store(part + ch, ch ? L : M, name);
+          continue;
+        }
+        for (int s0 = 1; s0 < a.splits; s0 += 4) {
+          uint4 ml[4];
+          uint2 ov[4];
+          until([&] {
+            bool ok = true;
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+              const int s = min(s0 + u, a.splits - 1);
+              ml[u] = named_load2(part + s * (HD + 2));
+              ov[u] = named_load(part + s * (HD + 2) + 2 + ch);
+              ok &= ml[u].y == name && ml[u].w == name && ov[u].y == name;
+            }
+            return ok;
+          });
+#pragma unroll
+          for (int u = 0; u < 4; u++) {
+            const float ms = s0 + u < a.splits ? __uint_as_float(ml[u].x) : -INFINITY, mn = fmaxf(M, ms);
+            if (mn == -INFINITY) continue;
+            const float f = M == -INFINITY ? 0.f : __expf(M - mn), e = ms == -INFINITY ? 0.f : __expf(ms - mn);
+            L = L * f + __uint_as_float(ml[u].z) * e; v = v * f + __uint_as_float(ov[u].x) * e; M = mn;
+          }
+        }
+        store_pair(a.att + head * (HD / 2), ch, v / L, name);
       }
       compute_sync();
     }
-    if (any) arrive(5 * l + 1);
     // ---- output projection ----
     if (int j2 = first_item(4 * l + 1); j2 < items.y) {
-      wait(5 * l + 1, min(n_attn, grid));
-      constexpr int U = 4;
-      for (int q0 = warp; q0 < B * a.H; q0 += WARPS * U) {       // a warp joins the ranges of a head, U heads at a time
-        float2 ml[U];
-        float4 v[U] = {};
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-          ml[u] = make_float2(-INFINITY, 0.f);
-          if (lane < a.splits && q0 + u * WARPS < B * a.H) ml[u] = __ldcg(a.att_ml + (long long)(q0 + u * WARPS) * a.splits + lane);
-        }
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-          ml[u].x = __expf(ml[u].x - warp_max(ml[u].x));      // 0 in the lanes without a range
-        }
-#pragma unroll 4
-        for (int s = 0; s < a.splits; s++) {
-          float4 p[U];
-#pragma unroll
-          for (int u = 0; u < U; u++)
-            p[u] = ld4(a.att + ((long long)min(q0 + u * WARPS, B * a.H - 1) * a.splits + s) * HD + lane * 4);
-#pragma unroll
-          for (int u = 0; u < U; u++) {
-            const float w = __shfl_sync(0xffffffffu, ml[u].x, s);
-            v[u].x += w * p[u].x; v[u].y += w * p[u].y; v[u].z += w * p[u].z; v[u].w += w * p[u].w;
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-          const int q = q0 + u * WARPS;
-          if (q >= B * a.H) break;
-          const float r = 1.f / warp_sum(ml[u].y * ml[u].x);
-          put4(X + q / a.H * xp, q % a.H * HD + lane * 4, pack2(v[u].x * r, v[u].y * r), pack2(v[u].z * r, v[u].w * r));
-        }
-      }
-      compute_sync();
+      rows_of(a.att, d / 2, name, false);
       for (; j2 < items.y; j2 += grid)
-        product(j2, false, [&](int b, int col, float v) { const long long at = (long long)b * d + col; a.xa[at] = __ldcg(a.xm + at) + v; });
-      arrive(5 * l + 2);
+        product(j2, false, [&](int b, int col) { return word(a.xm + (long long)b * d + col, name); },
+                [&](int b, int col, float v, float x) {
+                  v += x;
+                  named_store(a.xa + (long long)b * d + col, v, name);
+                  store_pair(a.xa2 + (long long)b * d / 2, col, v, name);
+                });
     }
     // ---- norm, MLP up ----
     if (int j2 = first_item(4 * l + 2); j2 < items.z) {
-      wait(5 * l + 2, blocks_of(4 * l + 1));
-      rows_of([&](int b, int col) { return ld4(a.xa + (long long)b * d + col); }, [](int, int, float4 v) { return v; });
+      rows_of(a.xa2, d / 2, name, true);
       for (; j2 < items.z; j2 += grid)
-        product(j2, true, [&](int b, int col, float v) { v = fmaxf(v, 0.f); a.up[(long long)b * 4 * d + col] = __float2bfloat16_rn(v * v); });
-      arrive(5 * l + 3);
+        product(j2, true, nothing, [&](int b, int col, float v, float) {
+          v = fmaxf(v, 0.f);
+          store_pair(a.up + (long long)b * 2 * d, col, v * v, name);
+        });
     }
     // ---- MLP down: a quarter of the inner rows an item ----
-    if (int j2 = first_item(4 * l + 3); j2 < items.w) {
-      wait(5 * l + 3, blocks_of(4 * l + 2));
+    if (int j2 = first_item(4 * l + 3), tiles = d >> 6; j2 < items.w) {
+      const int first = j2;
       for (; j2 < items.w; j2 += grid) {
-        const int tiles = d >> 6, ks = j2 / tiles, n8 = d >> 3;
-        constexpr int U = 4;
-        for (int i0 = tid; i0 < B * n8; i0 += THREADS * U) {
-          uint4 v[U];
-#pragma unroll
-          for (int u = 0; u < U; u++) {
-            const int i = min(i0 + u * THREADS, B * n8 - 1);
-            v[u] = __ldcg(reinterpret_cast<const uint4*>(a.up + (long long)(i / n8) * 4 * d + ks * d + i % n8 * 8));
-          }
-#pragma unroll
-          for (int u = 0; u < U; u++) {
-            const int i = i0 + u * THREADS;
-            if (i >= B * n8) break;
-            bf16* row = X + i / n8 * xp;
-            put4(row, i % n8 * 8, v[u].x, v[u].y);
-            put4(row, i % n8 * 8 + 4, v[u].z, v[u].w);
-          }
-        }
-        compute_sync();
-        product(j2 - ks * tiles, false, [&](int b, int col, float v) { a.part[ks * Bd + (long long)b * d + col] = v; });
+        const int ks = j2 / tiles;
+        rows_of(a.up + ks * (d / 2), 2 * d, name, false);
+        product(j2 - ks * tiles, false, nothing, [&](int b, int col, float v, float) { named_store(a.part + ks * Bd + (long long)b * d + col, v, name); });
       }
-      arrive(5 * l + 4);
+      // the stream after the block, by who had the first quarter of its columns: the next block's mix, or what the head reads
+      const bool end = l + 1 == a.L;
+      const float lb = end ? 0.f : a.theta[blocks[l + 1].lam_b], l0 = end ? -a.theta[a.off_lam_y] : a.theta[blocks[l + 1].lam_x0];
+      for (int t = first; t < tiles; t += grid) {
+#pragma unroll
+        for (int k = 0; k < 2 * NT; k++) {
+          const int o = tid + k * THREADS, b = o >> 6, col = t * 64 + (o & 63);
+          if (o >= 64 * B) break;
+          const long long at = (long long)b * d + col;
+          const float e = a.x0[at];
+          uint2 w[5];
+          until([&] {
+            w[0] = named_load(a.xa + at);
+            bool ok = w[0].y == name;
+#pragma unroll
+            for (int s = 0; s < 4; s++) { w[1 + s] = named_load(a.part + s * Bd + at); ok &= w[1 + s].y == name; }
+            return ok;
+          });
+          float x = __uint_as_float(w[0].x);
+#pragma unroll
+          for (int s = 0; s < 4; s++) x += __uint_as_float(w[1 + s].x);
+          if (l == a.backout && !end) named_store(a.xb + at, x, name);
+          if (end) x += l0 * (l == a.backout ? x : word(a.xb + at, launch * (a.L + 1) + a.backout + 1));
+          else { x = lb * x + l0 * e; named_store(a.xm + at, x, name + 1); }
+          store_pair(a.xn + (long long)b * d / 2, col, x, name + 1);
+        }
+      }
     }
   }
-  // ---- backout, norm, head ----
+  // ---- norm, head ----
   if (int j = first_item(4 * a.L); j < a.Vp >> 6) {
-    const float ly = a.theta[a.off_lam_y];
-    wait(5 * a.L - 1, blocks_of(4 * a.L - 1));
-    const bool same = a.backout == a.L - 1;
-    rows_of([&](int b, int col) {
-              const float4 x = stream(b, col), y = same ? x : ld4(a.xb + (long long)b * d + col);
-              return make_float4(x.x - ly * y.x, x.y - ly * y.y, x.z - ly * y.z, x.w - ly * y.w);
-            },
-            [](int, int, float4 v) { return v; });
+    rows_of(a.xn, d / 2, (launch + 1) * (a.L + 1), true);
     for (; j < a.Vp >> 6; j += grid)
-      product(j, true, [&](int b, int col, float v) { if (col < a.V) a.logits[(long long)b * a.V + col] = 15.f * tanhf(v / 15.f); });
+      product(j, true, nothing, [&](int b, int col, float v, float) { if (col < a.V) a.logits[(long long)b * a.V + col] = 15.f * tanhf(v / 15.f); });
   }
 }
 
@@ -564,7 +611,7 @@ template <int NT, int GMAX> int resident_blocks(size_t smem) {
   auto kernel = k_decode_step<NT, GMAX, ring_of<NT>()>;
   int per = 0;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, THREADS + 32, smem) != cudaSuccess) {
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, THREADS + 128, smem) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
@@ -601,11 +648,13 @@ void decode_step_carve(const femto_handle* h, char*& p, DecodeStepState& st) {
   const size_t d = h->d, n = st.columns;
   take(st.maps, sizeof(CUtensorMap) * (4 * h->L + 1));
   take(st.blocks, sizeof(DecodeBlock) * h->L);
-  take(st.counters, 4 * COUNTER_STRIDE * (size_t)(5 * h->L));
-  take(st.x0, 4 * n * d); take(st.xm, 4 * n * d); take(st.xa, 4 * n * d); take(st.xb, 4 * n * d);
-  take(st.part, 16 * n * d); take(st.qkv, 4 * n * h->dq); take(st.inv, 4 * n);
-  take(st.up, 2 * n * 4 * d);
-  take(st.att, 4 * n * h->H * MAX_SPLITS * HD); take(st.att_ml, 8 * n * h->H * MAX_SPLITS);
+  char* first = p;
+  take(st.launches, 8);
+  take(st.xn, 4 * n * d); take(st.xm, 8 * n * d); take(st.xa, 8 * n * d); take(st.xa2, 4 * n * d); take(st.xb, 8 * n * d);
+  take(st.part, 32 * n * d); take(st.qkv, 8 * n * h->dq); take(st.h16, 8 * 16 * n); take(st.up, 16 * n * d); take(st.att, 4 * n * d);
+  take(st.att_part, 8 * n * h->H * MAX_SPLITS * (HD + 2));
+  st.named_bytes = p - first;
+  take(st.x0, 4 * n * d);
 }
 
 int decode_step_setup(const femto_handle* h, DecodeStepState& st, const std::vector<void*>& K, const std::vector<void*>& V) {
@@ -629,14 +678,15 @@ int decode_step_setup(const femto_handle* h, DecodeStepState& st, const std::vec
   }
   FEMTO_TRY(put(h->sh_lm, h->d, h->Vp));
   CUDA_TRY(cudaMemcpy(st.blocks, bl.data(), sizeof(DecodeBlock) * bl.size(), cudaMemcpyHostToDevice));
+  CUDA_TRY(cudaMemset(st.launches, 0, st.named_bytes));      // no word has a name yet
   CUDA_TRY(cudaMemcpy(st.maps, maps.data(), sizeof(CUtensorMap) * maps.size(), cudaMemcpyHostToDevice));
   return 0;
 }
 
 int decode_step_run(const femto_handle* h, const DecodeStepState& st, DecodeStepArgs a, const int* tokens, const int* positions, cudaStream_t s) {
-  a.blocks = st.blocks; a.maps = st.maps; a.counters = st.counters; a.n_counters = 5 * h->L;
-  a.x0 = st.x0; a.xm = st.xm; a.xa = st.xa; a.xb = st.xb; a.part = st.part; a.qkv = st.qkv; a.inv = st.inv; a.up = st.up; a.att = st.att;
-  a.att_ml = st.att_ml;
+  a.blocks = st.blocks; a.maps = st.maps; a.launches = st.launches; a.x0 = st.x0;
+  a.xn = st.xn; a.xm = st.xm; a.xa = st.xa; a.xa2 = st.xa2; a.xb = st.xb; a.part = st.part; a.qkv = st.qkv; a.h16 = st.h16; a.up = st.up;
+  a.att = st.att; a.att_part = st.att_part;
   a.wte = (const bf16*)h->sh_wte; a.sin_t = h->sin_t; a.cos_t = h->cos_t; a.status = h->status;
   a.off_smear = h->off_smear; a.off_lam_s = h->off_lam_s; a.off_lam_y = h->off_lam_y;
   a.d = h->d; a.dq = h->dq; a.kv = h->kv; a.H = h->H; a.Hkv = h->Hkv; a.V = h->V; a.Vp = h->Vp; a.L = h->L; a.backout = h->backout; a.eps = h->eps;
@@ -651,7 +701,7 @@ int decode_step_run(const femto_handle* h, const DecodeStepState& st, DecodeStep
   const size_t smem = smem_bytes(a.d, a.L, nt, gmax);
   a.red_bytes = (int)red_bytes(nt, gmax);
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = st.blocks_n; cfg.blockDim = THREADS + 32; cfg.dynamicSmemBytes = smem; cfg.stream = s;
+  cfg.gridDim = st.blocks_n; cfg.blockDim = THREADS + 128; cfg.dynamicSmemBytes = smem; cfg.stream = s;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeCooperative;      // the blocks wait for one another: all of them are resident or none is
   at[0].val.cooperative = 1;

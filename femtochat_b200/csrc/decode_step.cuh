@@ -14,19 +14,20 @@ struct DecodeStepState {
   int blocks_n = 0, columns = 0;     // blocks of the kernel, and the columns it takes; 0: this model takes the chain of kernels
   CUtensorMap* maps = nullptr;       // four a block (QKV, wo, fc, proj), then the head
   DecodeBlock* blocks = nullptr;
-  unsigned int* counters = nullptr;
-  // [columns][width], fp32 unless noted: embedding, mixed stream, stream after the attention, stream for the backout,
-  // four partial sums of the MLP, projections, reciprocal norms, MLP inner (bf16), attention partials and their (max, sum)
-  float *x0 = nullptr, *xm = nullptr, *xa = nullptr, *xb = nullptr, *part = nullptr, *qkv = nullptr, *inv = nullptr, *att = nullptr;
-  float2* att_ml = nullptr;
-  bf16* up = nullptr;
+  unsigned int* launches = nullptr;
+  // Words of 8 bytes, data and name; [columns][width], a pair of bf16 a word (2) or one fp32 (4): what the QKV and the head read (2),
+  // the mixed stream (4), the stream after the attention (4, 2), the stream for the backout (4), four partial sums of the MLP (4),
+  // projections (4), the first 16 of the normalised row (4), MLP inner (2), attention (2) and its ranges (4: max, sum, channels)
+  uint2 *xn = nullptr, *xm = nullptr, *xa = nullptr, *xa2 = nullptr, *xb = nullptr, *part = nullptr, *qkv = nullptr, *h16 = nullptr,
+        *up = nullptr, *att = nullptr, *att_part = nullptr;
+  size_t named_bytes = 0;
+  float* x0 = nullptr;               // embedding
 };
 
 struct DecodeStepArgs {
-  const CUtensorMap* maps; const DecodeBlock* blocks; unsigned int* counters;
-  float *x0, *xm, *xa, *xb, *part, *qkv, *inv, *att;
-  float2* att_ml;
-  bf16* up;
+  const CUtensorMap* maps; const DecodeBlock* blocks; unsigned int* launches;
+  uint2 *xn, *xm, *xa, *xa2, *xb, *part, *qkv, *h16, *up, *att, *att_part;
+  float* x0;
   const float* theta;
   const bf16* wte; bf16* xe_prev;
   const float *sin_t, *cos_t;
@@ -34,7 +35,7 @@ struct DecodeStepArgs {
   float* logits;
   unsigned int* status;
   long long off_smear, off_lam_s, off_lam_y;
-  int d, dq, kv, H, Hkv, V, Vp, L, backout, B, t, maxT, docs, splits, n_counters, red_bytes;
+  int d, dq, kv, H, Hkv, V, Vp, L, backout, B, t, maxT, docs, splits, red_bytes;
   float eps;
 };
 
