@@ -165,8 +165,8 @@ struct GemmArgs {
   // fp32 split output: up to 3 column segments of C go to different destinations (fused QKV dW).
   int nseg = 0; int seg_col0[3] = {0, 0, 0}; int seg_ncol[3] = {0, 0, 0};
   float* seg_ptr[3] = {nullptr, nullptr, nullptr}; long long seg_ld[3] = {0, 0, 0};
-  // square symmetric result: tiles that lie entirely below the diagonal are not computed (the caller mirrors
-  // the upper triangle afterwards); honoured by the tensor-core kernel, ignored by the SIMT fallback
+  // square symmetric result (EPI_STORE, EPI_AXPBY): tiles that lie entirely below the diagonal are not computed.  The SIMT
+  // kernel stores the others a second time, transposed; after the tensor-core kernel the caller mirrors the upper triangle
   bool upper_only = false;
   // Grouped product (EPI_STORE, EPI_RELU2; batch 1): the rows of A come in runs of group_rows (128 or 256) rows, run i is
   // multiplied by matrix groups[1 + i] of B (strideB apart), and only the first groups[0] runs hold anything.  Device memory:

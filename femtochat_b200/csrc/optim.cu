@@ -429,7 +429,7 @@ int newton_schulz_t(T* S, T* S2, T* A, T* B2, int k, int in, int out, const floa
     g.C = A; g.ldc = r; g.strideC = rr; g.M = r; g.N = r; g.K = tall ? out : in; g.epi = EPI_STORE;
     g.upper_only = true;   // X X^T is symmetric: compute the tiles on and above the diagonal, mirror the rest
     FEMTO_TRY(gemm<T>(g, s));
-    FEMTO_TRY(mirror_upper<T>(A, r, rr, k, s));
+    if (sizeof(T) == 2 && gemm_tc_supported(g)) FEMTO_TRY(mirror_upper<T>(A, r, rr, k, s));
     // B2 = b A + c A A
     GemmArgs g2;
     g2.ws = ws; g2.ws_bytes = ws_bytes; g2.status = status; g2.batch = k;
@@ -438,7 +438,7 @@ int newton_schulz_t(T* S, T* S2, T* A, T* B2, int k, int in, int out, const floa
     g2.epi = EPI_AXPBY; g2.aux = A; g2.ldaux = r; g2.strideAux = rr; g2.alpha = b; g2.beta = c;
     g2.upper_only = true;  // a polynomial of a symmetric matrix is symmetric
     FEMTO_TRY(gemm<T>(g2, s));
-    FEMTO_TRY(mirror_upper<T>(B2, r, rr, k, s));
+    if (sizeof(T) == 2 && gemm_tc_supported(g2)) FEMTO_TRY(mirror_upper<T>(B2, r, rr, k, s));
     // X' = a X + B2 X   (stored orientation: S' = a S + B2 S when tall, S' = a S + S B2 otherwise)
     GemmArgs g3;
     g3.ws = ws; g3.ws_bytes = ws_bytes; g3.status = status; g3.batch = k;

@@ -40,6 +40,15 @@ def test_gemm_bf16_all_operand_layouts(ak, bk, shape):
     assert err <= 2.0 ** -8 * ref.abs().max()               # one bf16 rounding of the result
 
 
+@pytest.mark.parametrize("ak", [True, False])
+@pytest.mark.parametrize("bk", [True, False])
+@pytest.mark.parametrize("shape", [(1, 7, 5, 2), (63, 65, 17, 1), (66, 130, 127, 3), (129, 67, 1031, 1), (68, 60, 516, 2)])
+def test_gemm_simt_all_operand_layouts(ak, bk, shape):
+    """Pitches and sizes that the tensor-core kernel does not take: edges of the 64 x 64 tiles, groups of four elements that are
+    not aligned or reach past the end, K shared by the blocks of a cluster.  One bf16 rounding of the result, as above."""
+    test_gemm_bf16_all_operand_layouts(ak, bk, shape)
+
+
 def test_gemm_split_k_fp32_accumulate_is_deterministic():
     """Weight-gradient form: both operands MN-contiguous, K = tokens, fp32 C += ; split-K reduce in fixed order."""
     M, N, K = 1280, 1280, 8192
