@@ -118,6 +118,13 @@ def test_attention_forward_and_reverse(dtype, B, T, H, Hkv, hd, left, docs):
         assert rel <= (1e-2 if dtype == _lib.BF16 else 1e-5), rel
 
 
+@pytest.mark.parametrize("B,T,H,Hkv,hd,left,docs", [(2, 1, 2, 1, 24, 5, False), (1, 3, 2, 2, 32, 1, False), (2, 6, 3, 1, 50, 4, True),
+                                                    (1, 37, 2, 1, 128, 9, True), (1, 66, 2, 2, 200, 66, False)])
+def test_attention_of_fp32_widths(B, T, H, Hkv, hd, left, docs):
+    """Every width of the SIMT kernels' registers, and rows whose keys and queries do and do not fill groups of four."""
+    test_attention_forward_and_reverse(_lib.F32, B, T, H, Hkv, hd, left, docs)
+
+
 @pytest.mark.parametrize("B,T,H,Hkv,left,docs", [
     (2, 1, 2, 1, 1, False), (3, 5, 2, 2, 5, True), (2, 127, 2, 1, 127, False), (2, 129, 4, 2, 40, True), (3, 255, 2, 2, 255, True),
     (2, 257, 6, 2, 100, False), (1, 1000, 10, 5, 300, True), (2, 1153, 2, 1, 2000, False)])
