@@ -118,10 +118,11 @@ def test_attention_forward_and_reverse(dtype, B, T, H, Hkv, hd, left, docs):
         assert rel <= (1e-2 if dtype == _lib.BF16 else 1e-5), rel
 
 
-@pytest.mark.parametrize("B,T,H,Hkv,hd,left,docs", [(2, 1, 2, 1, 24, 5, False), (1, 3, 2, 2, 32, 1, False), (2, 6, 3, 1, 50, 4, True),
+@pytest.mark.parametrize("B,T,H,Hkv,hd,left,docs", [(2, 2, 2, 1, 24, 5, False), (1, 3, 2, 2, 32, 1, False), (2, 6, 3, 1, 50, 4, True),
                                                     (1, 37, 2, 1, 128, 9, True), (1, 66, 2, 2, 200, 66, False)])
 def test_attention_of_fp32_widths(B, T, H, Hkv, hd, left, docs):
-    """Every width of the SIMT kernels' registers, and rows whose keys and queries do and do not fill groups of four."""
+    """Every width of the SIMT kernels' registers, and rows whose keys and queries do and do not fill groups of four.
+    (Two tokens at least: the softmax of a single key is constant, so that dQ and dK are zero and have no relative error.)"""
     test_attention_forward_and_reverse(_lib.F32, B, T, H, Hkv, hd, left, docs)
 
 
