@@ -21,12 +21,15 @@ __device__ __forceinline__ float block_sum(float v) {
 }
 
 constexpr int RT = 256;   // threads of a row kernel: one row per block
+constexpr int FEW = 4;    // blocks that ask for the norms' weights ahead (one is enough; each asking cost a prompt of 4096 rows 1 %)
 
 template <typename T>
 __global__ void __launch_bounds__(RT) k_dec_embed(const T* __restrict__ table, const int* __restrict__ tokens, int ld_tok, int T_,
                                                   int base, int vocab, float scale, float* __restrict__ x, const NextNorms<T> nn, int d,
                                                   float eps, unsigned int* status) {
   pdl_trigger();
+  if (blockIdx.x < FEW) prefetch_l2(nn.w, 4ll * d, threadIdx.x, RT);
+  if (blockIdx.x < FEW && nn.h2) prefetch_l2(nn.w2, 4ll * d, threadIdx.x, RT);
   pdl_wait();
   const int row = blockIdx.x;
   int tk = tokens[(long long)(row / T_) * ld_tok + row % T_] - base;
@@ -71,6 +74,8 @@ template <typename T, int NV>
 __global__ void __launch_bounds__(RT) k_parallel_resid(float* __restrict__ x, const T* __restrict__ y, const T* __restrict__ y2, const MoeRows m,
                                                        const NextNorms<T> nn, int d, float eps) {
   pdl_trigger();
+  if (blockIdx.x < FEW && nn.h) prefetch_l2(nn.w, 4ll * d, threadIdx.x, RT);
+  if (blockIdx.x < FEW && nn.h2) prefetch_l2(nn.w2, 4ll * d, threadIdx.x, RT);
   pdl_wait();
   const long long row = blockIdx.x, base = row * d;
   auto expert_row = [&](int k, float& w) {
@@ -153,6 +158,8 @@ template <typename T, int NV>
 __global__ void __launch_bounds__(RT) k_resid_norm(float* __restrict__ x, const T* __restrict__ y, const float* __restrict__ w_post,
                                                    float m, const float* __restrict__ w_pre, T* __restrict__ h, int d, float eps) {
   pdl_trigger();
+  if (blockIdx.x < FEW) prefetch_l2(w_post, 4ll * d, threadIdx.x, RT);
+  if (blockIdx.x < FEW && h) prefetch_l2(w_pre, 4ll * d, threadIdx.x, RT);
   pdl_wait();
   const long long base = (long long)blockIdx.x * d;
   if constexpr (NV > 0) {
@@ -229,6 +236,7 @@ template <typename T>
 __global__ void __launch_bounds__(RT) k_gather_norm(const float* __restrict__ x, const int* __restrict__ want, int stride,
                                                     const float* __restrict__ w, T* __restrict__ h, int d, float eps) {
   pdl_trigger();
+  if (blockIdx.x < FEW) prefetch_l2(w, 4ll * d, threadIdx.x, RT);
   pdl_wait();
   const int i = blockIdx.x;
   const float* src = x + (long long)(want ? want[i] : (i + 1) * stride - 1) * d;
@@ -244,6 +252,7 @@ __global__ void __launch_bounds__(256) k_gated_norm(const T* __restrict__ in, co
                                                     const T* __restrict__ gate, long long ldg, T* __restrict__ out, long long n,
                                                     int groups, int size, float eps) {
   pdl_trigger();
+  if (blockIdx.x < FEW) prefetch_l2(w, 4ll * size * (w_all ? groups : 1), threadIdx.x, 256);
   pdl_wait();
   const int lane = threadIdx.x & (LG - 1);
   long long it = (long long)blockIdx.x * (256 / LG) + threadIdx.x / LG;
@@ -365,11 +374,12 @@ __global__ void __launch_bounds__(256) k_rows_mma(const bf16* __restrict__ X, lo
   const int* list = nullptr;
   if constexpr (LISTS) {
     pdl_wait();
-    if ((int)blockIdx.y >= bt.lists[0]) return;
     const int* g = bt.lists + 1 + 3 * blockIdx.y;
-    W += g[0] * bt.w;
-    list = bt.lists + 1 + 3 * bt.max_lists + g[1];
-    M = g[2];
+    const int n_lists = bt.lists[0], expert = g[0], start = g[1], length = g[2];      // four loads in flight; past n_lists they are not used
+    if ((int)blockIdx.y >= n_lists) return;
+    W += expert * bt.w;
+    list = bt.lists + 1 + 3 * bt.max_lists + start;
+    M = length;
   } else {
     X += blockIdx.y * bt.x;
     W += blockIdx.y * bt.w;
@@ -393,7 +403,14 @@ __global__ void __launch_bounds__(256) k_rows_mma(const bf16* __restrict__ X, lo
   const int kb = warp * 32 + c8;
 #pragma unroll
   for (int u = 0; u < U; u++) fetch(u, kb + u * 256);
-  if (!LISTS) pdl_wait();
+  if (!LISTS) {
+    // what does not fit the registers is on its way to L2: a line is 64 k, the share of two warps
+    if (!(warp & 1) && !(lane & 3))
+      for (int k = warp * 32 + U * 256; k < K; k += 256)
+#pragma unroll
+        for (int i = 0; i < 2 * RT; i++) prefetch_l2(wp[i] + k);
+    pdl_wait();
+  }
   const bf16* xp[NT];          // this lane's rows of X
 #pragma unroll
   for (int t = 0; t < NT; t++) {

@@ -187,10 +187,10 @@ template <typename T> int gemm_simt(const GemmArgs& g, cudaStream_t s) {
   const uintptr_t mask = 4 * sizeof(T) - 1;
   const bool vec_a = ((uintptr_t)g.A & mask) == 0 && ((g.lda | g.strideA) & 3) == 0;
   const bool vec_b = ((uintptr_t)g.B & mask) == 0 && ((g.ldb | g.strideB) & 3) == 0;
-  // K goes to as many blocks as bring about four to every multiprocessor, with at least 64 steps for each
+  // K goes to as many blocks as bring about four to every multiprocessor, with at least 128 steps for each
   const long long tiles = (long long)cdiv(g.N, TN) * cdiv(g.M, TM) * g.batch;
   int S = 1;
-  while (S < 8 && tiles * S < 4ll * device_sm_count() && g.K >= 2 * S * 64) S *= 2;
+  while (S < 8 && tiles * S < 4ll * device_sm_count() && g.K >= 2 * S * 128) S *= 2;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(cdiv(g.N, TN) * S, cdiv(g.M, TM), g.batch); cfg.blockDim = THREADS; cfg.stream = s;
   cudaLaunchAttribute at[2];

@@ -44,6 +44,9 @@ __device__ __forceinline__ void rotate(float u, float v, float pos, float freq, 
 template <typename T>
 __global__ void __launch_bounds__(256) k_latent_norms(const LatentArgs a) {
   pdl_trigger();
+  if (blockIdx.x < 4) prefetch_l2(a.dq_norm, 4ll * a.q_rank, threadIdx.x, 256);
+  if (blockIdx.x < 4) prefetch_l2(a.dkv_norm, 4ll * a.kv_rank, threadIdx.x, 256);
+  if (blockIdx.x < 4) prefetch_l2(a.freq, 4ll * (a.rot_dims / 2), threadIdx.x, 256);
   pdl_wait();
   constexpr int V = VecN<T>::n;
   const long long it = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -248,6 +251,11 @@ __global__ void __launch_bounds__(1024) k_absorb_q(const LatentArgs a) {
 template <int NK, int NP>
 __global__ void __launch_bounds__(256) k_latent_decode_mma(const LatentArgs a, int splits, int tiles_per, int KT, int width) {
   pdl_trigger();
+  {
+    const int n = a.first + (int)(blockIdx.z % a.T) + 1, k0 = blockIdx.y * tiles_per * KT, k1 = min(n, k0 + tiles_per * KT);
+    prefetch_l2(reinterpret_cast<const bf16*>(a.latent) + ((blockIdx.z / a.T) * (long long)a.maxT + k0) * a.ld, 2ll * a.ld * (k1 - k0), threadIdx.x, 256);
+    prefetch_l2(a.freq, 4ll * (a.rot_dims / 2), threadIdx.x, 256);
+  }
   pdl_wait();
   extern __shared__ __align__(16) uint8_t raw[];
   const int SP = KT + 4;

@@ -15,6 +15,8 @@ template <int NI> struct Tile { static constexpr int TOK = NI >= 8 ? 8 : 16; }; 
 template <typename T, bool DELTA, int NI>
 __global__ void __launch_bounds__(256) k_recurrence(const RecurrenceArgs a) {
   pdl_trigger();
+  prefetch_l2(a.S + (((long long)blockIdx.z * a.heads + blockIdx.y) * a.vdim + blockIdx.x * 32) * a.dim, 4ll * a.dim * min(32, a.vdim - (int)blockIdx.x * 32),
+              threadIdx.x, 256);
   pdl_wait();
   constexpr int DP = 32 * NI, TT = Tile<NI>::TOK;
   __shared__ __align__(16) float sq[TT][DP], sk[TT][DP], sg[DELTA ? TT : 1][DELTA ? DP : 4], sv[TT][32], sb[TT];
@@ -203,9 +205,29 @@ template <typename T> __device__ __forceinline__ float row_dot(const T* __restri
 template <typename T, int NI>
 __global__ void __launch_bounds__(1024) k_delta_decode(const DeltaDecodeArgs a) {
   pdl_trigger();
-  pdl_wait();
   constexpr int DP = 32 * NI;
   const DeltaPrepArgs& p = a.p;
+  {
+    // eight loads that wait for one another took 16 us a layer from memory
+    const int h = blockIdx.x, t = threadIdx.x, D = p.dim, E = p.vdim, n = p.taps, qh = h / (p.heads / p.kv_heads);
+    prefetch_l2(a.S + ((long long)blockIdx.y * p.heads + h) * E * D, 4ll * E * D, t, 1024);
+    prefetch_l2(reinterpret_cast<const T*>(a.w_a2) + (long long)h * D * a.ra, (long long)sizeof(T) * D * a.ra, t, 1024);
+    prefetch_l2(reinterpret_cast<const T*>(a.w_g2) + (long long)h * E * a.rg, (long long)sizeof(T) * E * a.rg, t, 1024);
+    prefetch_l2(p.conv_q + (long long)qh * D * n, 4ll * D * n, t, 1024);
+    prefetch_l2(p.conv_k + (long long)qh * D * n, 4ll * D * n, t, 1024);
+    prefetch_l2(p.conv_v + (long long)h * E * n, 4ll * E * n, t, 1024);
+    prefetch_l2(p.dt_bias + (long long)h * D, 4ll * D, t, 1024);
+    prefetch_l2(a.norm, 4ll * E, t, 1024);
+    if (t == 0) prefetch_l2(p.a_log + h);
+    const int channels = 2 * p.kv_heads * D + p.heads * E;
+    const T* tail = reinterpret_cast<const T*>(p.tail_in) + (long long)blockIdx.y * (n - 1) * channels;
+    for (int j = 0; j < n - 1; j++) {
+      prefetch_l2(tail + (long long)j * channels + qh * D, (long long)sizeof(T) * D, t, 1024);
+      prefetch_l2(tail + (long long)j * channels + (p.kv_heads + qh) * D, (long long)sizeof(T) * D, t, 1024);
+      prefetch_l2(tail + (long long)j * channels + 2 * p.kv_heads * D + h * E, (long long)sizeof(T) * E, t, 1024);
+    }
+  }
+  pdl_wait();
   extern __shared__ __align__(16) float sm[];
   float *sq = sm, *sk = sq + DP, *sg = sk + DP, *sv = sg + DP, *so = sv + p.vdim, *sz = so + p.vdim, *sa = sz + p.vdim, *sb = sa + a.ra;
   __shared__ float red[32], f_q, f_k;

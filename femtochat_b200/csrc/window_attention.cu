@@ -29,6 +29,8 @@ __global__ void __launch_bounds__(256) k_qk_norm(T* __restrict__ q, long long ld
                                                  int nq, int nk, int dim, const float* __restrict__ wq, const float* __restrict__ wk, float eps,
                                                  long long n) {
   pdl_trigger();
+  if (blockIdx.x < 4) prefetch_l2(wq, 4ll * dim, threadIdx.x, 256);
+  if (blockIdx.x < 4 && wk) prefetch_l2(wk, 4ll * dim, threadIdx.x, 256);
   pdl_wait();
   const int lane = threadIdx.x & (LG - 1);
   long long it = (long long)blockIdx.x * (256 / LG) + threadIdx.x / LG;
