@@ -21,15 +21,14 @@ __device__ __forceinline__ float block_sum(float v) {
 }
 
 constexpr int RT = 256;   // threads of a row kernel: one row per block
-constexpr int FEW = 4;    // blocks that ask for the norms' weights ahead (one is enough; each asking cost a prompt of 4096 rows 1 %)
+constexpr int FEW = 4;    // blocks that ask for the norms' weights ahead (one is enough; all of them asking cost a prompt of 4096 rows 1 %,
+                          // and any of k_parallel_resid's a prompt of 7108 rows 1.2 %)
 
 template <typename T>
 __global__ void __launch_bounds__(RT) k_dec_embed(const T* __restrict__ table, const int* __restrict__ tokens, int ld_tok, int T_,
                                                   int base, int vocab, float scale, float* __restrict__ x, const NextNorms<T> nn, int d,
                                                   float eps, unsigned int* status) {
   pdl_trigger();
-  if (blockIdx.x < FEW) prefetch_l2(nn.w, 4ll * d, threadIdx.x, RT);
-  if (blockIdx.x < FEW && nn.h2) prefetch_l2(nn.w2, 4ll * d, threadIdx.x, RT);
   pdl_wait();
   const int row = blockIdx.x;
   int tk = tokens[(long long)(row / T_) * ld_tok + row % T_] - base;
@@ -74,8 +73,6 @@ template <typename T, int NV>
 __global__ void __launch_bounds__(RT) k_parallel_resid(float* __restrict__ x, const T* __restrict__ y, const T* __restrict__ y2, const MoeRows m,
                                                        const NextNorms<T> nn, int d, float eps) {
   pdl_trigger();
-  if (blockIdx.x < FEW && nn.h) prefetch_l2(nn.w, 4ll * d, threadIdx.x, RT);
-  if (blockIdx.x < FEW && nn.h2) prefetch_l2(nn.w2, 4ll * d, threadIdx.x, RT);
   pdl_wait();
   const long long row = blockIdx.x, base = row * d;
   auto expert_row = [&](int k, float& w) {
