@@ -2,18 +2,20 @@
 // (the reference's Float32 path, src/gpt.jl:23-31) and of shapes the tcgen05 kernel does not
 // take (row pitches that are not multiples of 16 bytes, e.g. the 12 -> n_kv_head gate).
 //
-// 64 threads have a 64 x 64 tile, 8 x 8 results each as pairs (two multiply-adds an instruction): a step of k takes 32 of those
-// for four 16-byte loads from shared memory, which bound it (L1 68 % busy, fp32 pipe 34 %).  With so small a block even
-// 600 x 512 results are enough blocks once K is shared out: up to eight blocks of a cluster take ranges of K, and each adds
-// its share of the rows over the cluster's partial tiles, in order.  The next 16 steps of k are in registers while these run.
-// Newton-Schulz of four 512 x 2048 fp32 matrices: 22 TFLOP/s; a training step of 600 tokens, 512 wide (126 products): 14.4 ms
-// in them with 4 x 4 results a thread, scalar loads, one block a tile and nothing in flight (12 TFLOP/s), 7.9 ms so.
+// Every result is one chain of multiply-adds over k = 0, 1, ... in order, whatever the tile: a training step's results then are
+// the same bits at every tile size.  (K shared by the blocks of a cluster, partial sums added at the end, was as near to 64 bits, but over a
+// dozen updates of the same weights two orders of summation drift 1e-4 apart.)
+//
+// 64 threads have a W x W tile, 8 x 8 (W = 64) or 4 x 4 (32) results each as pairs (two multiply-adds an instruction): at 64 a step of k
+// takes 32 of those for four 16-byte loads from shared memory, which bound it.  The next steps of k are in registers while these run.
+// A training step of 600 tokens, 512 wide, four layers (126 products, most of them Newton-Schulz): 15.6 ms with 4 x 4 results a thread,
+// scalar loads and nothing in flight, 9.0 ms so; the introductory model (2 x 4 tokens, 32 wide) 1.45 -> 0.78 ms.
 #include "common.cuh"
 #include "sm100_ptx.cuh"
 
 namespace {
 
-constexpr int TM = 64, TN = 64, TK = 16, THREADS = 64;
+constexpr int THREADS = 64;
 
 // Four elements that follow each other in memory; those from `left` on are zero.
 template <typename T> __device__ __forceinline__ float4 load4(const T* p, bool vec, int left) {
@@ -34,51 +36,48 @@ template <typename T> __device__ __forceinline__ float4 load4(const T* p, bool v
   return v;
 }
 
-// A 64 x 16 piece of an operand: 16 elements a thread, into registers and from there to shared memory as [k][64].
-template <typename T> struct Piece {
-  float4 r[4];
-  // rows r0.. of n, steps k0.. up to k1
-  __device__ __forceinline__ void load(const T* p, long long ld, bool kmajor, bool vec, int r0, int n, int k0, int k1) {
-    const int t = threadIdx.x;
+// A W x TK piece of an operand in registers, and from there in shared memory as [k][W].  Of a k-contiguous operand, TK / 4 neighbouring
+// lanes read the TK elements of a row (one row a lane would be 32 lines an instruction), and the transposing stores of a warp
+// fall into 32 different banks because the columns of row k are permuted: m is at m ^ at(k).
+template <typename T, int W, int TK> struct Piece {
+  static constexpr int V = W * TK / (4 * THREADS), PER_M = TK / 4, PER_K = W / 4;      // lanes a row, a step of k
+  float4 r[V];
+  static __device__ __forceinline__ int at(int k) { return 32 / PER_M * (k >> 2); }
+  static __device__ __forceinline__ int row(int i, bool kmajor) { return kmajor ? threadIdx.x / PER_M + THREADS / PER_M * i : threadIdx.x % PER_K * 4; }
+  static __device__ __forceinline__ int step(int i, bool kmajor) { return kmajor ? threadIdx.x % PER_M * 4 : threadIdx.x / PER_K + THREADS / PER_K * i; }
+  // rows r0.. of n, steps k0.. of K
+  __device__ __forceinline__ void load(const T* p, long long ld, bool kmajor, bool vec, int r0, int n, int k0, int K) {
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const int row = kmajor ? r0 + t : r0 + (t & 15) * 4, k = kmajor ? k0 + 4 * i : k0 + (t >> 4) + 4 * i;
-      const int left = kmajor ? (row < n ? k1 - k : 0) : (k < k1 ? n - row : 0);
-      r[i] = load4<T>(p + (kmajor ? (long long)row * ld + k : (long long)k * ld + row), vec, left);
+    for (int i = 0; i < V; i++) {
+      const int m = r0 + row(i, kmajor), k = k0 + step(i, kmajor);
+      const int left = kmajor ? (m < n ? K - k : 0) : (k < K ? n - m : 0);
+      r[i] = load4<T>(p + (kmajor ? (long long)m * ld + k : (long long)k * ld + m), vec, left);
     }
   }
-  __device__ __forceinline__ void store(float (*s)[TM], bool kmajor) const {
-    const int t = threadIdx.x;
+  __device__ __forceinline__ void store(float (*s)[W], bool kmajor) const {
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
+    for (int i = 0; i < V; i++) {
+      const int k = step(i, kmajor), m = row(i, kmajor) ^ at(k);
       if (kmajor) {
-        s[4 * i][t] = r[i].x; s[4 * i + 1][t] = r[i].y; s[4 * i + 2][t] = r[i].z; s[4 * i + 3][t] = r[i].w;
+        s[k][m] = r[i].x; s[k + 1][m] = r[i].y; s[k + 2][m] = r[i].z; s[k + 3][m] = r[i].w;
       } else {
-        *reinterpret_cast<float4*>(&s[(t >> 4) + 4 * i][(t & 15) * 4]) = r[i];
+        *reinterpret_cast<float4*>(&s[k][m]) = r[i];
       }
     }
   }
 };
 
-__device__ __forceinline__ float4 cluster_load4(const float* p, int rank) {
-  uint32_t at;
-  float4 v;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(sm100::smem_u32(p)), "r"(rank));
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at) : "memory");
-  return v;
-}
-
-// The rows of blockIdx.y's tile, the columns of blockIdx.x / S's; block blockIdx.x % S of the cluster has a range of K.
-template <typename T>
-__global__ void __launch_bounds__(THREADS) gemm_simt_kernel(const GemmArgs g, int S, bool vec_a, bool vec_b) {
+template <typename T, int W, int TK>
+__global__ void __launch_bounds__(THREADS) gemm_simt_kernel(const GemmArgs g, bool vec_a, bool vec_b) {
   pdl_trigger();
-  __shared__ __align__(16) float tiles[2][2][TK][TM];       // A and B, two pieces each; afterwards the tile's partial sums
-  const int bz = blockIdx.z, rank = blockIdx.x % S;
-  const int m0 = blockIdx.y * TM, n0 = blockIdx.x / S * TN;
+  __shared__ __align__(16) float tiles[2][2][TK][W];       // A and B, two pieces each; afterwards the tile's results
+  constexpr int H = W / 32;                                // a thread's rows and columns: four of every 32
+  const int bz = blockIdx.z;
+  const int m0 = blockIdx.y * W, n0 = blockIdx.x * W;
   pdl_wait();
-  if (g.upper_only && m0 >= n0 + TN) return;                // the whole cluster
+  if (g.upper_only && m0 > n0) return;
   int bb = bz;
-  if (g.groups) {      // runs of rows are multiples of TM
+  if (g.groups) {      // runs of rows are multiples of W
     const int run = m0 / g.group_rows;
     if (run >= g.groups[0]) return;
     bb = g.groups[1 + run];
@@ -86,43 +85,50 @@ __global__ void __launch_bounds__(THREADS) gemm_simt_kernel(const GemmArgs g, in
   const T* A = reinterpret_cast<const T*>(g.A) + (long long)bz * g.strideA;
   const T* B = reinterpret_cast<const T*>(g.B) + (long long)bb * g.strideB;
   const int tid = threadIdx.x, tx = tid & 7, ty = tid >> 3;
-  const int per = ((g.K + TK - 1) / TK + S - 1) / S * TK, k_begin = rank * per, k_end = min(g.K, k_begin + per);
-  uint64_t acc[8][4] = {};       // rows 4 ty.. and 32 + 4 ty.., columns 4 tx.. and 32 + 4 tx.. in pairs
-  Piece<T> pa, pb;
+  uint64_t acc[4 * H][2 * H] = {};       // rows 4 ty.. of every 32, columns 4 tx.. of every 32 in pairs
+  Piece<T, W, TK> pa, pb;
   auto load = [&](int k) {
-    pa.load(A, g.lda, g.a_kmajor, vec_a, m0, g.M, k, k_end);
-    pb.load(B, g.ldb, g.b_kmajor, vec_b, n0, g.N, k, k_end);
+    pa.load(A, g.lda, g.a_kmajor, vec_a, m0, g.M, k, g.K);
+    pb.load(B, g.ldb, g.b_kmajor, vec_b, n0, g.N, k, g.K);
   };
-  if (k_begin < k_end) load(k_begin);
+  load(0);
   int at = 0;
-  for (int k = k_begin; k < k_end; k += TK, at ^= 1) {
+  for (int k = 0; k < g.K; k += TK, at ^= 1) {
     pa.store(tiles[at][0], g.a_kmajor);
     pb.store(tiles[at][1], g.b_kmajor);
     __syncthreads();           // the other two pieces are free: everybody has stored these after reading those
-    if (k + TK < k_end) load(k + TK);
+    if (k + TK < g.K) load(k + TK);
 #pragma unroll
-    for (int kk = 0; kk < TK; kk++) {
-      const float4 a0 = *reinterpret_cast<const float4*>(&tiles[at][0][kk][4 * ty]), a1 = *reinterpret_cast<const float4*>(&tiles[at][0][kk][32 + 4 * ty]);
-      const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(&tiles[at][1][kk][4 * tx]), b1 = *reinterpret_cast<const ulonglong2*>(&tiles[at][1][kk][32 + 4 * tx]);
-      const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+    for (int q = 0; q < TK; q += 16) {
+      if (q > 0 && k + q >= g.K) break;
 #pragma unroll
-      for (int i = 0; i < 8; i++) {
-        const uint64_t aa = sm100::pack2(a[i], a[i]);
-        acc[i][0] = sm100::fma2(aa, b0.x, acc[i][0]); acc[i][1] = sm100::fma2(aa, b0.y, acc[i][1]);
-        acc[i][2] = sm100::fma2(aa, b1.x, acc[i][2]); acc[i][3] = sm100::fma2(aa, b1.y, acc[i][3]);
+      for (int kk = q; kk < q + 16; kk++) {
+        float a[4 * H];
+        uint64_t b[2 * H];
+#pragma unroll
+        for (int h = 0; h < H; h++) {
+          const float4 v = *reinterpret_cast<const float4*>(&tiles[at][0][kk][32 * h + (4 * ty ^ Piece<T, W, TK>::at(kk))]);
+          const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(&tiles[at][1][kk][32 * h + (4 * tx ^ Piece<T, W, TK>::at(kk))]);
+          a[4 * h] = v.x; a[4 * h + 1] = v.y; a[4 * h + 2] = v.z; a[4 * h + 3] = v.w;
+          b[2 * h] = w.x; b[2 * h + 1] = w.y;
+        }
+#pragma unroll
+        for (int i = 0; i < 4 * H; i++) {
+          const uint64_t aa = sm100::pack2(a[i], a[i]);
+#pragma unroll
+          for (int j = 0; j < 2 * H; j++) acc[i][j] = sm100::fma2(aa, b[j], acc[i][j]);
+        }
       }
     }
   }
   __syncthreads();
-  float* sum = &tiles[0][0][0][0];       // [64][64]
+  float* sum = &tiles[0][0][0][0];       // [W][W]
 #pragma unroll
-  for (int i = 0; i < 8; i++) {
-    float* row = sum + ((i >> 2) * 32 + 4 * ty + (i & 3)) * TN;
-    *reinterpret_cast<ulonglong2*>(row + 4 * tx) = make_ulonglong2(acc[i][0], acc[i][1]);
-    *reinterpret_cast<ulonglong2*>(row + 32 + 4 * tx) = make_ulonglong2(acc[i][2], acc[i][3]);
-  }
-  if (S > 1) { sm100::cluster_arrive(); sm100::cluster_wait(); }
-  else __syncthreads();
+  for (int i = 0; i < 4 * H; i++)
+#pragma unroll
+    for (int h = 0; h < H; h++)
+      *reinterpret_cast<ulonglong2*>(sum + ((i >> 2) * 32 + 4 * ty + (i & 3)) * W + 32 * h + 4 * tx) = make_ulonglong2(acc[i][2 * h], acc[i][2 * h + 1]);
+  __syncthreads();
 
   T* C = reinterpret_cast<T*>(g.C) + (long long)bz * g.strideC;
   float* Cf = reinterpret_cast<float*>(g.C) + (long long)bz * g.strideC;
@@ -132,14 +138,9 @@ __global__ void __launch_bounds__(THREADS) gemm_simt_kernel(const GemmArgs g, in
     C[(long long)m * g.ldc + n] = v;
     if (both) C[(long long)n * g.ldc + m] = v;
   };
-  const int rows = TM / S;
-  for (int o = tid; o < rows * (TN / 4); o += THREADS) {
-    const int r = rank * rows + o / (TN / 4), m = m0 + r, c = o % (TN / 4) * 4;
-    float4 v4 = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int q = 0; q < S; q++) {
-      const float4 p = S > 1 ? cluster_load4(sum + r * TN + c, q) : *reinterpret_cast<const float4*>(sum + r * TN + c);
-      v4.x += p.x; v4.y += p.y; v4.z += p.z; v4.w += p.w;
-    }
+  for (int o = tid; o < W * W / 4; o += THREADS) {
+    const int r = o / (W / 4), m = m0 + r, c = o % (W / 4) * 4;
+    const float4 v4 = *reinterpret_cast<const float4*>(sum + r * W + c);
     if (m >= g.M) continue;
     const float e[4] = {v4.x, v4.y, v4.z, v4.w};
 #pragma unroll
@@ -175,7 +176,6 @@ __global__ void __launch_bounds__(THREADS) gemm_simt_kernel(const GemmArgs g, in
       }
     }
   }
-  if (S > 1) { sm100::cluster_arrive(); sm100::cluster_wait(); }      // nobody leaves while its sums are read
 }
 
 }  // namespace
@@ -187,19 +187,11 @@ template <typename T> int gemm_simt(const GemmArgs& g, cudaStream_t s) {
   const uintptr_t mask = 4 * sizeof(T) - 1;
   const bool vec_a = ((uintptr_t)g.A & mask) == 0 && ((g.lda | g.strideA) & 3) == 0;
   const bool vec_b = ((uintptr_t)g.B & mask) == 0 && ((g.ldb | g.strideB) & 3) == 0;
-  // K goes to as many blocks as bring about four to every multiprocessor, with at least 128 steps for each
-  const long long tiles = (long long)cdiv(g.N, TN) * cdiv(g.M, TM) * g.batch;
-  int S = 1;
-  while (S < 8 && tiles * S < 4ll * device_sm_count() && g.K >= 2 * S * 128) S *= 2;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(cdiv(g.N, TN) * S, cdiv(g.M, TM), g.batch); cfg.blockDim = THREADS; cfg.stream = s;
-  cudaLaunchAttribute at[2];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  at[1].id = cudaLaunchAttributeClusterDimension;
-  at[1].val.clusterDim.x = S; at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
-  cfg.attrs = at; cfg.numAttrs = S > 1 ? 2 : 1;
-  CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_simt_kernel<T>, g, S, vec_a, vec_b));
+  // Fewer than four blocks of two warps a multiprocessor leave it waiting: 32 x 32 tiles then.  The steps above take 12.5 and 1.19 ms with
+  // 64 x 64 alone, 9.04 and 0.78 with 32 x 32 alone, 8.97 and 0.78 by this rule (10.1 and 0.78 with the line at one block).
+  const long long tiles = (long long)cdiv(g.N, 64) * cdiv(g.M, 64) * g.batch / (g.upper_only ? 2 : 1);
+  auto launch = [&](auto kernel, int W) { return launch_dependent(kernel, dim3(cdiv(g.N, W), cdiv(g.M, W), g.batch), dim3(THREADS), 0, s, g, vec_a, vec_b); };
+  CUDA_TRY(tiles < 4ll * device_sm_count() ? launch(gemm_simt_kernel<T, 32, 32>, 32) : launch(gemm_simt_kernel<T, 64, 16>, 64));
   KERNEL_CHECK();
   return 0;
 }

@@ -44,9 +44,29 @@ def test_gemm_bf16_all_operand_layouts(ak, bk, shape):
 @pytest.mark.parametrize("bk", [True, False])
 @pytest.mark.parametrize("shape", [(1, 7, 5, 2), (63, 65, 17, 1), (66, 130, 127, 3), (129, 67, 1031, 1), (68, 60, 516, 2)])
 def test_gemm_simt_all_operand_layouts(ak, bk, shape):
-    """Pitches and sizes that the tensor-core kernel does not take: edges of the 64 x 64 tiles, groups of four elements that are
-    not aligned or reach past the end, K shared by the blocks of a cluster.  One bf16 rounding of the result, as above."""
+    """Pitches and sizes that the tensor-core kernel does not take: edges of the tiles, groups of four elements that are
+    not aligned or reach past the end.  One bf16 rounding of the result, as above."""
     test_gemm_bf16_all_operand_layouts(ak, bk, shape)
+
+
+@pytest.mark.parametrize("ak,bk", [(True, True), (False, True), (False, False)])
+@pytest.mark.parametrize("M,N,K,batch", [(33, 31, 17, 2), (68, 60, 516, 2), (129, 67, 1031, 1), (129, 67, 2052, 1), (602, 698, 70, 6)])
+def test_gemm_simt_sums_over_k_in_order(ak, bk, M, N, K, batch):
+    """Every result of the SIMT products is one chain of fp32 multiply-adds over k = 0, 1, ..., at every tile size (the last shape has
+    enough tiles for the large ones) and every K: products of two bf16 numbers are exact in fp32, so the chain can be followed here."""
+    g = torch.Generator(device="cuda").manual_seed(M * K)
+    A = torch.randn(batch, M, K, generator=g, device="cuda").bfloat16()
+    B = torch.randn(batch, K, N, generator=g, device="cuda").bfloat16()
+    As = A.contiguous() if ak else A.transpose(1, 2).contiguous()
+    Bs = B.transpose(1, 2).contiguous() if bk else B.contiguous()
+    C_ = torch.empty(batch, M, N, device="cuda")
+    _lib.check(_lib.lib().femto_gemm_bf16(_lib.ptr(As), int(ak), K if ak else M, _lib.ptr(Bs), int(bk), K if bk else N,
+                                          _lib.ptr(C_), N, M, N, K, batch, M * K, K * N, M * N, 1, 0, None))
+    torch.cuda.synchronize()
+    ref, a, b = torch.zeros(batch, M, N, device="cuda"), A.float(), B.float()
+    for k in range(K):
+        ref = ref + a[:, :, k, None] * b[:, k, None, :]
+    assert torch.equal(C_, ref)
 
 
 def test_gemm_split_k_fp32_accumulate_is_deterministic():
