@@ -146,6 +146,76 @@ def test_attention_of_fp32_widths(B, T, H, Hkv, hd, left, docs):
     test_attention_forward_and_reverse(_lib.F32, B, T, H, Hkv, hd, left, docs)
 
 
+def _fma(a, b, c):
+    """fp32 multiply-add: the product of two fp32 numbers is exact in fp64, whose sum is rounded once more (another result than the one
+    rounding's in 1 of 2^29)."""
+    return (a.double() * b.double() + c.double()).float()
+
+
+def _lane_sum(x, add=_fma):
+    """Sum over the last axis as a warp has it: channels lane, lane + 32, ... of x = (factor, factor) in a chain, then the lanes pairwise."""
+    a, b = (torch.nn.functional.pad(y, (0, -y.shape[-1] % 32)).unflatten(-1, (-1, 32)) for y in x)
+    s = torch.zeros_like(a[..., 0, :])
+    for e in range(a.shape[-2]):
+        s = add(a[..., e, :], b[..., e, :], s)
+    for half in (16, 8, 4, 2, 1):
+        s = s[..., :half] + s[..., half:2 * half]
+    return s[..., 0]
+
+
+@pytest.mark.parametrize("B,T,H,Hkv,hd,left,docs", [(2, 7, 2, 1, 24, 7, False), (1, 70, 2, 2, 50, 9, True), (1, 66, 2, 1, 128, 66, False), (1, 33, 3, 1, 200, 20, True)])
+def test_simt_attention_sums_key_by_key(B, T, H, Hkv, hd, left, docs):
+    """However many keys are in flight, a row of the SIMT kernels rescales and adds key by key (the reverse query by query), in
+    order and in fp32: the same bits as these recurrences, so that a training step does not depend on the kernels' grouping."""
+    Q, K, V, dO, ds = _attn_inputs(_lib.F32, B, T, H, Hkv, hd, seed=T, docs=docs)
+    Q, K, V, dO = (x.cuda() for x in (Q, K, V, dO))
+    dsd = ds.cuda() if ds is not None else None
+    O, dQ, dK, dV = (torch.empty_like(x) for x in (Q, Q, K, V))
+    l, m, lse = (torch.empty(B, H, T, device="cuda") for _ in range(3))
+    L = _lib.lib()
+    _lib.check(L.femto_attention_fwd(_lib.F32, _lib.ptr(O), _lib.ptr(l), _lib.ptr(m), _lib.ptr(lse), _lib.ptr(Q), _lib.ptr(K), _lib.ptr(V), B, T, H, Hkv,
+                                     hd, left, _lib.ptr(dsd), None))
+    _lib.check(L.femto_attention_bwd(_lib.F32, _lib.ptr(dQ), _lib.ptr(dK), _lib.ptr(dV), _lib.ptr(dO), _lib.ptr(Q), _lib.ptr(K), _lib.ptr(V), _lib.ptr(O),
+                                     _lib.ptr(lse), None, None, B, T, H, Hkv, hd, left, _lib.ptr(dsd), 0, None))
+    torch.cuda.synchronize()
+    q, k, v, do, o = (x.permute(0, 2, 1, 3).repeat_interleave(H // x.shape[2], 1) for x in (Q, K, V, dO, O))       # [B, H, T, hd]
+    t = torch.arange(T, device="cuda")
+    first = (t - left).clamp(min=0).expand(B, 1, T)
+    if ds is not None:
+        first = torch.maximum(first, dsd[:, None].long())
+    scale = torch.rsqrt(torch.tensor(float(hd), device="cuda"))
+    w = [_lane_sum((q, k[:, :, j:j + 1].expand_as(q))) for j in range(T)]                # of every query with key j
+    mr, lr, acc = torch.full_like(m, -math.inf), torch.zeros_like(l), torch.zeros_like(q)
+    dp = [_lane_sum((do, v[:, :, j:j + 1].expand_as(do))) for j in range(T)]
+    D = _lane_sum((do, o), lambda a, b, c: c + a * b)
+    dq = torch.zeros_like(q)
+    p, dsc = [], []
+    for j in range(T):
+        sees = (first <= j) & (t >= j)
+        s = w[j] * scale
+        mn = torch.maximum(mr, s)
+        a, e = torch.exp(mr - mn), torch.exp(s - mn)
+        lr = torch.where(sees, _fma(lr, a, e), lr)
+        acc = torch.where(sees[..., None], _fma(acc, a[..., None], e[..., None] * v[:, :, j:j + 1]), acc)
+        mr = torch.where(sees, mn, mr)
+        pj = torch.exp(_fma(w[j], scale, -lse))
+        p.append(torch.where(sees, pj, 0.0))
+        dsc.append(torch.where(sees, pj * (dp[j] - D) * scale, 0.0))
+        dq = _fma(dsc[j][..., None], k[:, :, j:j + 1], dq)
+    back = lambda x: x.permute(0, 2, 1, 3)
+    assert torch.equal(m, mr) and torch.equal(l, lr) and torch.equal(lse, mr + torch.log(lr))
+    assert torch.equal(O, back(acc * (1.0 / lr)[..., None]))
+    assert torch.equal(dQ, back(dq))
+    G = H // Hkv
+    dk, dv = torch.zeros(B, Hkv, T, hd, device="cuda"), torch.zeros(B, Hkv, T, hd, device="cuda")
+    P, S = torch.stack(p, -1), torch.stack(dsc, -1)                                     # [B, H, query, key]
+    for h in range(G):
+        for i in range(T):
+            dk = _fma(S[:, h::G, i, :, None], q[:, h::G, i:i + 1], dk)
+            dv = _fma(P[:, h::G, i, :, None], do[:, h::G, i:i + 1], dv)
+    assert torch.equal(dK, back(dk)) and torch.equal(dV, back(dv))
+
+
 @pytest.mark.parametrize("B,T,H,Hkv,left,docs", [
     (2, 1, 2, 1, 1, False), (3, 5, 2, 2, 5, True), (2, 127, 2, 1, 127, False), (2, 129, 4, 2, 40, True), (3, 255, 2, 2, 255, True),
     (2, 257, 6, 2, 100, False), (1, 1000, 10, 5, 300, True), (2, 1153, 2, 1, 2000, False)])
