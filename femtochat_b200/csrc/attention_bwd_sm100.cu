@@ -22,24 +22,15 @@ constexpr int TILE_BYTES = BT * HD * 2;  // two [128][64] swizzled slabs
 constexpr int BWD_SMEM = TILE_BYTES * 6 + 1024 + 256 + 2 * 3 * 128 * 4;
 constexpr float LOG2E = 1.4426950408889634f;
 
-// RAGGED below: T is not a multiple of the tile.  Tensor maps have one dimension per batch column, so that rows past a
-// column's end arrive as zeros and are clipped on the way out, and the row statistics are padded to whole tiles (a padding
-// query gets P = 0).  These lengths used to take the SIMT kernels, which keep P and dS in fp32, so here both are sums of two
-// bf16 numbers, whose low parts fill the rest of the columns of S and dP that they overwrite, and every product with them is two.
 struct BwdParams {
   AttnArgs a;
-  const float* D;   // [B][H][Tp] rowsum(dO*O)
-  const float* L2;  // [B][H][Tp] lse * log2(e)
-  const int* ds;    // [B][Tp] document starts, or null
-  int Tp;           // T in whole tiles
+  const float* D;   // [B][H][T] rowsum(dO*O)
+  const float* L2;  // [B][H][T] lse * log2(e)
 };
 
 __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&h);
-}
-__device__ __forceinline__ uint32_t rest2(float lo, float hi, uint32_t h) {   // what rounding to the pair h left over
-  return pack2(lo - __uint_as_float(h << 16), hi - __uint_as_float(h & 0xffff0000u));
 }
 // Eight results leave as one 16-byte store; with `accumulate` the eight bf16 values already there are added first
 // (Δattention!'s accumulate=true, ext/FemtoChatCUDAExt.jl:1775).
@@ -61,15 +52,13 @@ __device__ __forceinline__ void store8(bf16* dst, const uint32_t* r, float scale
 }
 
 // D[b][h][t] = sum_d dO*O and L2 = lse * log2(e): 16 lanes per (token, head) slice of 128 channels, 16-byte loads.
-template <bool RAGGED>
-__global__ void __launch_bounds__(256) attn_bwd_prep_kernel(AttnArgs a, float* D, float* L2, int* ds, int Tp) {
-  const long long total = (long long)a.B * Tp * a.H;
+__global__ void __launch_bounds__(256) attn_bwd_prep_kernel(AttnArgs a, float* D, float* L2) {
+  const long long total = (long long)a.B * a.T * a.H;
   const long long w0 = (long long)blockIdx.x * 16 + (threadIdx.x >> 4);
   const long long w = w0 < total ? w0 : total - 1;   // surplus half-warps recompute the last slice
   const int sub = threadIdx.x & 15;
   const int h = (int)(w % a.H);
-  const int b = (int)(w / a.H / Tp), t = (int)(w / a.H % Tp);
-  const long long row = (long long)b * a.T + (RAGGED ? min(t, a.T - 1) : t);
+  const long long row = w / a.H;
   const bf16* o = reinterpret_cast<const bf16*>(a.O) + row * a.o_stride + (long long)h * HD + sub * 8;
   const bf16* g = reinterpret_cast<const bf16*>(a.dO) + row * a.do_stride + (long long)h * HD + sub * 8;
   const uint4 ov = *reinterpret_cast<const uint4*>(o), gv = *reinterpret_cast<const uint4*>(g);
@@ -80,13 +69,11 @@ __global__ void __launch_bounds__(256) attn_bwd_prep_kernel(AttnArgs a, float* D
   for (int i = 0; i < 8; i++) acc += __bfloat162float(oh[i]) * __bfloat162float(gh[i]);
 #pragma unroll
   for (int off = 8; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+  const int b = (int)(row / a.T), t = (int)(row % a.T);
   if (sub == 0 && w0 < total) {
-    const long long si = ((long long)b * a.H + h) * Tp + t;
-    const bool pad = RAGGED && t >= a.T;
-    D[si] = pad ? 0.f : acc;
-    // the exponent's offset in base 2, so P = exp2(S c - L2) is one FMA + ex2
-    L2[si] = pad ? 1e30f : a.lse[((long long)b * a.H + h) * a.T + t] * LOG2E;
-    if (RAGGED && h == 0 && ds) ds[(long long)b * Tp + t] = a.doc_start[row];
+    const long long si = ((long long)b * a.H + h) * a.T + t;
+    D[si] = acc;
+    L2[si] = a.lse[si] * LOG2E;   // the exponent's offset in base 2, so P = exp2(S c - L2) is one FMA + ex2
   }
 }
 
@@ -120,7 +107,6 @@ __device__ __forceinline__ void stage_rows(uint8_t* stage, const uint32_t (&r0)[
 // ------------------------------------------------------------------------------------------------
 constexpr int DQ_SMEM = TILE_BYTES * 7 + 1024 + 256;
 
-template <bool RAGGED>
 __global__ void __launch_bounds__(384, 1)
 attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                    const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
@@ -153,11 +139,11 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   const int jhi = min(q0 + BT - 1, a.T - 1) / BT;
   int jlo = max(0, q0 - a.window_left) / BT;
   const long long row0 = (long long)b * a.T;
-  if (p.ds) {
+  if (a.doc_start) {
     // key tiles that lie before the earliest document start of these 128 queries are fully masked
     __shared__ int s_ds_min[4];
     if (threadIdx.x < 128) {
-      const int v = __reduce_min_sync(0xffffffffu, p.ds[(long long)b * p.Tp + q0 + threadIdx.x]);
+      const int v = __reduce_min_sync(0xffffffffu, a.doc_start[row0 + q0 + threadIdx.x]);
       if ((threadIdx.x & 31) == 0) s_ds_min[threadIdx.x >> 5] = v;
     }
     __syncthreads();
@@ -187,22 +173,22 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   if (warp == 0) {
     if (lane == 0) {
       mbar_expect_tx(qdo_full, 2 * TILE_BYTES);
-      tma_load_3d(sQ, &tmQ, qdo_full, h * HD, q0, b);
-      tma_load_3d(sQ + TILE_BYTES / 2, &tmQ, qdo_full, h * HD + 64, q0, b);
-      tma_load_3d(sdO, &tmdO, qdo_full, h * HD, q0, b);
-      tma_load_3d(sdO + TILE_BYTES / 2, &tmdO, qdo_full, h * HD + 64, q0, b);
+      tma_load_2d(sQ, &tmQ, qdo_full, h * HD, (int)(row0 + q0));
+      tma_load_2d(sQ + TILE_BYTES / 2, &tmQ, qdo_full, h * HD + 64, (int)(row0 + q0));
+      tma_load_2d(sdO, &tmdO, qdo_full, h * HD, (int)(row0 + q0));
+      tma_load_2d(sdO + TILE_BYTES / 2, &tmdO, qdo_full, h * HD + 64, (int)(row0 + q0));
       for (int i = 0; i < ntile; i++) {
         const int ks = i % 3, vs = i & 1;
-        const int krow = (jlo + i) * BT;
+        const int krow = (int)(row0 + (jlo + i) * BT);
         if (i >= 3 && !mbar_wait(&k_free[ks], ((i - 3) / 3) & 1, abort_flag, a.status)) break;
         mbar_expect_tx(&k_full[ks], TILE_BYTES);
-        tma_load_3d(sK + ks * TILE_BYTES, &tmK, &k_full[ks], kvh * HD, krow, b);
-        tma_load_3d(sK + ks * TILE_BYTES + TILE_BYTES / 2, &tmK, &k_full[ks], kvh * HD + 64, krow, b);
+        tma_load_2d(sK + ks * TILE_BYTES, &tmK, &k_full[ks], kvh * HD, krow);
+        tma_load_2d(sK + ks * TILE_BYTES + TILE_BYTES / 2, &tmK, &k_full[ks], kvh * HD + 64, krow);
         // the V stage of tile i-2 is free once its dP has been executed
         if (i >= 2 && !mbar_wait(&dp_full[vs], ((i - 2) >> 1) & 1, abort_flag, a.status)) break;
         mbar_expect_tx(&v_full[vs], TILE_BYTES);
-        tma_load_3d(sV + vs * TILE_BYTES, &tmV, &v_full[vs], kvh * HD, krow, b);
-        tma_load_3d(sV + vs * TILE_BYTES + TILE_BYTES / 2, &tmV, &v_full[vs], kvh * HD + 64, krow, b);
+        tma_load_2d(sV + vs * TILE_BYTES, &tmV, &v_full[vs], kvh * HD, krow);
+        tma_load_2d(sV + vs * TILE_BYTES + TILE_BYTES / 2, &tmV, &v_full[vs], kvh * HD + 64, krow);
       }
     }
   } else if (warp == 1) {
@@ -259,11 +245,6 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 #pragma unroll
         for (int k = 0; k < BT / 16; k++)  // 16 keys = 8 TMEM columns / 2048 B of K rows; dS of keys 64.. starts at column 64
           mma_ts(tdQ, tS[st] + (k >> 2) * 64 + (k & 3) * 8, smem_desc_sw128(k_addr + k * 2048, TILE_BYTES / 2, 1024), idesc_mn, (i > 0 || k > 0) ? 1u : 0u);
-        if constexpr (RAGGED) {   // the low parts, 32 columns further
-#pragma unroll
-          for (int k = 0; k < BT / 16; k++)
-            mma_ts(tdQ, tS[st] + 32 + (k >> 2) * 64 + (k & 3) * 8, smem_desc_sw128(k_addr + k * 2048, TILE_BYTES / 2, 1024), idesc_mn, 1u);
-        }
         tc_commit(&dq_done[st]);
         tc_commit(&k_free[ks]);
       }
@@ -277,8 +258,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     const float scale = rsqrtf((float)HD);
     const float c = scale * LOG2E;
     int lo = max(0, q - a.window_left);
-    if (p.ds) lo = max(lo, p.ds[(long long)b * p.Tp + q]);
-    const long long si = ((long long)b * a.H + h) * p.Tp + q;
+    if (a.doc_start) lo = max(lo, a.doc_start[row0 + q]);
+    const long long si = ((long long)b * a.H + h) * a.T + q;
     const float lse2 = p.L2[si];
     const float Dq = p.D[si];
     bool ok = true;
@@ -297,7 +278,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       uint32_t dr[2][32];
       tmem_ld32(tdP + lane_off + (2 * halfsel) * 32, dr[0]);
       tmem_ld32(tdP + lane_off + (2 * halfsel + 1) * 32, dr[1]);
-      uint32_t pk[2][16], pl[2][16];
+      uint32_t pk[2][16];
 #pragma unroll
       for (int u = 0; u < 2; u++) {
         const int cc = 2 * halfsel + u;
@@ -321,23 +302,17 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
               d2[e] = pv * (__uint_as_float(dr[u][j + e]) - Dq);
             }
             pk[u][j >> 1] = pack2(d2[0], d2[1]);
-            if constexpr (RAGGED) pl[u][j >> 1] = rest2(d2[0], d2[1], pk[u][j >> 1]);
           }
         } else {   // no mask edge crosses this warp's rows in this tile: the common case, without the compares
 #pragma unroll
           for (int j = 0; j < 32; j += 2) {
             const float p0 = fast_exp2(__uint_as_float(sr[j]) * c - lse2), p1 = fast_exp2(__uint_as_float(sr[j + 1]) * c - lse2);
-            const float d0 = p0 * (__uint_as_float(dr[u][j]) - Dq), d1 = p1 * (__uint_as_float(dr[u][j + 1]) - Dq);
-            pk[u][j >> 1] = pack2(d0, d1);
-            if constexpr (RAGGED) pl[u][j >> 1] = rest2(d0, d1, pk[u][j >> 1]);
+            pk[u][j >> 1] = pack2(p0 * (__uint_as_float(dr[u][j]) - Dq), p1 * (__uint_as_float(dr[u][j + 1]) - Dq));
           }
         }
       }
 #pragma unroll
-      for (int u = 0; u < 2; u++) {
-        tmem_st16(tS[st] + lane_off + halfsel * 64 + u * 16, pk[u]);
-        if constexpr (RAGGED) tmem_st16(tS[st] + lane_off + halfsel * 64 + 32 + u * 16, pl[u]);
-      }
+      for (int u = 0; u < 2; u++) tmem_st16(tS[st] + lane_off + halfsel * 64 + u * 16, pk[u]);
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
@@ -356,8 +331,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         stage_rows(stage, r0, r1, scale, lane);
         fence_proxy_async();
         __syncwarp();
-        if (lane == 0 && (!RAGGED || q0 + quad * 32 < a.T)) {
-          tma_store_3d(&tmdQ, stage, h * HD + halfsel * 64, q0 + quad * 32, b);
+        if (lane == 0) {
+          tma_store_3d(&tmdQ, stage, h * HD + halfsel * 64, (int)(row0 + q0 + quad * 32), 0);
           bulk_commit();
           bulk_wait_read<0>();   // shared memory is released when the CTA leaves
         }
@@ -369,8 +344,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           tmem_ld32(tdQ + lane_off + cc * 32, rr);
           tmem_ld_wait();
 #pragma unroll
-          for (int j = 0; j < 32; j += 8)
-            if (!RAGGED || q < a.T) store8(dq + cc * 32 + j, rr + j, scale, true);
+          for (int j = 0; j < 32; j += 8) store8(dq + cc * 32 + j, rr + j, scale, true);
         }
       }
     }
@@ -388,7 +362,6 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 // issues dV += P^T dO and dK += dS^T Q (one issuer per product: tcgen05.mma issue blocks while the
 // pipe is busy, so the barrier waits of one issuer overlap the issue of another).
 // ------------------------------------------------------------------------------------------------
-template <bool RAGGED>
 __global__ void __launch_bounds__(384, 1)
 attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                     const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
@@ -418,7 +391,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   const int g = a.H / a.Hkv;
   const int k0 = kt * BT;
   const int ilo = kt;
-  const int ihi = (int)min((long long)p.Tp / BT - 1, ((long long)k0 + BT - 1 + a.window_left) / BT);
+  const int ihi = (int)min((long long)a.T / BT - 1, ((long long)k0 + BT - 1 + a.window_left) / BT);
   const long long row0 = (long long)b * a.T;
   // query tiles whose earliest document start lies after this key tile are fully masked: keep a
   // compact list of the visible ones (document starts need not be monotone for arbitrary positions)
@@ -428,10 +401,10 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   __shared__ int s_nq;
   {
     const int cand = ihi - ilo + 1;
-    if (p.ds) {
+    if (a.doc_start) {
       for (int c = threadIdx.x >> 5; c < cand; c += 12) {
         const int base = (ilo + c) * BT + (threadIdx.x & 31) * 4;
-        const int4 v = *reinterpret_cast<const int4*>(p.ds + (long long)b * p.Tp + base);
+        const int4 v = *reinterpret_cast<const int4*>(a.doc_start + row0 + base);
         const int m = __reduce_min_sync(0xffffffffu, min(min(v.x, v.y), min(v.z, v.w)));
         int mx = max(max(v.x, v.y), max(v.z, v.w));   // 8 lanes hold 32 consecutive queries
         mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
@@ -445,7 +418,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     if (threadIdx.x == 0) {
       int n = 0;
       for (int c = 0; c < cand; c++)
-        if (!p.ds || s_tmin[c] <= k0 + BT - 1) s_qlist[n++] = ilo + c;
+        if (!a.doc_start || s_tmin[c] <= k0 + BT - 1) s_qlist[n++] = ilo + c;
       s_nq = n;
     }
     __syncthreads();
@@ -475,24 +448,24 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   if (warp == 0) {
     if (lane == 0) {
       mbar_expect_tx(kv_full, 2 * TILE_BYTES);
-      tma_load_3d(sK, &tmK, kv_full, kvh * HD, k0, b);
-      tma_load_3d(sK + TILE_BYTES / 2, &tmK, kv_full, kvh * HD + 64, k0, b);
-      tma_load_3d(sV, &tmV, kv_full, kvh * HD, k0, b);
-      tma_load_3d(sV + TILE_BYTES / 2, &tmV, kv_full, kvh * HD + 64, k0, b);
+      tma_load_2d(sK, &tmK, kv_full, kvh * HD, (int)(row0 + k0));
+      tma_load_2d(sK + TILE_BYTES / 2, &tmK, kv_full, kvh * HD + 64, (int)(row0 + k0));
+      tma_load_2d(sV, &tmV, kv_full, kvh * HD, (int)(row0 + k0));
+      tma_load_2d(sV + TILE_BYTES / 2, &tmV, kv_full, kvh * HD + 64, (int)(row0 + k0));
       for (int it = 0; it < nit; it++) {
         const int st = it & 1;
         const int h = kvh * g + it / nq;
-        const int qrow = s_qlist[it % nq] * BT;
+        const int qrow = (int)(row0 + s_qlist[it % nq] * BT);
         if (!mbar_wait(&qdo_empty[st], ((it >> 1) & 1) ^ 1, abort_flag, a.status)) break;
-        mbar_expect_tx(&qdo_full[st], 2 * TILE_BYTES + 1024 + (p.ds ? 512 : 0));
-        const long long srow = ((long long)b * a.H + h) * p.Tp + qrow;
+        mbar_expect_tx(&qdo_full[st], 2 * TILE_BYTES + 1024 + (a.doc_start ? 512 : 0));
+        const long long srow = ((long long)b * a.H + h) * a.T + s_qlist[it % nq] * BT;
         bulk_load_1d(stats + st * 384, p.L2 + srow, 512, &qdo_full[st]);
         bulk_load_1d(stats + st * 384 + 128, p.D + srow, 512, &qdo_full[st]);
-        if (p.ds) bulk_load_1d(stats + st * 384 + 256, p.ds + (long long)b * p.Tp + qrow, 512, &qdo_full[st]);
-        tma_load_3d(sQ + st * TILE_BYTES, &tmQ, &qdo_full[st], h * HD, qrow, b);
-        tma_load_3d(sQ + st * TILE_BYTES + TILE_BYTES / 2, &tmQ, &qdo_full[st], h * HD + 64, qrow, b);
-        tma_load_3d(sdO + st * TILE_BYTES, &tmdO, &qdo_full[st], h * HD, qrow, b);
-        tma_load_3d(sdO + st * TILE_BYTES + TILE_BYTES / 2, &tmdO, &qdo_full[st], h * HD + 64, qrow, b);
+        if (a.doc_start) bulk_load_1d(stats + st * 384 + 256, a.doc_start + qrow, 512, &qdo_full[st]);
+        tma_load_2d(sQ + st * TILE_BYTES, &tmQ, &qdo_full[st], h * HD, qrow);
+        tma_load_2d(sQ + st * TILE_BYTES + TILE_BYTES / 2, &tmQ, &qdo_full[st], h * HD + 64, qrow);
+        tma_load_2d(sdO + st * TILE_BYTES, &tmdO, &qdo_full[st], h * HD, qrow);
+        tma_load_2d(sdO + st * TILE_BYTES + TILE_BYTES / 2, &tmdO, &qdo_full[st], h * HD + 64, qrow);
       }
     }
   } else if (warp == 1 || warp == 3) {
@@ -533,13 +506,6 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 #pragma unroll
         for (int k = 0; k < 4; k++)
           mma_ts(tdK, tdP[bf] + (k >> 1) * 32 + (k & 1) * 8, smem_desc_sw128(q_addr + k * 2048, TILE_BYTES / 2, 1024), idesc_out, (h2 > 0 || k > 0) ? 1u : 0u);
-        if constexpr (RAGGED) {   // the low parts, 16 columns further
-#pragma unroll
-          for (int k = 0; k < 4; k++) {
-            mma_ts(tdV, tS[bf] + 16 + (k >> 1) * 32 + (k & 1) * 8, smem_desc_sw128(do_addr + k * 2048, TILE_BYTES / 2, 1024), idesc_out, 1u);
-            mma_ts(tdK, tdP[bf] + 16 + (k >> 1) * 32 + (k & 1) * 8, smem_desc_sw128(q_addr + k * 2048, TILE_BYTES / 2, 1024), idesc_out, 1u);
-          }
-        }
         tc_commit(&out_done[bf]);
         if (hf == 1) tc_commit(&qdo_empty[st]);
       }
@@ -564,7 +530,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       if (ok && !mbar_wait(&dp_full[bf], (h2 >> 1) & 1, abort_flag, a.status)) ok = false;
       if (!ok) continue;
       tc_fence_after();
-      uint32_t pp[16], pd[16], pp2[16], pd2[16];   // (pp2, pd2: the low parts)
+      uint32_t pp[16], pd[16];
       {
         const int cq = hf * 64 + halfsel * 32;   // first query (within the tile) of this thread's chunk
         const int qf = qi0 + halfsel * 32;       // its position in the sequence
@@ -573,7 +539,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         tmem_ld32(tdP[bf] + lane_off + halfsel * 32, dr);
         // the mask matters only when some key of this warp is above the chunk's first query (causal edge)
         // or below the largest lower bound of its 32 queries (window / document edge)
-        const int lo_max = max(max(0, qf + 31 - a.window_left), p.ds ? s_dsmax[qtile - ilo][cq >> 5] : 0);
+        const int lo_max = max(max(0, qf + 31 - a.window_left), a.doc_start ? s_dsmax[qtile - ilo][cq >> 5] : 0);
         const bool need_mask = __any_sync(0xffffffffu, key > qf || key < lo_max);
         tmem_ld_wait();
         if (need_mask) {
@@ -583,7 +549,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             const float4 d4 = *reinterpret_cast<const float4*>(sl + 128 + cq + j);
             const float ls[4] = {l4.x, l4.y, l4.z, l4.w}, dd[4] = {d4.x, d4.y, d4.z, d4.w};
             int los[4] = {0, 0, 0, 0};
-            if (p.ds) {
+            if (a.doc_start) {
               const int4 lo4 = *reinterpret_cast<const int4*>(sl + 256 + cq + j);
               los[0] = lo4.x; los[1] = lo4.y; los[2] = lo4.z; los[3] = lo4.w;
             }
@@ -598,13 +564,6 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             }
             pp[j >> 1] = pack2(p4[0], p4[1]); pp[(j >> 1) + 1] = pack2(p4[2], p4[3]);
             pd[j >> 1] = pack2(s4[0], s4[1]); pd[(j >> 1) + 1] = pack2(s4[2], s4[3]);
-            if constexpr (RAGGED) {
-#pragma unroll
-              for (int e = 0; e < 2; e++) {
-                pp2[(j >> 1) + e] = rest2(p4[2 * e], p4[2 * e + 1], pp[(j >> 1) + e]);
-                pd2[(j >> 1) + e] = rest2(s4[2 * e], s4[2 * e + 1], pd[(j >> 1) + e]);
-              }
-            }
           }
         } else {
 #pragma unroll
@@ -620,20 +579,12 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             }
             pp[j >> 1] = pack2(p4[0], p4[1]); pp[(j >> 1) + 1] = pack2(p4[2], p4[3]);
             pd[j >> 1] = pack2(s4[0], s4[1]); pd[(j >> 1) + 1] = pack2(s4[2], s4[3]);
-            if constexpr (RAGGED) {
-#pragma unroll
-              for (int e = 0; e < 2; e++) {
-                pp2[(j >> 1) + e] = rest2(p4[2 * e], p4[2 * e + 1], pp[(j >> 1) + e]);
-                pd2[(j >> 1) + e] = rest2(s4[2 * e], s4[2 * e + 1], pd[(j >> 1) + e]);
-              }
-            }
           }
         }
       }
       // P^T / dS^T of this thread's 32 queries go over the start of its own 32 columns of S^T / dP^T
       tmem_st16(tS[bf] + lane_off + halfsel * 32, pp);
       tmem_st16(tdP[bf] + lane_off + halfsel * 32, pd);
-      if constexpr (RAGGED) { tmem_st16(tS[bf] + lane_off + halfsel * 32 + 16, pp2); tmem_st16(tdP[bf] + lane_off + halfsel * 32 + 16, pd2); }
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
@@ -644,7 +595,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       tc_fence_after();
       if (!a.accumulate) {
         // every product has been executed: the two Q stages are free and stage dK and dV for TMA stores
-        const int out_row = key - lane;   // first of this warp's 32 key rows
+        const int out_row = (int)(row0 + key) - lane;   // first of this warp's 32 key rows
 #pragma unroll
         for (int which = 0; which < 2; which++) {
           uint32_t r0[32], r1[32];
@@ -656,8 +607,8 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           stage_rows(stage, r0, r1, which ? 1.f : scale, lane);
           fence_proxy_async();
           __syncwarp();
-          if (lane == 0 && (!RAGGED || out_row < a.T)) {
-            tma_store_3d(which ? &tmdV : &tmdK, stage, kvh * HD + halfsel * 64, out_row, b);
+          if (lane == 0) {
+            tma_store_3d(which ? &tmdV : &tmdK, stage, kvh * HD + halfsel * 64, out_row, 0);
             bulk_commit();
           }
         }
@@ -673,7 +624,6 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           tmem_ld_wait();
 #pragma unroll
           for (int j = 0; j < 32; j += 8) {
-            if (RAGGED && key >= a.T) continue;
             store8(dk + cc * 32 + j, rk + j, scale, true);
             store8(dv + cc * 32 + j, rv + j, 1.f, true);
           }
@@ -688,60 +638,44 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 
 }  // namespace
 
-// D and L2 of whole tiles, and for a ragged T the padded document starts.
-size_t attention_bwd_tc_ws_bytes(int B, int T, int H, int) {
-  const size_t Tp = (size_t)(T + BT - 1) / BT * BT;
-  return 2 * sizeof(float) * B * H * Tp + (T % BT ? sizeof(int) * B * Tp : 0);
-}
+size_t attention_bwd_tc_ws_bytes(int B, int T, int H, int) { return 2 * sizeof(float) * (size_t)B * H * T; }
 
-static bool bwd_aligned(const AttnArgs& a) {
-  return !((a.do_stride & 7) || (a.dq_stride & 7) || (a.dkv_stride & 7)) && aligned16(a.dO) && aligned16(a.dQ) && aligned16(a.dK) && aligned16(a.dV);
-}
-// Lengths that are no multiple of the tile take the tensor cores where these can: a caller with unaligned gradients, or with the
-// fixed scratch of 2 B H T floats and no room for the padding, keeps the SIMT kernels.
-bool attention_bwd_tc_supported(const AttnArgs& a) {
-  if (!attention_tc_supported(a)) return false;
-  return a.T % BT == 0 || (bwd_aligned(a) && a.ws && a.ws_bytes >= attention_bwd_tc_ws_bytes(a.B, a.T, a.H, a.hd));
-}
-
-template <bool RAGGED> static int bwd_launch(const AttnArgs& a, cudaStream_t s) {
+int attention_bwd_tc(const AttnArgs& a, cudaStream_t s) {
+  if (!attention_tc_supported(a) || !attention_whole_tiles(a)) return femto_fail(FEMTO_ERR_UNSUPPORTED, "attention_bwd_tc: unsupported shape");
+  if ((a.do_stride & 7) || (a.dq_stride & 7) || (a.dkv_stride & 7) || !aligned16(a.dO) || !aligned16(a.dQ) ||
+      !aligned16(a.dK) || !aligned16(a.dV))
+    return femto_fail(FEMTO_ERR_ALIGN, "attention_bwd_tc: gradient buffers must be 16-byte aligned");
+  const size_t need = attention_bwd_tc_ws_bytes(a.B, a.T, a.H, a.hd);
+  if (!a.ws || a.ws_bytes < need) return femto_fail(FEMTO_ERR_ARG, "attention_bwd_tc: workspace too small");
+  const long long N = (long long)a.B * a.T;
   BwdParams p;
   p.a = a;
-  p.Tp = (a.T + BT - 1) / BT * BT;
-  float *D = reinterpret_cast<float*>(a.ws), *L2 = D + (size_t)a.B * a.H * p.Tp;
-  int* ds = RAGGED && a.doc_start ? reinterpret_cast<int*>(L2 + (size_t)a.B * a.H * p.Tp) : nullptr;
-  p.D = D; p.L2 = L2; p.ds = RAGGED ? ds : a.doc_start;
-  attn_bwd_prep_kernel<RAGGED><<<cdiv((long long)a.B * p.Tp * a.H, 16), 256, 0, s>>>(a, D, L2, ds, p.Tp);
+  p.D = reinterpret_cast<const float*>(a.ws);
+  p.L2 = p.D + (size_t)a.B * a.H * a.T;
+  attn_bwd_prep_kernel<<<cdiv(N * a.H, 16), 256, 0, s>>>(a, reinterpret_cast<float*>(a.ws), reinterpret_cast<float*>(a.ws) + (size_t)a.B * a.H * a.T);
   KERNEL_CHECK();
-  // (columns, rows of one batch column, batch); results: 64-column x 32-row swizzled boxes, one per row-owning warp
-  CUtensorMap tmQ, tmK, tmV, tmdO, tmdQ, tmdK, tmdV;
-  const auto map = [&](CUtensorMap* m, const void* x, int heads, long long ld, int rows) {
-    return make_tmap_3d_bf16_sw(m, x, (uint64_t)heads * HD, a.T, a.B, ld, (uint64_t)a.T * ld, 64, rows, 3);
-  };
-  FEMTO_TRY(map(&tmQ, a.Q, a.H, a.q_stride, BT));
-  FEMTO_TRY(map(&tmK, a.K, a.Hkv, a.kv_stride, BT));
-  FEMTO_TRY(map(&tmV, a.V, a.Hkv, a.kv_stride, BT));
-  FEMTO_TRY(map(&tmdO, a.dO, a.H, a.do_stride, BT));
-  FEMTO_TRY(map(&tmdQ, a.dQ, a.H, a.dq_stride, 32));
-  FEMTO_TRY(map(&tmdK, a.dK, a.Hkv, a.dkv_stride, 32));
-  FEMTO_TRY(map(&tmdV, a.dV, a.Hkv, a.dkv_stride, 32));
+  CUtensorMap tmQ, tmK, tmV, tmdO;
+  FEMTO_TRY(make_tmap_2d_bf16(&tmQ, a.Q, (uint64_t)a.H * HD, N, a.q_stride, 64, BT));
+  FEMTO_TRY(make_tmap_2d_bf16(&tmK, a.K, (uint64_t)a.Hkv * HD, N, a.kv_stride, 64, BT));
+  FEMTO_TRY(make_tmap_2d_bf16(&tmV, a.V, (uint64_t)a.Hkv * HD, N, a.kv_stride, 64, BT));
+  FEMTO_TRY(make_tmap_2d_bf16(&tmdO, a.dO, (uint64_t)a.H * HD, N, a.do_stride, 64, BT));
   static PerDevice attr;
   const int dev = PerDevice::current();
   if (dev < 0 || !attr.done[dev]) {
-    CUDA_TRY(cudaFuncSetAttribute(attn_bwd_dq_kernel<RAGGED>, cudaFuncAttributeMaxDynamicSharedMemorySize, DQ_SMEM));
-    CUDA_TRY(cudaFuncSetAttribute(attn_bwd_dkv_kernel<RAGGED>, cudaFuncAttributeMaxDynamicSharedMemorySize, BWD_SMEM));
+    CUDA_TRY(cudaFuncSetAttribute(attn_bwd_dq_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DQ_SMEM));
+    CUDA_TRY(cudaFuncSetAttribute(attn_bwd_dkv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BWD_SMEM));
     if (dev >= 0) attr.done[dev] = true;
   }
-  attn_bwd_dq_kernel<RAGGED><<<dim3(p.Tp / BT, a.H, a.B), 384, DQ_SMEM, s>>>(tmQ, tmK, tmV, tmdO, tmdQ, p);
+  dim3 gq(a.T / BT, a.H, a.B);
+  // result maps: 64-column x 32-row swizzled boxes, one per row-owning warp
+  CUtensorMap tmdQ, tmdK, tmdV;
+  FEMTO_TRY(make_tmap_3d_bf16_sw(&tmdQ, a.dQ, (uint64_t)a.H * HD, N, 1, a.dq_stride, 0, 64, 32, 3));
+  FEMTO_TRY(make_tmap_3d_bf16_sw(&tmdK, a.dK, (uint64_t)a.Hkv * HD, N, 1, a.dkv_stride, 0, 64, 32, 3));
+  FEMTO_TRY(make_tmap_3d_bf16_sw(&tmdV, a.dV, (uint64_t)a.Hkv * HD, N, 1, a.dkv_stride, 0, 64, 32, 3));
+  attn_bwd_dq_kernel<<<gq, 384, DQ_SMEM, s>>>(tmQ, tmK, tmV, tmdO, tmdQ, p);
   KERNEL_CHECK();
-  attn_bwd_dkv_kernel<RAGGED><<<dim3(p.Tp / BT, a.Hkv, a.B), 384, BWD_SMEM, s>>>(tmQ, tmK, tmV, tmdO, tmdK, tmdV, p);
+  dim3 gk(a.T / BT, a.Hkv, a.B);
+  attn_bwd_dkv_kernel<<<gk, 384, BWD_SMEM, s>>>(tmQ, tmK, tmV, tmdO, tmdK, tmdV, p);
   KERNEL_CHECK();
   return 0;
-}
-
-int attention_bwd_tc(const AttnArgs& a, cudaStream_t s) {
-  if (!attention_tc_supported(a)) return femto_fail(FEMTO_ERR_UNSUPPORTED, "attention_bwd_tc: unsupported shape");
-  if (!bwd_aligned(a)) return femto_fail(FEMTO_ERR_ALIGN, "attention_bwd_tc: gradient buffers must be 16-byte aligned");
-  if (!a.ws || a.ws_bytes < attention_bwd_tc_ws_bytes(a.B, a.T, a.H, a.hd)) return femto_fail(FEMTO_ERR_ARG, "attention_bwd_tc: workspace too small");
-  return a.T % BT ? bwd_launch<true>(a, s) : bwd_launch<false>(a, s);
 }

@@ -1142,6 +1142,8 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 
 }  // namespace
 
+bool attention_whole_tiles(const AttnArgs& a) { return a.T % BQ == 0; }
+
 bool attention_tc_supported(const AttnArgs& a) {
   if (a.hd != HD) return false;
   if (a.T > 8192) return false;  // the dK/dV kernel lists at most 64 query tiles

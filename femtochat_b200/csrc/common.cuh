@@ -212,13 +212,14 @@ struct AttnArgs {
   bool accumulate = false;         // reverse pass: add to dQ / dK / dV instead of overwriting them
   int B = 0, T = 0, H = 0, Hkv = 0, hd = 0, window_left = 0;
   const int* doc_start = nullptr;  // [B][T] or null
+  bool reverse_follows = false;    // forward pass of a training step
   void* ws = nullptr; size_t ws_bytes = 0;
   unsigned int* status = nullptr;
 };
 template <typename T> int attention_fwd_simt(const AttnArgs& a, cudaStream_t s);
 template <typename T> int attention_bwd_simt(const AttnArgs& a, cudaStream_t s);
 bool attention_tc_supported(const AttnArgs& a);
-bool attention_bwd_tc_supported(const AttnArgs& a);
+bool attention_whole_tiles(const AttnArgs& a);
 int attention_fwd_tc(const AttnArgs& a, cudaStream_t s);
 int attention_bwd_tc(const AttnArgs& a, cudaStream_t s);
 size_t attention_bwd_tc_ws_bytes(int B, int T, int H, int hd);

@@ -329,9 +329,9 @@ static int step_t(femto_handle* h, const float* theta, float* delta, const int* 
   const float eps = h->eps;
   const bool mean = reduction == FEMTO_REDUCTION_MEAN;
   // with a side stream the GEMMs give up one ring stage (32 KB), so that streaming kernels of the other stream fit beside them
-  auto GA = [&]() { GemmArgs g; g.ws = h->gemm_ws; g.ws_bytes = h->gemm_ws_bytes; g.status = h->status; g.ring = (backward && side) ? 5 : 0; g.any_size = true; return g; };
+  auto GA = [&]() { GemmArgs g; g.ws = h->gemm_ws; g.ws_bytes = h->gemm_ws_bytes; g.status = h->status; g.ring = (backward && side) ? 5 : 0; g.any_size = !backward; return g; };
   // (any_size: fewer rows than a tile still are faster on the tensor cores than in the SIMT kernel, whose blocks walk K alone:
-  // 24 rows of d12 175 us a product, 17.4 us so)
+  // 24 rows of d12 175 us a product, 17.4 us so.  A training step keeps the SIMT kernel's order of summation there, see attention_simt.cu)
   // Y[N][out] = X[N][in] * W[in][out]
   auto lin_fwd = [&](const void* X, int in, const void* W, int out, void* Y, int ldy, int epi, const void* aux) {
     GemmArgs g = GA();
@@ -427,6 +427,7 @@ static int step_t(femto_handle* h, const float* theta, float* delta, const int* 
     a.Q = l.qkv; a.K = (const T*)l.qkv + d; a.V = (const T*)l.qkv + d + kv; a.q_stride = dq; a.kv_stride = dq;
     a.O = l.att; a.o_stride = d; a.lse = l.lse; a.B = B; a.T = Tl; a.H = H; a.Hkv = Hkv; a.hd = hd;
     a.window_left = p.window; a.doc_start = docs; a.ws = h->attn_ws; a.ws_bytes = h->attn_ws_bytes; a.status = h->status;
+    a.reverse_follows = backward;
     FEMTO_TRY(attention_fwd<T>(a, s));
     FEMTO_TRY(lin_fwd(l.att, d, l.sh_wo, d, h->xm, d, EPI_RESID, h->xm));
     FEMTO_TRY(S::norm((const T*)h->xm, (T*)l.xn2, l.r2, N, d, eps, s));

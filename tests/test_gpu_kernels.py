@@ -220,9 +220,9 @@ def test_simt_attention_sums_key_by_key(B, T, H, Hkv, hd, left, docs):
     (2, 1, 2, 1, 1, False), (3, 5, 2, 2, 5, True), (2, 127, 2, 1, 127, False), (2, 129, 4, 2, 40, True), (3, 255, 2, 2, 255, True),
     (2, 257, 6, 2, 100, False), (1, 1000, 10, 5, 300, True), (2, 1153, 2, 1, 2000, False)])
 def test_attention_of_ragged_lengths(B, T, H, Hkv, left, docs):
-    """Lengths that are no multiple of the 128-row tiles, several columns, on the tensor cores with P and dS in two bf16 parts: O is off
-    by its own rounding (2^-9 of it) and 2^-14 of the largest, the gradients by their rounding and that of the O they are computed from
-    (2^-9 each, rms below 4e-3); nothing past a column's end is read or written; accumulate adds."""
+    """Lengths that are no multiple of the 128-row tiles, several columns: the forward pass on the tensor cores with P in bf16 parts, the
+    reverse on the SIMT kernels.  O is off by its own rounding (2^-9 of it) and 2^-14 of the largest, the gradients by their rounding and
+    that of the O they are computed from (2^-9 each, rms below 4e-3); nothing past a column's end is read or written; accumulate adds."""
     Q, K, V, dO, ds = _attn_inputs(_lib.BF16, B, T, H, Hkv, 128, seed=T, docs=docs)
     Qd, Kd, Vd, dOd = (x.double() for x in (Q, K, V, dO))
     docs64 = ds.long() if ds is not None else None

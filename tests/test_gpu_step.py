@@ -1,4 +1,5 @@
 """GPU parity of the whole training step through the C ABI against the CPU oracle."""
+import hashlib
 import os
 
 import pytest
@@ -53,6 +54,32 @@ def run_both(cfgkw, B, dtype, short_window=0, doc_mask=False, reduction="sum", n
     assert st.status_word() == 0
     bitwise = torch.equal(g1, params.delta.cpu()) and l1 == l2
     return dict(l0=l0, l1=l1, g0=g0, g1=g1, lay=lay, st=st, params=params, bitwise=bitwise, inputs=(tok, tgt, pos))
+
+
+# SHA-256 (first 16 digits) of gradients and updated weights after two training steps, as sm_100a gives them with CUDA 12.9.
+STEP_BITS = {("float32", 3, 200): "2942202fdc1bae19", ("float32", 1, 5): "d967639a2c7aacfa", ("bfloat16", 1, 70): "c0a599044a8a3e29",
+             ("bfloat16", 3, 200): "a3587ac52d657278", ("bfloat16", 5, 27): "d81ff435c82e116b", ("bfloat16", 2, 128): "632affd8eb710a6d"}
+
+
+@pytest.mark.parametrize("dtype,B,T", STEP_BITS)
+def test_training_step_keeps_its_bits(dtype, B, T):
+    """A training step's results do not depend on which kernel runs it: fp32, and bf16 at lengths and row counts that do not
+    fill the tensor cores' tiles, keep the order of summation (and bf16 there P and dS in fp32).  A step from
+    the same weights that is off by roundings only is 1e-4 (fp32) off after a dozen updates, so this asks for the same bits."""
+    kw = dict(sequence_len=T, max_document_tokens=512, vocab_size=300, n_layer=3, n_head=4, n_kv_head=2, n_embed=512, window_pattern="SL")
+    cfg, ocfg = fb.GPTConfig(**kw), fo.GPTConfig(**kw)
+    lay, olay = fb.parameter_layout(cfg), fo.parameter_layout(ocfg)
+    th = torch.zeros(lay.nparams)
+    fo.initialize(th, ocfg, olay, 9, all_nonzero=True)
+    tok, tgt, pos = inputs(kw, B, seed=T)
+    params = fb.Params(th.cuda())
+    st = fb.gradient_state(params, cfg, lay, tok, tgt, pos, compute_type=dtype, short_window=30, doc_mask=True)
+    opt = fb.MuonAdamW(params, lay, st, compute_type=dtype)
+    for _ in range(2):
+        fb.loss_and_gradient_(params, st, lay, tok, tgt, pos, reduction="sum")
+        opt.step(Nt=float(tok.numel()))
+    got = hashlib.sha256(torch.cat([params.delta, params.theta]).cpu().numpy().tobytes()).hexdigest()[:16]
+    assert got == STEP_BITS[dtype, B, T]
 
 
 @pytest.mark.parametrize("nz", [False, True])
