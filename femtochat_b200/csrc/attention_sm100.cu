@@ -41,9 +41,12 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&h);
 }
 
-// What rounding (lo, hi) to the packed pair `h` left over, rounded in turn: together they hold 16 bits of each.
-__device__ __forceinline__ uint32_t rest_bf16(float lo, float hi, uint32_t h) {
-  return pack_bf16(lo - __uint_as_float(h << 16), hi - __uint_as_float(h & 0xffff0000u));
+// (lo, hi) as three pairs of bf16, 8 bits of each number in every one: their sum is the fp32 number itself.
+__device__ __forceinline__ void split_bf16(float lo, float hi, uint32_t& a, uint32_t& b, uint32_t& c) {
+  a = pack_bf16(lo, hi);
+  lo -= __uint_as_float(a << 16); hi -= __uint_as_float(a & 0xffff0000u);
+  b = pack_bf16(lo, hi);
+  c = pack_bf16(lo - __uint_as_float(b << 16), hi - __uint_as_float(b & 0xffff0000u));
 }
 
 // Optional cycle accounting of the roles of the persistent forward kernels (compiled in with -DFEMTO_ATTN_CYCLES,
@@ -345,8 +348,10 @@ constexpr int PF_SMEM = TILE_BYTES * 6 + 1024 + 256 + 3 * NS * 128 * 4;
 
 // RAGGED: T is not a multiple of the tile.  Tensor maps have one dimension per batch column, so the rows past a column's end
 // arrive as zeros and are clipped on the way out; causality masks them for every query of the column.  These lengths used to
-// take the SIMT kernel, which keeps P in fp32, so here P is the sum of two bf16 numbers: its high part lies over the first half
-// of S, its low part over the second, and P V is two products.  5 x 1000 tokens, 6 heads, causal: 2980 -> 25.6 us; 1500 tokens, 10 heads: 2230 -> 20.9 us.
+// take the SIMT kernel, which keeps P in fp32, so here P is the sum of three bf16 numbers, which is P to the last bit: two of them lie
+// over the halves of S, the third in columns of its own, and P V is three products.
+// 5 x 1000 tokens, 6 heads, causal: 2900 -> 31.0 us; 1500 tokens, 10 heads: 2230 -> 28.6 us (two parts: 26.7 and 23.8, but 1.1 - 2.4 in 1000
+// results on the wrong side of their bf16 rounding where fp32 has 0.1 - 0.4 and three parts 0.05 - 0.4, 1.6 past 1000 keys).
 
 __device__ __forceinline__ void pf_item(const AttnArgs& a, int item, int nqt, int& qt, int& h, int& b) {
   // heavy (late) query tiles first; within a query tile all heads and batch rows cost about the same
@@ -405,6 +410,7 @@ attn_fwd_persistent_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t tS[2] = {tmem_base, tmem_base + 128};
   const uint32_t tO = tmem_base + 256;
+  const uint32_t tR[2] = {tmem_base + 384, tmem_base + 448};   // RAGGED: the last 8 bits of P, written and read with S
 
   // Every role walks the same items in the same order.  n = number of this CTA's items so far (Q stage n & 1, phase
   // (n >> 1) & 1); tc = number of key tiles so far (K / V / S stage tc & 1, phase (tc >> 1) & 1).
@@ -527,6 +533,9 @@ attn_fwd_persistent_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid
 #pragma unroll
             for (int k = 0; k < BKV / 16; k++)
               mma_ts(tO, tS[st] + 64 + k * 8, smem_desc_sw128(v_addr + k * 2048, TILE_BYTES / 2, 1024), idesc_o, 1u);
+#pragma unroll
+            for (int k = 0; k < BKV / 16; k++)
+              mma_ts(tO, tR[st] + k * 8, smem_desc_sw128(v_addr + k * 2048, TILE_BYTES / 2, 1024), idesc_o, 1u);
           }
           tc_commit(&pv_done[st]);
           cy.lap(1);
@@ -627,18 +636,25 @@ attn_fwd_persistent_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid
         float sm[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
         for (int u = 0; u < CW / 32; u++) {
-          uint32_t pk[16], pl[16];
+          uint32_t pk[16], pl[16], pr[16];
 #pragma unroll
           for (int j = 0; j < 16; j += 2) {
             const float p0 = fast_exp2(fmaf(x[u * 32 + 2 * j], c, -mm)), p1 = fast_exp2(fmaf(x[u * 32 + 2 * j + 1], c, -mm));
             const float p2 = fast_exp2(fmaf(x[u * 32 + 2 * j + 2], c, -mm)), p3 = fast_exp2(fmaf(x[u * 32 + 2 * j + 3], c, -mm));
             sm[0] += p0; sm[1] += p1; sm[2] += p2; sm[3] += p3;
-            pk[j] = pack_bf16(p0, p1);
-            pk[j + 1] = pack_bf16(p2, p3);
-            if constexpr (RAGGED) { pl[j] = rest_bf16(p0, p1, pk[j]); pl[j + 1] = rest_bf16(p2, p3, pk[j + 1]); }
+            if constexpr (RAGGED) {
+              split_bf16(p0, p1, pk[j], pl[j], pr[j]);
+              split_bf16(p2, p3, pk[j + 1], pl[j + 1], pr[j + 1]);
+            } else {
+              pk[j] = pack_bf16(p0, p1);
+              pk[j + 1] = pack_bf16(p2, p3);
+            }
           }
           tmem_st16(tS[st] + lane_off + hs * (CW / 2) + u * 16, pk);
-          if constexpr (RAGGED) tmem_st16(tS[st] + lane_off + 64 + hs * (CW / 2) + u * 16, pl);
+          if constexpr (RAGGED) {
+            tmem_st16(tS[st] + lane_off + 64 + hs * (CW / 2) + u * 16, pl);
+            tmem_st16(tR[st] + lane_off + hs * (CW / 2) + u * 16, pr);
+          }
         }
         l += (sm[0] + sm[1]) + (sm[2] + sm[3]);
         cy.lap(4);

@@ -220,7 +220,7 @@ def test_simt_attention_sums_key_by_key(B, T, H, Hkv, hd, left, docs):
     (2, 1, 2, 1, 1, False), (3, 5, 2, 2, 5, True), (2, 127, 2, 1, 127, False), (2, 129, 4, 2, 40, True), (3, 255, 2, 2, 255, True),
     (2, 257, 6, 2, 100, False), (1, 1000, 10, 5, 300, True), (2, 1153, 2, 1, 2000, False)])
 def test_attention_of_ragged_lengths(B, T, H, Hkv, left, docs):
-    """Lengths that are no multiple of the 128-row tiles, several columns: the forward pass on the tensor cores with P in bf16 parts, the
+    """Lengths that are no multiple of the 128-row tiles, several columns: the forward pass on the tensor cores with P in three bf16 parts, the
     reverse on the SIMT kernels.  O is off by its own rounding (2^-9 of it) and 2^-14 of the largest, the gradients by their rounding and
     that of the O they are computed from (2^-9 each, rms below 4e-3); nothing past a column's end is read or written; accumulate adds."""
     Q, K, V, dO, ds = _attn_inputs(_lib.BF16, B, T, H, Hkv, 128, seed=T, docs=docs)
@@ -255,6 +255,24 @@ def test_attention_of_ragged_lengths(B, T, H, Hkv, left, docs):
         assert (got.float() - 2 * one.float()).norm() <= 4e-3 * 2 * one.float().norm() + 1e-6
     for h, x in zip(held, (Q, Q, K, V)):
         assert (h[x.numel():] == 7.0).all()
+
+
+@pytest.mark.parametrize("B,T,H,Hkv,left", [(16, 24, 6, 6, 24), (8, 77, 4, 2, 77), (2, 333, 10, 5, 100)])
+def test_ragged_attention_keeps_p_in_32_bits(B, T, H, Hkv, left):
+    """O is the exact result rounded to bf16 but where an error of e |O| moves it over a rounding boundary, about e 2^9 of all results.  With P, sums
+    and exponentials in fp32 e is some 2^-22 (1 to 3 results of 10000); P in 16 bits has 2^-18 and gives 12 to 18."""
+    g = torch.Generator(device="cuda").manual_seed(T)
+    Q, K, V = (torch.randn(B, T, n, 128, generator=g, device="cuda") for n in (H, Hkv, Hkv))
+    Q, K = (1.2 * x / x.square().mean(-1, keepdim=True).sqrt() for x in (Q, K))
+    Q, K, V = (x.bfloat16() for x in (Q, K, V))
+    O = torch.empty_like(Q)
+    _lib.check(_lib.lib().femto_attention_fwd(_lib.BF16, _lib.ptr(O), None, None, None, _lib.ptr(Q), _lib.ptr(K), _lib.ptr(V), B, T, H, Hkv, 128, left, None, None))
+    torch.cuda.synchronize()
+    q, k, v = (x.double().permute(0, 2, 1, 3).repeat_interleave(H // x.shape[2], 1) for x in (Q, K, V))
+    t = torch.arange(T, device="cuda")
+    hidden = (t[None] > t[:, None]) | (t[:, None] - t[None] > left)
+    ref = torch.softmax((q @ k.transpose(-1, -2) * 128 ** -0.5).masked_fill(hidden, -math.inf), -1) @ v
+    assert float((O != ref.permute(0, 2, 1, 3).bfloat16()).double().mean()) <= 6e-4
 
 
 def test_attention_at_benchmark_shape_geometric_documents():
