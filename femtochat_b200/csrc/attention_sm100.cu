@@ -572,7 +572,7 @@ attn_fwd_persistent_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid
       if (ok && lane == 0 && n >= 1) { bulk_wait_read<0>(); mbar_arrive(&q_free[(n - 1) & 1]); }
       int lo = max(0, q - a.window_left);
       if (a.doc_start) lo = max(lo, a.doc_start[row0 + (RAGGED ? min(q, a.T - 1) : q)]);
-      float m_used = -INFINITY, l = 0.f;
+      float m_used = -INFINITY, l = 0.f, m_row = -INFINITY;   // m_used moves only past 2^8; m_row is the row's maximum
       for (int i = 0; i < ntile; i++, tc++) {
         const int st = tc & 1;
         const uint32_t ph = (tc >> 1) & 1;
@@ -609,6 +609,7 @@ attn_fwd_persistent_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid
         cy.lap(2);
 #pragma unroll
         for (int o = 1; o < NS; o++) mt = fmaxf(mt, xmax[(tc & 1) * (NS * 128) + ((hs + o) % NS) * 128 + r]);
+        m_row = fmaxf(m_row, mt);
         const bool grow = mt > m_used + 8.f || (m_used == -INFINITY && mt > -INFINITY);
         if (__any_sync(0xffffffffu, grow)) {
           const float m_new = fmaxf(m_used, mt);
@@ -707,8 +708,8 @@ attn_fwd_persistent_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid
           const long long si = ((long long)b * a.H + h) * a.T + q;
           const float ln2 = 0.6931471805599453f;
           if (a.lse) a.lse[si] = (m_used + log2f(l)) * ln2;
-          if (a.l) a.l[si] = l;
-          if (a.m) a.m[si] = m_used * ln2;
+          if (a.l) a.l[si] = m_row == m_used ? l : l * exp2f(m_used - m_row);
+          if (a.m) a.m[si] = m_row * ln2;
         }
       }
       // the row's partner reads xl of this item before either thread may overwrite it for the next one

@@ -275,6 +275,23 @@ def test_ragged_attention_keeps_p_in_32_bits(B, T, H, Hkv, left):
     assert float((O != ref.permute(0, 2, 1, 3).bfloat16()).double().mean()) <= 6e-4
 
 
+@pytest.mark.parametrize("B,T,H,Hkv,left,docs", [(2, 77, 2, 1, 77, False), (1, 1000, 4, 2, 1000, False), (2, 450, 6, 6, 100, True), (2, 512, 4, 2, 512, True)])
+def test_attention_row_maximum_and_sum(B, T, H, Hkv, left, docs):
+    """l and m are the sum and the maximum of every row, in natural units, at ragged and at whole-tile lengths (scores up to some 50: their fp32
+    products are off by 1e-5 at most, and l, which is relative to the maximum, by as much)."""
+    Q, K, V, _, ds = _attn_inputs(_lib.BF16, B, T, H, Hkv, 128, seed=T, docs=docs)
+    Q = 3 * Q
+    _, l_ref, m_ref = fo.flash_attention_forward(Q.double(), K.double(), V.double(), (left, 0), ds.long() if ds is not None else None)
+    dev = [x.cuda() for x in (Q, K, V)]
+    dsd = ds.cuda() if ds is not None else None
+    O, l, m = torch.empty_like(dev[0]), torch.empty(B, H, T, device="cuda"), torch.empty(B, H, T, device="cuda")
+    _lib.check(_lib.lib().femto_attention_fwd(_lib.BF16, _lib.ptr(O), _lib.ptr(l), _lib.ptr(m), None, _lib.ptr(dev[0]), _lib.ptr(dev[1]), _lib.ptr(dev[2]),
+                                              B, T, H, Hkv, 128, left, _lib.ptr(dsd), None))
+    torch.cuda.synchronize()
+    assert (m.double().cpu() - m_ref).abs().max() <= 2e-5
+    assert ((l.double().cpu() - l_ref).abs() <= 4e-5 * l_ref).all()
+
+
 def test_attention_at_benchmark_shape_geometric_documents():
     """The benchmark's attention shape: T=2048, 10 query / 5 kv heads, head_dim 128, short window 1024, documents of
     geometric(512) length (B=1 so that the fp64 naive reference stays small)."""
