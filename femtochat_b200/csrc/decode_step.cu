@@ -606,12 +606,20 @@ size_t smem_bytes(int d, int L, int nt, int gmax) {
   return (size_t)(nt == 1 ? ring_of<1>() : ring_of<2>()) * SLOT + (size_t)8 * nt * (d + 16) * 2 + red_bytes(nt, gmax) + sizeof(DecodeBlock) * L;
 }
 
-// blocks that stay on the device together, or 0
+// blocks that stay on the device together, or 0.  The limit of dynamic shared memory belongs to the function and the device, not to
+// a model, so it is always set to all that a block may have: caches of several models decode in turn.
 template <int NT, int GMAX> int resident_blocks(size_t smem) {
   auto kernel = k_decode_step<NT, GMAX, ring_of<NT>()>;
-  int per = 0;
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, THREADS + 128, smem) != cudaSuccess) {
+  int per = 0, dev = 0, most = 0;
+  cudaFuncAttributes fixed;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
+      cudaFuncGetAttributes(&fixed, kernel) != cudaSuccess ||
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)fixed.sharedSizeBytes) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  if (smem + fixed.sharedSizeBytes > (size_t)most) return 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, THREADS + 128, smem) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }

@@ -480,6 +480,37 @@ def test_decode_step_of_bf16_columns_matches_the_oracle(B, H, G, L, doc_mask):
     kc.close()
 
 
+def _bf16_server(B, H, G, L, T, doc_mask, vocab=1000):
+    """A bf16 GPT with heads of 128 channels, tokens and positions of T tokens a column, and the oracle's logits of all of them."""
+    kw = dict(sequence_len=T, max_document_tokens=max(512, T), vocab_size=vocab, n_layer=L, n_head=H, n_kv_head=G, n_embed=128 * H, window_pattern="SL")
+    cfg, ocfg = fb.GPTConfig(**kw), fo.GPTConfig(**kw)
+    lay, olay = fb.parameter_layout(cfg), fo.parameter_layout(ocfg)
+    th = torch.zeros(lay.nparams)
+    fo.initialize(th, ocfg, olay, 17 + H, all_nonzero=True)
+    tok = torch.randint(1, vocab + 1, (B, T), generator=torch.Generator().manual_seed(B), dtype=torch.int32)
+    pos = torch.arange(T, dtype=torch.int32)[None, :].repeat(B, 1)
+    cache_o = {}
+    fo.Model(ocfg, fo.StepOptions(eps=fo.EPS_BF16, short_window=70, doc_mask=doc_mask)).forward(th, tok, tok, pos, cache=cache_o)
+    model = fb.GPT(fb.Params(th.cuda()), cfg, lay, compute_type="bfloat16", short_window=70, doc_mask=doc_mask)
+    return model, tok, pos, cache_o["z"].float().reshape(B, T, vocab)
+
+
+@pytest.mark.gpu
+def test_decode_steps_of_several_models_in_turn():
+    """Caches of a wide and of a narrow model are alive together and decode alternately: neither's size limits the other's launches."""
+    made = [_bf16_server(2, H, G, 2, 24, False) for H, G in ((8, 8), (2, 1), (4, 2))]
+    caches = []
+    for model, tok, pos, _ in made:
+        caches.append(fb.KVCache(model.state(2), 2, 24))
+        fb.prefill(model, caches[-1], tok[:, :20], pos[:, :20])
+    for t in range(20, 24):
+        for (model, tok, pos, ref), kc in zip(made, caches):
+            z = fb.decode_step(model, kc, tok[:, t], pos[:, t]).cpu()
+            assert (z - ref[:, t]).abs().max() <= 2.5e-2 * float(ref.abs().max()), t
+    for kc in caches:
+        kc.close()
+
+
 def test_generate_with_cache_equals_generate_by_recompute():
     """`generate` (src/generation.jl:26-56): greedy decoding (temperature 0) through the cache gives the tokens of
     the reference's recompute-everything loop; with sampling the same generator state gives the same tokens."""
