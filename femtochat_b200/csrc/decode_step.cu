@@ -37,19 +37,22 @@ __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t s) {
   asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(s));
   return r;
 }
-// Words that carry their name: two of them a load, straight from L2
+// Words that carry their name, straight from and to L2.  Each is ONE 64-bit scalar, which the memory model never tears: a vector of
+// 32-bit elements is several accesses without order, and a reader could see the new name beside the old data.  (Two words a load: a
+// vector of two such scalars, each with a name of its own.)
 __device__ __forceinline__ uint4 named_load2(const uint2* p) {
   uint4 v;
-  asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+  asm volatile("{\n\t.reg .b64 a, b;\n\tld.relaxed.gpu.global.v2.b64 {a, b}, [%4];\n\tmov.b64 {%0, %1}, a;\n\tmov.b64 {%2, %3}, b;\n\t}"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
   return v;
 }
 __device__ __forceinline__ uint2 named_load(const uint2* p) {
   uint2 v;
-  asm volatile("ld.volatile.global.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p) : "memory");
+  asm volatile("{\n\t.reg .b64 a;\n\tld.relaxed.gpu.global.b64 a, [%2];\n\tmov.b64 {%0, %1}, a;\n\t}" : "=r"(v.x), "=r"(v.y) : "l"(p) : "memory");
   return v;
 }
 __device__ __forceinline__ void named_store(uint2* p, uint32_t data, uint32_t name) {
-  asm volatile("st.volatile.global.v2.u32 [%0], {%1, %2};" ::"l"(p), "r"(data), "r"(name) : "memory");
+  asm volatile("{\n\t.reg .b64 a;\n\tmov.b64 a, {%1, %2};\n\tst.relaxed.gpu.global.b64 [%0], a;\n\t}" ::"l"(p), "r"(data), "r"(name) : "memory");
 }
 __device__ __forceinline__ void named_store(uint2* p, float data, uint32_t name) { named_store(p, __float_as_uint(data), name); }
 __device__ __forceinline__ float lo_f(uint32_t p) { return __uint_as_float(p << 16); }
@@ -282,19 +285,27 @@ __global__ void __launch_bounds__(THREADS + 128, 1) k_decode_step(const DecodeSt
     if (!(lane & 1)) named_store(row + (col >> 1), pack2(v, w), name);
   };
   // Rows of X: d columns of every row of `src` (pairs; `pitch` words a row), with the sums of squares of every 128 columns.
-  // All loads of a thread are in flight together (10: eight rows of 1280).
+  // All loads of a thread are in flight together (10: eight rows of 1280; one or two in most steps of few columns).  Every round of
+  // polls writes every v: what it left as it was would stay in registers beside the new (700 bytes of spills, 16 us more a token of d12).
   auto rows_of = [&](const uint2* src, int pitch, uint32_t name, bool squares) {
     constexpr int U = 10;
     for (int q0 = warp; q0 < B * steps; q0 += WARPS * U) {
       uint4 v[U];
       until([&] {
         bool ok = true;
-#pragma unroll
-        for (int u = 0; u < U; u++) {
+        auto ask = [&](int u) {
           const int q = q0 + u * WARPS;
-          if (q >= B * steps) break;
-          v[u] = named_load2(src + (long long)(q / steps) * pitch + q % steps * 64 + lane * 2);
+          v[u] = make_uint4(0, name, 0, name);
+          if (q < B * steps) v[u] = named_load2(src + (long long)(q / steps) * pitch + q % steps * 64 + lane * 2);
           ok &= v[u].y == name && v[u].w == name;
+        };
+        ask(0); ask(1);
+        if (q0 + 2 * WARPS < B * steps) {
+#pragma unroll
+          for (int u = 2; u < U; u++) ask(u);
+        } else {
+#pragma unroll
+          for (int u = 2; u < U; u++) v[u] = make_uint4(0, 0, 0, 0);
         }
         return ok;
       });

@@ -73,6 +73,13 @@ def test_schedules_match_oracle():
         assert (s["eta"], s["mu"], s["lam"]) == pytest.approx(fo.training_schedule(step, steps))
 
 
+def test_words_of_the_decode_step_are_single_accesses():
+    """Data and name of a word of the resident decode kernel travel as one 64-bit scalar (a vector of 32-bit elements may tear)."""
+    src = open(os.path.join(os.path.dirname(fb.__file__), "csrc", "decode_step.cu")).read()
+    accesses = re.findall(r"((?:ld|st)\.[a-z.]*global[a-z0-9.]*) ", src)
+    assert len(accesses) == 3 and all(a.endswith(".b64") for a in accesses), accesses
+
+
 def test_packed_batches_follow_loader_format():
     V, T, B = 4096, 256, 4
     pk = fb.PackedBatches(V, T, B, max_document_tokens=300, mean_doc_len=40, seed=1)
