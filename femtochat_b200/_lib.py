@@ -91,6 +91,7 @@ SIGNATURES = {
     "femto_kv_cache_create": (I32, [P, I32, I32, C.POINTER(P)]),
     "femto_kv_cache_destroy": (I32, [P]),
     "femto_kv_cache_length": (I32, [P]),
+    "femto_kv_cache_blocks": (I32, [P, I32]),
     "femto_prefill": (I32, [P, P, P, P, P, I32, I32, P, P]),
     "femto_decode_step": (I32, [P, P, P, P, P, I32, P, P]),
     "femto_kv_cache_reset": (I32, [P, P]),

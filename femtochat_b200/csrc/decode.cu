@@ -350,13 +350,18 @@ static int decode_t(femto_kv_cache* c, const float* theta, const int* tokens, co
   const int d = h->d, dq = h->dq, kv = h->kv, H = h->H, Hkv = h->Hkv, hd = h->hd, L = h->L;
   const float eps = h->eps;
   const int t = c->len;   // row of the new token in every column's cache
-  if (sizeof(T) == 2 && B <= c->step.columns) {
+  if (sizeof(T) == 2 && B <= c->step.columns && c->step.blocks_n > 0) {
     DecodeStepArgs a = {};
-    a.theta = theta; a.xe_prev = (bf16*)c->xe_prev; a.tok0 = c->tok0; a.pos = c->pos; a.doc_start = c->doc_start; a.lastpos = c->lastpos;
+    a.theta = theta; a.xe_prev = (bf16*)c->xe_prev; a.xe_new = (bf16*)c->xe_new; a.tok0 = c->tok0; a.pos = c->pos; a.doc_start = c->doc_start; a.lastpos = c->lastpos;
     a.logits = logits_out; a.B = B; a.t = t; a.maxT = c->maxT;
-    FEMTO_TRY(decode_step_run(h, c->step, a, tokens, positions, s));
-    c->len = t + 1;
-    return 0;
+    bool ran = false;
+    FEMTO_TRY(decode_step_run(h, c->step, a, tokens, positions, s, &ran));
+    if (ran) {
+      std::swap(c->xe_prev, c->xe_new);
+      std::swap(c->lastpos, c->pos);
+      c->len = t + 1;
+      return 0;
+    }
   }
   k_decode_prep<<<cdiv(B, 128), 128, 0, s>>>(tokens, positions, B, h->cfg.index_base, h->V, h->cfg.max_document_tokens, t, c->tok0,
                                              c->pos, c->doc_start, c->lastpos, h->status);
@@ -455,6 +460,13 @@ extern "C" int32_t femto_kv_cache_reset(femto_kv_cache* c, void* stream) {
   if (c->h->dec) return decoder_cache_reset(c, (cudaStream_t)stream);
   c->B = 0; c->len = 0;   // a GPT cache is written from its start by the next femto_prefill
   return 0;
+}
+
+extern "C" int32_t femto_kv_cache_blocks(femto_kv_cache* c, int32_t blocks) {
+  if (!c || !c->step.columns) return 0;
+  const int old = c->step.blocks_n;
+  if (blocks >= 0) c->step.blocks_n = blocks;
+  return old;
 }
 
 extern "C" int32_t femto_kv_cache_length(femto_kv_cache* c) { return c ? c->len : FEMTO_ERR_ARG; }

@@ -70,7 +70,9 @@ __device__ __forceinline__ void put4(bf16* row, int col, uint32_t lo, uint32_t h
 }
 
 // ---- the new token of every column: its id and position, normalised embedding and smear, and the first block's mixed stream ----
-// launches[0] counts the launches so far, launches[1] is this one's number for the blocks of the step.
+// launches[0] counts the launches so far, launches[1] is this one's number for the blocks of the step.  What the cache keeps from
+// token to token (xe_prev, lastpos) is read only, and the caller swaps the buffers once the step is launched: where that is refused, the
+// chain of kernels starts from the same state.
 __global__ void __launch_bounds__(THREADS) k_step_begin(const DecodeStepArgs a, const int* tokens, const int* positions, int base, int vocab,
                                                         int maxdoc) {
   const int b = blockIdx.x, tid = threadIdx.x;
@@ -99,7 +101,7 @@ __global__ void __launch_bounds__(THREADS) k_step_begin(const DecodeStepArgs a, 
   const float inv = rsqrtf(ss / a.d + a.eps);
   if (tid == 0) {
     const int p = pos_s;
-    a.tok0[b] = tk; a.pos[b] = p; a.lastpos[b] = p;
+    a.tok0[b] = tk; a.pos[b] = p;
     a.doc_start[b] = max(0, a.t - p);   // index (within the column) of the first token of this token's document
   }
   // every warp sums the smear gate's 24 inputs by itself
@@ -107,7 +109,8 @@ __global__ void __launch_bounds__(THREADS) k_step_begin(const DecodeStepArgs a, 
   float pre = lane < 24 ? __bfloat162float(__float2bfloat16_rn(__bfloat162float(src[lane]) * inv)) * a.theta[a.off_smear + lane] : 0.f;
   pre = warp_sum(pre);
   const float gate = a.theta[a.off_lam_s] * (1.f / (1.f + expf(-pre)));
-  bf16* prev = a.xe_prev + (long long)b * a.d;
+  const bf16* prev = a.xe_prev + (long long)b * a.d;
+  bf16* next = a.xe_new + (long long)b * a.d;
   const float mix = a.theta[a.blocks[0].lam_b] + a.theta[a.blocks[0].lam_x0];
   for (int c = 2 * tid; c < a.d; c += 2 * THREADS) {
     float x[2];
@@ -115,7 +118,7 @@ __global__ void __launch_bounds__(THREADS) k_step_begin(const DecodeStepArgs a, 
     for (int i = 0; i < 2; i++) {
       const bf16 e = __float2bfloat16_rn(__bfloat162float(src[c + i]) * inv);
       x[i] = __bfloat162float(e) + gate * __bfloat162float(prev[c + i]);
-      prev[c + i] = e;
+      next[c + i] = e;
       const long long at = (long long)b * a.d + c + i;
       a.x0[at] = x[i];
       x[i] *= mix;
@@ -702,7 +705,7 @@ int decode_step_setup(const femto_handle* h, DecodeStepState& st, const std::vec
   return 0;
 }
 
-int decode_step_run(const femto_handle* h, const DecodeStepState& st, DecodeStepArgs a, const int* tokens, const int* positions, cudaStream_t s) {
+int decode_step_run(const femto_handle* h, const DecodeStepState& st, DecodeStepArgs a, const int* tokens, const int* positions, cudaStream_t s, bool* ran) {
   a.blocks = st.blocks; a.maps = st.maps; a.launches = st.launches; a.x0 = st.x0;
   a.xn = st.xn; a.xm = st.xm; a.xa = st.xa; a.xa2 = st.xa2; a.xb = st.xb; a.part = st.part; a.qkv = st.qkv; a.h16 = st.h16; a.up = st.up;
   a.att = st.att; a.att_part = st.att_part;
@@ -725,10 +728,15 @@ int decode_step_run(const femto_handle* h, const DecodeStepState& st, DecodeStep
   at[0].id = cudaLaunchAttributeCooperative;      // the blocks wait for one another: all of them are resident or none is
   at[0].val.cooperative = 1;
   cfg.attrs = at; cfg.numAttrs = 1;
-#define LAUNCH(NT, GM) CUDA_TRY(cudaLaunchKernelEx(&cfg, k_decode_step<NT, GM, ring_of<NT>()>, a))
+  cudaError_t e;
+#define LAUNCH(NT, GM) e = cudaLaunchKernelEx(&cfg, k_decode_step<NT, GM, ring_of<NT>()>, a)
   if (nt == 1) { if (gmax == 2) LAUNCH(1, 2); else LAUNCH(1, 8); }
   else { if (gmax == 2) LAUNCH(2, 2); else LAUNCH(2, 8); }
 #undef LAUNCH
+  // a context or stream with fewer multiprocessors than the device has: nothing is lost, the caller takes the chain of kernels
+  *ran = e != cudaErrorCooperativeLaunchTooLarge;
+  if (!*ran) { cudaGetLastError(); return 0; }
+  CUDA_TRY(e);
   KERNEL_CHECK();
   return 0;
 }

@@ -29,7 +29,7 @@ struct DecodeStepArgs {
   uint2 *xn, *xm, *xa, *xa2, *xb, *part, *qkv, *h16, *up, *att, *att_part;
   float* x0;
   const float* theta;
-  const bf16* wte; bf16* xe_prev;
+  const bf16* wte; bf16 *xe_prev, *xe_new;
   const float *sin_t, *cos_t;
   int *tok0, *pos, *doc_start, *lastpos;
   float* logits;
@@ -43,4 +43,5 @@ void decode_step_plan(const femto_handle* h, int max_batch, DecodeStepState& st)
 size_t decode_step_bytes(const femto_handle* h, DecodeStepState st);
 void decode_step_carve(const femto_handle* h, char*& p, DecodeStepState& st);
 int decode_step_setup(const femto_handle* h, DecodeStepState& st, const std::vector<void*>& K, const std::vector<void*>& V);
-int decode_step_run(const femto_handle* h, const DecodeStepState& st, DecodeStepArgs a, const int* tokens, const int* positions, cudaStream_t s);
+int decode_step_run(const femto_handle* h, const DecodeStepState& st, DecodeStepArgs a, const int* tokens, const int* positions, cudaStream_t s,
+                    bool* ran);      // false: the launch was refused and nothing of the cache has changed

@@ -134,6 +134,11 @@ typedef struct femto_kv_cache femto_kv_cache;
 int32_t femto_kv_cache_create(femto_handle* h, int32_t max_batch, int32_t max_len, femto_kv_cache** h_out);
 int32_t femto_kv_cache_destroy(femto_kv_cache* c);
 int32_t femto_kv_cache_length(femto_kv_cache* c); /* tokens cached per column */
+/* A bf16 GPT's token is one kernel whose blocks, one per multiprocessor, wait for one another, so it starts when that many are
+ * free.  A program that keeps some busy with other work for long says how many blocks there may be: 0 takes the chain
+ * of kernels for every token, as a refused launch does for its own; a negative number only asks.  Returns the number before (0 too
+ * for models that always take the chain).  No counterpart in the reference. */
+int32_t femto_kv_cache_blocks(femto_kv_cache* c, int32_t blocks);
 /* tokens / positions: int32 [B][Tp] device arrays (positions NULL = 0..Tp-1); resets the cache to this prompt. */
 int32_t femto_prefill(femto_handle* h, femto_kv_cache* c, const float* theta, const int32_t* tokens,
                       const int32_t* positions, int32_t B, int32_t Tp, float* logits_out, void* stream);

@@ -6,6 +6,7 @@ import pytest
 import torch
 
 import femtochat_b200 as fb
+from femtochat_b200 import _lib
 from oracle import femto_oracle as fo
 
 pytestmark = pytest.mark.gpu
@@ -509,6 +510,24 @@ def test_decode_steps_of_several_models_in_turn():
             assert (z - ref[:, t]).abs().max() <= 2.5e-2 * float(ref.abs().max()), t
     for kc in caches:
         kc.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("blocks", [0, 1, 37, 1 << 20])
+def test_decode_step_with_fewer_blocks_than_multiprocessors(blocks):
+    """A cache may be told to take fewer blocks, or none (the chain of kernels); more than the device holds is what a context of fewer
+    multiprocessors meets: the launch is refused and the chain runs from the same state, step after step (positions continue by themselves)."""
+    model, tok, pos, ref = _bf16_server(3, 4, 2, 3, 90, True)
+    kc = fb.KVCache(model.state(3), 3, 90)
+    fb.prefill(model, kc, tok[:, :80], pos[:, :80])
+    n = _lib.lib().femto_kv_cache_blocks(kc.c, blocks)
+    assert n > 37 and _lib.lib().femto_kv_cache_blocks(kc.c, -1) == blocks
+    for t in range(80, 90):
+        if t == 85:
+            _lib.lib().femto_kv_cache_blocks(kc.c, n)
+        z = fb.decode_step(model, kc, tok[:, t]).cpu()
+        assert (z - ref[:, t]).abs().max() <= 2.5e-2 * float(ref.abs().max()), t
+    kc.close()
 
 
 def test_generate_with_cache_equals_generate_by_recompute():
