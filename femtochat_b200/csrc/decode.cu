@@ -342,6 +342,13 @@ template <typename T> int kv_cache_last_logits(femto_kv_cache* c, const T* xnf, 
 template int kv_cache_last_logits<float>(femto_kv_cache*, const float*, int, int, float*, cudaStream_t);
 template int kv_cache_last_logits<bf16>(femto_kv_cache*, const bf16*, int, int, float*, cudaStream_t);
 
+static DecodeStepArgs step_args(femto_kv_cache* c, const float* theta, int B, float* logits_out) {
+  DecodeStepArgs a = {};
+  a.theta = theta; a.xe_prev = (bf16*)c->xe_prev; a.xe_new = (bf16*)c->xe_new; a.tok0 = c->tok0; a.pos = c->pos; a.doc_start = c->doc_start; a.lastpos = c->lastpos;
+  a.logits = logits_out; a.B = B; a.t = c->len; a.maxT = c->maxT;
+  return a;
+}
+
 template <typename T>
 static int decode_t(femto_kv_cache* c, const float* theta, const int* tokens, const int* positions, int B, float* logits_out,
                     cudaStream_t s) {
@@ -351,11 +358,8 @@ static int decode_t(femto_kv_cache* c, const float* theta, const int* tokens, co
   const float eps = h->eps;
   const int t = c->len;   // row of the new token in every column's cache
   if (sizeof(T) == 2 && B <= c->step.columns && c->step.blocks_n > 0) {
-    DecodeStepArgs a = {};
-    a.theta = theta; a.xe_prev = (bf16*)c->xe_prev; a.xe_new = (bf16*)c->xe_new; a.tok0 = c->tok0; a.pos = c->pos; a.doc_start = c->doc_start; a.lastpos = c->lastpos;
-    a.logits = logits_out; a.B = B; a.t = t; a.maxT = c->maxT;
     bool ran = false;
-    FEMTO_TRY(decode_step_run(h, c->step, a, tokens, positions, s, &ran));
+    FEMTO_TRY(decode_step_run(h, c->step, step_args(c, theta, B, logits_out), tokens, positions, s, &ran));
     if (ran) {
       std::swap(c->xe_prev, c->xe_new);
       std::swap(c->lastpos, c->pos);
@@ -502,6 +506,29 @@ extern "C" int32_t femto_decode_step(femto_handle* h, femto_kv_cache* c, const f
   if (!h->weights_valid) return femto_fail(FEMTO_ERR_STATE, "call femto_refresh_weights before the first step");
   return h->bf ? decode_t<bf16>(c, theta, tokens, positions, B, logits_out, (cudaStream_t)stream)
                : decode_t<float>(c, theta, tokens, positions, B, logits_out, (cudaStream_t)stream);
+}
+
+extern "C" int32_t femto_selftest_decode_wait(femto_handle* h, femto_kv_cache* c, const float* theta, const int32_t* tokens, int32_t B, float* logits_out,
+                                              void* stream, int32_t* h_status) {
+  if (!h_status) return femto_fail(FEMTO_ERR_ARG, "NULL argument");
+  FEMTO_TRY(femto_decode_step(h, c, theta, tokens, nullptr, B, logits_out, stream));     // leaves positions and an embedding in place
+  if (h->dec || !h->bf || B > c->step.columns || c->step.blocks_n <= 0) return femto_fail(FEMTO_ERR_UNSUPPORTED, "this model's tokens take the chain of kernels");
+  if (c->len >= c->maxT) return femto_fail(FEMTO_ERR_SHAPE, "the cache is full (%d tokens per column)", c->maxT);
+  cudaStream_t s = (cudaStream_t)stream;
+  CUDA_TRY(cudaStreamSynchronize(s));
+  unsigned int launches = 0, before = 0, after = 0;
+  CUDA_TRY(cudaMemcpy(&launches, c->step.launches, 4, cudaMemcpyDeviceToHost));
+  CUDA_TRY(cudaMemcpy(&before, h->status, 4, cudaMemcpyDeviceToHost));
+  CUDA_TRY(cudaMemset(h->status, 0, 4));
+  bool ran = false;
+  FEMTO_TRY(decode_step_run(h, c->step, step_args(c, theta, B, logits_out), nullptr, nullptr, s, &ran));
+  CUDA_TRY(cudaStreamSynchronize(s));                    // the kernel returned by itself
+  if (!ran) return femto_fail(FEMTO_ERR_UNSUPPORTED, "the launch was refused");
+  CUDA_TRY(cudaMemcpy(&after, h->status, 4, cudaMemcpyDeviceToHost));
+  CUDA_TRY(cudaMemcpy(h->status, &before, 4, cudaMemcpyHostToDevice));
+  CUDA_TRY(cudaMemcpy(c->step.launches, &launches, 4, cudaMemcpyHostToDevice));
+  *h_status = (int32_t)after;
+  return 0;
 }
 
 extern "C" int32_t femto_decoder_step(femto_handle* h, femto_kv_cache* c, const float* theta, const int32_t* tokens, int32_t B, int32_t T,

@@ -717,8 +717,12 @@ int decode_step_run(const femto_handle* h, const DecodeStepState& st, DecodeStep
   int keys = 0;
   for (const LayerP& p : h->lp) keys = std::max(keys, std::min(a.t + 1, p.window + 1));
   a.splits = std::max(1, std::min({MAX_SPLITS, cdiv(keys, 64), st.blocks_n / (a.B * a.Hkv)}));
-  k_step_begin<<<a.B, THREADS, 0, s>>>(a, tokens, positions, h->cfg.index_base, h->V, h->cfg.max_document_tokens);
-  KERNEL_CHECK();
+  if (tokens) {
+    k_step_begin<<<a.B, THREADS, 0, s>>>(a, tokens, positions, h->cfg.index_base, h->V, h->cfg.max_document_tokens);
+    KERNEL_CHECK();
+  } else {      // the self test: words of a launch that nobody writes
+    CUDA_TRY(cudaMemsetAsync(st.launches + 1, 0x5a, 4, s));
+  }
   const int nt = a.B <= 8 ? 1 : 2, gmax = a.H / a.Hkv <= 2 ? 2 : 8;
   const size_t smem = smem_bytes(a.d, a.L, nt, gmax);
   a.red_bytes = (int)red_bytes(nt, gmax);

@@ -45,3 +45,4 @@ void decode_step_carve(const femto_handle* h, char*& p, DecodeStepState& st);
 int decode_step_setup(const femto_handle* h, DecodeStepState& st, const std::vector<void*>& K, const std::vector<void*>& V);
 int decode_step_run(const femto_handle* h, const DecodeStepState& st, DecodeStepArgs a, const int* tokens, const int* positions, cudaStream_t s,
                     bool* ran);      // false: the launch was refused and nothing of the cache has changed
+// (tokens NULL: the step alone, waiting for what k_step_begin would have left; see femto_selftest_decode_wait)

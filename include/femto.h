@@ -449,6 +449,11 @@ int64_t femto_launch_count(femto_handle* h);
  * waiting on the same barrier must leave through the abort flag, and the kernel must return by itself:
  * h_result2[0] = waiter timed out, h_result2[1] = second role unwound.  Nothing traps or hangs. */
 int32_t femto_selftest_bounded_wait(int32_t polls, int32_t* h_status, int32_t* h_result2);
+/* The same of a bf16 GPT's decode kernel: one token (as femto_decode_step), then the kernel once more without the one that feeds it, so
+ * that its blocks poll words that nobody writes.  They give up after about a second, raise status bit 2 (*h_status; the handle's own word
+ * stays as it was) and return by themselves; the cache goes on where it was. */
+int32_t femto_selftest_decode_wait(femto_handle* h, femto_kv_cache* c, const float* theta, const int32_t* tokens, int32_t B,
+                                   float* logits_out, void* stream, int32_t* h_status);
 
 /* Measurement aid (no counterpart in the reference): when enabled, every launch of the tensor-core
  * GEMM kernel is bracketed by CUDA events on its stream; the report returns the summed kernel time,

@@ -1,4 +1,5 @@
 """GPU parity of the whole training step through the C ABI against the CPU oracle."""
+import ctypes as C
 import hashlib
 import os
 
@@ -525,6 +526,25 @@ def test_decode_step_with_fewer_blocks_than_multiprocessors(blocks):
     for t in range(80, 90):
         if t == 85:
             _lib.lib().femto_kv_cache_blocks(kc.c, n)
+        z = fb.decode_step(model, kc, tok[:, t]).cpu()
+        assert (z - ref[:, t]).abs().max() <= 2.5e-2 * float(ref.abs().max()), t
+    kc.close()
+
+
+@pytest.mark.gpu
+def test_decode_kernel_gives_up_on_words_that_never_come():
+    """The polls of the resident decode kernel are bounded: without the kernel that feeds it, it raises the timeout bit and returns, and
+    the next token is right again."""
+    model, tok, pos, ref = _bf16_server(2, 4, 2, 2, 40, False)
+    st = model.state(2)
+    kc = fb.KVCache(st, 2, 40)
+    fb.prefill(model, kc, tok[:, :30], pos[:, :30])
+    z = torch.empty(2, 1000, device="cuda")
+    status = C.c_int32(0)
+    held = tok[:, 30].contiguous().cuda()
+    _lib.check(_lib.lib().femto_selftest_decode_wait(st.h, kc.c, _lib.ptr(model.params.theta), _lib.ptr(held), 2, _lib.ptr(z), None, C.byref(status)))
+    assert status.value & 2 and st.status_word() == 0 and len(kc) == 31
+    for t in range(31, 36):
         z = fb.decode_step(model, kc, tok[:, t]).cpu()
         assert (z - ref[:, t]).abs().max() <= 2.5e-2 * float(ref.abs().max()), t
     kc.close()
