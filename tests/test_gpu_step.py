@@ -550,6 +550,23 @@ def test_decode_kernel_gives_up_on_words_that_never_come():
     kc.close()
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("B,H,G,Tp,T", [
+    (1, 2, 1, 317, 326),           # five key ranges, then six: the ranges are added four at a time
+    (1, 1, 1, 2040, 2056),         # the cap of 32 ranges
+    (16, 8, 8, 60, 68), (16, 8, 8, 125, 132),      # one range: its 64 or 128 keys in flight are full, the new key is the first of the next
+    (8, 8, 8, 250, 262),           # two ranges, the same at their edge
+    (16, 4, 4, 125, 132)])
+def test_decode_step_at_the_edges_of_its_key_ranges(B, H, G, Tp, T):
+    model, tok, pos, ref = _bf16_server(B, H, G, 2, T, False, vocab=200)
+    kc = fb.KVCache(model.state(B), B, T)
+    fb.prefill(model, kc, tok[:, :Tp], pos[:, :Tp])
+    for t in range(Tp, T):
+        z = fb.decode_step(model, kc, tok[:, t]).cpu()
+        assert (z - ref[:, t]).abs().max() <= 2.5e-2 * float(ref.abs().max()), t
+    kc.close()
+
+
 def test_generate_with_cache_equals_generate_by_recompute():
     """`generate` (src/generation.jl:26-56): greedy decoding (temperature 0) through the cache gives the tokens of
     the reference's recompute-everything loop; with sampling the same generator state gives the same tokens."""
