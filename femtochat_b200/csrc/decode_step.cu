@@ -702,6 +702,7 @@ int decode_step_setup(const femto_handle* h, DecodeStepState& st, const std::vec
   CUDA_TRY(cudaMemcpy(st.blocks, bl.data(), sizeof(DecodeBlock) * bl.size(), cudaMemcpyHostToDevice));
   CUDA_TRY(cudaMemset(st.launches, 0, st.named_bytes));      // no word has a name yet
   CUDA_TRY(cudaMemcpy(st.maps, maps.data(), sizeof(CUtensorMap) * maps.size(), cudaMemcpyHostToDevice));
+  CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));      // the caller's stream may be one that does not wait for the legacy stream
   return 0;
 }
 
