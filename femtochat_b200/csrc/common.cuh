@@ -123,6 +123,7 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 // everything else out of L2 from token to token, a load after the wait costs 1 us from memory and a third of that from L2.
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 __device__ __forceinline__ void prefetch_l2(const void* p, long long bytes, int thread, int threads) {
+  if (bytes <= 0) return;      // a split without keys: p may lie past the end
   const char* first = reinterpret_cast<const char*>(reinterpret_cast<uintptr_t>(p) & ~(uintptr_t)127);
   const char* end = reinterpret_cast<const char*>(p) + bytes;
   for (const char* at = first + 128ll * thread; at < end; at += 128ll * threads) prefetch_l2(at < reinterpret_cast<const char*>(p) ? p : at);
