@@ -772,7 +772,6 @@ __global__ void __launch_bounds__(256) k_xent_rows(const float* __restrict__ log
   }
 }
 
-// dst [D][D+2kv] <- wq [D][D] | wk [D][kv] | wv [D][kv]
 // The compute-type copy of every weight in one launch: blocks of CAST_BLOCK elements, each of one job of the table.  Bound by HBM (4 bytes
 // in, 2 out per weight); one launch per tensor with one element per thread and step reached 3.7 TB/s, this 7.0 (d20: 1.55 -> 0.81 ms).
 template <typename T>
