@@ -260,7 +260,8 @@ template <> int attention_fwd<float>(const AttnArgs& a, cudaStream_t s) { return
 template <> int attention_bwd<float>(const AttnArgs& a, cudaStream_t s) { return attention_bwd_simt<float>(a, s); }
 // A training step whose length does not fill the 128-row tiles stays with these kernels, forward and reverse: they keep P and dS in
 // fp32, where the tensor cores multiply bf16 parts of them.  The difference is below a bf16 rounding of O, but a training step
-// magnifies it: single elements of a table's gradient by more than the rms of the table after a few updates.
+// magnifies it: single elements of a table's gradient by more than the rms of the table after a few updates.  (5 x 1000 tokens, 6 heads:
+// 1.7 ms forward, 2.0 and 2.3 reverse here; 0.03, 0.03 and 0.05 on the tensor cores.)
 template <> int attention_fwd<bf16>(const AttnArgs& a, cudaStream_t s) {
   if (attention_tc_supported(a) && (attention_whole_tiles(a) || !a.reverse_follows)) return attention_fwd_tc(a, s);
   return attention_fwd_simt<bf16>(a, s);

@@ -2,8 +2,10 @@
 // (src/generation.jl:26-56; "TODO" at src/gpt.jl:81): here the prompt is run once through the ordinary forward
 // pass, which leaves the post-RoPE, post-QK-norm keys and the gated values of every block in a per-layer cache,
 // and each further token runs a one-row-per-column forward (src/gpt.jl:129-170) whose attention reads that cache.
-// The decode step is bound by HBM: every weight is read once per token, so the matrix products are a
-// weight-streaming kernel (no tensor cores: M is the number of batch columns) and attention is a split-key kernel.
+// The decode step is bound by HBM: every weight is read once per token.  bf16 models with heads of 128 channels, up to 16 columns,
+// take one resident kernel for it (decode_step.cu).  Everything else, and a step whose launch is refused, takes the chain of kernels
+// below: the matrix products are a weight-streaming kernel (no tensor cores: M is the number of batch columns) and attention
+// is a split-key kernel.
 #include <algorithm>
 #include <vector>
 
