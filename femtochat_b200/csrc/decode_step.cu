@@ -12,7 +12,7 @@
 // reads until the name is right.  A store and a load carry a value across, where data, a fence, a counter and a poll (the
 // first form of this kernel) took 2 us a phase and 328 us a token of d12, 1136 us of eight columns of d20.  No buffer is
 // written again before its readers of the layer before are done, since every phase needs all of the one before it.
-// Measured a token, chain of launches -> now: d12, one column 1150 -> 210 us; d20, eight columns of 540 tokens 2600 -> 970 us.
+// Measured a token, chain of launches -> now: d12, one column 1150 -> 204 us; d20, eight columns of 540 tokens 2600 -> 873 us.
 //
 // Shares: an item is 64 output columns times d rows of a matrix, so that QKV, wo and fc have N / 64 items and proj four times
 // d / 64 (its four partial sums are added, in order, by the block that has the first).  Items go round the blocks without a restart

@@ -3,8 +3,8 @@
 // take (row pitches that are not multiples of 16 bytes, e.g. the 12 -> n_kv_head gate).
 //
 // Every result is one chain of multiply-adds over k = 0, 1, ... in order, whatever the tile: a training step's results then are
-// the same bits at every tile size.  (K shared by the blocks of a cluster, partial sums added at the end, was as near to 64 bits, but over a
-// dozen updates of the same weights two orders of summation drift 1e-4 apart.)
+// the same bits at every tile size.  (K shared by the blocks of a cluster, partial sums added at the end, was nearer to 64 bits, 5e-7 against 1.1e-6
+// over a step, but over a dozen updates of the same weights two orders of summation drift 1e-4 apart.)
 //
 // 64 threads have a W x W tile, 8 x 8 (W = 64) or 4 x 4 (32) results each as pairs (two multiply-adds an instruction): at 64 a step of k
 // takes 32 of those for four 16-byte loads from shared memory, which bound it.  The next steps of k are in registers while these run.
