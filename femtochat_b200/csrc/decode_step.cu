@@ -8,35 +8,41 @@
 // MLP down - passes from block to block.  (Copies issued by the eight computing warps themselves, cp.async, held up their loads of
 // activations: 400 us a token, d12.)
 //
-// What a phase leaves goes to global memory as words of 8 bytes, 4 of data and 4 that name the launch and the layer; who needs it
-// reads until the name is right.  A store and a load carry a value across, where data, a fence, a counter and a poll (the
+// What a phase leaves goes to global memory as words that carry a name, the launch and the layer, beside their data: 4 bytes of data in 8
+// (fp32 values that few read), 12 in 16 (the bf16 rows that every block reads; 16 bytes an access asked L2 half as often as 8 did).  Who
+// needs a word reads until its name is right.  A store and a load carry a value across, where data, a fence, a counter and a poll (the
 // first form of this kernel) took 2 us a phase and 328 us a token of d12, 1136 us of eight columns of d20.  No buffer is
 // written again before its readers of the layer before are done, since every phase needs all of the one before it.
-// Measured a token, chain of launches -> now: d12, one column 1150 -> 204 us; d20, eight columns of 540 tokens 2600 -> 873 us.
+// With many words a phase is waited for by ONE thread of a block, on a count of finished items that has no order of its own, and the
+// words are read once it says that they should be there: 148 blocks that polled 30 KB each kept the words from arriving, 5 to 11 us a
+// phase (d20, eight columns).  With few, a warp polls its first word and then reads the rest.
+// Measured a token: d12, one column, chain of launches 1150 us, named words of 8 bytes and 64-column items 204, now 179; d20, eight columns
+// of 540 tokens 2600, 873, 650.  Of a layer's 30 us there (6 would stream its weights), 1.9 are the read of the rows in each of four
+// phases, 1.4 to 2 each product, 5 the attention; 12 blocks have two items of the MLP's 160, which costs 4.
 //
-// Shares: an item is 64 output columns times d rows of a matrix, so that QKV, wo and fc have N / 64 items and proj four times
-// d / 64 (its four partial sums are added, in order, by the block that has the first).  Items go round the blocks without a restart
+// Shares: an item is 32 output columns times d rows of a matrix, so that QKV, wo and fc have N / 32 items and proj four times
+// d / 32 (its four partial sums are added, in order, by the block that has the first).  (64 columns left 108 of 148 blocks without a part
+// of QKV, 128 of wo.)  Items go round the blocks without a restart
 // from product to product, which balances the stream.  The rows of X are the 8-column operand of mma.m16n8k16, the
-// weights its 16-row operand: a lane takes 8 columns of the four rows of W that are its own in the fragment, and byte
-// permutations make the (k, k+1) pairs.  RMS norms have no weights here, so the reciprocal root multiplies the product.
+// weights its 16-row operand, turned by ldmatrix on its way from the ring.  RMS norms have no weights here, so the reciprocal root
+// multiplies the product.
 #include <algorithm>
 
 #include "decode_step.cuh"
+#include "named_words.cuh"
 #include "sm100_ptx.cuh"
 #include "warp_mma.cuh"
 
 namespace {
 
-constexpr int THREADS = 256, WARPS = 8, SLOT = 128 * 64 * 2,      // computing threads; a slot of the ring: 128 rows of 64 columns
-              HD = 128, MAX_SPLITS = 32;
-constexpr int RED_PITCH = 66;      // floats per fragment register pair of a warp's sums; 66: a column's eight land in eight banks
+constexpr int THREADS = 256, WARPS = 8, HD = 128, MAX_SPLITS = 32;      // computing threads
+constexpr int TILE = 32;           // columns of an item
+constexpr int RED_PITCH = 36;      // floats of a warp's sums of one row; 36: the four rows that eight lanes each store land in 32 banks
 constexpr int SPIN_LIMIT = 1 << 20;
+// How many items of a kind the step has finished, counted without order beside the words themselves: see rows_of
+// (what QKV and head read, QKV, attention, what the MLP reads, four quarters of its inside, its partial sums)
+enum { HINT_ROWS, HINT_QKV, HINT_ATT, HINT_MID, HINT_UP, HINT_PART = HINT_UP + 4, HINTS };
 
-__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t s) {
-  uint32_t r;
-  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(s));
-  return r;
-}
 // Words that carry their name, straight from and to L2.  Each is ONE 64-bit scalar, which the memory model never tears: a vector of
 // 32-bit elements is several accesses without order, and a reader could see the new name beside the old data.  (Two words a load: a
 // vector of two such scalars, each with a name of its own.)
@@ -54,6 +60,12 @@ __device__ __forceinline__ uint2 named_load(const uint2* p) {
 __device__ __forceinline__ void named_store(uint2* p, uint32_t data, uint32_t name) {
   asm volatile("{\n\t.reg .b64 a;\n\tmov.b64 a, {%1, %2};\n\tst.relaxed.gpu.global.b64 [%0], a;\n\t}" ::"l"(p), "r"(data), "r"(name) : "memory");
 }
+// 16 columns of a row are three words: columns 0 to 5, 6 to 11, and 12 to 15 (its third pair is not used).  A row has a word more than it
+// needs, in memory and in shared memory, where the words are copied as they are: the rows then start in different banks.
+__host__ __device__ constexpr int words_of(int columns) { return columns / 16 * 3; }
+__host__ __device__ constexpr int pitch_of(int d) { return words_of(d) + 1; }
+// where pair i of 16 columns is, in 32-bit units
+__device__ __forceinline__ int place(int i) { return i / 3 * 4 + i % 3; }
 __device__ __forceinline__ void named_store(uint2* p, float data, uint32_t name) { named_store(p, __float_as_uint(data), name); }
 __device__ __forceinline__ float lo_f(uint32_t p) { return __uint_as_float(p << 16); }
 __device__ __forceinline__ float hi_f(uint32_t p) { return __uint_as_float(p & 0xffff0000u); }
@@ -63,11 +75,6 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
 }
 // The computing warps only
 __device__ __forceinline__ void compute_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
-// Rows of X are permuted within every 16 columns so that the four a lane needs (2 c, 2 c + 1, 2 c + 8, 2 c + 9) lie together
-__device__ __forceinline__ void put4(bf16* row, int col, uint32_t lo, uint32_t hi) {      // col: a multiple of 4
-  uint32_t* w = reinterpret_cast<uint32_t*>(row + (col & ~15)) + (col & 4) + ((col >> 3) & 1);
-  w[0] = lo; w[2] = hi;
-}
 
 // ---- the new token of every column: its id and position, normalised embedding and smear, and the first block's mixed stream ----
 // launches[0] counts the launches so far, launches[1] is this one's number for the blocks of the step.  What the cache keeps from
@@ -78,6 +85,7 @@ __global__ void __launch_bounds__(THREADS) k_step_begin(const DecodeStepArgs a, 
   const int b = blockIdx.x, tid = threadIdx.x;
   const uint32_t launch = a.launches[0] + 1, name = launch * (a.L + 1) + 1;
   if (b == 0 && tid == 0) a.launches[1] = launch;
+  if (b == 0 && tid < HINTS) a.hints[tid * 32] = 0;
   int tk = tokens[b] - base;
   bool bad = tk < 0 || tk >= vocab;
   tk = min(max(tk, 0), vocab - 1);
@@ -124,29 +132,36 @@ __global__ void __launch_bounds__(THREADS) k_step_begin(const DecodeStepArgs a, 
       x[i] *= mix;
       named_store(a.xm + at, x[i], name);
     }
-    named_store(a.xn + ((long long)b * a.d + c) / 2, pack2(x[0], x[1]), name);
+    const uint32_t w0 = pack2(x[0], x[1]), w1 = __shfl_down_sync(0xffffffffu, w0, 1), w2 = __shfl_down_sync(0xffffffffu, w0, 2);   // whole warps: d / 2 is a multiple of 64
+    if ((tid & 7) % 3 == 0) named_store(a.xn + (long long)b * pitch_of(a.d) + words_of(c) + (tid & 7) / 3, w0, w1, w2, name);
   }
 }
 
+constexpr int slot_bytes(int ks) { return 128 * ks * TILE * 2; }
+constexpr int MAX_RING = 20, MIN_RING = 4;
+
 // ---- the step ----------------------------------------------------------------------------------------------------------
-template <int NT, int GMAX, int RING>
+// KS: steps of 16 rows that a warp has of a slot of the ring, which is 8 KS x 16 rows of a tile
+template <int NT, int GMAX, int KS>
 __global__ void __launch_bounds__(THREADS + 128, 1) k_decode_step(const DecodeStepArgs a) {
   extern __shared__ __align__(1024) unsigned char smem[];
+  constexpr int SLOT = slot_bytes(KS);
+  const int RING = a.ring;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, c = lane & 3, cta = blockIdx.x, grid = gridDim.x;
-  const int d = a.d, B = a.B, xp = d + 16;        // 16: the eight rows of an 8-byte fragment load fall into different banks
+  const int d = a.d, B = a.B, pitch = pitch_of(d);
   unsigned char* ring = smem;
-  bf16* X = reinterpret_cast<bf16*>(smem + RING * SLOT);
-  float* red = reinterpret_cast<float*>(X + 8 * NT * xp);
+  uint4* X = reinterpret_cast<uint4*>(smem + RING * SLOT);
+  float* red = reinterpret_cast<float*>(X + 8 * NT * pitch);
   const DecodeBlock* blocks = reinterpret_cast<const DecodeBlock*>(reinterpret_cast<unsigned char*>(red) + a.red_bytes);
-  __shared__ float ssp[8 * NT][33], inv_s[8 * NT], qs[GMAX][HD], kvs[2][HD];
+  __shared__ float ssp[8 * NT][WARPS + 1], inv_s[8 * NT], qs[GMAX][HD], kvs[2][HD];
   const uint32_t launch = a.launches[1];
   __shared__ int given_up;
-  __shared__ uint64_t full[RING], empty[RING];
-  const int steps = d >> 7, np = 4 * a.L + 1;
-  const int4 items = make_int4(a.dq >> 6, d >> 6, d >> 4, d >> 4);      // QKV, wo, fc, proj (a quarter of its rows each)
+  __shared__ uint64_t full[MAX_RING], empty[MAX_RING];
+  const int slots = d / (128 * KS), np = 4 * a.L + 1;
+  const int4 items = make_int4(a.dq / TILE, d / TILE, 4 * d / TILE, 4 * d / TILE);      // QKV, wo, fc, proj (a quarter of its rows each)
   const int per_block = items.x + items.y + items.z + items.w;
   // the matrix p of the step and the first of its items that is this block's
-  auto items_of = [&](int p) { const int k = p & 3; return p == np - 1 ? a.Vp >> 6 : k == 0 ? items.x : k == 1 ? items.y : k == 2 ? items.z : items.w; };
+  auto items_of = [&](int p) { const int k = p & 3; return p == np - 1 ? a.Vp / TILE : k == 0 ? items.x : k == 1 ? items.y : k == 2 ? items.z : items.w; };
   auto first_item = [&](int p) {
     const int k = p & 3, before = (p >> 2) * per_block + (k > 0 ? items.x : 0) + (k > 1 ? items.y : 0) + (k > 2 ? items.z : 0);
     const int j = cta - before % grid;
@@ -157,7 +172,7 @@ __global__ void __launch_bounds__(THREADS + 128, 1) k_decode_step(const DecodeSt
     uint32_t* dst = const_cast<uint32_t*>(reinterpret_cast<const uint32_t*>(blocks));
     for (int i = tid; i < a.L * (int)sizeof(DecodeBlock) / 4; i += THREADS + 128) dst[i] = src[i];
   }
-  for (int i = tid; i < 8 * NT * xp / 2; i += THREADS + 128) reinterpret_cast<uint32_t*>(X)[i] = 0;   // rows from B on stay zero
+  for (int i = tid; i < 8 * NT * pitch; i += THREADS + 128) X[i] = make_uint4(0, 0, 0, 0);   // rows from B on stay zero
   if (tid == 0) {
     if (cta == 0) a.launches[0] = launch;
     given_up = 0;
@@ -173,13 +188,13 @@ __global__ void __launch_bounds__(THREADS + 128, 1) k_decode_step(const DecodeSt
     if (warp > WARPS || lane) return;
     int n = 0, slot = 0, turn = 0;
     for (int p = 0; p < np; p++) {
-      const int tiles = (p & 3) == 3 ? d >> 6 : 1 << 30;
+      const int tiles = (p & 3) == 3 ? d / TILE : 1 << 30;
       for (int j = first_item(p); j < items_of(p); j += grid) {
         const int ks = j / tiles, tile = j - ks * tiles;
-        for (int s = 0; s < steps; s++) {
+        for (int s = 0; s < slots; s++) {
           if (turn && !sm100::mbar_wait(&empty[slot], (turn & 1) ^ 1, &given_up, a.status)) goto done;
           sm100::mbar_expect_tx(&full[slot], SLOT);
-          sm100::tma_load_2d(ring + slot * SLOT, a.maps + p, &full[slot], tile * 64, ks * d + s * 128);
+          sm100::tma_load_3d(ring + slot * SLOT, a.maps + p, &full[slot], tile * TILE, ks * d + s * 128 * KS, 0);
           n++;
           if (++slot == RING) { slot = 0; turn++; }
         }
@@ -207,103 +222,143 @@ __global__ void __launch_bounds__(THREADS + 128, 1) k_decode_step(const DecodeSt
     until([&] { v = named_load(p); return v.y == name; });
     return __uint_as_float(v.x);
   };
-  // One item: sums of this warp's steps over the ring, then over the warps in order; out(b, column, sum, what before(b, column) gave).
-  // A warp has 32 neighbouring columns of one row at a time.
-  auto product = [&](int tile, bool normed, auto&& before, auto&& out) {
-    float acc[4][NT][4] = {}, aux[2 * NT];
-#pragma unroll
-    for (int k = 0; k < 2 * NT; k++) {
-      const int o = tid + k * THREADS;
-      aux[k] = o < 64 * B ? before(o >> 6, tile * 64 + (o & 63)) : 0.f;
-    }
-    const bf16* xr = X + g * xp + warp * 16 + 4 * c;
-    // this lane's rows 2 c, 2 c + 1, 2 c + 8, 2 c + 9 of the warp's 16, 16-byte unit g of each where the 128-byte swizzle put it
-    const unsigned char* wl = ring + (warp * 16 + 2 * c) * 128;
-    const int u0 = (g ^ (2 * c)) * 16, u1 = (g ^ (2 * c + 1)) * 16;
-    auto step = [&](const uint4 (&w)[4], const uint2 (&x)[NT]) {
-      const uint32_t* w0 = &w[0].x; const uint32_t* w1 = &w[1].x; const uint32_t* w2 = &w[2].x; const uint32_t* w3 = &w[3].x;
-#pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const uint32_t f[4] = {prmt(w0[j], w1[j], 0x5410), prmt(w0[j], w1[j], 0x7632), prmt(w2[j], w3[j], 0x5410), prmt(w2[j], w3[j], 0x7632)};
-#pragma unroll
-        for (int t = 0; t < NT; t++) mma16816(acc[j][t], f, x[t].x, x[t].y);
-      }
-    };
-    auto fetch = [&](int s, uint4 (&w)[4], uint2 (&x)[NT]) {
+  // One item: sums of this warp's steps over the ring, then over the warps in order; out(k, b, column, sum).
+  // A warp has the 32 columns of one row b = warp + 8 k at a time.  `normed`: times the reciprocal root of the row's mean square, which the warps
+  // sum from the pieces of X that they multiply.
+  auto product = [&](int tile, bool normed, auto&& out) {
+    float acc[2][NT][4] = {}, ss[NT] = {};
+    const uint32_t* xr = reinterpret_cast<const uint32_t*>(X + g * pitch + warp * KS * 3);      // pairs c and c + 4 of every 16 columns
+    const int p0 = place(c), p1 = place(c + 4);
+    // this lane's row of a 16 x 16 piece, and its 16-byte unit of either piece where the 64-byte swizzle put it
+    const int row = warp * 16 * KS + (lane & 7) + ((lane >> 4) << 3), unit = (lane >> 3) & 1, turned = (row >> 1) & 3;      // 16 rows further: the same turn
+    const unsigned char* wl = ring + row * 64;
+    const int u0 = (unit ^ turned) * 16, u1 = ((2 + unit) ^ turned) * 16;
+    auto fetch = [&](int s, uint32_t (&f)[KS][2][4], uint2 (&x)[KS][NT]) {
       sm100::mbar_wait(&full[slot], parity, &given_up, a.status);
       const unsigned char* q = wl + slot * SLOT;
-      w[0] = *reinterpret_cast<const uint4*>(q + u0);        w[1] = *reinterpret_cast<const uint4*>(q + 128 + u1);
-      w[2] = *reinterpret_cast<const uint4*>(q + 1024 + u0); w[3] = *reinterpret_cast<const uint4*>(q + 1152 + u1);
 #pragma unroll
-      for (int t = 0; t < NT; t++) x[t] = *reinterpret_cast<const uint2*>(xr + 8 * t * xp + s * 128);
+      for (int k = 0; k < KS; k++) {
+        ldsm4t(f[k][0], q + k * 1024 + u0);
+        ldsm4t(f[k][1], q + k * 1024 + u1);
+#pragma unroll
+        for (int t = 0; t < NT; t++) {
+          const uint32_t* w = xr + (8 * t * pitch + (s * 8 * KS + k) * 3) * 4;
+          x[k][t] = make_uint2(w[p0], w[p1]);
+        }
+      }
       __syncwarp();
       if (lane == 0) sm100::mbar_arrive(&empty[slot]);
       if (++slot == RING) { slot = 0; parity ^= 1; }
     };
+    auto multiply = [&](const uint32_t (&f)[KS][2][4], const uint2 (&x)[KS][NT]) {
+#pragma unroll
+      for (int k = 0; k < KS; k++)
+#pragma unroll
+        for (int t = 0; t < NT; t++) {
+#pragma unroll
+          for (int i = 0; i < 2; i++) mma16816(acc[i][t], f[k][i], x[k][t].x, x[k][t].y);
+          if (!normed) continue;
+          const float e = lo_f(x[k][t].x), h = hi_f(x[k][t].x), u = lo_f(x[k][t].y), v = hi_f(x[k][t].y);
+          ss[t] += (e * e + h * h) + (u * u + v * v);
+        }
+    };
     int s = 0;
-    for (; s + 2 <= steps; s += 2) {
-      uint4 w[2][4];
-      uint2 x[2][NT];
-      fetch(s, w[0], x[0]);
-      fetch(s + 1, w[1], x[1]);
-      step(w[0], x[0]);
-      step(w[1], x[1]);
+    for (; s + 2 <= slots; s += 2) {
+      uint32_t f[2][KS][2][4];
+      uint2 x[2][KS][NT];
+      fetch(s, f[0], x[0]);
+      fetch(s + 1, f[1], x[1]);
+      multiply(f[0], x[0]);
+      multiply(f[1], x[1]);
     }
-    if (s < steps) {
-      uint4 w[4];
-      uint2 x[NT];
-      fetch(s, w, x);
-      step(w, x);
+    if (s < slots) {
+      uint32_t f[KS][2][4];
+      uint2 x[KS][NT];
+      fetch(s, f, x);
+      multiply(f, x);
     }
-    // register pair (j, i, t): column 8 g + 2 j + i of rows 8 t + 2 c and 8 t + 2 c + 1
+    // registers (i, t): columns 16 i + g and 16 i + g + 8 of rows 8 t + 2 c and 8 t + 2 c + 1
 #pragma unroll
-    for (int j = 0; j < 4; j++)
+    for (int i = 0; i < 2; i++)
 #pragma unroll
-      for (int i = 0; i < 2; i++)
+      for (int t = 0; t < NT; t++)
 #pragma unroll
-        for (int t = 0; t < NT; t++)
-          *reinterpret_cast<float2*>(red + ((warp * 8 + 2 * j + i) * NT + t) * RED_PITCH + 2 * lane) = make_float2(acc[j][t][2 * i], acc[j][t][2 * i + 1]);
-    if (normed && tid < B) {
-      float ss = 0.f;
-      for (int i = 0; i < steps; i++) ss += ssp[tid][i];
-      inv_s[tid] = 1.f / sqrtf(ss / d + a.eps);
+        for (int e = 0; e < 4; e++) red[((warp * NT + t) * 8 + 2 * c + (e & 1)) * RED_PITCH + 16 * i + g + 8 * (e >> 1)] = acc[i][t][e];
+    if (normed) {
+#pragma unroll
+      for (int t = 0; t < NT; t++) {
+        ss[t] += __shfl_xor_sync(0xffffffffu, ss[t], 1);
+        ss[t] += __shfl_xor_sync(0xffffffffu, ss[t], 2);
+        if (c == 0) ssp[8 * t + g][warp] = ss[t];
+      }
     }
     compute_sync();
 #pragma unroll
-    for (int k = 0; k < 2 * NT; k++) {
-      const int o = tid + k * THREADS, b = o >> 6, n = o & 63;
-      if (o >= 64 * B) break;
-      const float* p = red + ((n & 7) * NT + (b >> 3)) * RED_PITCH + (n >> 3) * 8 + (b & 7);
+    for (int k = 0; k < NT; k++) {
+      const int b = warp + 8 * k;
+      if (b >= B) break;
       float v = 0.f;
 #pragma unroll
-      for (int w = 0; w < WARPS; w++) v += p[w * 8 * NT * RED_PITCH];
-      out(b, tile * 64 + n, normed ? v * inv_s[b] : v, aux[k]);
+      for (int w = 0; w < WARPS; w++) v += red[(w * NT * 8 + b) * RED_PITCH + lane];
+      if (normed) {
+        float q = 0.f;
+#pragma unroll
+        for (int w = 0; w < WARPS; w++) q += ssp[b][w];
+        const float inv = rsqrtf(q * a.inv_d + a.eps);
+        if (lane == 0) inv_s[b] = inv;
+        v *= inv;
+      }
+      out(k, b, tile * TILE + lane, v);
     }
     compute_sync();
   };
-  auto nothing = [](int, int) { return 0.f; };
-  // two neighbouring columns of a row (neighbouring lanes) as one word of bf16
-  auto store_pair = [&](uint2* row, int col, float v, uint32_t name) {
-    const float w = __shfl_xor_sync(0xffffffffu, v, 1);
-    if (!(lane & 1)) named_store(row + (col >> 1), pack2(v, w), name);
+  auto finished = [&](int kind) {      // after the stores of all threads have been issued
+    if (tid == 0) count_one(a.hints + kind * 32);
   };
-  // Rows of X: d columns of every row of `src` (pairs; `pitch` words a row), with the sums of squares of every 128 columns.
-  // All loads of a thread are in flight together (10: eight rows of 1280; one or two in most steps of few columns).  Every round of
-  // polls writes every v: what it left as it was would stay in registers beside the new (700 bytes of spills, 16 us more a token of d12).
-  auto rows_of = [&](const uint2* src, int pitch, uint32_t name, bool squares) {
-    constexpr int U = 10;
-    for (int q0 = warp; q0 < B * steps; q0 += WARPS * U) {
+  // 32 neighbouring columns of a row, one a lane
+  auto store_row = [&](uint4* row, int col, float v, uint32_t name) {
+    const uint32_t w0 = pack2(v, __shfl_down_sync(0xffffffffu, v, 1)), w1 = __shfl_down_sync(0xffffffffu, w0, 2), w2 = __shfl_down_sync(0xffffffffu, w0, 4);
+    if ((lane & 15) % 6 == 0) named_store(row + words_of(col) + (lane & 15) / 6, w0, w1, w2, name);
+  };
+  // One thread waits until `count` items of a kind are done, so that the other 255, and all other blocks, do not keep asking L2 for
+  // words that nobody has written: that made a hand-over of eight rows of 1280 5 to 11 us long where 2 do (the more blocks waited, the
+  // longer).  The count carries no order: the words' names say what has arrived.
+  const bool counted = B * pitch > 2 * THREADS;
+  auto wait_for = [&](int kind, uint32_t count) {
+    if (!counted) return;
+    if (tid == 0) {
+      const unsigned int* p = a.hints + kind * 32;
+      for (int spin = 0; spin < SPIN_LIMIT >> 4; spin++) {
+        if (counted_so_far(p) >= count || ((spin & 63) == 63 && *(volatile int*)&given_up)) break;
+      }
+    }
+    compute_sync();
+  };
+  // Rows of X, all of `src`.  All loads of a thread are in flight together (8: eight rows of 1280 and a few; one in most steps of few columns).
+  // Every round of polls writes every v: what it left as it was would stay in registers beside the new (700 bytes of spills, 16 us more a
+  // token of d12).
+  auto rows_of = [&](const uint4* src, uint32_t name) {
+    constexpr int U = 8;
+    const int n = B * pitch, last = pitch - 1;      // (the word that a row has too much is nobody's)
+    for (int i0 = tid; i0 < n; i0 += THREADS * U) {
       uint4 v[U];
+      bool need[U];
+#pragma unroll
+      for (int u = 0; u < U; u++) need[u] = i0 + u * THREADS < n && (i0 + u * THREADS) % pitch != last;
+      if (!counted && need[0]) {
+        const int at = i0 & ~31;
+        const uint4* one = src + at + (at % pitch == last ? 1 : 0);
+        until([&] { return named_load(one).w == name; });
+      }
       until([&] {
         bool ok = true;
         auto ask = [&](int u) {
-          const int q = q0 + u * WARPS;
-          v[u] = make_uint4(0, name, 0, name);
-          if (q < B * steps) v[u] = named_load2(src + (long long)(q / steps) * pitch + q % steps * 64 + lane * 2);
-          ok &= v[u].y == name && v[u].w == name;
+          v[u] = make_uint4(0, 0, 0, name);
+          if (need[u]) v[u] = named_load(src + i0 + u * THREADS);
+          ok &= v[u].w == name;
         };
         ask(0); ask(1);
-        if (q0 + 2 * WARPS < B * steps) {
+        if (i0 - tid + 2 * THREADS < n) {
 #pragma unroll
           for (int u = 2; u < U; u++) ask(u);
         } else {
@@ -313,15 +368,8 @@ __global__ void __launch_bounds__(THREADS + 128, 1) k_decode_step(const DecodeSt
         return ok;
       });
 #pragma unroll
-      for (int u = 0; u < U; u++) {
-        const int q = q0 + u * WARPS;
-        if (q >= B * steps) break;
-        const int b = q / steps, k = q % steps;
-        put4(X + b * xp, k * 128 + lane * 4, v[u].x, v[u].z);
-        if (!squares) continue;
-        const float x = lo_f(v[u].x), y = hi_f(v[u].x), z = lo_f(v[u].z), w = hi_f(v[u].z), ss = warp_sum(x * x + y * y + z * z + w * w);
-        if (lane == 0) ssp[b][k] = ss;
-      }
+      for (int u = 0; u < U; u++)
+        if (need[u]) X[i0 + u * THREADS] = v[u];
     }
     compute_sync();
   };
@@ -333,14 +381,18 @@ __global__ void __launch_bounds__(THREADS + 128, 1) k_decode_step(const DecodeSt
     const uint32_t name = launch * (a.L + 1) + l + 1;
     // ---- norm, QKV ----
     if (int j = first_item(4 * l); j < items.x) {
-      rows_of(a.xn, d / 2, name, true);
+      wait_for(HINT_ROWS, l * (d / TILE));
+      rows_of(a.xn, name);
       const bool first = j == 0;
-      for (; j < items.x; j += grid)
-        product(j, true, nothing, [&](int b, int col, float v, float) { named_store(a.qkv + (long long)b * a.dq + col, v, name); });
+      for (; j < items.x; j += grid) {
+        product(j, true, [&](int, int b, int col, float v) { named_store(a.qkv + (long long)b * a.dq + col, v, name); });
+        finished(HINT_QKV);
+      }
       if (first)       // the first sixteen of the normalised row, for the gate of the value embeddings
         for (int i = tid; i < 16 * B; i += THREADS) {
-          const int b = i >> 4, k = i & 15, w = (k & 4) + ((k >> 3) & 1) + (k & 2);
-          named_store(a.h16 + i, __bfloat162float(X[b * xp + 2 * w + (k & 1)]) * inv_s[b], name);
+          const int b = i >> 4, k = i & 15;
+          const uint32_t pair = reinterpret_cast<const uint32_t*>(X + b * pitch)[place(k >> 1)];
+          named_store(a.h16 + i, (k & 1 ? hi_f(pair) : lo_f(pair)) * inv_s[b], name);
         }
       compute_sync();
     }
@@ -385,6 +437,7 @@ __global__ void __launch_bounds__(THREADS + 128, 1) k_decode_step(const DecodeSt
         if (lane < 12) wg = a.theta[blk.ve_gate + lane * a.Hkv + kvh];
       }
       cached(0);
+      wait_for(HINT_QKV, (l + 1) * items.x);
       // queries, and with the last range the new key and value: one warp a vector
       for (int v = warp; v < G + (last ? 2 : 0); v += WARPS) {
         const int col = v < G ? (kvh * G + v) * HD : d + (v - G) * a.kv + kvh * HD;
@@ -545,46 +598,68 @@ __global__ void __launch_bounds__(THREADS + 128, 1) k_decode_step(const DecodeSt
             L = L * f + __uint_as_float(ml[u].z) * e; v = v * f + __uint_as_float(ov[u].x) * e; M = mn;
           }
         }
-        store_pair(a.att + head * (HD / 2), ch, v / L, name);
+        store_row(a.att + (long long)b * pitch, (kvh * G + h) * HD + ch, v / L, name);
       }
       compute_sync();
+      if (sp == 0) finished(HINT_ATT);
     }
     // ---- output projection ----
     if (int j2 = first_item(4 * l + 1); j2 < items.y) {
-      rows_of(a.att, d / 2, name, false);
-      for (; j2 < items.y; j2 += grid)
-        product(j2, false, [&](int b, int col) { return word(a.xm + (long long)b * d + col, name); },
-                [&](int b, int col, float v, float x) {
-                  v += x;
-                  named_store(a.xa + (long long)b * d + col, v, name);
-                  store_pair(a.xa2 + (long long)b * d / 2, col, v, name);
-                });
+      float x[NT];      // the stream, on its way before the attention is waited for
+      auto stream = [&] {
+#pragma unroll
+        for (int k = 0; k < NT; k++) {
+          const int b = warp + 8 * k;
+          x[k] = b < B ? word(a.xm + (long long)b * d + j2 * TILE + lane, name) : 0.f;
+        }
+      };
+      wait_for(HINT_ROWS, l * (d / TILE));
+      stream();
+      wait_for(HINT_ATT, (l + 1) * B * a.Hkv);
+      rows_of(a.att, name);
+      for (;;) {
+        product(j2, false, [&](int k, int b, int col, float v) {
+          v += x[k];
+          named_store(a.xa + (long long)b * d + col, v, name);
+          store_row(a.xa2 + (long long)b * pitch, col, v, name);
+        });
+        finished(HINT_MID);
+        if ((j2 += grid) >= items.y) break;
+        stream();
+      }
     }
     // ---- norm, MLP up ----
     if (int j2 = first_item(4 * l + 2); j2 < items.z) {
-      rows_of(a.xa2, d / 2, name, true);
-      for (; j2 < items.z; j2 += grid)
-        product(j2, true, nothing, [&](int b, int col, float v, float) {
+      wait_for(HINT_MID, (l + 1) * (d / TILE));
+      rows_of(a.xa2, name);
+      for (; j2 < items.z; j2 += grid) {
+        product(j2, true, [&](int, int b, int col, float v) {
           v = fmaxf(v, 0.f);
-          store_pair(a.up + (long long)b * 2 * d, col, v * v, name);
+          const int ks = col / d;      // the same for the 32 columns
+          store_row(a.up + ((long long)ks * B + b) * pitch, col - ks * d, v * v, name);
         });
+        finished(HINT_UP + j2 / (d / TILE));
+      }
     }
     // ---- MLP down: a quarter of the inner rows an item ----
-    if (int j2 = first_item(4 * l + 3), tiles = d >> 6; j2 < items.w) {
+    if (int j2 = first_item(4 * l + 3), tiles = d / TILE; j2 < items.w) {
       const int first = j2;
       for (; j2 < items.w; j2 += grid) {
         const int ks = j2 / tiles;
-        rows_of(a.up + ks * (d / 2), 2 * d, name, false);
-        product(j2 - ks * tiles, false, nothing, [&](int b, int col, float v, float) { named_store(a.part + ks * Bd + (long long)b * d + col, v, name); });
+        wait_for(HINT_UP + ks, (l + 1) * tiles);
+        rows_of(a.up + ks * (long long)B * pitch, name);
+        product(j2 - ks * tiles, false, [&](int, int b, int col, float v) { named_store(a.part + ks * Bd + (long long)b * d + col, v, name); });
+        finished(HINT_PART);
       }
       // the stream after the block, by who had the first quarter of its columns: the next block's mix, or what the head reads
       const bool end = l + 1 == a.L;
       const float lb = end ? 0.f : a.theta[blocks[l + 1].lam_b], l0 = end ? -a.theta[a.off_lam_y] : a.theta[blocks[l + 1].lam_x0];
+      if (first < tiles) wait_for(HINT_PART, (l + 1) * items.w);
       for (int t = first; t < tiles; t += grid) {
 #pragma unroll
-        for (int k = 0; k < 2 * NT; k++) {
-          const int o = tid + k * THREADS, b = o >> 6, col = t * 64 + (o & 63);
-          if (o >= 64 * B) break;
+        for (int k = 0; k < NT; k++) {
+          const int b = warp + 8 * k, col = t * TILE + lane;
+          if (b >= B) break;
           const long long at = (long long)b * d + col;
           const float e = a.x0[at];
           uint2 w[5];
@@ -601,29 +676,30 @@ __global__ void __launch_bounds__(THREADS + 128, 1) k_decode_step(const DecodeSt
           if (l == a.backout && !end) named_store(a.xb + at, x, name);
           if (end) x += l0 * (l == a.backout ? x : word(a.xb + at, launch * (a.L + 1) + a.backout + 1));
           else { x = lb * x + l0 * e; named_store(a.xm + at, x, name + 1); }
-          store_pair(a.xn + (long long)b * d / 2, col, x, name + 1);
+          store_row(a.xn + (long long)b * pitch, col, x, name + 1);
         }
+        compute_sync();
+        finished(HINT_ROWS);
       }
     }
   }
   // ---- norm, head ----
-  if (int j = first_item(4 * a.L); j < a.Vp >> 6) {
-    rows_of(a.xn, d / 2, (launch + 1) * (a.L + 1), true);
-    for (; j < a.Vp >> 6; j += grid)
-      product(j, true, nothing, [&](int b, int col, float v, float) { if (col < a.V) a.logits[(long long)b * a.V + col] = 15.f * tanhf(v / 15.f); });
+  if (int j = first_item(4 * a.L); j < a.Vp / TILE) {
+    wait_for(HINT_ROWS, a.L * (d / TILE));
+    rows_of(a.xn, (launch + 1) * (a.L + 1));
+    for (; j < a.Vp / TILE; j += grid)
+      product(j, true, [&](int, int b, int col, float v) { if (col < a.V) a.logits[(long long)b * a.V + col] = 15.f * tanhf(v / 15.f); });
   }
 }
 
-template <int NT> constexpr int ring_of() { return NT == 1 ? 10 : 8; }
 size_t red_bytes(int nt, int gmax) { return std::max((size_t)4 * WARPS * 8 * nt * RED_PITCH, (size_t)4 * WARPS * gmax * (HD + 4)); }
-size_t smem_bytes(int d, int L, int nt, int gmax) {
-  return (size_t)(nt == 1 ? ring_of<1>() : ring_of<2>()) * SLOT + (size_t)8 * nt * (d + 16) * 2 + red_bytes(nt, gmax) + sizeof(DecodeBlock) * L;
-}
+size_t smem_bytes(int d, int L, int nt, int gmax) { return (size_t)8 * nt * pitch_of(d) * 16 + red_bytes(nt, gmax) + sizeof(DecodeBlock) * L; }      // beside the ring
 
 // blocks that stay on the device together, or 0.  The limit of dynamic shared memory belongs to the function and the device, not to
 // a model, so it is always set to all that a block may have: caches of several models decode in turn.
-template <int NT, int GMAX> int resident_blocks(size_t smem) {
-  auto kernel = k_decode_step<NT, GMAX, ring_of<NT>()>;
+// `ring`: slots that fit beside the rest, 160 KB of them at most (a share of the weights of two or three phases ahead).
+template <int NT, int GMAX, int KS> int resident_blocks(size_t smem, int& ring) {
+  auto kernel = k_decode_step<NT, GMAX, KS>;
   int per = 0, dev = 0, most = 0;
   cudaFuncAttributes fixed;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
@@ -632,16 +708,24 @@ template <int NT, int GMAX> int resident_blocks(size_t smem) {
     cudaGetLastError();
     return 0;
   }
-  if (smem + fixed.sharedSizeBytes > (size_t)most) return 0;
+  const long long left = most - (long long)fixed.sharedSizeBytes - (long long)smem;
+  ring = (int)std::min<long long>(left, 160 * 1024) / slot_bytes(KS);
+  if (left < 0 || ring < MIN_RING) return 0;
+  smem += (size_t)ring * slot_bytes(KS);
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, THREADS + 128, smem) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
   return per > 0 ? device_sm_count() : 0;
 }
-int resident(int nt, int gmax, size_t smem) {
-  if (nt == 1) return gmax == 2 ? resident_blocks<1, 2>(smem) : resident_blocks<1, 8>(smem);
-  return gmax == 2 ? resident_blocks<2, 2>(smem) : resident_blocks<2, 8>(smem);
+int steps_of(int d) { return d % 256 ? 1 : 2; }      // slots are 128 or 256 rows
+int resident(int nt, int gmax, int ks, size_t smem, int& ring) {
+  if (ks == 1) {
+    if (nt == 1) return gmax == 2 ? resident_blocks<1, 2, 1>(smem, ring) : resident_blocks<1, 8, 1>(smem, ring);
+    return gmax == 2 ? resident_blocks<2, 2, 1>(smem, ring) : resident_blocks<2, 8, 1>(smem, ring);
+  }
+  if (nt == 1) return gmax == 2 ? resident_blocks<1, 2, 2>(smem, ring) : resident_blocks<1, 8, 2>(smem, ring);
+  return gmax == 2 ? resident_blocks<2, 2, 2>(smem, ring) : resident_blocks<2, 8, 2>(smem, ring);
 }
 
 }  // namespace
@@ -650,10 +734,10 @@ int resident(int nt, int gmax, size_t smem) {
 // leave room for the ring (16 up to d = 2000 or so, 8 up to 3000); anything else takes the chain of kernels of decode.cu.
 void decode_step_plan(const femto_handle* h, int max_batch, DecodeStepState& st) {
   st.blocks_n = st.columns = 0;
-  if (!h->bf || h->hd != HD || (h->d & 127) || (h->Vp & 63) || h->H % h->Hkv || h->H / h->Hkv > 8 || h->d > 128 * 32) return;
+  if (!h->bf || h->hd != HD || (h->d & 127) || (h->Vp & (TILE - 1)) || h->H % h->Hkv || h->H / h->Hkv > 8 || h->d > 128 * 32) return;
   const int gmax = h->H / h->Hkv <= 2 ? 2 : 8;
   for (int nt = 1; nt <= (max_batch > 8 ? 2 : 1); nt++) {
-    const int n = resident(nt, gmax, smem_bytes(h->d, h->L, nt, gmax));
+    const int n = resident(nt, gmax, steps_of(h->d), smem_bytes(h->d, h->L, nt, gmax), st.ring[nt - 1]);
     if (!n) return;
     st.blocks_n = n; st.columns = std::min(max_batch, 8 * nt);
   }
@@ -671,9 +755,10 @@ void decode_step_carve(const femto_handle* h, char*& p, DecodeStepState& st) {
   take(st.maps, sizeof(CUtensorMap) * (4 * h->L + 1));
   take(st.blocks, sizeof(DecodeBlock) * h->L);
   char* first = p;
-  take(st.launches, 8);
-  take(st.xn, 4 * n * d); take(st.xm, 8 * n * d); take(st.xa, 8 * n * d); take(st.xa2, 4 * n * d); take(st.xb, 8 * n * d);
-  take(st.part, 32 * n * d); take(st.qkv, 8 * n * h->dq); take(st.h16, 8 * 16 * n); take(st.up, 16 * n * d); take(st.att, 4 * n * d);
+  take(st.launches, 8); take(st.hints, 128 * HINTS);
+  const size_t words = 16 * n * pitch_of(h->d);
+  take(st.xn, words); take(st.xm, 8 * n * d); take(st.xa, 8 * n * d); take(st.xa2, words); take(st.xb, 8 * n * d);
+  take(st.part, 32 * n * d); take(st.qkv, 8 * n * h->dq); take(st.h16, 8 * 16 * n); take(st.up, 4 * words); take(st.att, words);
   take(st.att_part, 8 * n * h->H * MAX_SPLITS * (HD + 2));
   st.named_bytes = p - first;
   take(st.x0, 4 * n * d);
@@ -682,11 +767,9 @@ void decode_step_carve(const femto_handle* h, char*& p, DecodeStepState& st) {
 int decode_step_setup(const femto_handle* h, DecodeStepState& st, const std::vector<void*>& K, const std::vector<void*>& V) {
   std::vector<CUtensorMap> maps;
   std::vector<DecodeBlock> bl;
-  auto put = [&](const void* W, int rows, int cols) {      // boxes of 128 rows and 64 columns: one slot of the ring
-    const uint64_t dims[2] = {(uint64_t)cols, (uint64_t)rows}, stride[1] = {(uint64_t)cols};
-    const uint32_t box[2] = {64, 128};
+  auto put = [&](const void* W, int rows, int cols) {      // boxes of 128 or 256 rows and 32 columns, 64-byte swizzle: one slot of the ring
     maps.emplace_back();
-    return make_tmap_nd_bf16(&maps.back(), W, 2, dims, stride, box);
+    return make_tmap_3d_bf16_sw(&maps.back(), W, cols, rows, 1, cols, 0, TILE, 128 * steps_of(h->d), 2);
   };
   for (int i = 0; i < h->L; i++) {
     const LayerBuf& l = h->lb[i];
@@ -707,7 +790,7 @@ int decode_step_setup(const femto_handle* h, DecodeStepState& st, const std::vec
 }
 
 int decode_step_run(const femto_handle* h, const DecodeStepState& st, DecodeStepArgs a, const int* tokens, const int* positions, cudaStream_t s, bool* ran) {
-  a.blocks = st.blocks; a.maps = st.maps; a.launches = st.launches; a.x0 = st.x0;
+  a.blocks = st.blocks; a.maps = st.maps; a.launches = st.launches; a.hints = st.hints; a.x0 = st.x0;
   a.xn = st.xn; a.xm = st.xm; a.xa = st.xa; a.xa2 = st.xa2; a.xb = st.xb; a.part = st.part; a.qkv = st.qkv; a.h16 = st.h16; a.up = st.up;
   a.att = st.att; a.att_part = st.att_part;
   a.wte = (const bf16*)h->sh_wte; a.sin_t = h->sin_t; a.cos_t = h->cos_t; a.status = h->status;
@@ -725,7 +808,8 @@ int decode_step_run(const femto_handle* h, const DecodeStepState& st, DecodeStep
     CUDA_TRY(cudaMemsetAsync(st.launches + 1, 0x5a, 4, s));
   }
   const int nt = a.B <= 8 ? 1 : 2, gmax = a.H / a.Hkv <= 2 ? 2 : 8;
-  const size_t smem = smem_bytes(a.d, a.L, nt, gmax);
+  a.ring = st.ring[nt - 1]; a.inv_d = 1.f / a.d;
+  const size_t smem = smem_bytes(a.d, a.L, nt, gmax) + (size_t)a.ring * slot_bytes(steps_of(a.d));
   a.red_bytes = (int)red_bytes(nt, gmax);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = st.blocks_n; cfg.blockDim = THREADS + 128; cfg.dynamicSmemBytes = smem; cfg.stream = s;
@@ -734,7 +818,7 @@ int decode_step_run(const femto_handle* h, const DecodeStepState& st, DecodeStep
   at[0].val.cooperative = 1;
   cfg.attrs = at; cfg.numAttrs = 1;
   cudaError_t e;
-#define LAUNCH(NT, GM) e = cudaLaunchKernelEx(&cfg, k_decode_step<NT, GM, ring_of<NT>()>, a)
+#define LAUNCH(NT, GM) e = steps_of(a.d) == 2 ? cudaLaunchKernelEx(&cfg, k_decode_step<NT, GM, 2>, a) : cudaLaunchKernelEx(&cfg, k_decode_step<NT, GM, 1>, a)
   if (nt == 1) { if (gmax == 2) LAUNCH(1, 2); else LAUNCH(1, 8); }
   else { if (gmax == 2) LAUNCH(2, 2); else LAUNCH(2, 8); }
 #undef LAUNCH

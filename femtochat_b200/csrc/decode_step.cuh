@@ -11,22 +11,24 @@
 struct DecodeBlock { bf16 *K, *V; const bf16* ve; long long lam_b, lam_x0, ve_gate; int window; };
 
 struct DecodeStepState {
+  int ring[2] = {0, 0};              // slots of its ring for up to 8 and up to 16 columns
   int blocks_n = 0, columns = 0;     // blocks of the kernel, and the columns it takes; 0: this model takes the chain of kernels
   CUtensorMap* maps = nullptr;       // four a block (QKV, wo, fc, proj), then the head
   DecodeBlock* blocks = nullptr;
-  unsigned int* launches = nullptr;
-  // Words of 8 bytes, data and name; [columns][width], a pair of bf16 a word (2) or one fp32 (4): what the QKV and the head read (2),
-  // the mixed stream (4), the stream after the attention (4, 2), the stream for the backout (4), four partial sums of the MLP (4),
-  // projections (4), the first 16 of the normalised row (4), MLP inner (2), attention (2) and its ranges (4: max, sum, channels)
-  uint2 *xn = nullptr, *xm = nullptr, *xa = nullptr, *xa2 = nullptr, *xb = nullptr, *part = nullptr, *qkv = nullptr, *h16 = nullptr,
-        *up = nullptr, *att = nullptr, *att_part = nullptr;
+  unsigned int *launches = nullptr, *hints = nullptr;      // hints: finished items by kind, 128 bytes apart
+  // Named words.  One fp32 in 8 bytes, [columns][width]: the mixed stream, the stream after the attention, the stream for the backout, four
+  // partial sums of the MLP, projections, the first 16 of the normalised row, ranges of the attention (max, sum, channels)
+  uint2 *xm = nullptr, *xa = nullptr, *xb = nullptr, *part = nullptr, *qkv = nullptr, *h16 = nullptr, *att_part = nullptr;
+  // Rows of bf16, three words of 16 bytes for 16 columns: what the QKV and the head read, what the MLP reads, its inside by quarters, attention
+  uint4 *xn = nullptr, *xa2 = nullptr, *up = nullptr, *att = nullptr;
   size_t named_bytes = 0;
   float* x0 = nullptr;               // embedding
 };
 
 struct DecodeStepArgs {
-  const CUtensorMap* maps; const DecodeBlock* blocks; unsigned int* launches;
-  uint2 *xn, *xm, *xa, *xa2, *xb, *part, *qkv, *h16, *up, *att, *att_part;
+  const CUtensorMap* maps; const DecodeBlock* blocks; unsigned int *launches, *hints;
+  uint2 *xm, *xa, *xb, *part, *qkv, *h16, *att_part;
+  uint4 *xn, *xa2, *up, *att;
   float* x0;
   const float* theta;
   const bf16* wte; bf16 *xe_prev, *xe_new;
@@ -35,8 +37,8 @@ struct DecodeStepArgs {
   float* logits;
   unsigned int* status;
   long long off_smear, off_lam_s, off_lam_y;
-  int d, dq, kv, H, Hkv, V, Vp, L, backout, B, t, maxT, docs, splits, red_bytes;
-  float eps;
+  int d, dq, kv, H, Hkv, V, Vp, L, backout, B, t, maxT, docs, splits, red_bytes, ring;
+  float eps, inv_d;
 };
 
 void decode_step_plan(const femto_handle* h, int max_batch, DecodeStepState& st);

@@ -80,6 +80,13 @@ def test_words_of_the_decode_step_are_single_accesses():
     assert len(accesses) == 3 and all(a.endswith(".b64") for a in accesses), accesses
 
 
+def test_wide_words_of_the_decode_step_are_single_accesses():
+    """The same for its words of 16 bytes: one 128-bit scalar."""
+    src = open(os.path.join(os.path.dirname(fb.__file__), "csrc", "named_words.cuh")).read()
+    accesses = re.findall(r"((?:ld|st)\.[a-z.]*global[a-z0-9.]*) ", src)
+    assert sorted(accesses) == ["ld.relaxed.gpu.global.b128", "ld.relaxed.gpu.global.u32", "st.relaxed.gpu.global.b128"], accesses
+
+
 def test_packed_batches_follow_loader_format():
     V, T, B = 4096, 256, 4
     pk = fb.PackedBatches(V, T, B, max_document_tokens=300, mean_doc_len=40, seed=1)
