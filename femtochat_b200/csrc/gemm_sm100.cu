@@ -261,65 +261,70 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     kb1 = min(p.kblocks, kb0 + p.kb_per_split);
   };
 
+  // The issuing warps run converged and one elected lane executes the instruction itself: addresses and descriptors then stay in uniform
+  // registers.  (In loops of a single lane a product took about 130 clocks to issue, 650 to 780 a k-block of four where the tensor cores
+  // need 512.  Persistent products: 65 -> 60.6 us at 5000 x 6912 x 1280, 60 -> 56.3 at 5000 x 1280 x 5120, the same bits.)
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    if (lane == 0) {
-      int stage = 0; uint32_t phase = 0;
-      uint32_t issued_mask = 0, last_parity = 0;
-      bool ok = true;
-      for (int u = first_unit; u < total_units && ok; u += unit_step) {
-        int bz, mt, nt, kb0, kb1;
-        unit_coords(u, bz, mt, nt, kb0, kb1);
-        if (below_diagonal(g, mt, nt, TILE_M)) continue;
-        const int m0 = mt * TILE_M + rank * BM;           // first row of A this CTA loads
-        const int n0 = nt * BN + rank * G::BN_LOCAL;      // first column of B this CTA loads (its half, in a pair)
-        const int bb = g.groups ? __ldg(g.groups + 1 + mt * TILE_M / g.group_rows) : g.strideB ? bz : 0;   // which matrix of B
-        for (int kb = kb0; kb < kb1; kb++) {
-          if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag, g.status)) { ok = false; break; }
-          uint8_t* sa = smem + stage * STAGE_BYTES;
-          uint8_t* sb = sa + A_BYTES;
+    int stage = 0; uint32_t phase = 0;
+    uint32_t issued_mask = 0, last_parity = 0;
+    bool ok = true;
+    for (int u = first_unit; u < total_units && ok; u += unit_step) {
+      int bz, mt, nt, kb0, kb1;
+      unit_coords(u, bz, mt, nt, kb0, kb1);
+      if (below_diagonal(g, mt, nt, TILE_M)) continue;
+      const int m0 = mt * TILE_M + rank * BM;           // first row of A this CTA loads
+      const int n0 = nt * BN + rank * G::BN_LOCAL;      // first column of B this CTA loads (its half, in a pair)
+      const int bb = g.groups ? __ldg(g.groups + 1 + mt * TILE_M / g.group_rows) : g.strideB ? bz : 0;   // which matrix of B
+      for (int kb = kb0; kb < kb1; kb++) {
+        if (!mbar_wait_warp(&empty[stage], phase ^ 1, abort_flag, g.status)) { ok = false; break; }
+        uint8_t* sa = smem + stage * STAGE_BYTES;
+        uint8_t* sb = sa + A_BYTES;
+        if (elect_one()) {
           if (PAIR) {
             // the leader announces the bytes of both CTAs; the loads of either CTA are counted on its barrier
             if (rank == 0) mbar_expect_tx(&full[stage], 2 * STAGE_BYTES);
             if (A_K) tma_load_3d_pair(sa, &tmA, &full[stage], kb * BK, m0, bz);
             else tma_load_4d_pair(sa, &tmA, &full[stage], 0, kb * BK, m0 / 64, bz);
             if (B_K) tma_load_3d_pair(sb, &tmB, &full[stage], kb * BK, n0, bb);
-            else tma_load_4d_pair(sb, &tmB, &full[stage], 0, kb * BK, n0 / 64, bz);
+            else tma_load_4d_pair(sb, &tmB, &full[stage], 0, kb * BK, n0 / 64, bb);
           } else {
-          mbar_expect_tx(&full[stage], STAGE_BYTES);
-          if (A_K) {
-            tma_load_3d(sa, &tmA, &full[stage], kb * BK, mt * BM, bz);
-          } else if (p.a_slabs) {
-            tma_load_4d(sa, &tmA, &full[stage], 0, kb * BK, mt * (BM / 64), bz);
-          } else {
+            mbar_expect_tx(&full[stage], STAGE_BYTES);
+            if (A_K) {
+              tma_load_3d(sa, &tmA, &full[stage], kb * BK, mt * BM, bz);
+            } else if (p.a_slabs) {
+              tma_load_4d(sa, &tmA, &full[stage], 0, kb * BK, mt * (BM / 64), bz);
+            } else {
 #pragma unroll
-            for (int j = 0; j < BM / 64; j++) tma_load_3d(sa + j * 8192, &tmA, &full[stage], mt * BM + j * 64, kb * BK, bz);
-          }
-          if (B_K) {
-            tma_load_3d(sb, &tmB, &full[stage], kb * BK, nt * BN, bb);
-          } else if (p.b_slabs) {
-            tma_load_4d(sb, &tmB, &full[stage], 0, kb * BK, nt * (BN / 64), bz);
-          } else {
+              for (int j = 0; j < BM / 64; j++) tma_load_3d(sa + j * 8192, &tmA, &full[stage], mt * BM + j * 64, kb * BK, bz);
+            }
+            if (B_K) {
+              tma_load_3d(sb, &tmB, &full[stage], kb * BK, nt * BN, bb);
+            } else if (p.b_slabs) {
+              tma_load_4d(sb, &tmB, &full[stage], 0, kb * BK, nt * (BN / 64), bb);
+            } else {
 #pragma unroll
-            for (int j = 0; j < BN / 64; j++) tma_load_3d(sb + j * 8192, &tmB, &full[stage], nt * BN + j * 64, kb * BK, bz);
+              for (int j = 0; j < BN / 64; j++) tma_load_3d(sb + j * 8192, &tmB, &full[stage], nt * BN + j * 64, kb * BK, bb);
+            }
           }
-          }
-          issued_mask |= 1u << stage;
-          last_parity = (last_parity & ~(1u << stage)) | (phase << stage);
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
-      }
-      if (*abort_flag && !PAIR) {
-        // let loads already in flight land before the CTA exits (a pair meets at the cluster barrier below, and
-        // only the leader's barriers see the bytes)
-        for (int i = 0; i < STAGES; i++)
-          if (issued_mask & (1u << i))
-            for (uint32_t it = 0; it < WAIT_LIMIT && !mbar_try_wait(&full[i], (last_parity >> i) & 1u); ++it) {}
+        __syncwarp();
+        issued_mask |= 1u << stage;
+        last_parity = (last_parity & ~(1u << stage)) | (phase << stage);
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
     }
+    if (*abort_flag && !PAIR) {
+      // let loads already in flight land before the CTA exits (a pair meets at the cluster barrier below, and
+      // only the leader's barriers see the bytes)
+      for (int i = 0; i < STAGES; i++)
+        if (issued_mask & (1u << i))
+          for (uint32_t it = 0; it < WAIT_LIMIT && !mbar_try_wait(&full[i], (last_parity >> i) & 1u); ++it) {}
+    }
+    __syncwarp();
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0 && rank == 0) {
+    if (rank == 0) {
       constexpr uint32_t idesc = idesc_bf16(TILE_M, BN, !A_K, !B_K);
       int stage = 0; uint32_t phase = 0;
       int acc = 0; uint32_t acc_phase = 0;
@@ -328,32 +333,36 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         int bz, mt, nt, kb0, kb1;
         unit_coords(u, bz, mt, nt, kb0, kb1);
         if (below_diagonal(g, mt, nt, TILE_M)) continue;
-        if (!mbar_wait(&tempty[acc], acc_phase ^ 1, abort_flag, g.status)) break;
+        if (!mbar_wait_warp(&tempty[acc], acc_phase ^ 1, abort_flag, g.status)) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
         for (int kb = kb0; kb < kb1; kb++) {
-          if (!mbar_wait(&full[stage], phase, abort_flag, g.status)) { ok = false; break; }
+          if (!mbar_wait_warp(&full[stage], phase, abort_flag, g.status)) { ok = false; break; }
           tc_fence_after();
           const uint32_t sa = smem_u32(smem + stage * STAGE_BYTES);
           const uint32_t sb = sa + A_BYTES;
+          if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < BK / 16; k++) {
-            // K-major: rows of 128 B, 8-row groups 1024 B apart, 16 k-elements = 32 B along the row.
-            // MN-major: [64 k][64 mn] slabs of 8192 B, 8-k groups 1024 B apart, 16 k = 2048 B.
-            const uint64_t ad = A_K ? smem_desc_sw128(sa + k * 32, 16, 1024) : smem_desc_sw128(sa + k * 2048, 8192, 1024);
-            const uint64_t bd = B_K ? smem_desc_sw128(sb + k * 32, 16, 1024) : smem_desc_sw128(sb + k * 2048, 8192, 1024);
-            if (PAIR) mma_ss_pair(d_tmem, ad, bd, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
-            else mma_ss(d_tmem, ad, bd, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+            for (int k = 0; k < BK / 16; k++) {
+              // K-major: rows of 128 B, 8-row groups 1024 B apart, 16 k-elements = 32 B along the row.
+              // MN-major: [64 k][64 mn] slabs of 8192 B, 8-k groups 1024 B apart, 16 k = 2048 B.
+              const uint64_t ad = A_K ? smem_desc_sw128(sa + k * 32, 16, 1024) : smem_desc_sw128(sa + k * 2048, 8192, 1024);
+              const uint64_t bd = B_K ? smem_desc_sw128(sb + k * 32, 16, 1024) : smem_desc_sw128(sb + k * 2048, 8192, 1024);
+              if (PAIR) mma_ss_pair(d_tmem, ad, bd, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+              else mma_ss(d_tmem, ad, bd, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+            }
+            if (PAIR) tc_commit_pair(&empty[stage]); else tc_commit(&empty[stage]);
+            if (kb + 1 == kb1) { if (PAIR) tc_commit_pair(&tfull[acc]); else tc_commit(&tfull[acc]); }
           }
-          if (PAIR) tc_commit_pair(&empty[stage]); else tc_commit(&empty[stage]);
+          __syncwarp();
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
         if (!ok) break;
-        if (PAIR) tc_commit_pair(&tfull[acc]); else tc_commit(&tfull[acc]);
         acc ^= 1;
         if (acc == 0) acc_phase ^= 1;
       }
     }
+    __syncwarp();
   } else {
     // ---------------- epilogue (warps 2..9) ----------------
     const int quad = warp & 3;           // TMEM lane quadrant this warp may read
