@@ -109,6 +109,7 @@ SIGNATURES = {
     "femto_comm_check": (I32, [P]),
     "femto_comm_abort": (I32, [P]),
     "femto_selftest_bounded_wait": (I32, [I32, C.POINTER(I32), C.POINTER(I32)]),
+    "femto_selftest_gemm_few_rows": (I32, [P, I64, P, I32, I64, P, I64, P, I64, P, I32, I32, I32, I32, I64, I64, I64, I32, I32, I32, P]),
     "femto_selftest_decode_wait": (I32, [P, P, P, P, I32, P, P, C.POINTER(I32)]),
     "femto_set_overlap": (I32, [P, I32]),
     "femto_optimizer_state_sizes": (I32, [P, C.POINTER(I64)]),

@@ -421,6 +421,27 @@ int32_t femto_gemm_bf16(const void* A, int32_t a_kmajor, int64_t lda, const void
   return standalone_finish(r, g.status, (cudaStream_t)stream);
 }
 
+int32_t femto_selftest_gemm_few_rows(const void* A, int64_t lda, const void* B, int32_t b_kmajor, int64_t ldb, void* C, int64_t ldc, const void* aux,
+                                     int64_t ldaux, const float* bias, int32_t M, int32_t N, int32_t K, int32_t batch, int64_t strideA, int64_t strideB,
+                                     int64_t strideC, int32_t epilogue, int32_t tile_columns, int32_t splits, void* stream) {
+  FEMTO_TRY(require_device());
+  if (!A || !B || !C || M <= 0 || N <= 0 || K <= 0) return femto_fail(FEMTO_ERR_ARG, "bad argument");
+  if (tile_columns != 64 && tile_columns != 128) return femto_fail(FEMTO_ERR_ARG, "tiles have 64 or 128 columns");
+  if (splits != 1 && splits != 2 && splits != 4 && splits != 8) return femto_fail(FEMTO_ERR_ARG, "clusters have 1, 2, 4 or 8 blocks");
+  if ((epilogue == EPI_RESID) != (aux != nullptr)) return femto_fail(FEMTO_ERR_ARG, "the residual epilogue, and no other, takes aux");
+  const int stages = cdiv(K, K & 63 ? 64 : 128);
+  if ((splits - 1) * cdiv(stages, splits) >= stages) return femto_fail(FEMTO_ERR_SHAPE, "K=%d leaves a block of the cluster without a part", K);
+  GemmArgs g;
+  g.A = A; g.lda = lda; g.B = B; g.ldb = ldb; g.b_kmajor = b_kmajor != 0; g.C = C; g.ldc = ldc; g.aux = aux; g.ldaux = ldaux; g.bias = bias;
+  g.M = M; g.N = N; g.K = K; g.batch = batch < 1 ? 1 : batch; g.strideA = strideA; g.strideB = strideB; g.strideC = g.strideAux = strideC;
+  g.epi = epilogue; g.beta = 0.f; g.any_size = true;
+  char* ws = nullptr;      // asked for by fp32 results of the persistent kernel only
+  FEMTO_TRY(standalone_scratch(256, &ws));
+  g.ws = ws; g.ws_bytes = 256;
+  FEMTO_TRY(standalone_status(&g.status));
+  return standalone_finish(gemm_split_bf16(g, tile_columns, splits, (cudaStream_t)stream), g.status, (cudaStream_t)stream);
+}
+
 int32_t femto_embedding_gradient(int32_t dtype, float* table, const void* dy, const int32_t* tokens0, int32_t N,
                                  int32_t D, int32_t rows, void* stream) {
   FEMTO_TRY(require_device());

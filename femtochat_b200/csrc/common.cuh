@@ -184,7 +184,8 @@ struct GemmArgs {
   const int* groups = nullptr;
   int group_rows = 0, n_groups = 0;   // n_groups: matrices in B
   const float* bias = nullptr;   // [N] added to the columns before the store (EPI_STORE)
-  bool any_size = false;   // take the tensor-core kernel for results smaller than one tile as well
+  bool any_size = false;   // no later step repeats this product bit for bit (no training step): results smaller than a tile take the
+                           // tensor cores as well, and K may be cut into ranges that are added at the end
   int ring = 0;   // depth of the operand ring of the tensor-core kernel; 0 = the deepest that fits (fewer stages leave
                   // shared memory free for kernels of another stream to run on the same SMs)
   // cross-entropy statistics epilogue
@@ -200,6 +201,9 @@ struct GemmArgs {
 template <typename T> int gemm_simt(const GemmArgs& g, cudaStream_t s);
 int gemm_tc_bf16(const GemmArgs& g, cudaStream_t s);       // tcgen05 path (gemm_sm100.cu)
 bool gemm_tc_supported(const GemmArgs& g);
+// few rows: narrow tiles, K over a cluster (gemm_split_sm100.cu)
+bool gemm_split_plan(const GemmArgs& g, int* bn, int* splits);
+int gemm_split_bf16(const GemmArgs& g, int bn, int splits, cudaStream_t s);
 template <typename T> int gemm(const GemmArgs& g, cudaStream_t s);  // dispatch
 
 // ---- attention --------------------------------------------------------------------------------

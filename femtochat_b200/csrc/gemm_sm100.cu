@@ -849,6 +849,7 @@ static int launch_tc(const GemmArgs& g, const CUtensorMap& tmA, const CUtensorMa
 
 int gemm_tc_bf16(const GemmArgs& g, cudaStream_t s) {
   if (!gemm_tc_supported(g)) return femto_fail(FEMTO_ERR_UNSUPPORTED, "gemm_tc: shape/alignment not supported");
+  if (int bn, splits; gemm_split_plan(g, &bn, &splits)) return gemm_split_bf16(g, bn, splits, s);
   TcParams p;
   p.g = g;
   const int nb = g.batch;

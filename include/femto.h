@@ -454,6 +454,14 @@ int32_t femto_selftest_bounded_wait(int32_t polls, int32_t* h_status, int32_t* h
  * stays as it was) and return by themselves; the cache goes on where it was. */
 int32_t femto_selftest_decode_wait(femto_handle* h, femto_kv_cache* c, const float* theta, const int32_t* tokens, int32_t B,
                                    float* logits_out, void* stream, int32_t* h_status);
+/* The product of few rows that prompts and evaluations take where it is the faster one (tiles of 128 rows and `tile_columns` = 64 or 128
+ * columns, K shared by a cluster of `splits` = 1, 2, 4 or 8 blocks), with every choice open: C = epilogue(A[M][K] * B) in bf16 with fp32
+ * accumulation, epilogue 0 store (+ bias), 1 + aux, 2 relu^2, 5 fp32, 7 silu(gate) * up of B's groups of 32 rows.  Waits.
+ * No counterpart in the reference. */
+int32_t femto_selftest_gemm_few_rows(const void* A, int64_t lda, const void* B, int32_t b_kmajor, int64_t ldb, void* C, int64_t ldc,
+                                     const void* aux, int64_t ldaux, const float* bias, int32_t M, int32_t N, int32_t K, int32_t batch,
+                                     int64_t strideA, int64_t strideB, int64_t strideC, int32_t epilogue, int32_t tile_columns,
+                                     int32_t splits, void* stream);
 
 /* Measurement aid (no counterpart in the reference): when enabled, every launch of the tensor-core
  * GEMM kernel is bracketed by CUDA events on its stream; the report returns the summed kernel time,

@@ -69,6 +69,38 @@ def test_gemm_simt_sums_over_k_in_order(ak, bk, M, N, K, batch):
     assert torch.equal(C_, ref)
 
 
+@pytest.mark.parametrize("bn,splits", [(64, 1), (64, 2), (64, 8), (128, 1), (128, 4)])
+@pytest.mark.parametrize("bk,epi,M,N,K,batch", [(False, 0, 1, 64, 1024, 2), (False, 1, 130, 192, 1984, 1), (False, 2, 255, 320, 1000, 1), (True, 0, 24, 72, 1000, 3),
+                                                (True, 5, 129, 100, 1984, 1), (True, 1, 100, 136, 1024, 1), (True, 7, 200, 384, 1984, 1)])
+def test_gemm_of_few_rows(bk, epi, M, N, K, batch, bn, splits):
+    """Narrow tiles with K shared by a cluster: one row, edges of tiles of 128 rows and 64 or 128 columns, columns that are no multiple of
+    eight (vector stores end), K that is and is not whole slabs of 64, an odd number of slabs, batches, both layouts of B, every epilogue.
+    One bf16 rounding of the result (of gate and up, too, where the result is their product); fp32: the sums' own rounding."""
+    L, P = _lib.lib(), _lib.ptr
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    A = torch.randn(batch, M, K, generator=g, device="cuda").bfloat16()
+    B = (torch.randn(batch, K, N, generator=g, device="cuda") * K ** -0.5).bfloat16()
+    Bs = B.transpose(1, 2).contiguous() if bk else B.contiguous()
+    n = N // 2 if epi == 7 else N
+    aux = torch.randn(batch, M, n, generator=g, device="cuda").bfloat16() if epi == 1 else None
+    bias = torch.randn(N, generator=g, device="cuda") if epi == 0 else None
+    out = torch.full((batch, M, n), float("nan"), device="cuda", dtype=torch.float32 if epi == 5 else torch.bfloat16)
+    _lib.check(L.femto_selftest_gemm_few_rows(P(A), K, P(Bs), int(bk), K if bk else N, P(out), n, P(aux), n, P(bias), M, N, K, batch, M * K, K * N,
+                                              M * n, epi, bn, splits, None))
+    ref = torch.bmm(A.double().cpu(), B.double().cpu())
+    if epi == 0:
+        ref += bias.double().cpu()
+    elif epi == 1:
+        ref += aux.double().cpu()
+    elif epi == 2:
+        ref = ref.clamp(min=0) ** 2
+    elif epi == 7:
+        gu = ref.view(batch, M, N // 64, 2, 32)
+        ref = (torch.nn.functional.silu(gu[..., 0, :]) * gu[..., 1, :]).reshape(batch, M, n)
+    err = (out.double().cpu() - ref).abs().max()
+    assert err <= (K * 2.0 ** -24 if epi == 5 else 2.0 ** -8) * ref.abs().max()
+
+
 def test_gemm_split_k_fp32_accumulate_is_deterministic():
     """Weight-gradient form: both operands MN-contiguous, K = tokens, fp32 C += ; split-K reduce in fixed order."""
     M, N, K = 1280, 1280, 8192
