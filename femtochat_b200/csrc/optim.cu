@@ -112,6 +112,11 @@ __global__ void __launch_bounds__(128) k_adamw_small(float* __restrict__ theta, 
 }
 
 // mom = mu*mom + (1-mu)*g ; X = (1-mu)*g + mu*mom  (src/optim.jl:206-207)
+__device__ __forceinline__ float momentum(float g, float& mom, float mu, float inv_nt) {
+  const float gv = g * inv_nt, mm = mu * mom + (1.f - mu) * gv;
+  mom = mm;
+  return (1.f - mu) * gv + mu * mm;
+}
 __global__ void __launch_bounds__(256) k_muon_momentum(const float* __restrict__ delta, const long long* __restrict__ offs,
                                                        float* __restrict__ mom, float* __restrict__ X, long long per,
                                                        float mu, float inv_nt) {
@@ -119,13 +124,26 @@ __global__ void __launch_bounds__(256) k_muon_momentum(const float* __restrict__
   const int k = blockIdx.y;
   const float* g = delta + offs[k];
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < per; i += (long long)gridDim.x * blockDim.x) {
-    float gv = g[i] * inv_nt;
-    float mm = mu * mom[k * per + i] + (1.f - mu) * gv;
-    mom[k * per + i] = mm;
-    X[k * per + i] = (1.f - mu) * gv + mu * mm;
+    float m = mom[k * per + i];
+    X[k * per + i] = momentum(g[i], m, mu, inv_nt);
+    mom[k * per + i] = m;
   }
 }
 
+template <typename T> __device__ __forceinline__ float column_sumsq(const T* p, int in, int ld) {
+  // eight independent partial sums (rows i mod 8), combined in a fixed order: eight loads in flight per thread
+  float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  int i = 0;
+  for (; i + 8 <= in; i += 8) {
+    float v[8];
+#pragma unroll
+    for (int u = 0; u < 8; u++) v[u] = to_f<T>(p[(long long)(i + u) * ld]);
+#pragma unroll
+    for (int u = 0; u < 8; u++) a[u] += v[u] * v[u];
+  }
+  for (; i < in; i++) { float v = to_f<T>(p[(long long)i * ld]); a[i & 7] += v * v; }
+  return ((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7]));
+}
 // vec[k][o] = sum_i X[k][i][o]^2 (thread per column, rows in order)
 template <typename T>
 __global__ void __launch_bounds__(256) k_sumsq_cols(const T* __restrict__ X, int in, int out, float* __restrict__ vec) {
@@ -133,19 +151,7 @@ __global__ void __launch_bounds__(256) k_sumsq_cols(const T* __restrict__ X, int
   const int k = blockIdx.y;
   const int o = blockIdx.x * 256 + threadIdx.x;
   if (o >= out) return;
-  const T* p = X + (long long)k * in * out + o;
-  // eight independent partial sums (rows i mod 8), combined in a fixed order: eight loads in flight per thread
-  float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  int i = 0;
-  for (; i + 8 <= in; i += 8) {
-    float v[8];
-#pragma unroll
-    for (int u = 0; u < 8; u++) v[u] = to_f<T>(p[(long long)(i + u) * out]);
-#pragma unroll
-    for (int u = 0; u < 8; u++) a[u] += v[u] * v[u];
-  }
-  for (; i < in; i++) { float v = to_f<T>(p[(long long)i * out]); a[i & 7] += v * v; }
-  vec[(long long)k * out + o] = ((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7]));
+  vec[(long long)k * out + o] = column_sumsq(X + (long long)k * in * out + o, in, out);
 }
 // vec[k][i] = sum_o X[k][i][o]^2 (warp per row)
 template <typename T>
@@ -163,11 +169,7 @@ __global__ void __launch_bounds__(256) k_sumsq_rows(const T* __restrict__ X, int
 
 // MuonEq + Polar-Express normalisation factors (src/optim.jl:210-212,135-136), one block per matrix:
 // fac[k][o] = sqrt(old/m)/max(sqrt(row[o]),1e-6) / (1.01*sqrt(sum_o fac0^2*row[o]) + 1e-6)
-__global__ void __launch_bounds__(256) k_muoneq_factors(const float* __restrict__ vec, int out, float* __restrict__ fac) {
-  pdl_trigger();
-  __shared__ float red[256];
-  const int k = blockIdx.x;
-  const float* row = vec + (long long)k * out;
+__device__ __forceinline__ void muoneq_factors(const float* row, int out, float* fac, float* red) {
   float acc = 0.f;
   for (int o = threadIdx.x; o < out; o += 256) acc += row[o];
   red[threadIdx.x] = acc;
@@ -185,7 +187,12 @@ __global__ void __launch_bounds__(256) k_muoneq_factors(const float* __restrict_
   __syncthreads();
   for (int s = 128; s > 0; s >>= 1) { if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s]; __syncthreads(); }
   const float scale = 1.01f * sqrtf(red[0]) + 1e-6f;
-  for (int o = threadIdx.x; o < out; o += 256) fac[(long long)k * out + o] = num / fmaxf(sqrtf(row[o]), 1e-6f) / scale;
+  for (int o = threadIdx.x; o < out; o += 256) fac[o] = num / fmaxf(sqrtf(row[o]), 1e-6f) / scale;
+}
+__global__ void __launch_bounds__(256) k_muoneq_factors(const float* __restrict__ vec, int out, float* __restrict__ fac) {
+  pdl_trigger();
+  __shared__ float red[256];
+  muoneq_factors(vec + (long long)blockIdx.x * out, out, fac + (long long)blockIdx.x * out, red);
 }
 
 template <typename T>
@@ -222,13 +229,7 @@ __global__ void __launch_bounds__(256) k_scale_cols_cast4(const float* __restric
 
 // Muon+ and NorMuon factors (src/optim.jl:218-233), one block per matrix.  vec = sums of X^2 along
 // the reduced axis (length dim, each over dsize elements); v is the persistent second moment.
-__global__ void __launch_bounds__(256) k_normuon_factors(const float* __restrict__ vec, int dim, int dsize, int rmin,
-                                                         float b2, float* __restrict__ v, float* __restrict__ fac) {
-  pdl_trigger();
-  __shared__ float red[256];
-  const int k = blockIdx.x;
-  const float* S = vec + (long long)k * dim;
-  float* vv = v + (long long)k * dim;
+__device__ __forceinline__ void normuon_factors(const float* S, int dim, int dsize, int rmin, float b2, float* vv, float* fac, float* red) {
   float acc = 0.f;
   for (int j = threadIdx.x; j < dim; j += 256) acc += S[j];
   red[threadIdx.x] = acc;
@@ -250,7 +251,14 @@ __global__ void __launch_bounds__(256) k_normuon_factors(const float* __restrict
   __syncthreads();
   for (int s = 128; s > 0; s >>= 1) { if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s]; __syncthreads(); }
   const float g = f1 * sqrtf(old) / fmaxf(sqrtf(red[0]), 1e-10f);
-  for (int j = threadIdx.x; j < dim; j += 256) fac[(long long)k * dim + j] = g * rsqrtf(fmaxf(vv[j], 1e-10f));
+  for (int j = threadIdx.x; j < dim; j += 256) fac[j] = g * rsqrtf(fmaxf(vv[j], 1e-10f));
+}
+__global__ void __launch_bounds__(256) k_normuon_factors(const float* __restrict__ vec, int dim, int dsize, int rmin,
+                                                         float b2, float* __restrict__ v, float* __restrict__ fac) {
+  pdl_trigger();
+  __shared__ float red[256];
+  const long long at = (long long)blockIdx.x * dim;
+  normuon_factors(vec + at, dim, dsize, rmin, b2, v + at, fac + at, red);
 }
 
 // theta -= eta*X + eta*lam*theta*[X*theta >= 0]  (src/optim.jl:244-245; ext/FemtoChatCUDAExt.jl:108-119)
@@ -323,6 +331,125 @@ __global__ void __launch_bounds__(256) k_muon_update2(float* __restrict__ theta,
         else *reinterpret_cast<float2*>(dst) = make_float2(r0, r1);
       }
     }
+  }
+}
+
+// ---- a whole Muon update of small matrices -------------------------------------------------------------------------------------------
+// One block a matrix, which stays in shared memory from its momentum to its new weights; all groups of small matrices in one launch.  As a
+// chain of launches a group was 23 (15 of them products of the iteration), 4 us each for the host and 2 to 5 for the device, whatever its
+// size: the introductory example's five groups 115 of its 203 launches a step, and the value gates (12 x heads) of every model half a
+// millisecond (15 products at 31 us).  Every sum is taken in the order of those launches' kernels (a product's result is one
+// chain of fp32 multiply-adds over k, its polynomial fma(alpha, aux, beta sum)), so the results are the same bits.  Training step of the
+// introductory example 792 -> 320 us, d12 (4 x 2048) 16.73 -> 16.53 ms, d20 (8 x 2048) 1.1 ms less.
+struct SmallMuon {
+  const long long* offs; float *mom, *v;       // of the first matrix this rank updates
+  void* const* shadow; const int* shadow_ld;
+  int k, in, out;
+  float mu, b2, eta, lam;
+};
+constexpr int SMALL_GROUPS = 8, SMALL_ELEMENTS = 4096, SMALL_SIDE = 1024;
+struct SmallMuonBatch { SmallMuon g[SMALL_GROUPS]; float coeffs[15]; int n, steps; float inv_nt; };
+// rows of an odd number of floats: neighbouring rows, and neighbouring columns, lie in different banks
+__host__ __device__ constexpr int odd(int n) { return n | 1; }
+inline size_t small_floats(int in, int out) {
+  const int r = std::min(in, out);
+  return 2 * (size_t)in * odd(out) + 2 * (size_t)r * odd(r) + 2 * (size_t)std::max(in, out);
+}
+
+// out(m, n, sum over k of a(m, k) b(k, n)): 2 x 4 results a thread
+template <typename FA, typename FB, typename FO> __device__ __forceinline__ void small_product(int M, int N, int K, FA&& a, FB&& b, FO&& out) {
+  const int mg = (M + 1) / 2, ng = (N + 3) / 4;
+  for (int u = threadIdx.x; u < mg * ng; u += 256) {
+    const int m0 = u / ng, n0 = u % ng;
+    int m[2], n[4];
+#pragma unroll
+    for (int i = 0; i < 2; i++) m[i] = min(m0 + i * mg, M - 1);
+#pragma unroll
+    for (int j = 0; j < 4; j++) n[j] = min(n0 + j * ng, N - 1);
+    float acc[2][4] = {};
+#pragma unroll 4
+    for (int k = 0; k < K; k++) {
+      float x[2], y[4];
+#pragma unroll
+      for (int i = 0; i < 2; i++) x[i] = a(m[i], k);
+#pragma unroll
+      for (int j = 0; j < 4; j++) y[j] = b(k, n[j]);
+#pragma unroll
+      for (int i = 0; i < 2; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc[i][j] = fmaf(x[i], y[j], acc[i][j]);
+    }
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+        if (m0 + i * mg < M && n0 + j * ng < N) out(m[i], n[j], acc[i][j]);
+  }
+  __syncthreads();
+}
+
+template <typename T, typename S>
+__global__ void __launch_bounds__(256) k_muon_small(float* __restrict__ theta, const float* __restrict__ delta, const __grid_constant__ SmallMuonBatch batch) {
+  pdl_trigger();
+  extern __shared__ float smem[];
+  __shared__ float red[256];
+  int k = blockIdx.x, gi = 0;
+  while (k >= batch.g[gi].k) k -= batch.g[gi++].k;
+  const SmallMuon& g = batch.g[gi];
+  const int in = g.in, out = g.out, per = in * out, ld = odd(out), r = min(in, out), lr = odd(r), tid = threadIdx.x;
+  float *cur = smem, *nxt = cur + in * ld, *A = nxt + in * ld, *B = A + r * lr, *vec = B + r * lr, *fac = vec + max(in, out);
+  const float* d = delta + g.offs[k];
+  float* mom = g.mom + (long long)k * per;
+  for (int i = tid; i < per; i += 256) {
+    float m = mom[i];
+    cur[i / out * ld + i % out] = momentum(d[i], m, g.mu, batch.inv_nt);
+    mom[i] = m;
+  }
+  __syncthreads();
+  for (int o = tid; o < out; o += 256) vec[o] = column_sumsq(cur + o, in, ld);
+  __syncthreads();
+  muoneq_factors(vec, out, fac, red);
+  __syncthreads();
+  // what the launches keep in the compute type has its values here
+  for (int i = tid; i < per; i += 256) { const int at = i / out * ld + i % out; cur[at] = round_to<T>(cur[at] * fac[i % out]); }
+  __syncthreads();
+  const bool tall = out > in;
+  for (int t = 0; t < batch.steps; t++) {
+    const float ca = batch.coeffs[3 * t], cb = batch.coeffs[3 * t + 1], cc = batch.coeffs[3 * t + 2];
+    auto put_a = [&](int m, int n, float v) { A[m * lr + n] = round_to<T>(v); };
+    if (tall) small_product(r, r, out, [&](int m, int q) { return cur[m * ld + q]; }, [&](int q, int n) { return cur[n * ld + q]; }, put_a);
+    else small_product(r, r, in, [&](int m, int q) { return cur[q * ld + m]; }, [&](int q, int n) { return cur[q * ld + n]; }, put_a);
+    small_product(r, r, r, [&](int m, int q) { return A[m * lr + q]; }, [&](int q, int n) { return A[n * lr + q]; },
+                  [&](int m, int n, float v) { B[m * lr + n] = round_to<T>(__fmaf_rn(cb, A[m * lr + n], __fmul_rn(cc, v))); });
+    auto put_x = [&](int m, int n, float v) { nxt[m * ld + n] = round_to<T>(__fmaf_rn(ca, cur[m * ld + n], v)); };
+    if (tall) small_product(r, out, r, [&](int m, int q) { return B[m * lr + q]; }, [&](int q, int n) { return cur[q * ld + n]; }, put_x);
+    else small_product(in, r, r, [&](int m, int q) { return cur[m * ld + q]; }, [&](int q, int n) { return B[n * lr + q]; }, put_x);
+    float* swap = cur; cur = nxt; nxt = swap;
+  }
+  const bool by_col = out >= in;
+  const int dim = by_col ? out : in;
+  if (by_col) {
+    for (int o = tid; o < out; o += 256) vec[o] = column_sumsq(cur + o, in, ld);
+  } else {
+    for (int i = tid >> 5; i < in; i += 8) {
+      float acc = 0.f;
+      for (int o = tid & 31; o < out; o += 32) { const float v = cur[i * ld + o]; acc += v * v; }
+      acc = warp_sum(acc);
+      if ((tid & 31) == 0) vec[i] = acc;
+    }
+  }
+  __syncthreads();
+  normuon_factors(vec, dim, by_col ? in : out, r, g.b2, g.v + (long long)k * dim, fac, red);
+  __syncthreads();
+  float* th = theta + g.offs[k];
+  S* sh = g.shadow ? reinterpret_cast<S*>(g.shadow[k]) : nullptr;
+  const int sld = g.shadow ? g.shadow_ld[k] : 0;
+  for (int i = tid; i < per; i += 256) {
+    const int row = i / out, col = i % out;
+    const float x = cur[row * ld + col] * fac[by_col ? col : row], t = th[i];
+    const float tn = t - (g.eta * x + g.eta * g.lam * t * ((x * t) >= 0.f ? 1.f : 0.f));
+    th[i] = tn;
+    if (sh) sh[(long long)row * sld + col] = from_f<S>(tn);
   }
 }
 
@@ -749,7 +876,43 @@ int optimizer_step(femto_optimizer* o, float* theta, const float* delta, float e
   }
   FEMTO_TRY(flush_small());
   int rc = 0;
+  // small matrices: 4096 elements are 25 us of a block, about what the 23 launches of a group take the device; more would wait for one block
+  auto small = [&](const MuonGroup& g) { return (long long)g.in * g.out <= SMALL_ELEMENTS && std::max(g.in, g.out) <= SMALL_SIDE; };
+  auto step_small = [&](SmallMuonBatch& b, size_t floats) -> int {
+    if (!b.n) return 0;
+    int blocks = 0;
+    for (int i = 0; i < b.n; i++) blocks += b.g[i].k;
+    const size_t bytes = floats * sizeof(float);
+    auto launch = [&](auto kernel) -> int {
+      if (bytes > 48 << 10) CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+      kernel<<<blocks, 256, bytes, s>>>(theta, delta, b);
+      KERNEL_CHECK();
+      return 0;
+    };
+    b.n = 0;
+    if (o->cfg.compute_dtype == FEMTO_BF16) return h->bf ? launch(k_muon_small<bf16, bf16>) : launch(k_muon_small<bf16, float>);
+    return h->bf ? launch(k_muon_small<float, bf16>) : launch(k_muon_small<float, float>);
+  };
+  SmallMuonBatch sb = {};
+  sb.steps = o->cfg.ns_steps; sb.inv_nt = 1.f / n_tokens;
+  std::copy(o->cfg.ns_coeffs, o->cfg.ns_coeffs + 15, sb.coeffs);
+  size_t floats = 0;
+  for (auto& g : o->muon) {
+    if (!small(g) || g.k1 <= g.k0) continue;
+    SmallMuon& m = sb.g[sb.n++];
+    const long long per = (long long)g.in * g.out;
+    m.k = g.k1 - g.k0; m.in = g.in; m.out = g.out; m.offs = g.d_offs + g.k0;
+    m.mom = o->muon_m + g.moff + g.k0 * per; m.v = o->muon_v + g.voff + (long long)g.k0 * std::max(g.in, g.out);
+    m.shadow = g.d_shadow ? g.d_shadow + g.k0 : nullptr; m.shadow_ld = g.d_shadow_ld ? g.d_shadow_ld + g.k0 : nullptr;
+    m.mu = has_mu ? mu : g.mu; m.b2 = g.b2; m.lam = has_lambda ? lambda : g.lam;
+    m.eta = eta * g.alpha * sqrtf(std::max(1.f, (float)g.out / (float)g.in));
+    floats = std::max(floats, small_floats(g.in, g.out));
+    if (sb.n == SMALL_GROUPS && (rc = step_small(sb, floats))) break;
+  }
+  if (!rc) rc = step_small(sb, floats);
   for (auto& g : o->muon) {  // src/optim.jl:434-438
+    if (rc) break;
+    if (small(g)) continue;
     const float m_ = has_mu ? mu : g.mu, l_ = has_lambda ? lambda : g.lam;
     if (o->cfg.compute_dtype == FEMTO_BF16) rc = muon_group_step<bf16>(o, g, theta, delta, eta * g.alpha, m_, l_, n_tokens, s);
     else rc = muon_group_step<float>(o, g, theta, delta, eta * g.alpha, m_, l_, n_tokens, s);

@@ -653,6 +653,44 @@ def test_muon_direction_matches_oracle_two_steps(dtype, k, m, n):
         assert (v.cpu().reshape(st.v.shape) - st.v).abs().max() <= (6e-2 if dtype == _lib.BF16 else 1e-5) * float(st.v.abs().max())
 
 
+@pytest.mark.parametrize("ctype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("d,heads,kv,steps", [(28, 2, 1, 5), (24, 1, 1, 4), (32, 2, 1, 5), (32, 4, 4, 1), (40, 5, 1, 5)])
+def test_small_muon_matrices_take_the_same_bits_in_one_launch(ctype, d, heads, kv, steps):
+    """An update whose matrices are small is one launch; `femto_muon_direction` on the same stack is the chain of launches.  Moments are the
+    same bits and so is the direction: the new weights follow from it with two roundings.  Square, tall and wide matrices, one row (value
+    gates), a width that is no multiple of four, an even number of iterations (the stack ends where it began), and 4096 elements, beside
+    matrices of 6400 (40 wide) that keep the chain."""
+    cfg = fb.GPTConfig(sequence_len=4, max_document_tokens=16, vocab_size=16, n_layer=3, n_head=heads, n_kv_head=kv, n_embed=d, window_pattern="L")
+    lay = fb.parameter_layout(cfg)
+    g = torch.Generator(device="cuda").manual_seed(d + steps)
+    params = fb.Params(torch.randn(lay.nparams, device="cuda", generator=g) * 0.1)
+    params.delta.normal_(0.0, 3.0, generator=g)
+    tok = torch.ones(1, 4, dtype=torch.int32, device="cuda")
+    st = fb.gradient_state(params, cfg, lay, tok, tok, compute_type=ctype)
+    coeffs = fo.POLAR_EXPRESS_COEFFS[:steps]
+    opt = fb.MuonAdamW(params, lay, st, compute_type=ctype, matrix_lr=0.02, coeffs=coeffs)
+    opt.muon_m.normal_(0.0, 1.0, generator=g)
+    opt.muon_v.uniform_(0.001, 0.01, generator=g)
+    flat = (C.c_float * 15)(*[c for abc in coeffs for c in abc])
+    eta, lam, want = 0.7, 0.03, []
+    for group in opt.muon:
+        m, v = group.m.clone(), group.v.clone()
+        k, rows, cols = m.shape
+        G = torch.stack([params.delta[s.offset:s.offset + s.size].view(rows, cols) for s in group.specs]).contiguous()
+        X = torch.zeros_like(G)
+        _lib.check(_lib.lib().femto_muon_direction(_lib.F32 if ctype == "float32" else _lib.BF16, _lib.ptr(X), _lib.ptr(G), _lib.ptr(m), _lib.ptr(v), k, rows,
+                                                   cols, 0.9, 0.9, 64.0, flat, steps, None))
+        old = torch.stack([params.theta[s.offset:s.offset + s.size].view(rows, cols) for s in group.specs]).double()
+        rate = eta * 0.02 * max(1.0, cols / rows) ** 0.5
+        want.append((m, v, old - (rate * X.double() + rate * lam * old * (X * old >= 0))))
+    opt.step(eta=eta, mu=0.9, lam=lam, Nt=64.0)
+    torch.cuda.synchronize()
+    for group, (m, v, theta) in zip(opt.muon, want):
+        assert torch.equal(group.m, m) and torch.equal(group.v, v)
+        got = torch.stack([params.theta[s.offset:s.offset + s.size].view(m.shape[1:]) for s in group.specs]).double()
+        assert (got - theta).abs().max() <= 2.0 ** -22 * theta.abs().max()
+
+
 def test_muon_adamw_three_steps_bf16_against_oracle():
     """The whole MuonAdamW step with the Polar-Express chain in bf16 (the training configuration) against the oracle
     run with compute_dtype=bfloat16, on 256- and 512-wide matrices that take the tensor-core GEMM.  bf16 Newton-Schulz
