@@ -82,7 +82,7 @@ SIGNATURES = {
     "femto_nccl_unique_id": (I32, [P]),
     "femto_create": (I32, [C.POINTER(FemtoConfig), I32, I32, P, C.POINTER(P)]),
     "femto_destroy": (I32, [P]),
-    "femto_refresh_weights": (I32, [P, P, P]),
+    "femto_refresh_weights": (I32, [P, P, P]), "femto_weights_changed": (I32, [P]),
     "femto_loss_and_gradient": (I32, [P, P, P, P, P, P, I32, I32, I32, P, P, P]),
     "femto_forward_loss": (I32, [P, P, P, P, P, I32, I32, P, P, P]),
     "femto_forward_logits": (I32, [P, P, P, P, I32, P, P]),

@@ -210,6 +210,13 @@ int32_t femto_refresh_weights(femto_handle* h, const float* theta, void* stream)
   return h->dec ? decoder_refresh(h, theta, (cudaStream_t)stream) : model_refresh(h, theta, (cudaStream_t)stream);
 }
 
+int32_t femto_weights_changed(femto_handle* h) {
+  if (!h) return femto_fail(FEMTO_ERR_ARG, "NULL handle");
+  if (h->dec) return femto_fail(FEMTO_ERR_UNSUPPORTED, "a decoder that lists its layers takes femto_refresh_weights");
+  h->weights_changed = true;
+  return 0;
+}
+
 int32_t femto_loss_and_gradient(femto_handle* h, const float* theta, float* delta, const int32_t* tokens,
                                 const int32_t* targets, const int32_t* positions, int32_t B, int32_t reduction,
                                 int32_t accumulate, float* loss_out, int32_t* n_valid_out, void* stream) {

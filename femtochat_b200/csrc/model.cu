@@ -216,16 +216,17 @@ int cast_table(femto_handle* h) {
     jobs.push_back({src, rows * cols, cols, ldd, dst, h->cast_blocks, cols % 8 == 0 && ldd % 8 == 0 && aligned16(dst)});
     h->cast_blocks += cdiv(rows * cols, CAST_BLOCK);
   };
-  add(h->off_wte, h->sh_wte, Vp, d, d);
-  add(h->off_lm, h->sh_lm, Vp, d, d);
   for (int i = 0; i < h->L; i++) {
     const LayerP& p = h->lp[i];
     const LayerBuf& l = h->lb[i];
     char* qkv = reinterpret_cast<char*>(l.sh_wqkv);
     add(p.wq, qkv, d, d, dq); add(p.wk, qkv + d * es, d, kv, dq); add(p.wv, qkv + (d + kv) * es, d, kv, dq);
     add(p.wo, l.sh_wo, d, d, d); add(p.fc, l.sh_fc, d, 4 * d, 4 * d); add(p.proj, l.sh_proj, 4 * d, d, d);
-    if (p.ve) add(p.ve_table, l.sh_ve, Vp, kv, kv);
   }
+  add(h->off_lm, h->sh_lm, Vp, d, d);
+  h->cast_tables = h->cast_blocks;      // the tables last: a call that does not train can read their rows from Theta
+  add(h->off_wte, h->sh_wte, Vp, d, d);
+  for (int i = 0; i < h->L; i++) if (h->lp[i].ve) add(h->lp[i].ve_table, h->lb[i].sh_ve, Vp, kv, kv);
   h->n_cast_jobs = (int)jobs.size();
   CUDA_TRY(cudaMemcpy(h->cast_jobs, jobs.data(), sizeof(CastJob) * jobs.size(), cudaMemcpyHostToDevice));
   return 0;
@@ -293,10 +294,30 @@ void model_free(femto_handle* h) {
   h->arena = nullptr;
 }
 
+// blocks [from, to) of the cast table
+static int cast_range(femto_handle* h, const float* theta, int from, int to, cudaStream_t s) {
+  return h->bf ? Stream<bf16>::cast_all(theta, h->cast_jobs, h->n_cast_jobs, from, to, s) : Stream<float>::cast_all(theta, h->cast_jobs, h->n_cast_jobs, from, to, s);
+}
 int model_refresh(femto_handle* h, const float* theta, cudaStream_t s) {
-  FEMTO_TRY(h->bf ? Stream<bf16>::cast_all(theta, h->cast_jobs, h->n_cast_jobs, h->cast_blocks, s)
-                  : Stream<float>::cast_all(theta, h->cast_jobs, h->n_cast_jobs, h->cast_blocks, s));
+  FEMTO_TRY(cast_range(h, theta, 0, h->cast_blocks, s));
   h->weights_valid = true;
+  h->weights_changed = h->tables_live = false;
+  return 0;
+}
+int model_ensure_weights(femto_handle* h, const float* theta, bool tables, cudaStream_t s) {
+  if (h->weights_changed) {
+    if (tables) return model_refresh(h, theta, s);
+    // More than half of the weights are embedding tables, of which a call reads the rows of its tokens: those it takes from Theta, as it
+    // takes the gates and scalars.  d20: 0.81 -> 0.40 ms a call, d12 0.42 -> 0.12.  (The cast beside the pass on the other stream, in
+    // pieces that the blocks wait for, was slower than before it: 3.80 against 3.77 ms a prompt of 1500 tokens of d20.)
+    FEMTO_TRY(cast_range(h, theta, 0, h->cast_tables, s));
+    h->weights_valid = h->tables_live = true;
+    h->weights_changed = false;
+  }
+  if (tables && h->tables_live) {
+    FEMTO_TRY(cast_range(h, theta, h->cast_tables, h->cast_blocks, s));
+    h->tables_live = false;
+  }
   return 0;
 }
 
@@ -412,7 +433,8 @@ static int step_t(femto_handle* h, const float* theta, float* delta, const int* 
   const int* docs = h->cfg.doc_mask ? h->doc_start : nullptr;
 
   // ---- forward (src/gpt.jl:129-170) ----
-  FEMTO_TRY(S::embed_norm((const T*)h->sh_wte, h->tok0, (T*)h->xe, N, d, eps, s));
+  const bool live = h->tables_live;      // rows of the tables come from Theta
+  FEMTO_TRY(S::embed_norm((const T*)h->sh_wte, h->tok0, (T*)h->xe, N, d, eps, s, live ? theta + h->off_wte : nullptr));
   FEMTO_TRY(S::smear((const T*)h->xe, theta + h->off_smear, theta + h->off_lam_s, N, Tl, d, h->sg, (T*)h->x0, s));
   for (int i = 0; i < L; i++) {
     const LayerP& p = h->lp[i];
@@ -422,7 +444,7 @@ static int step_t(femto_handle* h, const float* theta, float* delta, const int* 
     FEMTO_TRY(lin_fwd(l.xn1, d, l.sh_wqkv, dq, l.qkv, dq, EPI_STORE, nullptr));
     FEMTO_TRY(S::qkv_post((T*)l.qkv, dq, (const T*)l.xn1, d, p.ve ? theta + p.ve_gate : nullptr,
                           p.ve ? (const T*)l.sh_ve : nullptr, h->tok0, h->pos, h->sin_t, h->cos_t, N, H, Hkv, hd, eps,
-                          l.rqk, l.sv, s));
+                          l.rqk, l.sv, s, live && p.ve ? theta + p.ve_table : nullptr));
     AttnArgs a;
     a.Q = l.qkv; a.K = (const T*)l.qkv + d; a.V = (const T*)l.qkv + d + kv; a.q_stride = dq; a.kv_stride = dq;
     a.O = l.att; a.o_stride = d; a.lse = l.lse; a.B = B; a.T = Tl; a.H = H; a.Hkv = Hkv; a.hd = hd;
@@ -612,11 +634,12 @@ int model_step(femto_handle* h, const float* theta, float* delta, const int* tok
   if (B <= 0 || B > h->maxB) return femto_fail(FEMTO_ERR_SHAPE, "B=%d outside 1..max_batch=%d", B, h->maxB);
   if (reduction != FEMTO_REDUCTION_SUM && reduction != FEMTO_REDUCTION_MEAN)
     return femto_fail(FEMTO_ERR_ARG, "reduction must be FEMTO_REDUCTION_SUM or FEMTO_REDUCTION_MEAN");
-  if (!h->weights_valid) return femto_fail(FEMTO_ERR_STATE, "call femto_refresh_weights before the first step");
+  if (!h->weights_valid && !h->weights_changed) return femto_fail(FEMTO_ERR_STATE, "call femto_refresh_weights before the first step");
   if (!aligned16(theta) || (delta && !aligned16(delta))) return femto_fail(FEMTO_ERR_ALIGN, "Theta/delta must be 16-byte aligned");
   // A training step runs on the handle's own two streams, bracketed by the caller's stream on both sides; every
   // other call (loss only, logits, a prompt) is one dependency chain and stays on the caller's stream.
   const bool two = backward && h->hi && h->lo && !gemm_profiling();
+  FEMTO_TRY(model_ensure_weights(h, theta, backward, s));
   cudaStream_t chain = two ? h->hi : s;
   if (two) {
     cudaEvent_t e = h->ev_fork[h->ev_next++ % femto_handle::N_FORK];

@@ -40,8 +40,10 @@ struct femto_handle {
   void *sh_wte = nullptr, *sh_lm = nullptr;
   char *weights_begin = nullptr, *weights_end = nullptr;   // the contiguous range holding every compute-type weight
   bool weights_valid = false;
+  bool weights_changed = false;   // Theta was written since: the next call that reads the copies makes them from the Theta it is given
+  bool tables_live = false;       // ... all but those of the embedding tables, whose rows calls that do not train read from their Theta
   struct CastJob* cast_jobs = nullptr;   // device table of model_refresh
-  int n_cast_jobs = 0, cast_blocks = 0;
+  int n_cast_jobs = 0, cast_blocks = 0, cast_tables = 0;      // blocks from cast_tables on are the embedding tables
   int *tok0 = nullptr, *tgt0 = nullptr, *pos = nullptr, *doc_start = nullptr, *raw_tok = nullptr, *raw_tgt = nullptr,
       *raw_pos = nullptr;
   void *xe = nullptr, *x0 = nullptr, *xm = nullptr, *xnf = nullptr;
@@ -95,6 +97,7 @@ int model_fill(femto_handle* h, const femto_config* cfg);  // derived sizes + la
 int model_alloc(femto_handle* h);
 void model_free(femto_handle* h);
 int model_refresh(femto_handle* h, const float* theta, cudaStream_t s);
+int model_ensure_weights(femto_handle* h, const float* theta, bool tables, cudaStream_t s);   // makes the copies that have to be made
 int model_step(femto_handle* h, const float* theta, float* delta, const int* tokens, const int* targets,
                const int* positions, int B, int reduction, bool backward, bool accumulate, float* loss_out,
                int* nvalid_out, cudaStream_t s, float* logits_out = nullptr, float* token_losses_out = nullptr,

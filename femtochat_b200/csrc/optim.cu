@@ -839,6 +839,7 @@ int optimizer_step(femto_optimizer* o, float* theta, const float* delta, float e
   if (!(n_tokens > 0.f)) return femto_fail(FEMTO_ERR_ARG, "n_tokens must be positive");
   const bool sharded = o->shard_world > 1;
   femto_handle* h = o->h;
+  FEMTO_TRY(model_ensure_weights(h, theta, true, s));      // the update writes the copies of what it updates only
   const size_t es_model = h->bf ? 2 : 4;
   // The AdamW tables are pure HBM streaming and touch nothing the Muon groups touch: on the handle's low-priority
   // stream they run under the Polar Express GEMMs of the Muon groups instead of before them.

@@ -47,16 +47,30 @@ __global__ void k_prep_tokens(const int* tokens, const int* targets, const int* 
   doc_start[i] = max(0, t - p);
 }
 
-template <typename T, int V>
-__global__ void __launch_bounds__(256) k_embed_norm(const T* __restrict__ table, const int* __restrict__ tok0,
+// V neighbouring values of a table of T, or of fp32 values that become T here (pairs: Theta's tensors start at even offsets)
+template <typename T, int V, typename E> __device__ __forceinline__ void load_table(const E* p, float (&f)[V]) {
+  if constexpr (sizeof(E) == sizeof(T)) {
+    load_vec<T, V>(reinterpret_cast<const T*>(p), f);
+  } else if constexpr (V == 1) {
+    f[0] = round_to<T>(p[0]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < V; i += 2) {
+      const float2 q = *reinterpret_cast<const float2*>(p + i);
+      f[i] = round_to<T>(q.x); f[i + 1] = round_to<T>(q.y);
+    }
+  }
+}
+template <typename T, int V, typename E>
+__global__ void __launch_bounds__(256) k_embed_norm(const E* __restrict__ table, const int* __restrict__ tok0,
                                                     T* __restrict__ xe, int N, int D, float eps) {
   pdl_trigger();
   ROW_SETUP();
-  const T* src = table + (long long)tok0[row] * D;
+  const E* src = table + (long long)tok0[row] * D;
   float ss = 0.f;
   for (int c = lane * V; c < D; c += 32 * V) {
     float f[V];
-    load_vec<T, V>(src + c, f);
+    load_table<T, V, E>(src + c, f);
 #pragma unroll
     for (int i = 0; i < V; i++) ss += f[i] * f[i];
   }
@@ -65,7 +79,7 @@ __global__ void __launch_bounds__(256) k_embed_norm(const T* __restrict__ table,
   T* dst = xe + row * D;
   for (int c = lane * V; c < D; c += 32 * V) {
     float f[V];
-    load_vec<T, V>(src + c, f);
+    load_table<T, V, E>(src + c, f);
 #pragma unroll
     for (int i = 0; i < V; i++) f[i] *= inv;
     store_vec<T, V>(dst + c, f);
@@ -208,10 +222,10 @@ __global__ void __launch_bounds__(256) k_backout_norm(const T* __restrict__ xl, 
 }
 
 // One warp per (token, slot): slots [0,H) = query heads, [H,H+Hkv) = key heads, then value heads.
-template <typename T>
+template <typename T, typename E>
 __global__ void __launch_bounds__(256) k_qkv_post(T* __restrict__ qkv, long long ldq, const T* __restrict__ xn1,
                                                   int D, const float* __restrict__ ve_gate,
-                                                  const T* __restrict__ ve_table, const int* __restrict__ tok0,
+                                                  const E* __restrict__ ve_table, const int* __restrict__ tok0,
                                                   const int* __restrict__ pos, const float* __restrict__ sin_t,
                                                   const float* __restrict__ cos_t, long long N, int H, int Hkv,
                                                   int hd, float eps, float* __restrict__ rqk,
@@ -253,8 +267,12 @@ __global__ void __launch_bounds__(256) k_qkv_post(T* __restrict__ qkv, long long
     pre = warp_sum(pre);
     const float sig = 1.f / (1.f + expf(-pre));
     if (lane == 0) sv[n * Hkv + kvh] = sig;
-    const T* ve = ve_table + (long long)tok0[n] * (Hkv * hd) + (long long)kvh * hd;
-    for (int d = lane; d < hd; d += 32) base[d] = from_f<T>(to_f<T>(base[d]) + 3.f * sig * to_f<T>(ve[d]));
+    const E* ve = ve_table + (long long)tok0[n] * (Hkv * hd) + (long long)kvh * hd;
+    for (int d = lane; d < hd; d += 32) {
+      float v[1];
+      load_table<T, 1, E>(ve + d, v);
+      base[d] = from_f<T>(to_f<T>(base[d]) + 3.f * sig * v[0]);
+    }
   }
 }
 
@@ -343,9 +361,9 @@ template <typename T> __device__ __forceinline__ void store8(T* p, const float (
   }
 }
 
-template <typename T>
+template <typename T, typename E>
 __global__ void __launch_bounds__(256) k_qkv_post_128(T* __restrict__ qkv, long long ldq, const T* __restrict__ xn1, int D,
-                                                      const float* __restrict__ ve_gate, const T* __restrict__ ve_table,
+                                                      const float* __restrict__ ve_gate, const E* __restrict__ ve_table,
                                                       const int* __restrict__ tok0, const int* __restrict__ pos,
                                                       const float* __restrict__ sin_t, const float* __restrict__ cos_t,
                                                       long long N, int H, int Hkv, float eps, float* __restrict__ rqk,
@@ -390,10 +408,11 @@ __global__ void __launch_bounds__(256) k_qkv_post_128(T* __restrict__ qkv, long 
     pre = oct_sum(pre);
     const float sig = 1.f / (1.f + expf(-pre));
     if (live && sub == 0) sv[n * Hkv + kvh] = sig;
-    const T* ve = ve_table + (long long)tok0[n] * (Hkv * hd) + (long long)kvh * hd + sub * 16;
+    const E* ve = ve_table + (long long)tok0[n] * (Hkv * hd) + (long long)kvh * hd + sub * 16;
     float a[8], b[8], e0[8], e1[8];
     load8<T>(base + sub * 16, a); load8<T>(base + sub * 16 + 8, b);
-    load8<T>(ve, e0); load8<T>(ve + 8, e1);
+    if constexpr (sizeof(E) == sizeof(T)) { load8<T>(reinterpret_cast<const T*>(ve), e0); load8<T>(reinterpret_cast<const T*>(ve) + 8, e1); }
+    else { load_table<T, 8, E>(ve, e0); load_table<T, 8, E>(ve + 8, e1); }
 #pragma unroll
     for (int i = 0; i < 8; i++) { a[i] += 3.f * sig * e0[i]; b[i] += 3.f * sig * e1[i]; }
     if (live) { store8<T>(base + sub * 16, a); store8<T>(base + sub * 16 + 8, b); }
@@ -775,17 +794,18 @@ __global__ void __launch_bounds__(256) k_xent_rows(const float* __restrict__ log
 // The compute-type copy of every weight in one launch: blocks of CAST_BLOCK elements, each of one job of the table.  Bound by HBM (4 bytes
 // in, 2 out per weight); one launch per tensor with one element per thread and step reached 3.7 TB/s, this 7.0 (d20: 1.55 -> 0.81 ms).
 template <typename T>
-__global__ void __launch_bounds__(256) k_cast_all(const float* __restrict__ theta, const CastJob* __restrict__ jobs, int n_jobs) {
+__global__ void __launch_bounds__(256) k_cast_all(const float* __restrict__ theta, const CastJob* __restrict__ jobs, int n_jobs, int first) {
   pdl_trigger();
+  const int block = first + blockIdx.x;
   int lo = 0, hi = n_jobs - 1;
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
-    if (jobs[mid].first_block <= (int)blockIdx.x) lo = mid; else hi = mid - 1;
+    if (jobs[mid].first_block <= block) lo = mid; else hi = mid - 1;
   }
   const CastJob j = jobs[lo];
   const float* src = theta + j.src;
   T* dst = reinterpret_cast<T*>(j.dst);
-  const long long i0 = (long long)((int)blockIdx.x - j.first_block) * CAST_BLOCK;
+  const long long i0 = (long long)(block - j.first_block) * CAST_BLOCK;
   constexpr int V = 8, STEPS = CAST_BLOCK / (256 * V);
   if (j.vec && (reinterpret_cast<uintptr_t>(src) & 7) == 0) {       // Theta's tensors start at even offsets
     float2 f[STEPS][V / 2];
@@ -807,7 +827,6 @@ __global__ void __launch_bounds__(256) k_cast_all(const float* __restrict__ thet
   }
   for (long long i = i0 + threadIdx.x; i < i0 + CAST_BLOCK && i < j.n; i += 256) dst[i / j.cols * j.ldd + i % j.cols] = from_f<T>(src[i]);
 }
-
 __global__ void __launch_bounds__(1024) k_sum_rows(const float* __restrict__ rows, int n, float* out,
                                                    const int* __restrict__ tgt0, int* n_valid_out,
                                                    float scale_by_valid) {
@@ -929,8 +948,10 @@ int Stream<T>::prep_tokens(const int* tokens, const int* targets, const int* pos
   return 0;
 }
 template <typename T>
-int Stream<T>::embed_norm(const T* table, const int* tok0, T* xe, int N, int D, float eps, cudaStream_t s) {
-  DISPATCH_V(D % VecN<T>::n == 0, k_embed_norm<T, V><<<row_grid(N), 256, 0, s>>>(table, tok0, xe, N, D, eps);)
+int Stream<T>::embed_norm(const T* table, const int* tok0, T* xe, int N, int D, float eps, cudaStream_t s, const float* table32) {
+  // (fp32 rows as T = fp32 are read 16 bytes at a time)
+  if (table32) DISPATCH_V(D % VecN<T>::n == 0 && (reinterpret_cast<uintptr_t>(table32) & (sizeof(T) == 4 ? 15 : 7)) == 0, (k_embed_norm<T, V, float><<<row_grid(N), 256, 0, s>>>(table32, tok0, xe, N, D, eps));)
+  else DISPATCH_V(D % VecN<T>::n == 0, (k_embed_norm<T, V, T><<<row_grid(N), 256, 0, s>>>(table, tok0, xe, N, D, eps));)
   KERNEL_CHECK();
   return 0;
 }
@@ -957,14 +978,16 @@ template <typename T> int Stream<T>::norm(const T* x, T* xn, float* r, int N, in
 template <typename T>
 int Stream<T>::qkv_post(T* qkv, long long ldq, const T* xn1, int D, const float* ve_gate, const T* ve_table,
                         const int* tok0, const int* pos, const float* sin_t, const float* cos_t, int N, int H,
-                        int Hkv, int hd, float eps, float* rqk, float* sv, cudaStream_t s) {
+                        int Hkv, int hd, float eps, float* rqk, float* sv, cudaStream_t s, const float* ve32) {
   long long warps = (long long)N * (H + 2 * Hkv);
-  if (hd == 128 && ldq % 8 == 0 && aligned16(qkv) && (!ve_table || aligned16(ve_table)))
-    k_qkv_post_128<T><<<cdiv(warps, 32), 256, 0, s>>>(qkv, ldq, xn1, D, ve_gate, ve_table, tok0, pos, sin_t, cos_t, N, H,
-                                                     Hkv, eps, rqk, sv);
-  else
-    k_qkv_post<T><<<cdiv(warps, WPB), 256, 0, s>>>(qkv, ldq, xn1, D, ve_gate, ve_table, tok0, pos, sin_t, cos_t, N, H,
-                                                  Hkv, hd, eps, rqk, sv);
+  const bool wide = hd == 128 && ldq % 8 == 0 && aligned16(qkv);
+  auto launch = [&](auto* ve, bool aligned) {
+    typedef std::remove_const_t<std::remove_pointer_t<decltype(ve)>> E;
+    if (wide && aligned) k_qkv_post_128<T, E><<<cdiv(warps, 32), 256, 0, s>>>(qkv, ldq, xn1, D, ve_gate, ve, tok0, pos, sin_t, cos_t, N, H, Hkv, eps, rqk, sv);
+    else k_qkv_post<T, E><<<cdiv(warps, WPB), 256, 0, s>>>(qkv, ldq, xn1, D, ve_gate, ve, tok0, pos, sin_t, cos_t, N, H, Hkv, hd, eps, rqk, sv);
+  };
+  if (ve32) launch(ve32, (reinterpret_cast<uintptr_t>(ve32) & (sizeof(T) == 4 ? 15 : 7)) == 0);
+  else launch(ve_table, !ve_table || aligned16(ve_table));
   KERNEL_CHECK();
   return 0;
 }
@@ -1065,8 +1088,9 @@ int Stream<T>::xent_rows(const float* logits, long long ldl, const int* tgt0, in
   KERNEL_CHECK();
   return 0;
 }
-template <typename T> int Stream<T>::cast_all(const float* theta, const CastJob* jobs, int n_jobs, int blocks, cudaStream_t s) {
-  k_cast_all<T><<<blocks, 256, 0, s>>>(theta, jobs, n_jobs);
+template <typename T> int Stream<T>::cast_all(const float* theta, const CastJob* jobs, int n_jobs, int from, int to, cudaStream_t s) {
+  if (to <= from) return 0;
+  k_cast_all<T><<<to - from, 256, 0, s>>>(theta, jobs, n_jobs, from);
   KERNEL_CHECK();
   return 0;
 }

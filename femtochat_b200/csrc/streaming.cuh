@@ -16,7 +16,8 @@ template <typename T> struct Stream {
   static int prep_tokens(const int* tokens, const int* targets, const int* positions, int B, int Tlen,
                          int index_base, int vocab, int maxdoc, int* tok0, int* tgt0, int* pos, int* doc_start,
                          unsigned int* status, cudaStream_t s);
-  static int embed_norm(const T* table, const int* tok0, T* xe, int N, int D, float eps, cudaStream_t s);
+  // `table` of T, or fp32 rows (`table32`) that are rounded to T on their way
+  static int embed_norm(const T* table, const int* tok0, T* xe, int N, int D, float eps, cudaStream_t s, const float* table32 = nullptr);
   static int smear(const T* xe, const float* w_s, const float* lam_s, int N, int Tlen, int D, float* sg, T* x0,
                    cudaStream_t s);
   static int mix_norm(const T* xin, const T* x0, const float* lam_b, const float* lam_x0, T* xm, T* xn, float* r,
@@ -24,7 +25,7 @@ template <typename T> struct Stream {
   static int norm(const T* x, T* xn, float* r, int N, int D, float eps, cudaStream_t s);
   static int qkv_post(T* qkv, long long ldq, const T* xn1, int D, const float* ve_gate, const T* ve_table,
                       const int* tok0, const int* pos, const float* sin_t, const float* cos_t, int N, int H,
-                      int Hkv, int hd, float eps, float* rqk, float* sv, cudaStream_t s);
+                      int Hkv, int hd, float eps, float* rqk, float* sv, cudaStream_t s, const float* ve32 = nullptr);
   static int qkv_post_bwd(T* dqkv, const T* qkv, long long ldq, const T* ve_table, const int* tok0,
                           const int* pos, const float* sin_t, const float* cos_t, int N, int H, int Hkv, int hd,
                           const float* rqk, const float* sv, T* dve, float* dpre, cudaStream_t s);
@@ -49,7 +50,7 @@ template <typename T> struct Stream {
   static int xent_rows(const float* logits, long long ldl, const int* tgt0, int n, int V, float w,
                        const float* w_dev, T* dlogit,
                        long long lddl, float* loss_rows, cudaStream_t s);
-  static int cast_all(const float* theta, const CastJob* jobs, int n_jobs, int blocks, cudaStream_t s);
+  static int cast_all(const float* theta, const CastJob* jobs, int n_jobs, int from, int to, cudaStream_t s);      // blocks [from, to) of the jobs
 };
 
 int sum_rows_to_scalar(const float* rows, int n, float* out, const int* tgt0, int* n_valid_out, float scale_by_valid,

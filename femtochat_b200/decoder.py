@@ -189,6 +189,8 @@ class DecoderState(Handle):
             super().refresh_weights(theta)
             self._packed = now
 
+    refresh_for = refresh_weights
+
 
 class Decoder:
     """The model: Θ (flat fp32 on the device), its configuration and layout.  Same face as GPT towards `prefill`,

@@ -45,7 +45,7 @@ def prefill(model, cache: KVCache, tokens, positions=None):
     tok, pos = _dev_i32(tokens), _dev_i32(positions)
     B, Tp = tok.shape
     st = cache.state
-    st.refresh_weights(model.params.theta)
+    st.refresh_for(model.params.theta)
     out = torch.empty(B, model.config.vocab_size, device="cuda", dtype=torch.float32)
     _lib.check(_lib.lib().femto_prefill(st.h, cache.c, _lib.ptr(model.params.theta), _lib.ptr(tok), _lib.ptr(pos), B, Tp,
                                         _lib.ptr(out), _lib.stream_ptr()))

@@ -174,7 +174,7 @@ class GPT:
             return self.logits(tokens, positions)
         tok, tgt, pos = _dev_i32(tokens), _dev_i32(targets), _dev_i32(positions)
         st = self.state(tok.shape[0])
-        st.refresh_weights(self.params.theta)
+        st.refresh_for(self.params.theta)
         if reduction == "none":   # per-token losses [B][T] (src/gpt.jl:191-193)
             import torch
             out = torch.empty(tok.shape[0], tok.shape[1], device="cuda", dtype=torch.float32)
@@ -191,7 +191,7 @@ class GPT:
         import torch
         tok, pos = _dev_i32(tokens), _dev_i32(positions)
         st = self.state(tok.shape[0])
-        st.refresh_weights(self.params.theta)
+        st.refresh_for(self.params.theta)
         out = torch.empty(tok.shape[0], tok.shape[1], self.config.vocab_size, device="cuda", dtype=torch.float32)
         _lib.check(_lib.lib().femto_forward_logits(st.h, _lib.ptr(self.params.theta), _lib.ptr(tok), _lib.ptr(pos),
                                                    tok.shape[0], _lib.ptr(out), _lib.stream_ptr()))

@@ -13,6 +13,10 @@ class Handle:
     def refresh_weights(self, theta) -> None:
         _lib.check(_lib.lib().femto_refresh_weights(self.h, _lib.ptr(theta), _lib.stream_ptr()))
 
+    def refresh_for(self, theta) -> None:
+        """For the library call with this Θ that follows: it makes the compute-type weights that it needs from it."""
+        _lib.check(_lib.lib().femto_weights_changed(self.h))
+
     def status_word(self) -> int:
         out = C.c_int32(0)
         _lib.check(_lib.lib().femto_status_word(self.h, C.byref(out)))

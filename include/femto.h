@@ -93,6 +93,10 @@ int32_t femto_window_sizes(const femto_config* h_cfg, int32_t* h_left, int32_t* 
  * master weights on every Linear call (src/gpt.jl:27); here the cast happens once per update.
  * Call after any external write to Theta; femto_optimizer_step does it itself. */
 int32_t femto_refresh_weights(femto_handle* h, const float* theta, void* stream);
+/* Says that Theta was written: the next call that needs the copies makes them from the Theta it is given, as if femto_refresh_weights had
+ * been called with it just before.  Calls that do not train need none of the embedding tables: until one that does, or
+ * femto_refresh_weights, they read the rows of their tokens from the Theta they are given, as they read gates and scalars. */
+int32_t femto_weights_changed(femto_handle* h);
 
 /* loss_and_gradient! (ext/FemtoChatEnzymeExt.jl:38-44) with the training script's accumulation
  * (scripts/train.jl:117-131): delta = (accumulate ? delta : 0) + d loss / d Theta.

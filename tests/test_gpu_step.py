@@ -498,6 +498,54 @@ def _bf16_server(B, H, G, L, T, doc_mask, vocab=1000):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("ctype,d,heads,kv", [("bfloat16", 256, 2, 1), ("bfloat16", 96, 3, 3), ("float32", 256, 2, 1), ("float32", 64, 4, 2)])
+def test_calls_that_do_not_train_read_embedding_rows_from_theta(ctype, d, heads, kv):
+    """After Theta was written, a loss, a prompt and the tokens after it leave the compute-type copies of the embedding tables as they were
+    and read rows of Theta instead: the same bits as a handle whose copies were all made.  A training step on that handle makes
+    them first.  Heads of 128 and of other sizes (both kernels behind the projections, the resident and the other decode step)."""
+    cfg = fb.GPTConfig(sequence_len=40, max_document_tokens=64, vocab_size=300, n_layer=3, n_head=heads, n_kv_head=kv, n_embed=d, window_pattern="SL")
+    lay = fb.parameter_layout(cfg)
+    theta = torch.zeros(lay.nparams, device="cuda")
+    fb.initialize_(theta, lay, seed=5, all_nonzero=True)
+    params = fb.Params(theta)
+    g = torch.Generator(device="cuda").manual_seed(9)
+    tok, tgt = (torch.randint(1, 301, (2, 40), generator=g, device="cuda", dtype=torch.int32) for _ in range(2))
+
+    def fresh():
+        model = fb.GPT(params, cfg, lay, compute_type=ctype)
+        model.state(2).refresh_weights(theta)
+        return model
+
+    def serve(model, whole):
+        kc = fb.KVCache(model.state(2), 2, 40)
+        out = [fb.prefill(model, kc, tok[:, :20])]
+        if whole:
+            model.state(2).refresh_weights(theta)
+        out += [fb.decode_step(model, kc, tok[:, t]) for t in range(20, 24)]
+        kc.close()
+        return torch.stack(out)
+
+    model = fb.GPT(params, cfg, lay, compute_type=ctype)
+    model(tok, tgt, reduction="none")
+    theta[lay.embedding.offset:lay.embedding.offset + lay.embedding.size].mul_(-0.5)
+    for b in lay.blocks:
+        if b["ve_table"] is not None:
+            theta[b["ve_table"].offset:b["ve_table"].offset + b["ve_table"].size].add_(0.3)
+    served = serve(model, False)
+    assert torch.equal(served, serve(fresh(), True))
+    other = fresh()
+    _lib.check(_lib.lib().femto_forward_loss(other.state(2).h, _lib.ptr(theta), _lib.ptr(tok), _lib.ptr(tgt), None, 2, _lib.REDUCTION["sum"],
+                                             _lib.ptr(other.state(2)._loss), _lib.ptr(other.state(2)._nvalid), None))
+    assert model(tok, tgt, reduction="sum") == float(other.state(2)._loss)
+    deltas = []
+    for m in (model, other):
+        params.delta.zero_()
+        fb.loss_and_gradient_(params, m.state(2), lay, tok, tgt)
+        deltas.append(params.delta.clone())
+    assert torch.equal(deltas[0], deltas[1]) and float(deltas[0].abs().max()) > 0
+
+
+@pytest.mark.gpu
 def test_decode_steps_of_several_models_in_turn():
     """Caches of a wide and of a narrow model are alive together and decode alternately: neither's size limits the other's launches."""
     made = [_bf16_server(2, H, G, 2, 24, False) for H, G in ((8, 8), (2, 1), (4, 2))]
