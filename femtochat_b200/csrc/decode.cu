@@ -66,19 +66,6 @@ __global__ void k_kv_append(const T* __restrict__ qkv, long long ldq, int d, int
   Kc[((long long)b * maxT + t) * kv + c] = row[d + c];
   Vc[((long long)b * maxT + t) * kv + c] = row[d + kv + c];
 }
-// The prompt's K / V rows [B][Tp] of one block into the cache.
-template <typename T>
-__global__ void k_kv_prefill(const T* __restrict__ qkv, long long ldq, int d, int kv, T* __restrict__ Kc, T* __restrict__ Vc,
-                             int maxT, int Tp, int B) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (long long)B * Tp * kv) return;
-  const int c = (int)(i % kv);
-  const long long bt = i / kv;
-  const int b = (int)(bt / Tp), t = (int)(bt % Tp);
-  const T* row = qkv + bt * ldq;
-  Kc[((long long)b * maxT + t) * kv + c] = row[d + c];
-  Vc[((long long)b * maxT + t) * kv + c] = row[d + kv + c];
-}
 template <typename T>
 __global__ void k_take_last_rows(const T* __restrict__ x, int Tp, int D, int B, T* __restrict__ out) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -313,11 +300,7 @@ static int decode_attention(femto_kv_cache* c, int layer, const T* qkv, long lon
 template <typename T> int kv_cache_store_prompt(femto_kv_cache* c, int B, int Tp, cudaStream_t s) {
   femto_handle* h = c->h;
   if (B > c->maxB || Tp > c->maxT) return femto_fail(FEMTO_ERR_SHAPE, "prompt [%d][%d] exceeds the cache [%d][%d]", B, Tp, c->maxB, c->maxT);
-  for (int i = 0; i < h->L; i++) {
-    const long long n = (long long)B * Tp * h->kv;
-    k_kv_prefill<T><<<cdiv(n, 256), 256, 0, s>>>((const T*)h->lb[i].qkv, h->dq, h->d, h->kv, (T*)c->K[i], (T*)c->V[i], c->maxT, Tp, B);
-    KERNEL_CHECK();
-  }
+  // (the blocks' keys and values are there: the kernel behind the projections leaves them, see PromptCache)
   k_take_last_rows<T><<<cdiv((long long)B * h->d, 256), 256, 0, s>>>((const T*)h->xe, Tp, h->d, B, (T*)c->xe_prev);
   KERNEL_CHECK();
   k_take_last_pos<<<cdiv(B, 128), 128, 0, s>>>(h->pos, Tp, B, c->lastpos);
@@ -489,7 +472,7 @@ extern "C" int32_t femto_prefill(femto_handle* h, femto_kv_cache* c, const float
   }
   if ((long long)B * Tp > h->maxN) return femto_fail(FEMTO_ERR_SHAPE, "prompt of %d x %d tokens exceeds the workspace (%d tokens)", B, Tp, h->maxN);
   StepExtra ex;
-  ex.T = Tp; ex.cache = c; ex.last_logits = logits_out;
+  ex.T = Tp; ex.cache = c; ex.last_logits = logits_out; ex.K = c->K.data(); ex.V = c->V.data(); ex.maxT = c->maxT;
   return model_step(h, theta, nullptr, tokens, nullptr, positions, B, FEMTO_REDUCTION_SUM, false, false, nullptr, nullptr,
                     (cudaStream_t)stream, nullptr, nullptr, &ex);
 }

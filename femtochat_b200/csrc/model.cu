@@ -442,9 +442,11 @@ static int step_t(femto_handle* h, const float* theta, float* delta, const int* 
     const T* xin = i == 0 ? (const T*)h->x0 : (const T*)h->lb[i - 1].xout;
     FEMTO_TRY(S::mix_norm(xin, (const T*)h->x0, theta + p.lam_b, theta + p.lam_x0, (T*)h->xm, (T*)l.xn1, l.r1, N, d, eps, s));
     FEMTO_TRY(lin_fwd(l.xn1, d, l.sh_wqkv, dq, l.qkv, dq, EPI_STORE, nullptr));
+    PromptCache<T> pc;
+    if (ex && ex->cache) { pc.K = (T*)ex->K[i]; pc.V = (T*)ex->V[i]; pc.T_ = Tl; pc.maxT = ex->maxT; }
     FEMTO_TRY(S::qkv_post((T*)l.qkv, dq, (const T*)l.xn1, d, p.ve ? theta + p.ve_gate : nullptr,
                           p.ve ? (const T*)l.sh_ve : nullptr, h->tok0, h->pos, h->sin_t, h->cos_t, N, H, Hkv, hd, eps,
-                          l.rqk, l.sv, s, live && p.ve ? theta + p.ve_table : nullptr));
+                          l.rqk, l.sv, s, live && p.ve ? theta + p.ve_table : nullptr, pc));
     AttnArgs a;
     a.Q = l.qkv; a.K = (const T*)l.qkv + d; a.V = (const T*)l.qkv + d + kv; a.q_stride = dq; a.kv_stride = dq;
     a.O = l.att; a.o_stride = d; a.lse = l.lse; a.B = B; a.T = Tl; a.H = H; a.Hkv = Hkv; a.hd = hd;

@@ -88,6 +88,8 @@ struct femto_kv_cache;
 struct StepExtra {
   int T = 0;                        // rows per column of this call (0 = sequence_len)
   femto_kv_cache* cache = nullptr;  // filled from the prompt when set
+  void* const *K = nullptr, * const *V = nullptr;   // the cache's keys and values of every block, maxT rows a column
+  int maxT = 0;
   float* last_logits = nullptr;     // fp32 [B][vocab_size]: soft-capped logits of each column's last position
 };
 template <typename T> int kv_cache_store_prompt(femto_kv_cache* c, int B, int Tp, cudaStream_t s);

@@ -229,7 +229,7 @@ __global__ void __launch_bounds__(256) k_qkv_post(T* __restrict__ qkv, long long
                                                   const int* __restrict__ pos, const float* __restrict__ sin_t,
                                                   const float* __restrict__ cos_t, long long N, int H, int Hkv,
                                                   int hd, float eps, float* __restrict__ rqk,
-                                                  float* __restrict__ sv) {
+                                                  float* __restrict__ sv, const PromptCache<T> pc) {
   pdl_trigger();
   const int lane = threadIdx.x & 31;
   const int nslot = H + 2 * Hkv;
@@ -259,6 +259,7 @@ __global__ void __launch_bounds__(256) k_qkv_post(T* __restrict__ qkv, long long
       float y1 = round_to<T>(x1 * c + x2 * s), y2 = round_to<T>(-x1 * s + x2 * c);
       base[p] = from_f<T>(y1 * g);
       base[p + half] = from_f<T>(y2 * g);
+      if (slot >= H && pc.K) { T* k = pc.row(pc.K, n, Hkv * hd) + (slot - H) * hd; k[p] = from_f<T>(y1 * g); k[p + half] = from_f<T>(y2 * g); }
     }
   } else if (ve_table != nullptr) {
     const int kvh = slot - H - Hkv;
@@ -272,7 +273,11 @@ __global__ void __launch_bounds__(256) k_qkv_post(T* __restrict__ qkv, long long
       float v[1];
       load_table<T, 1, E>(ve + d, v);
       base[d] = from_f<T>(to_f<T>(base[d]) + 3.f * sig * v[0]);
+      if (pc.V) pc.row(pc.V, n, Hkv * hd)[kvh * hd + d] = base[d];
     }
+  } else if (pc.V) {
+    T* v = pc.row(pc.V, n, Hkv * hd) + (slot - H - Hkv) * hd;
+    for (int d = lane; d < hd; d += 32) v[d] = base[d];
   }
 }
 
@@ -367,7 +372,7 @@ __global__ void __launch_bounds__(256) k_qkv_post_128(T* __restrict__ qkv, long 
                                                       const int* __restrict__ tok0, const int* __restrict__ pos,
                                                       const float* __restrict__ sin_t, const float* __restrict__ cos_t,
                                                       long long N, int H, int Hkv, float eps, float* __restrict__ rqk,
-                                                      float* __restrict__ sv) {
+                                                      float* __restrict__ sv, const PromptCache<T> pc) {
   pdl_trigger();
   constexpr int hd = 128, half = 64;
   const int sub = threadIdx.x & 7;
@@ -400,6 +405,10 @@ __global__ void __launch_bounds__(256) k_qkv_post_128(T* __restrict__ qkv, long 
 #pragma unroll
     for (int i = 0; i < 8; i++) { x1[i] *= g; x2[i] *= g; }
     if (live) { store8<T>(base + sub * 8, x1); store8<T>(base + half + sub * 8, x2); }
+    if (live && slot >= H && pc.K) {
+      T* k = pc.row(pc.K, n, Hkv * hd) + (slot - H) * hd + sub * 8;
+      store8<T>(k, x1); store8<T>(k + half, x2);
+    }
   } else if (ve_table != nullptr) {
     const int kvh = slot - H - Hkv;
     // gate input: the first 12 channels of the normed block input, two per lane for lanes 0-3
@@ -416,6 +425,11 @@ __global__ void __launch_bounds__(256) k_qkv_post_128(T* __restrict__ qkv, long 
 #pragma unroll
     for (int i = 0; i < 8; i++) { a[i] += 3.f * sig * e0[i]; b[i] += 3.f * sig * e1[i]; }
     if (live) { store8<T>(base + sub * 16, a); store8<T>(base + sub * 16 + 8, b); }
+    if (live && pc.V) { T* v = pc.row(pc.V, n, Hkv * hd) + kvh * hd + sub * 16; store8<T>(v, a); store8<T>(v + 8, b); }
+  } else if (pc.V) {
+    float a[8], b[8];
+    load8<T>(base + sub * 16, a); load8<T>(base + sub * 16 + 8, b);
+    if (live) { T* v = pc.row(pc.V, n, Hkv * hd) + (slot - H - Hkv) * hd + sub * 16; store8<T>(v, a); store8<T>(v + 8, b); }
   }
 }
 
@@ -978,13 +992,13 @@ template <typename T> int Stream<T>::norm(const T* x, T* xn, float* r, int N, in
 template <typename T>
 int Stream<T>::qkv_post(T* qkv, long long ldq, const T* xn1, int D, const float* ve_gate, const T* ve_table,
                         const int* tok0, const int* pos, const float* sin_t, const float* cos_t, int N, int H,
-                        int Hkv, int hd, float eps, float* rqk, float* sv, cudaStream_t s, const float* ve32) {
+                        int Hkv, int hd, float eps, float* rqk, float* sv, cudaStream_t s, const float* ve32, const PromptCache<T>& pc) {
   long long warps = (long long)N * (H + 2 * Hkv);
-  const bool wide = hd == 128 && ldq % 8 == 0 && aligned16(qkv);
+  const bool wide = hd == 128 && ldq % 8 == 0 && aligned16(qkv) && aligned16(pc.K) && aligned16(pc.V);
   auto launch = [&](auto* ve, bool aligned) {
     typedef std::remove_const_t<std::remove_pointer_t<decltype(ve)>> E;
-    if (wide && aligned) k_qkv_post_128<T, E><<<cdiv(warps, 32), 256, 0, s>>>(qkv, ldq, xn1, D, ve_gate, ve, tok0, pos, sin_t, cos_t, N, H, Hkv, eps, rqk, sv);
-    else k_qkv_post<T, E><<<cdiv(warps, WPB), 256, 0, s>>>(qkv, ldq, xn1, D, ve_gate, ve, tok0, pos, sin_t, cos_t, N, H, Hkv, hd, eps, rqk, sv);
+    if (wide && aligned) k_qkv_post_128<T, E><<<cdiv(warps, 32), 256, 0, s>>>(qkv, ldq, xn1, D, ve_gate, ve, tok0, pos, sin_t, cos_t, N, H, Hkv, eps, rqk, sv, pc);
+    else k_qkv_post<T, E><<<cdiv(warps, WPB), 256, 0, s>>>(qkv, ldq, xn1, D, ve_gate, ve, tok0, pos, sin_t, cos_t, N, H, Hkv, hd, eps, rqk, sv, pc);
   };
   if (ve32) launch(ve32, (reinterpret_cast<uintptr_t>(ve32) & (sizeof(T) == 4 ? 15 : 7)) == 0);
   else launch(ve_table, !ve_table || aligned16(ve_table));

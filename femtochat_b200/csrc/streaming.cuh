@@ -12,6 +12,12 @@ struct CastJob {
 };
 constexpr int CAST_BLOCK = 8192;
 
+// Where keys and values of a prompt go beside the projections, [B][maxT][kv]: row n is token n % T of column n / T.  NULL: nowhere.
+template <typename T> struct PromptCache {
+  T *K = nullptr, *V = nullptr;
+  int T_ = 1, maxT = 0;
+  __device__ __forceinline__ T* row(T* base, long long n, int kv) const { return base + ((n / T_) * maxT + n % T_) * kv; }
+};
 template <typename T> struct Stream {
   static int prep_tokens(const int* tokens, const int* targets, const int* positions, int B, int Tlen,
                          int index_base, int vocab, int maxdoc, int* tok0, int* tgt0, int* pos, int* doc_start,
@@ -25,7 +31,7 @@ template <typename T> struct Stream {
   static int norm(const T* x, T* xn, float* r, int N, int D, float eps, cudaStream_t s);
   static int qkv_post(T* qkv, long long ldq, const T* xn1, int D, const float* ve_gate, const T* ve_table,
                       const int* tok0, const int* pos, const float* sin_t, const float* cos_t, int N, int H,
-                      int Hkv, int hd, float eps, float* rqk, float* sv, cudaStream_t s, const float* ve32 = nullptr);
+                      int Hkv, int hd, float eps, float* rqk, float* sv, cudaStream_t s, const float* ve32 = nullptr, const PromptCache<T>& pc = {});
   static int qkv_post_bwd(T* dqkv, const T* qkv, long long ldq, const T* ve_table, const int* tok0,
                           const int* pos, const float* sin_t, const float* cos_t, int N, int H, int Hkv, int hd,
                           const float* rqk, const float* sv, T* dve, float* dpre, cudaStream_t s);
