@@ -303,6 +303,8 @@ int decoder_create(const femto_decoder_config* cfg, femto_handle** out) {
 void decoder_free(DecoderStack* d) {
   if (!d) return;
   if (d->arena) cudaFree(d->arena);
+  if (d->step.exec) cudaGraphExecDestroy(d->step.exec);
+  if (d->step.stream) cudaStreamDestroy(d->step.stream);
   delete d;
 }
 
@@ -612,6 +614,54 @@ static int logits_t(DecoderStack* d, const float* theta, const int* want, int st
   return rows_linear<T>(d, d->hn, w, d->head, w, out, d->cfg.vocab, n, d->cfg.vocab, w, EPI_F32, s, ro);
 }
 
+// One token per column as one launch.  A step is 170 to 190 dependent kernels of 2 to 10 us, and the host took as long for their launches as
+// the device for their work.  Recording one costs it a fraction of launching it, and the position, the token, the weights and the logits
+// of this step go into the graph as they are: nothing is kept from the step before but the shape of the graph.  A first step, columns that
+// change from step to step, and kernels that change with the position so that the graph has to be made again (about 1 ms) take plain launches
+// for a while; so do steps that the caller records.  ran stays false, and the cache as it was, where plain launches are to do the step.
+static int step_by_graph(DecoderStack* d, femto_kv_cache* c, const float* theta, const int* tokens, int B, float* logits_out, cudaStream_t s, bool& ran) {
+  StepGraph& g = d->step;
+  g.streak = B == g.B ? std::min(g.streak + 1, 1 << 20) : 0;
+  g.B = B;
+  if (g.streak < g.wait) return 0;
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &status) != cudaSuccess) { cudaGetLastError(); return 0; }
+  if (status != cudaStreamCaptureStatusNone) return 0;
+  if (!g.stream) CUDA_TRY(cudaStreamCreateWithFlags(&g.stream, cudaStreamNonBlocking));
+  std::vector<int> tails;
+  for (const auto& l : c->state) tails.push_back(l.tail_now);
+  const long long launches = g_femto_launches;
+  auto leave = [&] {
+    for (size_t i = 0; i < tails.size(); i++) c->state[i].tail_now = tails[i];
+    g_femto_launches = launches;
+    cudaGetLastError();
+    g.streak = 0; g.wait = 64;
+    return 0;
+  };
+  CUDA_TRY(cudaStreamBeginCapture(g.stream, cudaStreamCaptureModeThreadLocal));
+  int r = d->bf ? pass_t<bf16>(d, c, theta, tokens, 1, B, 1, nullptr, g.stream) : pass_t<float>(d, c, theta, tokens, 1, B, 1, nullptr, g.stream);
+  if (r == 0 && logits_out)
+    r = d->bf ? logits_t<bf16>(d, theta, nullptr, 1, B, logits_out, g.stream) : logits_t<float>(d, theta, nullptr, 1, B, logits_out, g.stream);
+  cudaGraph_t graph = nullptr;
+  const cudaError_t end = cudaStreamEndCapture(g.stream, &graph);
+  if (r != 0 || end != cudaSuccess || !graph) {
+    if (graph) cudaGraphDestroy(graph);
+    return leave();
+  }
+  cudaGraphExecUpdateResultInfo info;
+  if (g.exec && cudaGraphExecUpdate(g.exec, graph, &info) != cudaSuccess) {
+    cudaGetLastError();
+    cudaGraphExecDestroy(g.exec);
+    g.exec = nullptr;
+    g.streak = 0; g.wait = std::min(64, 2 * g.wait);
+  }
+  if (!g.exec && cudaGraphInstantiate(&g.exec, graph, 0) != cudaSuccess) g.exec = nullptr;
+  cudaGraphDestroy(graph);
+  if (!g.exec || cudaGraphLaunch(g.exec, s) != cudaSuccess) return leave();
+  ran = true;
+  return 0;
+}
+
 int decoder_step(femto_handle* h, femto_kv_cache* c, const float* theta, const int* tokens, int B, int T, const int* h_want, int n_want,
                  float* logits_out, float* residuals_out, cudaStream_t s) {
   DecoderStack* d = h->dec;
@@ -628,6 +678,11 @@ int decoder_step(femto_handle* h, femto_kv_cache* c, const float* theta, const i
   const int portion = d->cfg.max_rows / B;
   if (residuals_out && T > portion) return femto_fail(FEMTO_ERR_SHAPE, "residuals of %d x %d tokens exceed max_rows", B, T);
   c->B = B;
+  if (T == 1 && portion >= 1 && !h_want && !residuals_out) {
+    bool ran = false;
+    FEMTO_TRY(step_by_graph(d, c, theta, tokens, B, logits_out, s, ran));
+    if (ran) { c->len++; return 0; }
+  }
   for (int t0 = 0; t0 < T; t0 += portion) {
     const int n = std::min(portion, T - t0);
     FEMTO_TRY(d->bf ? pass_t<bf16>(d, c, theta, tokens + t0, T, B, n, residuals_out, s)

@@ -35,7 +35,16 @@ struct DecLayer {
   int qk_heads() const { return c.mixer == FEMTO_MIXER_CHANNEL_DELTA ? c.kv_heads : c.heads; }
 };
 
+// The graph of a decode step: its kernels are recorded anew for every token (their arguments change with the position) and the
+// executable graph is brought up to date, see step_by_graph.
+struct StepGraph {
+  cudaStream_t stream = nullptr;      // records, never runs
+  cudaGraphExec_t exec = nullptr;
+  int B = 0, streak = 0, wait = 1;    // columns of the last step, steps before it with as many, steps to let pass before recording
+};
+
 struct DecoderStack {
+  StepGraph step;
   femto_decoder_config cfg;
   std::vector<DecLayer> layers;
   std::vector<femto_decoder_tensor> tensors;

@@ -102,6 +102,47 @@ def test_columns_equal_each_alone(dtype):
     ok(model)
 
 
+@BOTH
+@pytest.mark.parametrize("name", ["mixed", "large"])
+def test_steps_as_one_launch_equal_plain_launches(name, dtype):
+    """From a handle's second step on, a step is one launch of a graph; a step whose wanted positions are listed is launched kernel by
+    kernel.  The same bits, for caches of different sizes in turn, after a reset, on another stream, and inside a caller's own graph."""
+    cfg, ranks = (dc.MIXED, dc.MIXED_RANKS) if name == "mixed" else (dc.LARGE, dc.LARGE_RANKS)
+    model, _ = dc.model_and_weights(cfg, ranks, dtype, seed=12)
+    state = model.state(3)
+    t = torch.stack([dc.tokens(90, cfg["vocab"], 30 + b) for b in range(3)]).int().cuda()
+    caches = {k: (fb.KVCache(state, B, 90), fb.KVCache(state, B, 90), B, n) for k, (B, n) in enumerate([(1, 40), (3, 5), (3, 64)])}
+
+    def step(k, at):
+        a, b, B, _ = caches[k]
+        got, want = fb.decode_step(model, a, t[:B, at]), fb.extend(model, b, t[:B, at:at + 1], want=list(range(B)))
+        assert torch.equal(got, want), (k, at)
+
+    for again in range(2):
+        for k, (a, b, B, n) in caches.items():
+            assert torch.equal(fb.prefill(model, a, t[:B, :n]), fb.prefill(model, b, t[:B, :n]))
+            for at in range(n, n + 8):
+                step(k, at)
+        for i in range(3):
+            for k, (a, b, B, n) in caches.items():      # columns that change from step to step
+                step(k, n + 8 + i)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        for at in range(51, 55):
+            step(0, at)
+    torch.cuda.current_stream().wait_stream(side)
+    a, b, B, n = caches[0]
+    token, graph = t[:1, 55].clone(), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = fb.decode_step(model, a, token)
+    graph.replay()
+    assert torch.equal(got, fb.extend(model, b, t[:1, 55:56], want=[0]))
+    for at in range(56, 60):
+        step(0, at)
+    ok(model)
+
+
 def test_wanted_positions_and_internal_portions():
     """A prompt longer than one internal pass, several columns, a ragged choice of positions."""
     cfg, ranks = dc.MIXED, dc.MIXED_RANKS
