@@ -357,11 +357,11 @@ __global__ void __launch_bounds__(256) k_latent_decode_mma(const LatentArgs a, i
       float x0 = 0.f, x1 = 0.f;
 #pragma unroll
       for (int k = 0; k < 8; k++) {
-        x0 += ss[(k * 16 + r) * SP + lane];
+        if (lane < KT) x0 += ss[(k * 16 + r) * SP + lane];
         if (KT > 32) x1 += ss[(k * 16 + r) * SP + lane + 32];
       }
       const int key = tile * KT + lane;
-      x0 = key < n ? x0 * a.scale : -INFINITY;
+      x0 = lane < KT && key < n ? x0 * a.scale : -INFINITY;
       x1 = KT > 32 && key + 32 < n ? x1 * a.scale : -INFINITY;
       const float m = sml[2 * r], mn = fmaxf(m, warp_max(fmaxf(x0, x1)));      // finite: the first key of a tile is always seen
       const float p0 = __expf(x0 - mn), p1 = __expf(x1 - mn), f = __expf(m - mn);
@@ -577,7 +577,10 @@ static int latent_decode_tc(const LatentArgs& a, cudaStream_t s, bool& done) {
   const int N = a.first + a.T, rows = a.B * a.T, H = a.heads, hd = a.dim + a.rot_dim;
   const int width = round_up(a.ld, 64), nk = cdiv(width, 128), np = cdiv(a.lp, 128);
   auto bytes = [&](int kt) { return (size_t)2 * kt * width * 2 + 2 * 16 * 64 * 2 + 4 * (size_t)(8 * 16 * (kt + 4) + 48); };
-  const int KT = bytes(64) <= 227 * 1024 ? 64 : 32;
+  // The tiles of a split follow one another, so a short context takes narrow ones, one a split, while these run at once and 32 splits are enough.
+  const int blocks = cdiv(H, 16) * rows, widest = bytes(64) <= 227 * 1024 ? 64 : 32;
+  int KT = 16;
+  while (KT < widest && (cdiv(N, KT) > 32 || (long long)cdiv(N, KT) * blocks > device_sm_count() || a.rot_dim > 8 * (KT + 4))) KT *= 2;
   // the rotated queries (16 x rot_dim) pass through the space of the scores
   done = bytes(KT) <= 227 * 1024 && (hd & 7) == 0 && (a.dim & 7) == 0 && nk <= 9 && a.rot_dim <= 8 * (KT + 4);
   if (!done) return 0;
@@ -588,7 +591,7 @@ static int latent_decode_tc(const LatentArgs& a, cudaStream_t s, bool& done) {
     FEMTO_TRY(rows_stream(q + (long long)r0 * H * hd, (long long)H * hd, (const bf16*)a.w_ukt, a.dp, a.qabs + (long long)r0 * H * a.lp, (long long)H * a.lp,
                           std::min(ROWS_STREAM, rows - r0), a.lp, a.dim, EPI_F32, H, bt, s));
   }
-  const int tiles = cdiv(N, KT), blocks = cdiv(H, 16) * rows;
+  const int tiles = cdiv(N, KT);
   int per = std::max(1, cdiv(tiles, std::max(1, device_sm_count() / blocks)));      // as many splits as fill the device once
   while ((size_t)rows * H * cdiv(tiles, per) * (a.lp + 2) > a.part_floats) per++;
   const int splits = cdiv(tiles, per);

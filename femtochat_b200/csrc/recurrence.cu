@@ -2,6 +2,7 @@
 // the gated delta rule with one decay per key channel.  The state is kept as [vdim][dim]: its vdim columns are independent
 // recurrences that share q, k and the decays, so a block owns 32 of them, eight lanes each, for any number of tokens.
 #include "decoder.cuh"
+#include "sm100_ptx.cuh"
 
 namespace {
 
@@ -187,169 +188,203 @@ __global__ void __launch_bounds__(256) k_conv_tail(const DeltaPrepArgs a) {
 
 // ---- one token -----------------------------------------------------------------------------------------------------------
 // The whole mixer between the packed projection and the output projection for one new token: convolutions, unit vectors,
-// both low-rank projections, state update, read-out, norm and gate.  One block per (head, column).
+// both low-rank projections, state update, read-out, norm and gate.  grid (heads x cluster, columns).  Bound by the chain of
+// dependent loads and sums, so a head's E rows of state and its D + E low-rank rows are shared by the CTAs of a cluster: each makes
+// q, k and its own v, decays and gates; the decays reach the others through distributed shared memory, the state's rows are
+// on their way to registers meanwhile, and the squares for the norm meet the same way.  A warp has whole rows of the state.
 __device__ __forceinline__ float sigmoid_f(float z) { return 1.f / (1.f + expf(-z)); }
 
-template <typename T> __device__ __forceinline__ float row_dot(const T* __restrict__ w, const float* x, int n, int lane) {
-  constexpr int V = VecN<T>::n;      // rows are padded to multiples of 8 with zeros
-  float acc = 0.f;
-  for (int c = lane * V; c < n; c += 32 * V) {
-    float f[V];
-    load_vec<T, V>(w + c, f);
-#pragma unroll
-    for (int e = 0; e < V; e++) acc = fmaf(f[e], x[c + e], acc);
-  }
-  return warp_sum(acc);
+__device__ __forceinline__ void store_peer(const float* p, uint32_t rank, float v) {
+  uint32_t at;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(sm100::smem_u32(p)), "r"(rank));
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(at), "f"(v) : "memory");
 }
 
-template <typename T, int NI>
-__global__ void __launch_bounds__(1024) k_delta_decode(const DeltaDecodeArgs a) {
+// SI: 128 channels of a row of the state each
+template <typename T, int SI>
+__global__ void __launch_bounds__(1024) k_delta_decode(const DeltaDecodeArgs a, int cl, int staged) {
   pdl_trigger();
-  constexpr int DP = 32 * NI;
+  constexpr int V = VecN<T>::n, ROWS = 4 / SI, HELD = 2;      // rows of the state a warp has in flight; low-rank rows loaded before the wait
   const DeltaPrepArgs& p = a.p;
-  {
-    // eight loads that wait for one another took 16 us a layer from memory
-    const int h = blockIdx.x, t = threadIdx.x, D = p.dim, E = p.vdim, n = p.taps, qh = h / (p.heads / p.kv_heads);
-    prefetch_l2(a.S + ((long long)blockIdx.y * p.heads + h) * E * D, 4ll * E * D, t, 1024);
-    prefetch_l2(reinterpret_cast<const T*>(a.w_a2) + (long long)h * D * a.ra, (long long)sizeof(T) * D * a.ra, t, 1024);
-    prefetch_l2(reinterpret_cast<const T*>(a.w_g2) + (long long)h * E * a.rg, (long long)sizeof(T) * E * a.rg, t, 1024);
-    prefetch_l2(p.conv_q + (long long)qh * D * n, 4ll * D * n, t, 1024);
-    prefetch_l2(p.conv_k + (long long)qh * D * n, 4ll * D * n, t, 1024);
-    prefetch_l2(p.conv_v + (long long)h * E * n, 4ll * E * n, t, 1024);
-    prefetch_l2(p.dt_bias + (long long)h * D, 4ll * D, t, 1024);
-    prefetch_l2(a.norm, 4ll * E, t, 1024);
-    if (t == 0) prefetch_l2(p.a_log + h);
-    const int channels = 2 * p.kv_heads * D + p.heads * E;
-    const T* tail = reinterpret_cast<const T*>(p.tail_in) + (long long)blockIdx.y * (n - 1) * channels;
-    for (int j = 0; j < n - 1; j++) {
-      prefetch_l2(tail + (long long)j * channels + qh * D, (long long)sizeof(T) * D, t, 1024);
-      prefetch_l2(tail + (long long)j * channels + (p.kv_heads + qh) * D, (long long)sizeof(T) * D, t, 1024);
-      prefetch_l2(tail + (long long)j * channels + 2 * p.kv_heads * D + h * E, (long long)sizeof(T) * E, t, 1024);
-    }
-  }
-  pdl_wait();
-  extern __shared__ __align__(16) float sm[];
-  float *sq = sm, *sk = sq + DP, *sg = sk + DP, *sv = sg + DP, *so = sv + p.vdim, *sz = so + p.vdim, *sa = sz + p.vdim, *sb = sa + a.ra;
-  __shared__ float red[32], f_q, f_k;
-  const int h = blockIdx.x, b = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int h = blockIdx.x / cl, rank = blockIdx.x % cl, b = blockIdx.y, tid = threadIdx.x, threads = blockDim.x, warp = tid >> 5, warps = threads >> 5, lane = tid & 31;
   const int H = p.heads, G = p.kv_heads, D = p.dim, E = p.vdim, n = p.taps, keep = n - 1;
   const int qh = h / (H / G), channels = 2 * G * D + H * E;
-  const T* proj = reinterpret_cast<const T*>(p.proj) + (long long)b * p.ldp;
+  // this CTA's decays, and its rows of state, values and gates
+  const int dn = (D + cl - 1) / cl, d0 = min(D, rank * dn), d1 = min(D, d0 + dn), en = (E + cl - 1) / cl, e0 = min(E, rank * en), e1 = min(E, e0 + en);
+  const int low = d1 - d0 + e1 - e0;
+  extern __shared__ __align__(16) float sm[];
+  float *sq = sm, *sk = sq + D, *sg = sk + D, *sv = sg + D, *so = sv + en, *sz = so + en, *sa = sz + en, *sb = sa + a.ra, *st = sb + a.rg;
+  __shared__ float f_q, f_k, squares[8];
   const T* tin = reinterpret_cast<const T*>(p.tail_in) + (long long)b * keep * channels;
   T* tout = reinterpret_cast<T*>(p.tail_out) + (long long)b * keep * channels;
-  for (int i = tid; i < a.ra; i += 1024) sa[i] = to_f<T>(proj[a.s_a1 + i]);
-  for (int i = tid; i < a.rg; i += 1024) sb[i] = to_f<T>(proj[a.s_g1 + i]);
-  for (int i = tid; i < 2 * DP + E; i += 1024) {
-    const int which = i < DP ? 0 : i < 2 * DP ? 1 : 2, c = which == 2 ? i - 2 * DP : i - which * DP;
-    const int size = which == 2 ? E : D, head = which == 2 ? h : qh;
-    float y = 0.f;
-    if (c < size) {
-      const int at = head * size + c, chan = (which == 0 ? 0 : which == 1 ? G * D : 2 * G * D) + at;
-      const float* taps = (which == 0 ? p.conv_q : which == 1 ? p.conv_k : p.conv_v) + (long long)at * n;
-      const T now = proj[(which == 0 ? p.s_q : which == 1 ? p.s_k : p.s_v) + at];
-      const bool writes = which == 2 || h % (H / G) == 0;      // the heads of a group share q and k
-      float acc = 0.f;
-      for (int j0 = 0; j0 < keep; j0 += 4) {          // four loads in flight before the first store
-        T x[4];
-#pragma unroll
-        for (int j = 0; j < 4; j++) if (j0 + j < keep) x[j] = tin[(long long)(j0 + j) * channels + chan];
-#pragma unroll
-        for (int j = 0; j < 4; j++)
-          if (j0 + j < keep) {
-            acc = fmaf(taps[j0 + j], to_f<T>(x[j]), acc);
-            if (writes && j0 + j > 0) tout[(long long)(j0 + j - 1) * channels + chan] = x[j];
-          }
-      }
-      if (writes && keep > 0) tout[(long long)(keep - 1) * channels + chan] = now;
-      y = silu_f(fmaf(taps[keep], to_f<T>(now), acc));
-      if (which == 2) y = round_to<T>(y);
-    }
-    (which == 0 ? sq : which == 1 ? sk : sv)[c] = y;
+  float* S = a.S + (((long long)b * H + h) * E + e0) * D;
+  // low-rank row i of this CTA
+  auto low_row = [&](int i) {
+    const bool decay = i < d1 - d0;
+    const int c = decay ? d0 + i : e0 + i - (d1 - d0);
+    return decay ? reinterpret_cast<const T*>(a.w_a2) + (long long)(h * D + c) * a.ra : reinterpret_cast<const T*>(a.w_g2) + (long long)(h * E + c) * a.rg;
+  };
+  auto low_rank = [&](int i) { return i < d1 - d0 ? a.ra : a.rg; };
+  prefetch_l2(S, 4ll * (e1 - e0) * D, tid, threads);
+  prefetch_l2(p.dt_bias + (long long)h * D + d0, 4ll * (d1 - d0), tid, threads);
+  prefetch_l2(a.norm + e0, 4ll * (e1 - e0), tid, threads);
+  if (tid == 0) prefetch_l2(p.a_log + h);
+  for (int j = 0; j < keep; j++) {
+    prefetch_l2(tin + (long long)j * channels + qh * D, (long long)sizeof(T) * D, tid, threads);
+    prefetch_l2(tin + (long long)j * channels + (G + qh) * D, (long long)sizeof(T) * D, tid, threads);
+    prefetch_l2(tin + (long long)j * channels + 2 * G * D + h * E + e0, (long long)sizeof(T) * (e1 - e0), tid, threads);
   }
+  prefetch_l2(reinterpret_cast<const T*>(a.w_a2) + (long long)(h * D + d0) * a.ra, (long long)sizeof(T) * (d1 - d0) * a.ra, tid, threads);
+  prefetch_l2(reinterpret_cast<const T*>(a.w_g2) + (long long)(h * E + e0) * a.rg, (long long)sizeof(T) * (e1 - e0) * a.rg, tid, threads);
+  // weights, which no kernel of the chain writes: taps, and the first low-rank rows of each warp
+  for (int i = tid; staged && i < (2 * D + e1 - e0) * n; i += threads)
+    st[i] = i < D * n ? p.conv_q[(long long)qh * D * n + i] : i < 2 * D * n ? p.conv_k[(long long)qh * D * n + i - D * n] : p.conv_v[(long long)(h * E + e0) * n + i - 2 * D * n];
+  uint4 held[HELD];
+#pragma unroll
+  for (int u = 0; u < HELD; u++) {
+    const int i = warp + u * warps;
+    if (i < low && lane * V < low_rank(i)) held[u] = *reinterpret_cast<const uint4*>(low_row(i) + lane * V);
+  }
+  if (cl > 1) sm100::cluster_arrive();        // the others have started
+  pdl_wait();
+  __syncthreads();      // the taps
+  const T* proj = reinterpret_cast<const T*>(p.proj) + (long long)b * p.ldp;
+  for (int i = tid; i < a.ra + a.rg; i += threads) sa[i] = to_f<T>(i < a.ra ? proj[a.s_a1 + i] : proj[a.s_g1 + i - a.ra]);
+  for (int i = tid; i < 2 * D + e1 - e0; i += threads) {
+    const int which = i < D ? 0 : i < 2 * D ? 1 : 2, c = which == 2 ? i - 2 * D : i - which * D;
+    const int at = which == 2 ? h * E + e0 + c : qh * D + c, chan = (which == 0 ? 0 : which == 1 ? G * D : 2 * G * D) + at;
+    const float* taps = staged ? st + i * n : (which == 0 ? p.conv_q : which == 1 ? p.conv_k : p.conv_v) + (long long)at * n;
+    const T now = proj[(which == 0 ? p.s_q : which == 1 ? p.s_k : p.s_v) + at];
+    const bool writes = which == 2 || (rank == 0 && h % (H / G) == 0);      // the heads of a group share q and k
+    float acc = 0.f;
+    for (int j0 = 0; j0 < keep; j0 += 4) {          // four loads in flight before the first store
+      T x[4];
+#pragma unroll
+      for (int j = 0; j < 4; j++) if (j0 + j < keep) x[j] = tin[(long long)(j0 + j) * channels + chan];
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+        if (j0 + j < keep) {
+          acc = fmaf(taps[j0 + j], to_f<T>(x[j]), acc);
+          if (writes && j0 + j > 0) tout[(long long)(j0 + j - 1) * channels + chan] = x[j];
+        }
+    }
+    if (writes && keep > 0) tout[(long long)(keep - 1) * channels + chan] = now;
+    const float y = silu_f(fmaf(taps[keep], to_f<T>(now), acc));
+    if (which == 2) sv[c] = round_to<T>(y);
+    else (which ? sk : sq)[c] = y;
+  }
+  if (cl > 1) sm100::cluster_wait();
   __syncthreads();
-  if (warp < 2) {
-    const float* x = warp ? sk : sq;
+  if (warp >= warps - 2) {
+    const float* x = warp & 1 ? sk : sq;
     float ss = 0.f;
     for (int c = lane; c < D; c += 32) ss += x[c] * x[c];
     ss = 1.f / sqrtf(warp_sum(ss) + 1e-6f);
-    if (lane == 0) { if (warp) f_k = ss; else f_q = ss * (1.f / sqrtf((float)D)); }
+    if (lane == 0) { if (warp & 1) f_k = ss; else f_q = ss * (1.f / sqrtf((float)D)); }
   }
   const float rate = expf(p.a_log[h]);
-#pragma unroll 4
-  for (int i = warp; i < D + E; i += 32) {
-    const bool decay = i < D;
-    const int c = decay ? i : i - D, r = decay ? a.ra : a.rg;
-    const T* w = reinterpret_cast<const T*>(decay ? a.w_a2 : a.w_g2) + (long long)(h * (decay ? D : E) + c) * r;
-    const float z = row_dot<T>(w, decay ? sa : sb, r, lane);
-    if (lane == 0) (decay ? sg : sz)[c] = z;
-  }
-  __syncthreads();
-  for (int i = tid; i < DP + E; i += 1024) {
-    if (i < DP) sg[i] = i < D ? expf(-rate * softplus_f(sg[i] + p.dt_bias[h * D + i])) : 0.f;
-    else sz[i - DP] = sigmoid_f(round_to<T>(sz[i - DP]));
-  }
-  __syncthreads();
-  const float beta = sigmoid_f(to_f<T>(proj[p.s_b + h])), fk = f_k, fq = f_q;
-  const int sub = tid & 7;
-  const bool vec = (D & 3) == 0;
-  for (int e = tid >> 3; e < (E + 127) / 128 * 128; e += 128) {
-    float* Sp = a.S + (((long long)b * H + h) * E + min(e, E - 1)) * D;
-    float s[NI][4], dot = 0.f;
+  for (int i0 = warp, u = 0; i0 < low; i0 += warps, u++) {
+    const bool decay = i0 < d1 - d0;
+    const float* x = decay ? sa : sb;
+    const int r = low_rank(i0);
+    const T* w = low_row(i0);
+    float z = 0.f;
+    for (int c = lane * V; c < r; c += 32 * V) {       // rows are padded to multiples of 8 with zeros
+      const uint4 q = c < 32 * V && u < HELD ? (u ? held[1] : held[0]) : *reinterpret_cast<const uint4*>(w + c);
+      const T* f = reinterpret_cast<const T*>(&q);
 #pragma unroll
-    for (int i = 0; i < NI; i++) {
-      const int d = 4 * (sub + 8 * i);
-      if (vec) {
-        const float4 v = d < D && e < E ? *reinterpret_cast<const float4*>(Sp + d) : make_float4(0.f, 0.f, 0.f, 0.f);
-        s[i][0] = v.x; s[i][1] = v.y; s[i][2] = v.z; s[i][3] = v.w;
-      } else {
-#pragma unroll
-        for (int j = 0; j < 4; j++) s[i][j] = d + j < D && e < E ? Sp[d + j] : 0.f;
-      }
+      for (int e = 0; e < V; e++) z = fmaf(to_f<T>(f[e]), x[c + e], z);
     }
+    z = warp_sum(z);
+    if (decay) {
+      const int c = d0 + i0;
+      z = expf(-rate * softplus_f(z + p.dt_bias[h * D + c]));
+      if (cl == 1) { if (lane == 0) sg[c] = z; }
+      else if (lane < cl) store_peer(sg + c, lane, z);
+    } else if (lane == 0) {
+      sz[i0 - (d1 - d0)] = sigmoid_f(round_to<T>(z));
+    }
+  }
+  if (cl > 1) sm100::cluster_arrive(); else __syncthreads();
+  const float beta = sigmoid_f(to_f<T>(proj[p.s_b + h]));
+  const bool vec = (D & 3) == 0;
+  bool waited = cl == 1;
+  for (int r0 = 0; r0 < en; r0 += ROWS * warps) {
+    float s[ROWS][SI][4];
 #pragma unroll
-    for (int i = 0; i < NI; i++)
+    for (int r = 0; r < ROWS; r++)
 #pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const int d = 4 * (sub + 8 * i) + j;
-        s[i][j] *= sg[d];
-        dot = fmaf(s[i][j], sk[d] * fk, dot);
-      }
-    dot += __shfl_xor_sync(0xffffffffu, dot, 1); dot += __shfl_xor_sync(0xffffffffu, dot, 2); dot += __shfl_xor_sync(0xffffffffu, dot, 4);
-    const float u = beta * ((e < E ? sv[e] : 0.f) - dot);
-    float o = 0.f;
-#pragma unroll
-    for (int i = 0; i < NI; i++)
-#pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const int d = 4 * (sub + 8 * i) + j;
-        s[i][j] = fmaf(sk[d] * fk, u, s[i][j]);
-        o = fmaf(s[i][j], sq[d] * fq, o);
-      }
-    o += __shfl_xor_sync(0xffffffffu, o, 1); o += __shfl_xor_sync(0xffffffffu, o, 2); o += __shfl_xor_sync(0xffffffffu, o, 4);
-    if (e < E) {
-#pragma unroll
-      for (int i = 0; i < NI; i++) {
-        const int d = 4 * (sub + 8 * i);
+      for (int i = 0; i < SI; i++) {
+        const int e = r0 + r * warps + warp, d = 4 * lane + 128 * i;
+        const float* Sp = S + (long long)e * D + d;
         if (vec) {
-          if (d < D) *reinterpret_cast<float4*>(Sp + d) = make_float4(s[i][0], s[i][1], s[i][2], s[i][3]);
+          const float4 v = d < D && e < e1 - e0 ? *reinterpret_cast<const float4*>(Sp) : make_float4(0.f, 0.f, 0.f, 0.f);
+          s[r][i][0] = v.x; s[r][i][1] = v.y; s[r][i][2] = v.z; s[r][i][3] = v.w;
         } else {
 #pragma unroll
-          for (int j = 0; j < 4; j++) if (d + j < D) Sp[d + j] = s[i][j];
+          for (int j = 0; j < 4; j++) s[r][i][j] = d + j < D && e < e1 - e0 ? Sp[j] : 0.f;
         }
       }
-      if (sub == 0) so[e] = round_to<T>(o);
+    if (!waited) { sm100::cluster_wait(); waited = true; }       // all decays are here, and with them f_q and f_k
+    float dot[ROWS] = {}, o[ROWS] = {};
+#pragma unroll
+    for (int r = 0; r < ROWS; r++)
+#pragma unroll
+      for (int i = 0; i < SI; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          const int d = 4 * lane + 128 * i + j;
+          if (d >= D) continue;
+          s[r][i][j] *= sg[d];
+          dot[r] = fmaf(s[r][i][j], sk[d] * f_k, dot[r]);
+        }
+#pragma unroll
+    for (int r = 0; r < ROWS; r++) {
+      const int e = r0 + r * warps + warp;
+      const float u = beta * ((e < e1 - e0 ? sv[e] : 0.f) - warp_sum(dot[r]));
+#pragma unroll
+      for (int i = 0; i < SI; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          const int d = 4 * lane + 128 * i + j;
+          if (d >= D) continue;
+          s[r][i][j] = fmaf(sk[d] * f_k, u, s[r][i][j]);
+          o[r] = fmaf(s[r][i][j], sq[d] * f_q, o[r]);
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < ROWS; r++) {
+      const int e = r0 + r * warps + warp;
+      o[r] = warp_sum(o[r]);
+      if (e >= e1 - e0) continue;
+      if (lane == 0) so[e] = round_to<T>(o[r]);
+#pragma unroll
+      for (int i = 0; i < SI; i++) {
+        const int d = 4 * lane + 128 * i;
+        float* Sp = S + (long long)e * D + d;
+        if (vec) {
+          if (d < D) *reinterpret_cast<float4*>(Sp) = make_float4(s[r][i][0], s[r][i][1], s[r][i][2], s[r][i][3]);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 4; j++) if (d + j < D) Sp[j] = s[r][i][j];
+        }
+      }
     }
   }
   __syncthreads();
+  if (warp == 0) {
+    float ss = 0.f;
+    for (int c = lane; c < e1 - e0; c += 32) ss += so[c] * so[c];
+    ss = warp_sum(ss);
+    if (cl == 1) { if (lane == 0) squares[0] = ss; }
+    else if (lane < cl) store_peer(squares + rank, lane, ss);
+  }
+  if (cl > 1) { sm100::cluster_arrive(); sm100::cluster_wait(); } else __syncthreads();
   float ss = 0.f;
-  for (int c = tid; c < E; c += 1024) ss += so[c] * so[c];
-  ss = warp_sum(ss);
-  if (lane == 0) red[warp] = ss;
-  __syncthreads();
-  ss = warp_sum(red[lane]);
+  for (int r = 0; r < cl; r++) ss += squares[r];
   const float inv = 1.f / sqrtf(ss / E + a.eps);
-  T* out = reinterpret_cast<T*>(a.out) + ((long long)b * H + h) * E;
-  for (int c = tid; c < E; c += 1024) out[c] = from_f<T>(so[c] * inv * a.norm[c] * sz[c]);
+  T* out = reinterpret_cast<T*>(a.out) + ((long long)b * H + h) * E + e0;
+  for (int c = tid; c < e1 - e0; c += threads) out[c] = from_f<T>(so[c] * inv * a.norm[e0 + c] * sz[c]);
 }
 
 }  // namespace
@@ -390,18 +425,31 @@ template <typename T> int delta_prep(const DeltaPrepArgs& a, cudaStream_t s) {
 template int delta_prep<float>(const DeltaPrepArgs&, cudaStream_t);
 template int delta_prep<bf16>(const DeltaPrepArgs&, cudaStream_t);
 
+// Heads and columns that leave multiprocessors idle share a head among up to eight of them.
 template <typename T> int delta_decode(const DeltaDecodeArgs& a, cudaStream_t s) {
-  const dim3 grid(a.p.heads, a.p.B);
-  const int ni = a.p.dim <= 32 ? 1 : a.p.dim <= 64 ? 2 : a.p.dim <= 128 ? 4 : 8;
   if (a.p.dim > 256 || a.p.vdim > 256) return femto_fail(FEMTO_ERR_UNSUPPORTED, "delta rule: dim %d / vdim %d > 256", a.p.dim, a.p.vdim);
-  const size_t smem = 4 * (size_t)(3 * 32 * ni + 3 * a.p.vdim + a.ra + a.rg);
-  if (smem > 48 * 1024) return femto_fail(FEMTO_ERR_UNSUPPORTED, "delta rule: ranks %d and %d are too large", a.ra, a.rg);
-#define LAUNCH(NI) CUDA_TRY(launch_dependent(k_delta_decode<T, NI>, grid, 1024, smem, s, a))
-  if (ni == 1) LAUNCH(1);
-  else if (ni == 2) LAUNCH(2);
-  else if (ni == 4) LAUNCH(4);
-  else LAUNCH(8);
-#undef LAUNCH
+  int cl = 1;
+  while (cl < 8 && 2ll * cl * a.p.heads * a.p.B <= device_sm_count()) cl *= 2;
+  const int en = cdiv(a.p.vdim, cl), threads = cl >= 4 ? 512 : 1024;
+  size_t smem = 4 * ((size_t)3 * a.p.dim + 3 * en + a.ra + a.rg);
+  const size_t taps = 4 * (2 * (size_t)a.p.dim + en) * a.p.taps;
+  const int staged = smem + taps <= 47 * 1024;      // many taps are read where they lie
+  if (staged) smem += taps;
+  if (smem > 48 * 1024 - 64) return femto_fail(FEMTO_ERR_UNSUPPORTED, "delta rule: ranks %d and %d are too large", a.ra, a.rg);
+  auto launch = [&](auto kernel) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(a.p.heads * cl, a.p.B); cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem; cfg.stream = s;
+    static const bool off = [] { const char* e = getenv("FEMTO_PDL"); return e && e[0] == '0'; }();   // measurement aid: fully serialised
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = cl; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at; cfg.numAttrs = off ? 1 : 2;
+    return cudaLaunchKernelEx(&cfg, kernel, a, cl, staged);
+  };
+  if (a.p.dim <= 128) CUDA_TRY(launch(k_delta_decode<T, 1>));
+  else CUDA_TRY(launch(k_delta_decode<T, 2>));
   KERNEL_CHECK();
   return 0;
 }
