@@ -305,6 +305,9 @@ void decoder_free(DecoderStack* d) {
   if (d->arena) cudaFree(d->arena);
   if (d->step.exec) cudaGraphExecDestroy(d->step.exec);
   if (d->step.stream) cudaStreamDestroy(d->step.stream);
+  if (d->step.side) cudaStreamDestroy(d->step.side);
+  if (d->step.fork) cudaEventDestroy(d->step.fork);
+  if (d->step.join) cudaEventDestroy(d->step.join);
   delete d;
 }
 
@@ -545,7 +548,7 @@ static int feed_forward(DecoderStack* d, const DecLayer& l, const float* theta, 
       RowsBatch bt;
       bt.lists = d->moe_lists; bt.max_lists = a.max_lists; bt.x_div = q.top; bt.w = (long long)l.ffp * w;
       FEMTO_TRY(rows_stream((const bf16*)h, w, (const bf16*)l.w_gu, w, d->moe_act, l.ffp, R, l.ffp, w, EPI_RELU2, a.max_lists, bt, s));
-      bt.x_div = 1;
+      bt.x_div = 1; bt.ready = 1;
       FEMTO_TRY(rows_stream((const bf16*)d->moe_act, l.ffp, (const bf16*)l.w_down, l.ffp, d->moe_out, w, R, w, l.ffp, EPI_STORE, a.max_lists, bt, s));
       return 0;
     }
@@ -564,10 +567,18 @@ static int feed_forward(DecoderStack* d, const DecLayer& l, const float* theta, 
   return gemm<T>(g, s);
 }
 
-// Tokens [t0, t0 + Tn) of every column.
+// Whether a parallel block's attention has no workspace in common with its feed-forward: its products stream, or are those of RL_ROWS rows.
+template <typename T> static bool attention_stands_alone(const DecoderStack* d, const DecLayer& l, int R) {
+  const int w = d->cfg.width, n = l.c.heads * l.c.vdim;
+  return l.c.mixer == FEMTO_MIXER_ATTENTION &&
+         (R <= 8 || (sizeof(T) == 2 && R <= ROWS_STREAM && ((w | n) & 7) == 0 && aligned16(d->hn) && aligned16(d->mixg) && aligned16(l.w_in) && aligned16(l.w_o)));
+}
+
+// Tokens [t0, t0 + Tn) of every column.  g: the pass is recorded into a graph, where a parallel block's feed-forward becomes a branch
+// beside its attention: the one streams the weights of experts, the other is a chain of short kernels.
 template <typename T>
 static int pass_t(DecoderStack* d, femto_kv_cache* c, const float* theta, const int* tokens, int ld_tok, int B, int Tn, float* residuals,
-                  cudaStream_t s) {
+                  cudaStream_t s, const StepGraph* g = nullptr) {
   typedef DecStream<T> S;
   const int R = B * Tn, w = d->cfg.width, L = d->cfg.n_layer;
   const float eps = d->cfg.norm_eps, m = d->cfg.residual_mult;
@@ -587,10 +598,18 @@ static int pass_t(DecoderStack* d, femto_kv_cache* c, const float* theta, const 
     const bool mlp = l.c.ff > 0;
     const NextNorms<T> next = norms_of(i + 1);
     MoeRows mr;
+    const bool branch = g && parallel && mlp && attention_stands_alone<T>(d, l, R);
+    if (branch) {
+      CUDA_TRY(cudaEventRecord(g->fork, s));
+      CUDA_TRY(cudaStreamWaitEvent(g->side, g->fork, 0));
+      FEMTO_TRY(feed_forward<T>(d, l, theta, d->hn2, d->y2, R, mr, g->side));
+      CUDA_TRY(cudaEventRecord(g->join, g->side));
+    }
     FEMTO_TRY(mixer_t<T>(d, c, i, theta, B, Tn, c->len, s));
+    if (branch) CUDA_TRY(cudaStreamWaitEvent(s, g->join, 0));
     if (parallel) {
-      if (mlp) FEMTO_TRY(feed_forward<T>(d, l, theta, d->hn2, d->y2, R, mr, s));
-      FEMTO_TRY(S::parallel_resid(d->x, (const T*)d->y, mlp && !l.c.experts ? (const T*)d->y2 : nullptr, mr, next, R, w, eps, s));
+      if (mlp && !branch) FEMTO_TRY(feed_forward<T>(d, l, theta, d->hn2, d->y2, R, mr, s));
+      FEMTO_TRY(S::parallel_resid(d->x, (const T*)d->y, mlp && !l.c.experts ? (const T*)d->y2 : nullptr, mr, next, R, w, eps, branch, s));
     } else {
       FEMTO_TRY(S::resid_norm(d->x, (const T*)d->y, theta + l.norm1b, m, mlp ? theta + l.norm2 : next.w, mlp || next.h ? (T*)d->hn : nullptr, R, w, eps, s));
       if (mlp) {
@@ -627,7 +646,14 @@ static int step_by_graph(DecoderStack* d, femto_kv_cache* c, const float* theta,
   cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s, &status) != cudaSuccess) { cudaGetLastError(); return 0; }
   if (status != cudaStreamCaptureStatusNone) return 0;
-  if (!g.stream) CUDA_TRY(cudaStreamCreateWithFlags(&g.stream, cudaStreamNonBlocking));
+  if (!g.stream) {
+    int low = 0, high = 0;      // the attention's short kernels go before the blocks of the experts' products
+    CUDA_TRY(cudaDeviceGetStreamPriorityRange(&low, &high));
+    if (!g.side) CUDA_TRY(cudaStreamCreateWithPriority(&g.side, cudaStreamNonBlocking, low));
+    if (!g.fork) CUDA_TRY(cudaEventCreateWithFlags(&g.fork, cudaEventDisableTiming));
+    if (!g.join) CUDA_TRY(cudaEventCreateWithFlags(&g.join, cudaEventDisableTiming));
+    CUDA_TRY(cudaStreamCreateWithPriority(&g.stream, cudaStreamNonBlocking, high));
+  }
   std::vector<int> tails;
   for (const auto& l : c->state) tails.push_back(l.tail_now);
   const long long launches = g_femto_launches;
@@ -639,7 +665,7 @@ static int step_by_graph(DecoderStack* d, femto_kv_cache* c, const float* theta,
     return 0;
   };
   CUDA_TRY(cudaStreamBeginCapture(g.stream, cudaStreamCaptureModeThreadLocal));
-  int r = d->bf ? pass_t<bf16>(d, c, theta, tokens, 1, B, 1, nullptr, g.stream) : pass_t<float>(d, c, theta, tokens, 1, B, 1, nullptr, g.stream);
+  int r = d->bf ? pass_t<bf16>(d, c, theta, tokens, 1, B, 1, nullptr, g.stream, &g) : pass_t<float>(d, c, theta, tokens, 1, B, 1, nullptr, g.stream, &g);
   if (r == 0 && logits_out)
     r = d->bf ? logits_t<bf16>(d, theta, nullptr, 1, B, logits_out, g.stream) : logits_t<float>(d, theta, nullptr, 1, B, logits_out, g.stream);
   cudaGraph_t graph = nullptr;

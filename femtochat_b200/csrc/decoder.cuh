@@ -38,7 +38,8 @@ struct DecLayer {
 // The graph of a decode step: its kernels are recorded anew for every token (their arguments change with the position) and the
 // executable graph is brought up to date, see step_by_graph.
 struct StepGraph {
-  cudaStream_t stream = nullptr;      // records, never runs
+  cudaStream_t stream = nullptr, side = nullptr;      // record, never run
+  cudaEvent_t fork = nullptr, join = nullptr;
   cudaGraphExec_t exec = nullptr;
   int B = 0, streak = 0, wait = 1;    // columns of the last step, steps before it with as many, steps to let pass before recording
 };
@@ -99,7 +100,7 @@ template <typename T> struct DecStream {
                    const NextNorms<T>& n, int d, float eps, unsigned int* status, cudaStream_t s);
   // x += y + (y2, or the weighted sum of the experts' rows, or nothing), then the norms
   static int parallel_resid(float* x, const T* y, const T* y2, const MoeRows& m, const NextNorms<T>& n, int rows, int d, float eps,
-                            cudaStream_t s);
+                            bool joins, cudaStream_t s);
   // x += m rms_norm(y) w_post;  h = rms_norm(x) w_pre (skipped when h is NULL)
   static int resid_norm(float* x, const T* y, const float* w_post, float m, const float* w_pre, T* h, int rows, int d, float eps,
                         cudaStream_t s);
@@ -144,7 +145,8 @@ struct RowsBatch {
   // Experts: the batch are the lists of k_moe_choose_few (lists[0] of them, each expert, start, length); list entry p is row
   // p / x_div of X and row p of C; EPI_RELU2 squares the positive part of the result.
   const int* lists = nullptr;
-  int max_lists = 0, x_div = 1;
+  // ready: the kernel before this one is a product over the same lists, which starts its dependents only when it has seen them.
+  int max_lists = 0, x_div = 1, ready = 0;
 };
 int rows_stream(const bf16* X, long long ldx, const bf16* W, long long ldw, void* C, long long ldc, int M, int N, int K, int epi, int batch,
                 const RowsBatch& bt, cudaStream_t s);

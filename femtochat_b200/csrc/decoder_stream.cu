@@ -367,12 +367,15 @@ __global__ void __launch_bounds__(256) k_rows_linear(const T* __restrict__ X, lo
 template <int NT, bool GATED, bool LISTS>
 __global__ void __launch_bounds__(256) k_rows_mma(const bf16* __restrict__ X, long long ldx, const bf16* __restrict__ W, long long ldw,
                                                   void* __restrict__ C, long long ldc, int M, int N, int K, int epi, const RowsBatch bt) {
-  pdl_trigger();
   const int* list = nullptr;
+  // The first product over lists waits for them before it lets its dependents start; the second starts its weights with the lists
+  // that are there then, while the first one's last blocks run.
+  if (LISTS && !bt.ready) pdl_wait();
+  pdl_trigger();
   if constexpr (LISTS) {
-    pdl_wait();
     const int* g = bt.lists + 1 + 3 * blockIdx.y;
-    const int n_lists = bt.lists[0], expert = g[0], start = g[1], length = g[2];      // four loads in flight; past n_lists they are not used
+    // four loads in flight, from L2 (L1 may hold the lists of a layer before); past n_lists they are not used
+    const int n_lists = __ldcg(bt.lists), expert = __ldcg(g), start = __ldcg(g + 1), length = __ldcg(g + 2);
     if ((int)blockIdx.y >= n_lists) return;
     W += expert * bt.w;
     list = bt.lists + 1 + 3 * bt.max_lists + start;
@@ -400,7 +403,7 @@ __global__ void __launch_bounds__(256) k_rows_mma(const bf16* __restrict__ X, lo
   const int kb = warp * 32 + c8;
 #pragma unroll
   for (int u = 0; u < U; u++) fetch(u, kb + u * 256);
-  if (!LISTS) {
+  if (!LISTS || bt.ready) {
     // what does not fit the registers is on its way to L2: a line is 64 k, the share of two warps
     if (!(warp & 1) && !(lane & 3))
       for (int k = warp * 32 + U * 256; k < K; k += 256)
@@ -412,7 +415,7 @@ __global__ void __launch_bounds__(256) k_rows_mma(const bf16* __restrict__ X, lo
 #pragma unroll
   for (int t = 0; t < NT; t++) {
     const int m = 8 * t + g;
-    xp[t] = X + (m < M ? (LISTS ? list[m] / bt.x_div : m) : 0) * ldx;
+    xp[t] = X + (m < M ? (LISTS ? __ldcg(list + m) / bt.x_div : m) : 0) * ldx;
   }
   float acc[RT][NT][4] = {};
   for (int k0 = kb; k0 < K + c8; k0 += U * 256) {       // the four lanes of a row leave together
@@ -462,7 +465,7 @@ __global__ void __launch_bounds__(256) k_rows_mma(const bf16* __restrict__ X, lo
       reinterpret_cast<bf16*>(out.C2)[(m / out.T2) * out.stride2 + (m % out.T2) * out.ld2 + n - out.n2] = __float2bfloat16_rn(v);
       continue;
     }
-    const long long at = LISTS ? list[m] * ldc + n : m * ldc + blockIdx.y * bt.c + n;
+    const long long at = LISTS ? __ldcg(list + m) * ldc + n : m * ldc + blockIdx.y * bt.c + n;
     if (epi == EPI_F32) reinterpret_cast<float*>(C)[at] = v;
     else reinterpret_cast<bf16*>(C)[at] = __float2bfloat16_rn(v);
   }
@@ -479,12 +482,14 @@ int DecStream<T>::embed(const T* table, const int* tokens, int ld_tok, int B, in
 }
 template <typename T>
 int DecStream<T>::parallel_resid(float* x, const T* y, const T* y2, const MoeRows& m, const NextNorms<T>& n, int rows, int d, float eps,
-                                 cudaStream_t s) {
+                                 bool joins, cudaStream_t s) {
   bool vec = (d & 3) == 0;
   for (const void* p : {(const void*)x, (const void*)y, (const void*)y2, m.out, (const void*)n.w, (const void*)n.h, (const void*)n.w2, (const void*)n.h2})
     vec = vec && aligned16(p);
   const int nv = vec ? cdiv(d, RT * 4) : 0;
-#define LAUNCH(NV) CUDA_TRY(launch_dependent(k_parallel_resid<T, NV>, rows, RT, 0, s, x, y, y2, m, n, d, eps))
+  // behind two branches it waits for both, as an ordinary launch does
+#define LAUNCH(NV) do { if (joins) k_parallel_resid<T, NV><<<rows, RT, 0, s>>>(x, y, y2, m, n, d, eps); \
+                        else CUDA_TRY(launch_dependent(k_parallel_resid<T, NV>, rows, RT, 0, s, x, y, y2, m, n, d, eps)); } while (0)
   if (nv == 1) LAUNCH(1);
   else if (nv == 2) LAUNCH(2);
   else if (nv == 3 || nv == 4) LAUNCH(4);

@@ -368,6 +368,12 @@ __global__ void __launch_bounds__(32 * DW, KS <= 8 ? 3 : 1) k_window_decode_mma(
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
   const int first = blockIdx.y * sh.tiles_per, last = min(first + sh.tiles_per, (vis.n + DT - 1) / DT);
+  for (int t = first + warp; t < last; t += DW)      // a lane a key
+    if (lane < vis.n - t * DT) {
+      const long long at = (long long)vis.key(t * DT + lane) * a.ld;
+      prefetch_l2(ksrc + at, 2ll * MD, 0, 1);
+      prefetch_l2(vsrc + at, 2ll * E, 0, 1);
+    }
   pdl_wait();
   uint32_t qa[KS][4];
   float o[NE][2][4] = {}, m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
