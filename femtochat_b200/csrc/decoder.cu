@@ -69,6 +69,7 @@ int decoder_fill(DecoderStack* d, const femto_decoder_config* cfg) {
     DecLayer& l = d->layers[i];
     l.c = cfg->h_layers[i];
     l.own = i;
+    d->mixture = d->mixture || l.c.experts > 0;
     for (int hops = 0; d->layer_cfg[l.own].weights_of >= 0; hops++) {
       if (hops > cfg->n_layer) return femto_fail(FEMTO_ERR_SHAPE, "layer %d: weights_of goes round in a circle", i);
       l.own = d->layer_cfg[l.own].weights_of;
@@ -557,7 +558,7 @@ static int feed_forward(DecoderStack* d, const DecLayer& l, const float* theta, 
   FEMTO_TRY(moe_sort<T>(a, s));
   mr.slot = d->moe_slot;
   GemmArgs g;
-  g.ws = d->gemm_ws; g.ws_bytes = d->gemm_ws_bytes; g.status = d->status; g.any_size = true;
+  g.ws = d->gemm_ws; g.ws_bytes = d->gemm_ws_bytes; g.status = d->status; g.any_size = true; g.whole_k = true;
   g.groups = d->moe_groups; g.group_rows = a.group_rows; g.n_groups = q.experts;
   g.M = (int)moe_max_slots(R, q.experts, q.top, a.group_rows);
   g.A = d->moe_x; g.lda = w; g.B = l.w_gu; g.ldb = w; g.strideB = (long long)l.ffp * w; g.C = d->moe_act; g.ldc = l.ffp;

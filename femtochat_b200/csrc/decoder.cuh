@@ -51,7 +51,7 @@ struct DecoderStack {
   std::vector<femto_decoder_tensor> tensors;
   std::vector<femto_layer_config> layer_cfg;
   long long nparams = 0, off_embed = 0, off_final = 0;
-  bool bf = false, weights_valid = false;
+  bool bf = false, weights_valid = false, mixture = false;      // mixture: some layer has experts
   char* arena = nullptr;
   unsigned int* status = nullptr;
   void* embed = nullptr;              // [vocab][width] compute type: input table

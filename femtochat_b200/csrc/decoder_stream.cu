@@ -594,7 +594,7 @@ int rows_linear(DecoderStack* d, const void* X, long long ldx, const void* W, lo
   GemmArgs g;
   g.ws = d->gemm_ws; g.ws_bytes = d->gemm_ws_bytes; g.status = d->status;
   g.A = X; g.lda = ldx; g.a_kmajor = true; g.B = W; g.ldb = ldw; g.b_kmajor = true;
-  g.C = C; g.ldc = ldc; g.M = M; g.N = N; g.K = K; g.epi = epi; g.beta = 0.f; g.any_size = true; g.bias = out.bias;
+  g.C = C; g.ldc = ldc; g.M = M; g.N = N; g.K = K; g.epi = epi; g.beta = 0.f; g.any_size = true; g.whole_k = d->mixture; g.bias = out.bias;
   if (out.n2) {      // two products: this part, and the rest as a batch over the columns of tokens
     g.N = out.n2;
     FEMTO_TRY(gemm<T>(g, s));

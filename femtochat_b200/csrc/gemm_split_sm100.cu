@@ -331,7 +331,7 @@ bool gemm_split_plan(const GemmArgs& g, int* bn, int* splits) {
   double best = 0.95 * (5.6 + 0.33 * waves * kb + (g.epi == EPI_RESID && waves == 1 ? 2.0 : 0.0));
   bool found = false;
   for (int w = 64; w <= 128; w *= 2)
-    for (int s = 1, doublings = 0; s <= 8; s *= 2, doublings++) {
+    for (int s = 1, doublings = 0; s <= (g.whole_k ? 1 : 8); s *= 2, doublings++) {
       const int stages = cdiv(g.K, 2 * BK), per = cdiv(stages, s);      // of two k-blocks
       if ((s - 1) * per >= stages || (long long)cdiv(g.M, BM) * cdiv(g.N, w) * g.batch * s > cluster_ctas(s)) continue;
       const double cost = (w == 64 ? 4.2 + 0.45 * per : 5.4 + 0.58 * per) + 0.45 * doublings;

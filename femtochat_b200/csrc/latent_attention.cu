@@ -663,7 +663,7 @@ template <typename T> int latent_attention(const LatentArgs& a, cudaStream_t s) 
   GemmArgs g;
   g.ws = a.d->gemm_ws; g.ws_bytes = a.d->gemm_ws_bytes; g.status = a.d->status;
   g.A = a.latent; g.lda = a.ld; g.strideA = (long long)a.maxT * a.ld; g.B = a.w_kv; g.ldb = a.lp; g.strideB = 0;
-  g.C = a.kv; g.ldc = wide; g.strideC = (long long)a.maxT * wide; g.M = N; g.N = wide; g.K = a.lp; g.epi = EPI_STORE; g.any_size = true;
+  g.C = a.kv; g.ldc = wide; g.strideC = (long long)a.maxT * wide; g.M = N; g.N = wide; g.K = a.lp; g.epi = EPI_STORE; g.any_size = true; g.whole_k = a.d->mixture;
   g.batch = a.B;
   FEMTO_TRY(gemm<T>(g, s));
   if (sizeof(T) == 2 && latent_attention_tc_supported(a)) return latent_attention_tc(a, s);
