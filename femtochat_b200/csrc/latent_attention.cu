@@ -300,20 +300,27 @@ __global__ void __launch_bounds__(256) k_latent_decode_mma(const LatentArgs a, i
   }
   __syncthreads();
   // this warp's steps of the queries: latent channels from qabs, then the rotated part, zeros in the padding
+  // (all loads first: one behind the other they took 4 us of the kernel's 10)
+  float2 qf[NK][4];
+#pragma unroll
+  for (int s = 0; s < NK; s++)
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+      const int h = h0 + g + 8 * (e & 1), c = (warp + 8 * s) * 16 + 8 * (e >> 1) + c2;
+      const bool in = h < a.heads && c < a.lp;
+      const float2 v = *reinterpret_cast<const float2*>(a.qabs + (row * a.heads + min(h, a.heads - 1)) * a.lp + min(c, a.lp - 2));
+      qf[s][e] = in ? v : make_float2(0.f, 0.f);
+    }
   uint32_t qa[NK][4], ql[NK][4];
 #pragma unroll
   for (int s = 0; s < NK; s++)
 #pragma unroll
     for (int e = 0; e < 4; e++) {
-      const int r = g + 8 * (e & 1), h = h0 + r, c = (warp + 8 * s) * 16 + 8 * (e >> 1) + c2;
-      float2 f = make_float2(0.f, 0.f);
-      if (h < a.heads) {
-        if (c < a.lp) {
-          f = *reinterpret_cast<const float2*>(a.qabs + (row * a.heads + h) * a.lp + c);
-        } else {
-          if (c < a.lp + a.rot_dim) f.x = qr[r * a.rot_dim + c - a.lp];
-          if (c + 1 < a.lp + a.rot_dim) f.y = qr[r * a.rot_dim + c + 1 - a.lp];
-        }
+      const int r = g + 8 * (e & 1), c = (warp + 8 * s) * 16 + 8 * (e >> 1) + c2;
+      float2 f = qf[s][e];
+      if (c >= a.lp && h0 + r < a.heads) {
+        if (c < a.lp + a.rot_dim) f.x = qr[r * a.rot_dim + c - a.lp];
+        if (c + 1 < a.lp + a.rot_dim) f.y = qr[r * a.rot_dim + c + 1 - a.lp];
       }
       const __nv_bfloat162 hi = __floats2bfloat162_rn(f.x, f.y);
       const __nv_bfloat162 lo = __floats2bfloat162_rn(f.x - __bfloat162float(hi.x), f.y - __bfloat162float(hi.y));

@@ -191,7 +191,9 @@ __global__ void __launch_bounds__(256) k_conv_tail(const DeltaPrepArgs a) {
 // both low-rank projections, state update, read-out, norm and gate.  grid (heads x cluster, columns).  Bound by the chain of
 // dependent loads and sums, so a head's E rows of state and its D + E low-rank rows are shared by the CTAs of a cluster: each makes
 // q, k and its own v, decays and gates; the decays reach the others through distributed shared memory, the state's rows are
-// on their way to registers meanwhile, and the squares for the norm meet the same way.  A warp has whole rows of the state.
+// on their way to registers meanwhile, and the squares for the norm meet the same way.  A warp has whole rows of the state.  Clocks of
+// one block's thread (10 heads, 128 x 128) found what to mend: four rows a warp where it has one, and 4-way bank conflicts, were 5.5 us of 14.
+// From the projections' end, one column: one block a head 18 us, so 8.3.
 __device__ __forceinline__ float sigmoid_f(float z) { return 1.f / (1.f + expf(-z)); }
 
 __device__ __forceinline__ void store_peer(const float* p, uint32_t rank, float v) {
@@ -200,11 +202,11 @@ __device__ __forceinline__ void store_peer(const float* p, uint32_t rank, float 
   asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(at), "f"(v) : "memory");
 }
 
-// SI: 128 channels of a row of the state each
-template <typename T, int SI>
+// SI: 128 channels of a row of the state each; ROWS: rows of the state a warp has in flight
+template <typename T, int SI, int ROWS>
 __global__ void __launch_bounds__(1024) k_delta_decode(const DeltaDecodeArgs a, int cl, int staged) {
   pdl_trigger();
-  constexpr int V = VecN<T>::n, ROWS = 4 / SI, HELD = 2;      // rows of the state a warp has in flight; low-rank rows loaded before the wait
+  constexpr int V = VecN<T>::n, HELD = 2;      // low-rank rows of a warp loaded before the wait
   const DeltaPrepArgs& p = a.p;
   const int h = blockIdx.x / cl, rank = blockIdx.x % cl, b = blockIdx.y, tid = threadIdx.x, threads = blockDim.x, warp = tid >> 5, warps = threads >> 5, lane = tid & 31;
   const int H = p.heads, G = p.kv_heads, D = p.dim, E = p.vdim, n = p.taps, keep = n - 1;
@@ -213,7 +215,7 @@ __global__ void __launch_bounds__(1024) k_delta_decode(const DeltaDecodeArgs a, 
   const int dn = (D + cl - 1) / cl, d0 = min(D, rank * dn), d1 = min(D, d0 + dn), en = (E + cl - 1) / cl, e0 = min(E, rank * en), e1 = min(E, e0 + en);
   const int low = d1 - d0 + e1 - e0;
   extern __shared__ __align__(16) float sm[];
-  float *sq = sm, *sk = sq + D, *sg = sk + D, *sv = sg + D, *so = sv + en, *sz = so + en, *sa = sz + en, *sb = sa + a.ra, *st = sb + a.rg;
+  float *sa = sm, *sb = sa + a.ra, *sq = sb + a.rg, *sk = sq + D, *sg = sk + D, *sv = sg + D, *so = sv + en, *sz = so + en, *st = sz + en;      // ranks are padded to 8
   __shared__ float f_q, f_k, squares[8];
   const T* tin = reinterpret_cast<const T*>(p.tail_in) + (long long)b * keep * channels;
   T* tout = reinterpret_cast<T*>(p.tail_out) + (long long)b * keep * channels;
@@ -245,9 +247,36 @@ __global__ void __launch_bounds__(1024) k_delta_decode(const DeltaDecodeArgs a, 
     const int i = warp + u * warps;
     if (i < low && lane * V < low_rank(i)) held[u] = *reinterpret_cast<const uint4*>(low_row(i) + lane * V);
   }
+  const float rate = expf(p.a_log[h]);
+  auto bias_of = [&](int i) { return i < d1 - d0 ? p.dt_bias[h * D + d0 + i] : 0.f; };
+  float bias[HELD];
+#pragma unroll
+  for (int u = 0; u < HELD; u++) bias[u] = bias_of(warp + u * warps);
+  const float norm = tid < e1 - e0 ? a.norm[e0 + tid] : 0.f;
   if (cl > 1) sm100::cluster_arrive();        // the others have started
   pdl_wait();
   __syncthreads();      // the taps
+  const bool vec = (D & 3) == 0;
+  // rows r0 + r warps + warp of this CTA's part of the state
+  float s[ROWS][SI][4];
+  auto load_state = [&](int r0) {
+#pragma unroll
+    for (int r = 0; r < ROWS; r++)
+#pragma unroll
+      for (int i = 0; i < SI; i++) {
+        const int e = r0 + r * warps + warp, d = 4 * lane + 128 * i;
+        const bool there = e < e1 - e0;
+        const float* Sp = S + (long long)e * D + d;
+        if (vec) {
+          const float4 v = d < D && there ? *reinterpret_cast<const float4*>(Sp) : make_float4(0.f, 0.f, 0.f, 0.f);
+          s[r][i][0] = v.x; s[r][i][1] = v.y; s[r][i][2] = v.z; s[r][i][3] = v.w;
+        } else {
+#pragma unroll
+          for (int j = 0; j < 4; j++) s[r][i][j] = d + j < D && there ? Sp[j] : 0.f;
+        }
+      }
+  };
+  if (ROWS == 1) load_state(0);       // on its way from here on
   const T* proj = reinterpret_cast<const T*>(p.proj) + (long long)b * p.ldp;
   for (int i = tid; i < a.ra + a.rg; i += threads) sa[i] = to_f<T>(i < a.ra ? proj[a.s_a1 + i] : proj[a.s_g1 + i - a.ra]);
   for (int i = tid; i < 2 * D + e1 - e0; i += threads) {
@@ -282,7 +311,6 @@ __global__ void __launch_bounds__(1024) k_delta_decode(const DeltaDecodeArgs a, 
     ss = 1.f / sqrtf(warp_sum(ss) + 1e-6f);
     if (lane == 0) { if (warp & 1) f_k = ss; else f_q = ss * (1.f / sqrtf((float)D)); }
   }
-  const float rate = expf(p.a_log[h]);
   for (int i0 = warp, u = 0; i0 < low; i0 += warps, u++) {
     const bool decay = i0 < d1 - d0;
     const float* x = decay ? sa : sb;
@@ -293,12 +321,15 @@ __global__ void __launch_bounds__(1024) k_delta_decode(const DeltaDecodeArgs a, 
       const uint4 q = c < 32 * V && u < HELD ? (u ? held[1] : held[0]) : *reinterpret_cast<const uint4*>(w + c);
       const T* f = reinterpret_cast<const T*>(&q);
 #pragma unroll
-      for (int e = 0; e < V; e++) z = fmaf(to_f<T>(f[e]), x[c + e], z);
+      for (int e = 0; e < V; e += 4) {
+        const float4 v = *reinterpret_cast<const float4*>(x + c + e);
+        z = fmaf(to_f<T>(f[e]), v.x, z); z = fmaf(to_f<T>(f[e + 1]), v.y, z); z = fmaf(to_f<T>(f[e + 2]), v.z, z); z = fmaf(to_f<T>(f[e + 3]), v.w, z);
+      }
     }
     z = warp_sum(z);
     if (decay) {
       const int c = d0 + i0;
-      z = expf(-rate * softplus_f(z + p.dt_bias[h * D + c]));
+      z = expf(-rate * softplus_f(z + (u < HELD ? (u ? bias[1] : bias[0]) : bias_of(i0))));
       if (cl == 1) { if (lane == 0) sg[c] = z; }
       else if (lane < cl) store_peer(sg + c, lane, z);
     } else if (lane == 0) {
@@ -307,36 +338,34 @@ __global__ void __launch_bounds__(1024) k_delta_decode(const DeltaDecodeArgs a, 
   }
   if (cl > 1) sm100::cluster_arrive(); else __syncthreads();
   const float beta = sigmoid_f(to_f<T>(proj[p.s_b + h]));
-  const bool vec = (D & 3) == 0;
   bool waited = cl == 1;
   for (int r0 = 0; r0 < en; r0 += ROWS * warps) {
-    float s[ROWS][SI][4];
-#pragma unroll
-    for (int r = 0; r < ROWS; r++)
-#pragma unroll
-      for (int i = 0; i < SI; i++) {
-        const int e = r0 + r * warps + warp, d = 4 * lane + 128 * i;
-        const float* Sp = S + (long long)e * D + d;
-        if (vec) {
-          const float4 v = d < D && e < e1 - e0 ? *reinterpret_cast<const float4*>(Sp) : make_float4(0.f, 0.f, 0.f, 0.f);
-          s[r][i][0] = v.x; s[r][i][1] = v.y; s[r][i][2] = v.z; s[r][i][3] = v.w;
-        } else {
-#pragma unroll
-          for (int j = 0; j < 4; j++) s[r][i][j] = d + j < D && e < e1 - e0 ? Sp[j] : 0.f;
-        }
-      }
+    if (ROWS > 1 || r0 > 0) load_state(r0);
     if (!waited) { sm100::cluster_wait(); waited = true; }       // all decays are here, and with them f_q and f_k
-    float dot[ROWS] = {}, o[ROWS] = {};
+    float dot[ROWS] = {}, o[ROWS] = {}, cg[SI][4], ck[SI][4], cq[SI][4];      // decay, key and query of this lane's channels
+#pragma unroll
+    for (int i = 0; i < SI; i++) {
+      const int d = 4 * lane + 128 * i;
+      if (vec && d < D) {
+        const float4 vg = *reinterpret_cast<const float4*>(sg + d), vk = *reinterpret_cast<const float4*>(sk + d), vq = *reinterpret_cast<const float4*>(sq + d);
+        cg[i][0] = vg.x; cg[i][1] = vg.y; cg[i][2] = vg.z; cg[i][3] = vg.w;
+        ck[i][0] = vk.x; ck[i][1] = vk.y; ck[i][2] = vk.z; ck[i][3] = vk.w;
+        cq[i][0] = vq.x; cq[i][1] = vq.y; cq[i][2] = vq.z; cq[i][3] = vq.w;
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; j++) { const bool in = d + j < D; cg[i][j] = in ? sg[d + j] : 0.f; ck[i][j] = in ? sk[d + j] : 0.f; cq[i][j] = in ? sq[d + j] : 0.f; }
+      }
+#pragma unroll
+      for (int j = 0; j < 4; j++) { ck[i][j] *= f_k; cq[i][j] *= f_q; }
+    }
 #pragma unroll
     for (int r = 0; r < ROWS; r++)
 #pragma unroll
       for (int i = 0; i < SI; i++)
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-          const int d = 4 * lane + 128 * i + j;
-          if (d >= D) continue;
-          s[r][i][j] *= sg[d];
-          dot[r] = fmaf(s[r][i][j], sk[d] * f_k, dot[r]);
+          s[r][i][j] *= cg[i][j];
+          dot[r] = fmaf(s[r][i][j], ck[i][j], dot[r]);
         }
 #pragma unroll
     for (int r = 0; r < ROWS; r++) {
@@ -346,10 +375,8 @@ __global__ void __launch_bounds__(1024) k_delta_decode(const DeltaDecodeArgs a, 
       for (int i = 0; i < SI; i++)
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-          const int d = 4 * lane + 128 * i + j;
-          if (d >= D) continue;
-          s[r][i][j] = fmaf(sk[d] * f_k, u, s[r][i][j]);
-          o[r] = fmaf(s[r][i][j], sq[d] * f_q, o[r]);
+          s[r][i][j] = fmaf(ck[i][j], u, s[r][i][j]);
+          o[r] = fmaf(s[r][i][j], cq[i][j], o[r]);
         }
     }
 #pragma unroll
@@ -384,7 +411,7 @@ __global__ void __launch_bounds__(1024) k_delta_decode(const DeltaDecodeArgs a, 
   for (int r = 0; r < cl; r++) ss += squares[r];
   const float inv = 1.f / sqrtf(ss / E + a.eps);
   T* out = reinterpret_cast<T*>(a.out) + ((long long)b * H + h) * E + e0;
-  for (int c = tid; c < e1 - e0; c += threads) out[c] = from_f<T>(so[c] * inv * a.norm[e0 + c] * sz[c]);
+  for (int c = tid; c < e1 - e0; c += threads) out[c] = from_f<T>(so[c] * inv * (c == tid ? norm : a.norm[e0 + c]) * sz[c]);
 }
 
 }  // namespace
@@ -448,8 +475,9 @@ template <typename T> int delta_decode(const DeltaDecodeArgs& a, cudaStream_t s)
     cfg.attrs = at; cfg.numAttrs = off ? 1 : 2;
     return cudaLaunchKernelEx(&cfg, kernel, a, cl, staged);
   };
-  if (a.p.dim <= 128) CUDA_TRY(launch(k_delta_decode<T, 1>));
-  else CUDA_TRY(launch(k_delta_decode<T, 2>));
+  const bool once = en <= threads / 32;      // a warp has one row of the state
+  if (a.p.dim <= 128) CUDA_TRY(once ? launch(k_delta_decode<T, 1, 1>) : launch(k_delta_decode<T, 1, 4>));
+  else CUDA_TRY(once ? launch(k_delta_decode<T, 2, 1>) : launch(k_delta_decode<T, 2, 2>));
   KERNEL_CHECK();
   return 0;
 }
