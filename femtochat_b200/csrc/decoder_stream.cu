@@ -69,10 +69,21 @@ template <typename T> __device__ __forceinline__ void store4(T* p, float a, floa
 }
 
 // NV 4-element vectors per thread stay in registers between the sum and the norms (NV = 0: any width, through memory).
-template <typename T, int NV>
-__global__ void __launch_bounds__(RT) k_parallel_resid(float* __restrict__ x, const T* __restrict__ y, const T* __restrict__ y2, const MoeRows m,
+// AHEAD, up to a row a multiprocessor: the norms' weights are in registers before the wait, and x is on its way with y (a token of Zurevik d20,
+// 4 rows: 876 -> 860 us; a prompt of 7108 rows is 1.5 % slower so, its blocks have fewer registers to hide behind).  y is not __restrict__:
+// what the compiler holds for constant it may load before the wait.
+template <typename T, int NV, bool AHEAD>
+__global__ void __launch_bounds__(RT) k_parallel_resid(float* __restrict__ x, const T* y, const T* y2, const MoeRows m,
                                                        const NextNorms<T> nn, int d, float eps) {
   pdl_trigger();
+  float4 ahead[NV > 0 ? NV : 1], ahead2[NV > 0 ? NV : 1];
+#pragma unroll
+  for (int i = 0; i < (AHEAD ? NV : 0); i++) {
+    const int c = (i * RT + threadIdx.x) * 4;
+    ahead[i] = ahead2[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (c < d && nn.h) ahead[i] = *reinterpret_cast<const float4*>(nn.w + c);
+    if (c < d && nn.h && nn.h2) ahead2[i] = *reinterpret_cast<const float4*>(nn.w2 + c);
+  }
   pdl_wait();
   const long long row = blockIdx.x, base = row * d;
   auto expert_row = [&](int k, float& w) {
@@ -82,7 +93,12 @@ __global__ void __launch_bounds__(RT) k_parallel_resid(float* __restrict__ x, co
   };
   float ss = 0.f;
   if constexpr (NV > 0) {
-    float r[NV][4], f[4];
+    float r[NV][4], f[4], xs[NV][4];
+#pragma unroll
+    for (int i = 0; i < NV; i++) {
+      const int c = (i * RT + threadIdx.x) * 4;
+      if (AHEAD && c < d) load4<float>(x + base + c, xs[i]);
+    }
 #pragma unroll
     for (int i = 0; i < NV; i++) {
       const int c = (i * RT + threadIdx.x) * 4;
@@ -111,9 +127,9 @@ __global__ void __launch_bounds__(RT) k_parallel_resid(float* __restrict__ x, co
     for (int i = 0; i < NV; i++) {
       const int c = (i * RT + threadIdx.x) * 4;
       if (c >= d) continue;
-      load4<float>(x + base + c, f);
+      if (!AHEAD) load4<float>(x + base + c, xs[i]);
 #pragma unroll
-      for (int e = 0; e < 4; e++) { r[i][e] += f[e]; ss += r[i][e] * r[i][e]; }
+      for (int e = 0; e < 4; e++) { r[i][e] += xs[i][e]; ss += r[i][e] * r[i][e]; }
       store4<float>(x + base + c, r[i][0], r[i][1], r[i][2], r[i][3]);
     }
     if (!nn.h) return;
@@ -122,11 +138,11 @@ __global__ void __launch_bounds__(RT) k_parallel_resid(float* __restrict__ x, co
     for (int i = 0; i < NV; i++) {
       const int c = (i * RT + threadIdx.x) * 4;
       if (c >= d) continue;
-      load4<float>(nn.w + c, f);
-      store4<T>(nn.h + base + c, r[i][0] * inv * f[0], r[i][1] * inv * f[1], r[i][2] * inv * f[2], r[i][3] * inv * f[3]);
+      if (!AHEAD) ahead[i] = *reinterpret_cast<const float4*>(nn.w + c);
+      store4<T>(nn.h + base + c, r[i][0] * inv * ahead[i].x, r[i][1] * inv * ahead[i].y, r[i][2] * inv * ahead[i].z, r[i][3] * inv * ahead[i].w);
       if (!nn.h2) continue;
-      load4<float>(nn.w2 + c, f);
-      store4<T>(nn.h2 + base + c, r[i][0] * inv * f[0], r[i][1] * inv * f[1], r[i][2] * inv * f[2], r[i][3] * inv * f[3]);
+      if (!AHEAD) ahead2[i] = *reinterpret_cast<const float4*>(nn.w2 + c);
+      store4<T>(nn.h2 + base + c, r[i][0] * inv * ahead2[i].x, r[i][1] * inv * ahead2[i].y, r[i][2] * inv * ahead2[i].z, r[i][3] * inv * ahead2[i].w);
     }
   } else {
     for (int c = threadIdx.x; c < d; c += RT) {
@@ -498,12 +514,14 @@ int DecStream<T>::parallel_resid(float* x, const T* y, const T* y2, const MoeRow
     vec = vec && aligned16(p);
   const int nv = vec ? cdiv(d, RT * 4) : 0;
   // behind two branches it waits for both, as an ordinary launch does
-#define LAUNCH(NV) do { if (joins) k_parallel_resid<T, NV><<<rows, RT, 0, s>>>(x, y, y2, m, n, d, eps); \
-                        else CUDA_TRY(launch_dependent(k_parallel_resid<T, NV>, rows, RT, 0, s, x, y, y2, m, n, d, eps)); } while (0)
+#define LAUNCH2(NV, AHEAD) do { if (joins) k_parallel_resid<T, NV, AHEAD><<<rows, RT, 0, s>>>(x, y, y2, m, n, d, eps); \
+                                else CUDA_TRY(launch_dependent(k_parallel_resid<T, NV, AHEAD>, rows, RT, 0, s, x, y, y2, m, n, d, eps)); } while (0)
+#define LAUNCH(NV) do { if (rows <= device_sm_count()) LAUNCH2(NV, true); else LAUNCH2(NV, false); } while (0)
   if (nv == 1) LAUNCH(1);
   else if (nv == 2) LAUNCH(2);
   else if (nv == 3 || nv == 4) LAUNCH(4);
-  else LAUNCH(0);
+  else LAUNCH2(0, false);
+#undef LAUNCH2
 #undef LAUNCH
   KERNEL_CHECK();
   return 0;

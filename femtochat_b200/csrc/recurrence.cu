@@ -28,13 +28,18 @@ __global__ void __launch_bounds__(256) k_recurrence(const RecurrenceArgs a) {
   const int D = a.dim, E = a.vdim;
   float* Sp = a.S + (((long long)b * a.heads + h) * E + min(e, E - 1)) * D;
   float s[NI * 4];
+  const bool vec = (D & 3) == 0;
 #pragma unroll
-  for (int i = 0; i < NI; i++)
+  for (int i = 0; i < NI; i++) {
+    const int d = 4 * (sub + 8 * i);
+    if (vec) {
+      const float4 v = e < E && d < D ? *reinterpret_cast<const float4*>(Sp + d) : make_float4(0.f, 0.f, 0.f, 0.f);
+      s[i * 4] = v.x; s[i * 4 + 1] = v.y; s[i * 4 + 2] = v.z; s[i * 4 + 3] = v.w;
+    } else {
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const int d = 4 * (sub + 8 * i) + j;
-      s[i * 4 + j] = (e < E && d < D) ? Sp[d] : 0.f;
+      for (int j = 0; j < 4; j++) s[i * 4 + j] = (e < E && d + j < D) ? Sp[d + j] : 0.f;
     }
+  }
   const float decay = DELTA ? 1.f : a.decay[h];
   for (int t0 = 0; t0 < a.T; t0 += TT) {
     const int n = min(TT, a.T - t0);
@@ -95,12 +100,16 @@ __global__ void __launch_bounds__(256) k_recurrence(const RecurrenceArgs a) {
     }
   }
 #pragma unroll
-  for (int i = 0; i < NI; i++)
+  for (int i = 0; i < NI; i++) {
+    const int d = 4 * (sub + 8 * i);
+    if (e >= E) continue;
+    if (vec) {
+      if (d < D) *reinterpret_cast<float4*>(Sp + d) = make_float4(s[i * 4], s[i * 4 + 1], s[i * 4 + 2], s[i * 4 + 3]);
+    } else {
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const int d = 4 * (sub + 8 * i) + j;
-      if (e < E && d < D) Sp[d] = s[i * 4 + j];
+      for (int j = 0; j < 4; j++) if (d + j < D) Sp[d + j] = s[i * 4 + j];
     }
+  }
 }
 
 // Input x[t - back] of channel c: from this call's rows, or from the inputs kept of earlier calls (zeros before the start).

@@ -103,6 +103,41 @@ def test_columns_equal_each_alone(dtype):
 
 
 @BOTH
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim,conv,ranks,B", [
+    (4, 2, 128, 128, 4, (64, 128), 1),        # eight CTAs a head, a row of the state a warp
+    (4, 2, 128, 130, 4, (300, 520), 1),       # more rows than warps, ranks beyond what is loaded ahead
+    (4, 2, 66, 40, 3, (8, 8), 7),             # four; channels that are no multiple of four
+    (4, 4, 200, 136, 4, (40, 24), 10),        # two
+    (4, 2, 256, 256, 2, (128, 128), 20),      # one
+    (2, 1, 256, 72, 40, (16, 16), 3)])        # taps that do not fit shared memory
+def test_one_token_of_the_delta_rule(heads, kv_heads, dim, vdim, conv, ranks, B, dtype):
+    """Every cluster size and every form of the one-token kernel, token by token from the first on."""
+    cfg = dc.config(dc.delta(heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim, conv=conv, ff=0))
+    model, w = dc.model_and_weights(cfg, ranks, dtype, seed=13)
+    n = 12
+    t = torch.stack([dc.tokens(n, cfg["vocab"], 60 + b) for b in range(B)])
+    want = torch.stack([lo.Sequence(cfg, w).feed(t[b]) for b in range(B)])
+    c = cache_for(model, n, B)
+    for k in range(n):
+        z = fb.extend(model, c, t[:, k:k + 1], want=list(range(B)))
+        assert dc.rel_error(z, want[:, k]) < TOL[dtype], k
+    ok(model)
+
+
+@pytest.mark.parametrize("edge", [16, 32, 512, 1024])
+def test_latent_attention_at_the_edges_of_its_tiles(edge):
+    """Contexts around which the one-token kernel takes another tile, and wider ones (16 keys up to 512, then 32, then 64)."""
+    cfg, ranks = dc.SINGLE["latent, dim 64"]
+    model, w = dc.model_and_weights(cfg, ranks, "bfloat16", seed=14)
+    n = edge + 4
+    t = dc.tokens(n, cfg["vocab"], 70)
+    want = lo.Sequence(cfg, w).feed(t)
+    c = cache_for(model, n)
+    assert dc.rel_error(dc.feed(model, c, t, (edge - 3,) + (1,) * 7), want) < TOL["bfloat16"]
+    ok(model)
+
+
+@BOTH
 @pytest.mark.parametrize("name", ["mixed", "large"])
 def test_steps_as_one_launch_equal_plain_launches(name, dtype):
     """From a handle's second step on, a step is one launch of a graph; a step whose wanted positions are listed is launched kernel by
