@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(RT) k_resid_norm(float* __restrict__ x, const 
   pdl_trigger();
   const long long base = (long long)blockIdx.x * d;
   if constexpr (NV > 0) {
-    // The weights are in registers before the wait: behind the sums they were 0.5 of a token's 2.9 us.
+    // The weights are in registers before the wait: behind the sums, in 40 norms of one block, they were 46 of a token's 646 us.
     float4 post[NV], pre[NV];
 #pragma unroll
     for (int i = 0; i < NV; i++) {
