@@ -649,11 +649,12 @@ static int step_by_graph(DecoderStack* d, femto_kv_cache* c, const float* theta,
   if (status != cudaStreamCaptureStatusNone) return 0;
   if (!g.stream) {
     int low = 0, high = 0;      // the attention's short kernels go before the blocks of the experts' products
-    CUDA_TRY(cudaDeviceGetStreamPriorityRange(&low, &high));
-    if (!g.side) CUDA_TRY(cudaStreamCreateWithPriority(&g.side, cudaStreamNonBlocking, low));
-    if (!g.fork) CUDA_TRY(cudaEventCreateWithFlags(&g.fork, cudaEventDisableTiming));
-    if (!g.join) CUDA_TRY(cudaEventCreateWithFlags(&g.join, cudaEventDisableTiming));
-    CUDA_TRY(cudaStreamCreateWithPriority(&g.stream, cudaStreamNonBlocking, high));
+    const bool made = cudaDeviceGetStreamPriorityRange(&low, &high) == cudaSuccess &&
+                      (g.side || cudaStreamCreateWithPriority(&g.side, cudaStreamNonBlocking, low) == cudaSuccess) &&
+                      (g.fork || cudaEventCreateWithFlags(&g.fork, cudaEventDisableTiming) == cudaSuccess) &&
+                      (g.join || cudaEventCreateWithFlags(&g.join, cudaEventDisableTiming) == cudaSuccess) &&
+                      cudaStreamCreateWithPriority(&g.stream, cudaStreamNonBlocking, high) == cudaSuccess;
+    if (!made) { cudaGetLastError(); g.streak = 0; g.wait = 64; return 0; }
   }
   std::vector<int> tails;
   for (const auto& l : c->state) tails.push_back(l.tail_now);
@@ -665,7 +666,7 @@ static int step_by_graph(DecoderStack* d, femto_kv_cache* c, const float* theta,
     g.streak = 0; g.wait = 64;
     return 0;
   };
-  CUDA_TRY(cudaStreamBeginCapture(g.stream, cudaStreamCaptureModeThreadLocal));
+  if (cudaStreamBeginCapture(g.stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) return leave();
   int r = d->bf ? pass_t<bf16>(d, c, theta, tokens, 1, B, 1, nullptr, g.stream, &g) : pass_t<float>(d, c, theta, tokens, 1, B, 1, nullptr, g.stream, &g);
   if (r == 0 && logits_out)
     r = d->bf ? logits_t<bf16>(d, theta, nullptr, 1, B, logits_out, g.stream) : logits_t<float>(d, theta, nullptr, 1, B, logits_out, g.stream);
