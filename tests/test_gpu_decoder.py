@@ -137,6 +137,19 @@ def test_latent_attention_at_the_edges_of_its_tiles(edge):
     ok(model)
 
 
+def test_models_with_experts_sum_in_one_order():
+    """Products of 44 rows would share K among the blocks of a cluster, those of 352 would not: with experts the same columns give the
+    same bits in both, so that a router does not choose by the number of its neighbours."""
+    layer = dict(heads=8, kv_heads=4, dim=128, vdim=128, size=70, scale=0.09)
+    cfg = dc.zurevik(dc.sinks(mlp=dc.moe(ff=1024, experts=4), **layer), dc.sinks(mlp=dc.moe(ff=1024, experts=4), **layer), width=1024, vocab=512)
+    model, _ = dc.model_and_weights(cfg, (8, 8), "bfloat16", seed=15)
+    t = torch.stack([dc.tokens(11, cfg["vocab"], 80 + b) for b in range(4)])
+    few = fb.prefill(model, cache_for(model, 11, 4), t)
+    many = fb.prefill(model, cache_for(model, 11, 32), t.repeat(8, 1))
+    assert torch.equal(many[:4], few)
+    ok(model)
+
+
 @BOTH
 @pytest.mark.parametrize("name", ["mixed", "large"])
 def test_steps_as_one_launch_equal_plain_launches(name, dtype):
