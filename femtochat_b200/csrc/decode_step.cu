@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(THREADS + 128, 1) k_decode_step(const DecodeSt
         float q = 0.f;
 #pragma unroll
         for (int w = 0; w < WARPS; w++) q += ssp[b][w];
-        const float inv = rsqrtf(q * a.inv_d + a.eps);
+        const float inv = 1.f / sqrtf(q / d + a.eps);      // correctly rounded, as every other norm of the model
         if (lane == 0) inv_s[b] = inv;
         v *= inv;
       }
@@ -816,7 +816,7 @@ int decode_step_run(const femto_handle* h, const DecodeStepState& st, DecodeStep
     CUDA_TRY(cudaMemsetAsync(st.launches + 1, 0x5a, 4, s));
   }
   const int nt = a.B <= 8 ? 1 : 2, gmax = a.H / a.Hkv <= 2 ? 2 : 8;
-  a.ring = st.ring[nt - 1]; a.inv_d = 1.f / a.d;
+  a.ring = st.ring[nt - 1];
   const size_t smem = smem_bytes(a.d, a.L, nt, gmax) + (size_t)a.ring * slot_bytes(steps_of(a.d));
   a.red_bytes = (int)red_bytes(nt, gmax);
   cudaLaunchConfig_t cfg = {};

@@ -38,8 +38,7 @@ struct DecodeStepArgs {
   unsigned int* status;
   long long off_wte, off_smear, off_lam_s, off_lam_y;
   int d, dq, kv, H, Hkv, V, Vp, L, backout, B, t, maxT, docs, splits, red_bytes, ring, live;      // live: rows of the tables come from Theta
- 
-  float eps, inv_d;
+  float eps;
 };
 
 void decode_step_plan(const femto_handle* h, int max_batch, DecodeStepState& st);

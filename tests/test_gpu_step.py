@@ -599,6 +599,41 @@ def test_decode_kernel_gives_up_on_words_that_never_come():
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("B", [16, 4])
+def test_decode_step_takes_the_reciprocal_root_in_correctly_rounded_operations(B):
+    """The norm before the head, bit for bit.  Blocks that add nothing hand it the embedding: k channels of one bf16 value, whose squares
+    sum exactly in any order, and a head that reads one channel times a power of two, so small that the soft cap's tanh gives back its
+    argument.  What is left of a logit is 1 / sqrt(mean + eps) and three more operations, here in numpy's fp32, which rounds correctly."""
+    import numpy as np
+    f, d, scale = np.float32, 512, 2.0 ** -16
+    cfg = fb.GPTConfig(sequence_len=80, max_document_tokens=128, vocab_size=300, n_layer=2, n_head=4, n_kv_head=2, n_embed=d, window_pattern="L")
+    lay = fb.parameter_layout(cfg)
+    theta = torch.zeros(lay.nparams, device="cuda")
+    fb.initialize_(theta, lay, seed=3)       # the projections back into the stream are zero
+    for block in lay.blocks:
+        theta[block["lam_b"].offset], theta[block["lam_x0"].offset] = 1.0, 0.0
+    theta[lay.lam_y.offset] = 0.0
+    vp = lay.embedding.shape[1]
+    theta[lay.embedding.offset:lay.embedding.offset + lay.embedding.size] = (torch.arange(d)[None, :] < torch.arange(1, vp + 1)[:, None]).float().flatten().cuda()
+    theta[lay.lm_head.offset:lay.lm_head.offset + lay.lm_head.size] = 0.0
+    theta[lay.lm_head.offset:lay.lm_head.offset + vp] = scale
+    model = fb.GPT(fb.Params(theta, delta=False), cfg, lay, compute_type="bfloat16")
+    eps = f(fo.EPS_BF16)
+    kc = fb.KVCache(model.state(B), B, 80)
+    fb.prefill(model, kc, torch.ones(B, 1, dtype=torch.int32))
+    for first in range(1, 257, B):
+        ids = torch.arange(first, first + B, dtype=torch.int32)      # token k has k channels
+        z = fb.decode_step(model, kc, ids)
+        k = ids.numpy().astype(np.float32)
+        e = torch.from_numpy(f(1) / np.sqrt(k / f(d) + eps)).bfloat16().float().numpy()
+        inv = f(1) / np.sqrt(k * e * e / f(d) + eps)
+        want = f(15) * (e * f(scale) * inv / f(15))
+        assert want.dtype == np.float32
+        assert torch.equal(z, torch.from_numpy(want).cuda()[:, None].expand_as(z)), first
+    kc.close()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("B,H,G,Tp,T", [
     (1, 2, 1, 317, 326),           # five key ranges, then six: the ranges are added four at a time
     (1, 1, 1, 2040, 2056),         # the cap of 32 ranges
