@@ -141,6 +141,23 @@ static inline cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3
   cfg.attrs = at; cfg.numAttrs = off ? 0 : 1;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
+// Lets a kernel's launches have `bytes` of dynamic shared memory.  The limit belongs to the function and the device, not to a model or a
+// call: it is set once, to all that a block may have beside the kernel's own.  (Set to each launch's size, as it was, two threads that
+// step two models lower each other's between setting and launch; and 48 KB without setting it leave no room for the kernel's own.)
+template <auto KERNEL> static int allow_smem(size_t bytes) {
+  static PerDevice attr;
+  const int dev = PerDevice::current();
+  if (dev < 0 || !attr.done[dev]) {
+    cudaFuncAttributes fixed;
+    int device = 0, most = 0;
+    CUDA_TRY(cudaGetDevice(&device));
+    CUDA_TRY(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
+    CUDA_TRY(cudaFuncGetAttributes(&fixed, KERNEL));
+    CUDA_TRY(cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)fixed.sharedSizeBytes));
+    if (dev >= 0) attr.done[dev] = true;
+  }
+  return bytes <= 227 * 1024 ? 0 : femto_fail(FEMTO_ERR_UNSUPPORTED, "a block would need %zu bytes of shared memory", bytes);
+}
 #endif
 int device_sm_count();   // multiprocessors of the current device (cached per device)
 

@@ -563,12 +563,6 @@ __global__ void __launch_bounds__(1024) k_latent_decode_out(const LatentArgs a, 
 }
 
 // Opt-in to more than 48 KB of dynamic shared memory, once per kernel and device.
-template <typename K> int allow_smem(K kernel, size_t bytes) {
-  if (bytes > 227 * 1024) return femto_fail(FEMTO_ERR_UNSUPPORTED, "latent attention: a tile needs %zu bytes of shared memory", bytes);
-  if (bytes > 48 * 1024) CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-  return 0;
-}
-
 }  // namespace
 
 template <typename T> int latent_norms(const LatentArgs& a, cudaStream_t s) {
@@ -602,7 +596,7 @@ static int latent_decode_tc(const LatentArgs& a, cudaStream_t s, bool& done) {
   int per = std::max(1, cdiv(tiles, std::max(1, device_sm_count() / blocks)));      // as many splits as fill the device once
   while ((size_t)rows * H * cdiv(tiles, per) * (a.lp + 2) > a.part_floats) per++;
   const int splits = cdiv(tiles, per);
-#define LAUNCH(NK, NP) do { FEMTO_TRY(allow_smem(k_latent_decode_mma<NK, NP>, bytes(KT))); \
+#define LAUNCH(NK, NP) do { FEMTO_TRY((allow_smem<k_latent_decode_mma<NK, NP>>(bytes(KT)))); \
   CUDA_TRY(launch_dependent(k_latent_decode_mma<NK, NP>, dim3(cdiv(H, 16), splits, rows), 256, bytes(KT), s, a, splits, per, KT, width)); } while (0)
   if (nk <= 1) LAUNCH(1, 1);
   else if (nk <= 2) LAUNCH(2, 2);
@@ -632,7 +626,7 @@ template <typename T> static int latent_decode(const LatentArgs& a, cudaStream_t
   constexpr int V = VecN<T>::n;
   const int N = a.first + a.T, rows = a.B * a.T;
   const size_t absorb = 4 * (size_t)(a.dim + a.rot_dim + 1024 / (a.lp / V) * a.lp);
-  FEMTO_TRY(allow_smem(k_absorb_q<T>, absorb));
+  FEMTO_TRY(allow_smem<k_absorb_q<T>>(absorb));
   CUDA_TRY(launch_dependent(k_absorb_q<T>, dim3(a.heads, rows), 1024, absorb, s, a));
   KERNEL_CHECK();
   const int blocks = cdiv(a.heads, 8) * rows;
@@ -641,7 +635,7 @@ template <typename T> static int latent_decode(const LatentArgs& a, cudaStream_t
   const size_t smem = 4 * (size_t)(32 * (a.ld + 1) + 8 * a.ld);
   const int per = cdiv(a.lp, 32);
   const dim3 grid(cdiv(a.heads, 8), splits, rows);
-#define LAUNCH(PER) do { FEMTO_TRY(allow_smem(k_latent_decode<T, PER>, smem)); CUDA_TRY(launch_dependent(k_latent_decode<T, PER>, grid, 256, smem, s, a, splits)); } while (0)
+#define LAUNCH(PER) do { FEMTO_TRY((allow_smem<k_latent_decode<T, PER>>(smem))); CUDA_TRY(launch_dependent(k_latent_decode<T, PER>, grid, 256, smem, s, a, splits)); } while (0)
   if (per <= 4) LAUNCH(4);
   else if (per <= 8) LAUNCH(8);
   else if (per <= 16) LAUNCH(16);
@@ -675,7 +669,7 @@ template <typename T> int latent_attention(const LatentArgs& a, cudaStream_t s) 
   FEMTO_TRY(gemm<T>(g, s));
   if (sizeof(T) == 2 && latent_attention_tc_supported(a)) return latent_attention_tc(a, s);
   const size_t smem = 4 * (size_t)((SQ + SK) * (a.dim + a.rot_dim + 1) + SK * a.vdim + SQ * (SK + 1) + 2 * SQ);
-  FEMTO_TRY(allow_smem(k_latent_attn_simt<T>, smem));
+  FEMTO_TRY(allow_smem<k_latent_attn_simt<T>>(smem));
   k_latent_attn_simt<T><<<dim3(cdiv(a.T, SQ), a.heads, a.B), 128, smem, s>>>(a, N);
   KERNEL_CHECK();
   return 0;

@@ -884,15 +884,17 @@ int optimizer_step(femto_optimizer* o, float* theta, const float* delta, float e
     int blocks = 0;
     for (int i = 0; i < b.n; i++) blocks += b.g[i].k;
     const size_t bytes = floats * sizeof(float);
-    auto launch = [&](auto kernel) -> int {
-      if (bytes > 48 << 10) CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    auto launch = [&](auto kernel, int allowed) -> int {
+      FEMTO_TRY(allowed);
       kernel<<<blocks, 256, bytes, s>>>(theta, delta, b);
       KERNEL_CHECK();
       return 0;
     };
     b.n = 0;
-    if (o->cfg.compute_dtype == FEMTO_BF16) return h->bf ? launch(k_muon_small<bf16, bf16>) : launch(k_muon_small<bf16, float>);
-    return h->bf ? launch(k_muon_small<float, bf16>) : launch(k_muon_small<float, float>);
+#define LAUNCH(T, S) launch(k_muon_small<T, S>, allow_smem<k_muon_small<T, S>>(bytes))
+    if (o->cfg.compute_dtype == FEMTO_BF16) return h->bf ? LAUNCH(bf16, bf16) : LAUNCH(bf16, float);
+    return h->bf ? LAUNCH(float, bf16) : LAUNCH(float, float);
+#undef LAUNCH
   };
   SmallMuonBatch sb = {};
   sb.steps = o->cfg.ns_steps; sb.inv_nt = 1.f / n_tokens;

@@ -571,12 +571,6 @@ __global__ void __launch_bounds__(512) k_window_combine(const WindowAttnArgs a, 
   }
 }
 
-template <typename K> int allow_smem(K kernel, size_t bytes) {
-  if (bytes > 227 * 1024) return femto_fail(FEMTO_ERR_UNSUPPORTED, "attention: a tile needs %zu bytes of shared memory", bytes);
-  if (bytes > 48 * 1024) CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-  return 0;
-}
-
 template <typename T> int window_decode(const WindowAttnArgs& a, cudaStream_t s) {
   constexpr int V = VecN<T>::n;
   const int rows = a.B * a.T, es = sizeof(T);
@@ -612,7 +606,7 @@ template <typename T> int window_decode(const WindowAttnArgs& a, cudaStream_t s)
   if (floats() > a.part_floats) return femto_fail(FEMTO_ERR_STATE, "attention: no room for the partial results of %d rows", rows);
   sh.splits = cdiv(tiles, sh.tiles_per);
   const dim3 grid(a.kv_heads * sh.groups, sh.splits, rows);
-#define LAUNCH(KERNEL, THREADS) do { FEMTO_TRY(allow_smem(KERNEL, smem)); CUDA_TRY(launch_dependent(KERNEL, grid, THREADS, smem, s, a, sh)); } while (0)
+#define LAUNCH(KERNEL, THREADS) do { FEMTO_TRY((allow_smem<KERNEL>(smem))); CUDA_TRY(launch_dependent(KERNEL, grid, THREADS, smem, s, a, sh)); } while (0)
   if (tc) {
     if (sh.pk <= 64 && sh.pv <= 64) LAUNCH((k_window_decode_mma<4, 4>), 32 * DW);
     else if (sh.pk <= 128 && sh.pv <= 128) LAUNCH((k_window_decode_mma<8, 8>), 32 * DW);
@@ -665,10 +659,10 @@ template <typename T> int window_attention(const WindowAttnArgs& a, cudaStream_t
   const size_t smem = 4 * (size_t)((SQ + SK) * (a.dim + 1) + SK * a.vdim + SQ * (SK + 1) + 2 * SQ + 4);
   const dim3 grid(cdiv(a.T, SQ), a.heads, a.B);
   if (a.maps == 2) {
-    FEMTO_TRY(allow_smem(k_window_attn<T, 2>, smem));
+    FEMTO_TRY((allow_smem<k_window_attn<T, 2>>(smem)));
     k_window_attn<T, 2><<<grid, 128, smem, s>>>(a);
   } else {
-    FEMTO_TRY(allow_smem(k_window_attn<T, 1>, smem));
+    FEMTO_TRY((allow_smem<k_window_attn<T, 1>>(smem)));
     k_window_attn<T, 1><<<grid, 128, smem, s>>>(a);
   }
   KERNEL_CHECK();

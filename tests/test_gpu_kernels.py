@@ -653,13 +653,49 @@ def test_muon_direction_matches_oracle_two_steps(dtype, k, m, n):
         assert (v.cpu().reshape(st.v.shape) - st.v).abs().max() <= (6e-2 if dtype == _lib.BF16 else 1e-5) * float(st.v.abs().max())
 
 
+def test_small_muon_matrices_of_two_models_in_two_threads():
+    """The limit of a kernel's shared memory is the function's, not a model's: updates of 64 x 64 and of 60 x 60 matrices, from two
+    threads at once, are all launched, and give what the same updates give one after the other."""
+    import threading
+
+    def model(d):
+        cfg = fb.GPTConfig(sequence_len=4, max_document_tokens=16, vocab_size=16, n_layer=1, n_head=2, n_kv_head=2, n_embed=d, window_pattern="L")
+        lay = fb.parameter_layout(cfg)
+        g = torch.Generator(device="cuda").manual_seed(d)
+        params = fb.Params(torch.randn(lay.nparams, device="cuda", generator=g) * 0.1)
+        params.delta.normal_(0.0, 3.0, generator=g)
+        tok = torch.ones(1, 4, dtype=torch.int32, device="cuda")
+        return params, fb.MuonAdamW(params, lay, fb.gradient_state(params, cfg, lay, tok, tok))
+
+    failed = []
+
+    def train(opt):
+        try:
+            for _ in range(500):
+                opt.step(Nt=64.0)
+        except Exception as e:
+            failed.append(e)
+
+    alone, both = [model(d) for d in (64, 60)], [model(d) for d in (64, 60)]
+    for _, opt in alone:
+        train(opt)
+    threads = [threading.Thread(target=train, args=(opt,)) for _, opt in both]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not failed, failed[0]
+    assert all(torch.equal(a[0].theta, b[0].theta) for a, b in zip(alone, both))
+
+
 @pytest.mark.parametrize("ctype", ["float32", "bfloat16"])
-@pytest.mark.parametrize("d,heads,kv,steps", [(28, 2, 1, 5), (24, 1, 1, 4), (32, 2, 1, 5), (32, 4, 4, 1), (40, 5, 1, 5)])
+@pytest.mark.parametrize("d,heads,kv,steps", [(28, 2, 1, 5), (24, 1, 1, 4), (32, 2, 1, 5), (32, 4, 4, 1), (40, 5, 1, 5), (88, 2, 1, 5)])
 def test_small_muon_matrices_take_the_same_bits_in_one_launch(ctype, d, heads, kv, steps):
     """An update whose matrices are small is one launch; `femto_muon_direction` on the same stack is the chain of launches.  Moments are the
     same bits and so is the direction: the new weights follow from it with two roundings.  Square, tall and wide matrices, one row (value
-    gates), a width that is no multiple of four, an even number of iterations (the stack ends where it began), and 4096 elements, beside
-    matrices of 6400 (40 wide) that keep the chain."""
+    gates), a width that is no multiple of four, an even number of iterations (the stack ends where it began), 4096 elements, beside
+    matrices of 6400 (40 wide) that keep the chain, and 88 x 44, which fill 48 KB of shared memory but for less than the kernel's own."""
     cfg = fb.GPTConfig(sequence_len=4, max_document_tokens=16, vocab_size=16, n_layer=3, n_head=heads, n_kv_head=kv, n_embed=d, window_pattern="L")
     lay = fb.parameter_layout(cfg)
     g = torch.Generator(device="cuda").manual_seed(d + steps)
