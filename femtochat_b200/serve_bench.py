@@ -114,8 +114,9 @@ def measure(model, B, T, vocab, n_decode=32, kernels=False):
     import femtochat_b200 as fb
     g = torch.Generator(device="cuda").manual_seed(2)
     tok = torch.randint(model.index_base, vocab + model.index_base, (B, T), generator=g, device="cuda", dtype=torch.int32)
-    model.state(B).refresh_weights(model.params.theta)
-    model.state(B).refresh_weights = lambda theta: None      # Θ does not change: no cast inside the timed calls
+    state = model.state(B)
+    state.refresh_weights(model.params.theta)
+    state.refresh_weights = state.refresh_for = lambda theta: None      # Θ does not change: no cast inside the timed calls
     c = fb.KVCache(model.state(B), B, T + 4 * n_decode + 64)
     pre = timed(lambda: fb.prefill(model, c, tok), 5)
     one = tok[:, 0].contiguous()

@@ -694,3 +694,20 @@ def test_update_kernels_refresh_the_compute_type_weights(cfgkw, ctype):
         after_refresh = fb.loss_and_gradient_(params, st, lay, tok, tgt, pos)
         assert after_update == after_refresh, step
         assert torch.equal(delta_a, params.delta)
+
+
+@pytest.mark.gpu
+def test_serving_times_hold_no_cast_of_weights(capsys):
+    """The serving benchmark says that its timed calls cast no weights: none of the kernels that it lists is a cast, and the model's next
+    own prompt has one."""
+    from femtochat_b200 import serve_bench
+    size = dict(width=256, n_layer=2, heads=2, kv_heads=1, vocab=300)
+    model = serve_bench.random_gpt(size, 256)
+    serve_bench.measure(model, 2, 40, size["vocab"], n_decode=4, kernels=True)
+    listed = capsys.readouterr().out
+    assert "k_qkv_post" in listed and "k_cast_all" not in listed, listed
+    del model.state(2).refresh_for
+    kc = fb.KVCache(model.state(2), 2, 40)
+    tok = torch.ones(2, 20, dtype=torch.int32, device="cuda")
+    assert any("k_cast_all" in name for name, _, _ in serve_bench.kernel_times(lambda: fb.prefill(model, kc, tok)))
+    kc.close()
