@@ -293,4 +293,13 @@ struct XentArgs {
   cudaEvent_t ev_read[2] = {nullptr, nullptr}; cudaEvent_t ev_fork[2] = {nullptr, nullptr};
 };
 template <typename T> int xent_tail(const XentArgs& x, cudaStream_t s);
-bool gemm_profiling();   // per-launch GEMM timing is on: every launch stays on one stream so that the times add up
+bool gemm_profiling();   // per-launch GEMM timing is on: every launch stays on one stream, and out of graphs, so that the times add up
+// While it is on, brackets the launch of a tensor-core GEMM (either kernel) with events.
+struct GemmSpan {
+  cudaStream_t s;
+  cudaEvent_t first = nullptr, last = nullptr;
+  double flops;
+  GemmSpan(const GemmArgs& g, cudaStream_t s);
+  ~GemmSpan();
+  GemmSpan(const GemmSpan&) = delete;
+};

@@ -641,6 +641,7 @@ static int logits_t(DecoderStack* d, const float* theta, const int* want, int st
 // for a while; so do steps that the caller records.  ran stays false, and the cache as it was, where plain launches are to do the step.
 static int step_by_graph(DecoderStack* d, femto_kv_cache* c, const float* theta, const int* tokens, int B, float* logits_out, cudaStream_t s, bool& ran) {
   StepGraph& g = d->step;
+  if (gemm_profiling()) return 0;      // events of a recording have no times
   g.streak = B == g.B ? std::min(g.streak + 1, 1 << 20) : 0;
   g.B = B;
   if (g.streak < g.wait) return 0;

@@ -740,6 +740,17 @@ struct GemmProfile {
 }  // namespace
 
 bool gemm_profiling() { return g_prof.on; }
+GemmSpan::GemmSpan(const GemmArgs& g, cudaStream_t s) : s(s), flops(2.0 * g.M * (double)g.N * g.K * g.batch) {
+  if (!g_prof.on) return;
+  cudaEventCreate(&first); cudaEventCreate(&last);
+  cudaEventRecord(first, s);
+}
+GemmSpan::~GemmSpan() {
+  if (!first) return;
+  cudaEventRecord(last, s);
+  g_prof.ev.push_back(first); g_prof.ev.push_back(last);
+  g_prof.flops += flops;
+}
 extern "C" int32_t femto_profile_gemm(int32_t enable) {
   for (auto e : g_prof.ev) cudaEventDestroy(e);
   g_prof.ev.clear();
@@ -927,17 +938,9 @@ int gemm_tc_bf16(const GemmArgs& g, cudaStream_t s) {
     p.tma_store = 1;
   }
   const int grid = pair ? 2 * std::min(p.total_units, workers) : std::min(p.total_units, sms);
-  cudaEvent_t e0 = nullptr, e1 = nullptr;
-  if (g_prof.on) {
-    cudaEventCreate(&e0); cudaEventCreate(&e1);
-    cudaEventRecord(e0, s);
-  }
-  if (pair) FEMTO_TRY(launch_tc<true>(g, tmA, tmB, tmC, p, grid, s));
-  else FEMTO_TRY(launch_tc<false>(g, tmA, tmB, tmC, p, grid, s));
-  if (g_prof.on) {
-    cudaEventRecord(e1, s);
-    g_prof.ev.push_back(e0); g_prof.ev.push_back(e1);
-    g_prof.flops += 2.0 * g.M * (double)g.N * g.K * g.batch;
+  {
+    GemmSpan span(g, s);
+    FEMTO_TRY(pair ? launch_tc<true>(g, tmA, tmB, tmC, p, grid, s) : launch_tc<false>(g, tmA, tmB, tmC, p, grid, s));
   }
   KERNEL_CHECK();
   if (splits > 1) {

@@ -375,10 +375,13 @@ int gemm_split_bf16(const GemmArgs& g, int bn, int splits, cudaStream_t s) {
                         : g.b_kmajor        ? launch_split<true, S, false, KS>(tmA, tmB, p, grid, smem, s) \
                                             : launch_split<false, S, false, KS>(tmA, tmB, p, grid, smem, s))
 #define LAUNCH(S) (ks == 2 ? LAUNCH2(S, 2) : LAUNCH2(S, 1))
-  if (splits == 1) r = LAUNCH(1);
-  else if (splits == 2) r = LAUNCH(2);
-  else if (splits == 4) r = LAUNCH(4);
-  else r = LAUNCH(8);
+  {
+    GemmSpan span(g, s);
+    if (splits == 1) r = LAUNCH(1);
+    else if (splits == 2) r = LAUNCH(2);
+    else if (splits == 4) r = LAUNCH(4);
+    else r = LAUNCH(8);
+  }
 #undef LAUNCH
 #undef LAUNCH2
   FEMTO_TRY(r);

@@ -467,8 +467,8 @@ int32_t femto_selftest_gemm_few_rows(const void* A, int64_t lda, const void* B, 
                                      int64_t strideA, int64_t strideB, int64_t strideC, int32_t epilogue, int32_t tile_columns,
                                      int32_t splits, void* stream);
 
-/* Measurement aid (no counterpart in the reference): when enabled, every launch of the tensor-core
- * GEMM kernel is bracketed by CUDA events on its stream; the report returns the summed kernel time,
+/* Measurement aid (no counterpart in the reference): when enabled, every launch of a tensor-core
+ * GEMM kernel (the persistent one, or that of few rows) is bracketed by CUDA events on its stream; the report returns the summed kernel time,
  * the summed 2*M*N*K and the launch count since the last femto_profile_gemm call. */
 int32_t femto_profile_gemm(int32_t enable);
 int32_t femto_profile_gemm_report(double* h_ms, double* h_flops, int32_t* h_launches);

@@ -711,3 +711,41 @@ def test_serving_times_hold_no_cast_of_weights(capsys):
     tok = torch.ones(2, 20, dtype=torch.int32, device="cuda")
     assert any("k_cast_all" in name for name, _, _ in serve_bench.kernel_times(lambda: fb.prefill(model, kc, tok)))
     kc.close()
+
+
+def _profiled(fn):
+    """(milliseconds, FLOPs, launches) of the tensor-core products of one call."""
+    ms, flops, n = C.c_double(0), C.c_double(0), C.c_int32(0)
+    _lib.lib().femto_profile_gemm(1)
+    fn()
+    torch.cuda.synchronize()
+    _lib.lib().femto_profile_gemm_report(C.byref(ms), C.byref(flops), C.byref(n))
+    _lib.lib().femto_profile_gemm(0)
+    return ms.value, flops.value, n.value
+
+
+@pytest.mark.gpu
+def test_profile_of_products_counts_those_of_few_rows():
+    """A prompt of 24 tokens: four products a block, all on the tensor cores, whichever of the two kernels takes them."""
+    model, tok, pos, _ = _bf16_server(1, 4, 2, 2, 40, False)
+    kc = fb.KVCache(model.state(1), 1, 40)
+    ms, flops, n = _profiled(lambda: fb.prefill(model, kc, tok[:, :24], pos[:, :24]))
+    assert n == 8 and flops == 2 * 2.0 * 24 * 512 * (1024 + 512 + 2048 + 2048) and ms > 0
+    kc.close()
+
+
+@pytest.mark.gpu
+def test_profile_of_products_times_every_step():
+    """Forty columns of a decoder, whose steps are launches of a graph otherwise: each step's products are timed, and the next call is in order."""
+    import decoder_cases as dc
+    model, _ = dc.model_and_weights(dc.LARGE, dc.LARGE_RANKS, "bfloat16", seed=12)
+    kc = fb.KVCache(model.state(40), 40, 20)
+    t = torch.stack([dc.tokens(20, dc.LARGE["vocab"], b) for b in range(40)]).int().cuda()
+    fb.prefill(model, kc, t[:, :8])
+    for at in range(8, 11):
+        fb.decode_step(model, kc, t[:, at])
+    seen = [_profiled(lambda: fb.decode_step(model, kc, t[:, at])) for at in range(11, 15)]
+    assert len({(flops, n) for _, flops, n in seen}) == 1 and seen[0][2] > 0 and all(ms > 0.002 * n for ms, _, n in seen)
+    fb.decode_step(model, kc, t[:, 15])
+    assert model.state(40).status_word() == 0
+    kc.close()
