@@ -54,14 +54,11 @@ __device__ __forceinline__ void finish8(const GemmArgs& g, float (&v)[8], long l
     const bool vec = full && (reinterpret_cast<uintptr_t>(C) & 15) == 0;
     if (vec) {
 #pragma unroll
-      for (int j = 0; j < 8; j += 4) {
-        float4 o = make_float4(g.alpha * v[j], g.alpha * v[j + 1], g.alpha * v[j + 2], g.alpha * v[j + 3]);
-        if (g.beta != 0.f) { const float4 q = *reinterpret_cast<const float4*>(C + j); o.x += q.x; o.y += q.y; o.z += q.z; o.w += q.w; }
-        *reinterpret_cast<float4*>(C + j) = o;
-      }
+      for (int j = 0; j < 8; j += 4)
+        *reinterpret_cast<float4*>(C + j) = make_float4(g.alpha * v[j], g.alpha * v[j + 1], g.alpha * v[j + 2], g.alpha * v[j + 3]);
     } else {
 #pragma unroll
-      for (int j = 0; j < 8; j++) if (n + j < g.N) C[j] = (g.beta != 0.f ? C[j] : 0.f) + g.alpha * v[j];
+      for (int j = 0; j < 8; j++) if (n + j < g.N) C[j] = g.alpha * v[j];
     }
     return;
   }
@@ -313,6 +310,7 @@ static int cluster_ctas(int splits) {
 static bool split_supported(const GemmArgs& g) {
   if (!g.any_size || !g.a_kmajor || g.upper_only || g.nseg) return false;
   if (g.epi != EPI_STORE && g.epi != EPI_RESID && g.epi != EPI_RELU2 && g.epi != EPI_F32 && g.epi != EPI_SWIGLU) return false;
+  if (g.epi == EPI_F32 && g.beta != 0.f) return false;      // sums of several products are a training step's
   return g.b_kmajor || !(g.N & 63);
 }
 
