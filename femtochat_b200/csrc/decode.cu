@@ -506,6 +506,7 @@ extern "C" int32_t femto_selftest_decode_wait(femto_handle* h, femto_kv_cache* c
   CUDA_TRY(cudaMemcpy(&launches, c->step.launches, 4, cudaMemcpyDeviceToHost));
   CUDA_TRY(cudaMemcpy(&before, h->status, 4, cudaMemcpyDeviceToHost));
   CUDA_TRY(cudaMemset(h->status, 0, 4));
+  CUDA_TRY(cudaMemset(c->step.hints, 0, c->step.hint_bytes));      // the counts of that step would end the waits for them
   bool ran = false;
   FEMTO_TRY(decode_step_run(h, c->step, step_args(c, theta, B, logits_out), nullptr, nullptr, s, &ran));
   CUDA_TRY(cudaStreamSynchronize(s));                    // the kernel returned by itself

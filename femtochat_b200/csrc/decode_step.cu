@@ -762,7 +762,8 @@ void decode_step_carve(const femto_handle* h, char*& p, DecodeStepState& st) {
   take(st.maps, sizeof(CUtensorMap) * (4 * h->L + 1));
   take(st.blocks, sizeof(DecodeBlock) * h->L);
   char* first = p;
-  take(st.launches, 8); take(st.hints, 128 * HINTS);
+  st.hint_bytes = 128 * HINTS;
+  take(st.launches, 8); take(st.hints, st.hint_bytes);
   const size_t words = 16 * n * pitch_of(h->d);
   take(st.xn, words); take(st.xm, 8 * n * d); take(st.xa, 8 * n * d); take(st.xa2, words); take(st.xb, 8 * n * d);
   take(st.part, 32 * n * d); take(st.qkv, 8 * n * h->dq); take(st.h16, 8 * 16 * n); take(st.up, 4 * words); take(st.att, words);

@@ -21,7 +21,7 @@ struct DecodeStepState {
   uint2 *xm = nullptr, *xa = nullptr, *xb = nullptr, *part = nullptr, *qkv = nullptr, *h16 = nullptr, *att_part = nullptr;
   // Rows of bf16, three words of 16 bytes for 16 columns: what the QKV and the head read, what the MLP reads, its inside by quarters, attention
   uint4 *xn = nullptr, *xa2 = nullptr, *up = nullptr, *att = nullptr;
-  size_t named_bytes = 0;
+  size_t named_bytes = 0, hint_bytes = 0;
   float* x0 = nullptr;               // embedding
 };
 

@@ -580,17 +580,18 @@ def test_decode_step_with_fewer_blocks_than_multiprocessors(blocks):
 
 
 @pytest.mark.gpu
-def test_decode_kernel_gives_up_on_words_that_never_come():
+@pytest.mark.parametrize("B", [2, 8])
+def test_decode_kernel_gives_up_on_words_that_never_come(B):
     """The polls of the resident decode kernel are bounded: without the kernel that feeds it, it raises the timeout bit and returns, and
-    the next token is right again."""
-    model, tok, pos, ref = _bf16_server(2, 4, 2, 2, 40, False)
-    st = model.state(2)
-    kc = fb.KVCache(st, 2, 40)
+    the next token is right again.  Two columns poll the words themselves (194 of 16 bytes), eight wait on counts of finished items first (776)."""
+    model, tok, pos, ref = _bf16_server(B, 4, 2, 2, 40, False)
+    st = model.state(B)
+    kc = fb.KVCache(st, B, 40)
     fb.prefill(model, kc, tok[:, :30], pos[:, :30])
-    z = torch.empty(2, 1000, device="cuda")
+    z = torch.empty(B, 1000, device="cuda")
     status = C.c_int32(0)
     held = tok[:, 30].contiguous().cuda()
-    _lib.check(_lib.lib().femto_selftest_decode_wait(st.h, kc.c, _lib.ptr(model.params.theta), _lib.ptr(held), 2, _lib.ptr(z), None, C.byref(status)))
+    _lib.check(_lib.lib().femto_selftest_decode_wait(st.h, kc.c, _lib.ptr(model.params.theta), _lib.ptr(held), B, _lib.ptr(z), None, C.byref(status)))
     assert status.value & 2 and st.status_word() == 0 and len(kc) == 31
     for t in range(31, 36):
         z = fb.decode_step(model, kc, tok[:, t]).cpu()
