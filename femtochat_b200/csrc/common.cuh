@@ -130,16 +130,28 @@ __device__ __forceinline__ void prefetch_l2(const void* p, long long bytes, int 
 }
 // Launches a kernel that calls pdl_wait() in every thread: its blocks may be scheduled while the previous kernel of the
 // stream drains, so the launch latency of a chain of small kernels (a decode step) is hidden.
+// `cluster`: neighbouring blocks along x that form one.
 template <typename... P, typename... A>
-static inline cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+static inline cudaError_t launch_dependent_clusters(void (*kernel)(P...), int cluster, dim3 grid, dim3 block, size_t smem, cudaStream_t s, const A&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = s;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
   static const bool off = [] { const char* e = getenv("FEMTO_PDL"); return e && e[0] == '0'; }();   // measurement aid: fully serialised
-  cfg.attrs = at; cfg.numAttrs = off ? 0 : 1;
+  cudaLaunchAttribute at[2];
+  int n = 0;
+  if (cluster > 1) {
+    at[n].id = cudaLaunchAttributeClusterDimension;
+    at[n].val.clusterDim.x = cluster; at[n].val.clusterDim.y = 1; at[n++].val.clusterDim.z = 1;
+  }
+  if (!off) {
+    at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[n++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  cfg.attrs = at; cfg.numAttrs = n;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+template <typename... P, typename... A>
+static inline cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, const A&... args) {
+  return launch_dependent_clusters(kernel, 1, grid, block, smem, s, args...);
 }
 // Lets a kernel's launches have `bytes` of dynamic shared memory.  The limit belongs to the function and the device, not to a model or a
 // call: it is set once, to all that a block may have beside the kernel's own.  (Set to each launch's size, as it was, two threads that

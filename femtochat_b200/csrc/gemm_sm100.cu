@@ -837,23 +837,14 @@ static int launch_tc(const GemmArgs& g, const CUtensorMap& tmA, const CUtensorMa
     CUDA_TRY(cudaFuncSetAttribute(gemm_tc_kernel<false, false, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM_BYTES));
     if (dev >= 0) attr.done[dev] = true;
   }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid); cfg.blockDim = dim3(NTHREADS); cfg.stream = s;
-  cfg.dynamicSmemBytes = G::SMEM_BYTES - (G::STAGES - p.stages) * G::STAGE_BYTES;
-  static int pdl = -1;   // FEMTO_PDL=0 in the environment launches fully serialised (measurement aid)
-  if (pdl < 0) { const char* e = getenv("FEMTO_PDL"); pdl = (e && e[0] == '0') ? 0 : 1; }
-  cudaLaunchAttribute at[2];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = PAIR ? 2 : 1; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at; cfg.numAttrs = pdl ? 2 : 1;
+  const size_t smem = G::SMEM_BYTES - (G::STAGES - p.stages) * G::STAGE_BYTES;
+  auto launch = [&](auto kernel) { return launch_dependent_clusters(kernel, PAIR ? 2 : 1, grid, NTHREADS, smem, s, tmA, tmB, tmC, p); };
   cudaError_t e;
-  if (g.epi == EPI_SWIGLU) e = cudaLaunchKernelEx(&cfg, gemm_tc_kernel<true, true, PAIR, true>, tmA, tmB, tmC, p);
-  else if (g.a_kmajor && g.b_kmajor) e = cudaLaunchKernelEx(&cfg, gemm_tc_kernel<true, true, PAIR>, tmA, tmB, tmC, p);
-  else if (g.a_kmajor) e = cudaLaunchKernelEx(&cfg, gemm_tc_kernel<true, false, PAIR>, tmA, tmB, tmC, p);
-  else if (g.b_kmajor) e = cudaLaunchKernelEx(&cfg, gemm_tc_kernel<false, true, PAIR>, tmA, tmB, tmC, p);
-  else e = cudaLaunchKernelEx(&cfg, gemm_tc_kernel<false, false, PAIR>, tmA, tmB, tmC, p);
+  if (g.epi == EPI_SWIGLU) e = launch(gemm_tc_kernel<true, true, PAIR, true>);
+  else if (g.a_kmajor && g.b_kmajor) e = launch(gemm_tc_kernel<true, true, PAIR>);
+  else if (g.a_kmajor) e = launch(gemm_tc_kernel<true, false, PAIR>);
+  else if (g.b_kmajor) e = launch(gemm_tc_kernel<false, true, PAIR>);
+  else e = launch(gemm_tc_kernel<false, false, PAIR>);
   if (e != cudaSuccess) return femto_fail((int)e, "gemm_tc launch failed: %s", cudaGetErrorString(e));
   return 0;
 }

@@ -268,16 +268,7 @@ int launch_split(const CUtensorMap& tmA, const CUtensorMap& tmB, const SplitPara
     CUDA_TRY(cudaFuncSetAttribute(gemm_split_kernel<B_K, S, ACT, KS>, cudaFuncAttributeMaxDynamicSharedMemorySize, RING_BYTES + 1024));
     if (dev >= 0) attr.done[dev] = true;
   }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid; cfg.blockDim = dim3(NTHREADS); cfg.dynamicSmemBytes = smem; cfg.stream = s;
-  static const bool off = [] { const char* e = getenv("FEMTO_PDL"); return e && e[0] == '0'; }();   // measurement aid: fully serialised
-  cudaLaunchAttribute at[2];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = S; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at; cfg.numAttrs = off ? 1 : 2;
-  CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_split_kernel<B_K, S, ACT, KS>, tmA, tmB, p));
+  CUDA_TRY(launch_dependent_clusters(gemm_split_kernel<B_K, S, ACT, KS>, S, grid, NTHREADS, smem, s, tmA, tmB, p));
   return 0;
 }
 

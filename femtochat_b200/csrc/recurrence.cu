@@ -472,18 +472,7 @@ template <typename T> int delta_decode(const DeltaDecodeArgs& a, cudaStream_t s)
   const int staged = smem + taps <= 47 * 1024;      // many taps are read where they lie
   if (staged) smem += taps;
   if (smem > 48 * 1024 - 64) return femto_fail(FEMTO_ERR_UNSUPPORTED, "delta rule: ranks %d and %d are too large", a.ra, a.rg);
-  auto launch = [&](auto kernel) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(a.p.heads * cl, a.p.B); cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem; cfg.stream = s;
-    static const bool off = [] { const char* e = getenv("FEMTO_PDL"); return e && e[0] == '0'; }();   // measurement aid: fully serialised
-    cudaLaunchAttribute at[2];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = cl; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at; cfg.numAttrs = off ? 1 : 2;
-    return cudaLaunchKernelEx(&cfg, kernel, a, cl, staged);
-  };
+  auto launch = [&](auto kernel) { return launch_dependent_clusters(kernel, cl, dim3(a.p.heads * cl, a.p.B), threads, smem, s, a, cl, staged); };
   const bool once = en <= threads / 32;      // a warp has one row of the state
   if (a.p.dim <= 128) CUDA_TRY(once ? launch(k_delta_decode<T, 1, 1>) : launch(k_delta_decode<T, 1, 4>));
   else CUDA_TRY(once ? launch(k_delta_decode<T, 2, 1>) : launch(k_delta_decode<T, 2, 2>));
