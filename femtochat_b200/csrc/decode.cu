@@ -356,7 +356,7 @@ static int decode_t(femto_kv_cache* c, const float* theta, const int* tokens, co
                                              c->pos, c->doc_start, c->lastpos, h->status);
   KERNEL_CHECK();
   const int* docs = h->cfg.doc_mask ? c->doc_start : nullptr;
-  FEMTO_TRY(S::embed_norm((const T*)h->sh_wte, c->tok0, (T*)c->xe_new, B, d, eps, s, h->tables_live ? theta + h->off_wte : nullptr));
+  FEMTO_TRY(S::embed_norm((const T*)h->sh_wte, c->tok0, (T*)c->xe_new, B, d, eps, s));
   k_smear_decode<T><<<cdiv(B, 8), 256, 0, s>>>((const T*)c->xe_new, (T*)c->xe_prev, theta + h->off_smear, theta + h->off_lam_s, B, d,
                                                (T*)h->x0);
   KERNEL_CHECK();
@@ -376,7 +376,7 @@ static int decode_t(femto_kv_cache* c, const float* theta, const int* tokens, co
     FEMTO_TRY(S::mix_norm(xin, (const T*)h->x0, theta + p.lam_b, theta + p.lam_x0, (T*)h->xm, (T*)l.xn1, l.r1, B, d, eps, s));
     FEMTO_TRY(product(l.xn1, d, l.sh_wqkv, dq, l.qkv, EPI_STORE, nullptr));
     FEMTO_TRY(S::qkv_post((T*)l.qkv, dq, (const T*)l.xn1, d, p.ve ? theta + p.ve_gate : nullptr, p.ve ? (const T*)l.sh_ve : nullptr,
-                          c->tok0, c->pos, h->sin_t, h->cos_t, B, H, Hkv, hd, eps, l.rqk, l.sv, s, h->tables_live && p.ve ? theta + p.ve_table : nullptr));
+                          c->tok0, c->pos, h->sin_t, h->cos_t, B, H, Hkv, hd, eps, l.rqk, l.sv, s));
     k_kv_append<T><<<cdiv((long long)B * kv, 256), 256, 0, s>>>((const T*)l.qkv, dq, d, kv, (T*)c->K[i], (T*)c->V[i], c->maxT, t, B);
     KERNEL_CHECK();
     FEMTO_TRY(decode_attention<T>(c, i, (const T*)l.qkv, dq, (T*)l.att, d, B, t, p.window, docs, s));
@@ -432,6 +432,7 @@ extern "C" int32_t femto_kv_cache_create(femto_handle* h, int32_t max_batch, int
     decode_step_carve(h, p, c->step);
     if (const int r = decode_step_setup(h, c->step, c->K, c->V)) { cudaFree(c->mem); delete c; return r; }
   }
+  h->decodes = true;
   *out = c;
   return 0;
 }
@@ -488,7 +489,7 @@ extern "C" int32_t femto_decode_step(femto_handle* h, femto_kv_cache* c, const f
     if (positions) return femto_fail(FEMTO_ERR_UNSUPPORTED, "this model counts positions from the start of the sequence");
     return decoder_step(h, c, theta, tokens, B, 1, nullptr, 0, logits_out, nullptr, (cudaStream_t)stream);
   }
-  FEMTO_TRY(model_ensure_weights(h, theta, false, (cudaStream_t)stream));
+  FEMTO_TRY(model_ensure_weights(h, theta, true, (cudaStream_t)stream));
   if (!h->weights_valid) return femto_fail(FEMTO_ERR_STATE, "call femto_refresh_weights before the first step");
   return h->bf ? decode_t<bf16>(c, theta, tokens, positions, B, logits_out, (cudaStream_t)stream)
                : decode_t<float>(c, theta, tokens, positions, B, logits_out, (cudaStream_t)stream);

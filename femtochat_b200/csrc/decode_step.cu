@@ -97,8 +97,8 @@ __global__ void __launch_bounds__(THREADS) k_step_begin(const DecodeStepArgs a, 
     if (bad) atomicOr(a.status, ST_BAD_TOKEN);
     pos_s = p;
   }
-  const long long row = (long long)tk * a.d;
-  auto src = [&](int c) { return a.live ? round_to<bf16>(a.theta[a.off_wte + row + c]) : __bfloat162float(a.wte[row + c]); };
+  const bf16* row = a.wte + (long long)tk * a.d;
+  auto src = [&](int c) { return __bfloat162float(row[c]); };
   float ss = 0.f;
   for (int c = tid; c < a.d; c += THREADS) { const float f = src(c); ss += f * f; }
   ss = warp_sum(ss);
@@ -434,13 +434,7 @@ __global__ void __launch_bounds__(THREADS + 128, 1) k_decode_step(const DecodeSt
       uint2 ve = make_uint2(0, 0);
       float wg = 0.f;
       if (last && blk.ve) {
-        const long long at = (long long)a.tok0[b] * a.kv + (long long)kvh * HD + 4 * lane;
-        if (a.live) {      // (Theta's tensors start at even offsets)
-          const float2 lo = *reinterpret_cast<const float2*>(a.theta + blk.ve_table + at), hi = *reinterpret_cast<const float2*>(a.theta + blk.ve_table + at + 2);
-          ve = make_uint2(pack2(lo.x, lo.y), pack2(hi.x, hi.y));
-        } else {
-          ve = *reinterpret_cast<const uint2*>(blk.ve + at);
-        }
+        ve = *reinterpret_cast<const uint2*>(blk.ve + (long long)a.tok0[b] * a.kv + (long long)kvh * HD + 4 * lane);
         if (lane < 12) wg = a.theta[blk.ve_gate + lane * a.Hkv + kvh];
       }
       cached(0);
@@ -786,7 +780,7 @@ int decode_step_setup(const femto_handle* h, DecodeStepState& st, const std::vec
     FEMTO_TRY(put(l.sh_fc, h->d, 4 * h->d)); FEMTO_TRY(put(l.sh_proj, 4 * h->d, h->d));
     DecodeBlock b = {};
     b.K = (bf16*)K[i]; b.V = (bf16*)V[i]; b.ve = p.ve ? (const bf16*)l.sh_ve : nullptr;
-    b.lam_b = p.lam_b; b.lam_x0 = p.lam_x0; b.ve_gate = p.ve_gate; b.ve_table = p.ve_table; b.window = p.window;
+    b.lam_b = p.lam_b; b.lam_x0 = p.lam_x0; b.ve_gate = p.ve_gate; b.window = p.window;
     bl.push_back(b);
   }
   FEMTO_TRY(put(h->sh_lm, h->d, h->Vp));
@@ -802,7 +796,6 @@ int decode_step_run(const femto_handle* h, const DecodeStepState& st, DecodeStep
   a.xn = st.xn; a.xm = st.xm; a.xa = st.xa; a.xa2 = st.xa2; a.xb = st.xb; a.part = st.part; a.qkv = st.qkv; a.h16 = st.h16; a.up = st.up;
   a.att = st.att; a.att_part = st.att_part;
   a.wte = (const bf16*)h->sh_wte; a.sin_t = h->sin_t; a.cos_t = h->cos_t; a.status = h->status;
-  a.live = h->tables_live; a.off_wte = h->off_wte;
   a.off_smear = h->off_smear; a.off_lam_s = h->off_lam_s; a.off_lam_y = h->off_lam_y;
   a.d = h->d; a.dq = h->dq; a.kv = h->kv; a.H = h->H; a.Hkv = h->Hkv; a.V = h->V; a.Vp = h->Vp; a.L = h->L; a.backout = h->backout; a.eps = h->eps;
   a.docs = h->cfg.doc_mask ? 1 : 0;

@@ -8,7 +8,7 @@
 #include "model.cuh"
 
 // What a block of the model needs beside its matrices
-struct DecodeBlock { bf16 *K, *V; const bf16* ve; long long lam_b, lam_x0, ve_gate, ve_table; int window; };
+struct DecodeBlock { bf16 *K, *V; const bf16* ve; long long lam_b, lam_x0, ve_gate; int window; };
 
 struct DecodeStepState {
   int ring[2] = {0, 0};              // slots of its ring for up to 8 and up to 16 columns
@@ -36,8 +36,8 @@ struct DecodeStepArgs {
   int *tok0, *pos, *doc_start, *lastpos;
   float* logits;
   unsigned int* status;
-  long long off_wte, off_smear, off_lam_s, off_lam_y;
-  int d, dq, kv, H, Hkv, V, Vp, L, backout, B, t, maxT, docs, splits, red_bytes, ring, live;      // live: rows of the tables come from Theta
+  long long off_smear, off_lam_s, off_lam_y;
+  int d, dq, kv, H, Hkv, V, Vp, L, backout, B, t, maxT, docs, splits, red_bytes, ring;
   float eps;
 };
 

@@ -307,9 +307,10 @@ int model_refresh(femto_handle* h, const float* theta, cudaStream_t s) {
 int model_ensure_weights(femto_handle* h, const float* theta, bool tables, cudaStream_t s) {
   if (h->weights_changed) {
     if (tables) return model_refresh(h, theta, s);
-    // More than half of the weights are embedding tables, of which a call reads the rows of its tokens: those it takes from Theta, as it
-    // takes the gates and scalars.  d20: 0.81 -> 0.40 ms a call, d12 0.42 -> 0.12.  (The cast beside the pass on the other stream, in
-    // pieces that the blocks wait for, was slower than before it: 3.80 against 3.77 ms a prompt of 1500 tokens of d20.)
+    // More than half of the weights are embedding tables, of which an evaluation reads the rows of its tokens: those it takes from Theta, as
+    // it takes the gates and scalars.  d20: 0.81 -> 0.40 ms a call, d12 0.42 -> 0.12.  (The tables of a prompt cannot be left out, see
+    // model_step.  Their cast beside the pass on another stream, with 24 to 296 blocks at a time or all, took as long as before it: a prompt of
+    // 1500 tokens of d20 3.61 to 4.29 ms, 3.65 before it, 3.22 without.)
     FEMTO_TRY(cast_range(h, theta, 0, h->cast_tables, s));
     h->weights_valid = h->tables_live = true;
     h->weights_changed = false;
@@ -641,7 +642,9 @@ int model_step(femto_handle* h, const float* theta, float* delta, const int* tok
   // A training step runs on the handle's own two streams, bracketed by the caller's stream on both sides; every
   // other call (loss only, logits, a prompt) is one dependency chain and stays on the caller's stream.
   const bool two = backward && h->hi && h->lo && !gemm_profiling();
-  FEMTO_TRY(model_ensure_weights(h, theta, backward, s));
+  // The tokens behind a prompt, or behind an evaluation between them, read the copies, whatever is written to Theta meanwhile: where there is
+  // a cache, those of the tables are made too.
+  FEMTO_TRY(model_ensure_weights(h, theta, backward || h->decodes, s));
   cudaStream_t chain = two ? h->hi : s;
   if (two) {
     cudaEvent_t e = h->ev_fork[h->ev_next++ % femto_handle::N_FORK];

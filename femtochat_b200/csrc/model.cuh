@@ -42,6 +42,7 @@ struct femto_handle {
   bool weights_valid = false;
   bool weights_changed = false;   // Theta was written since: the next call that reads the copies makes them from the Theta it is given
   bool tables_live = false;       // ... all but those of the embedding tables, whose rows calls that do not train read from their Theta
+  bool decodes = false;           // a cache was made: its tokens read the copies that the call before them left, those of the tables too
   struct CastJob* cast_jobs = nullptr;   // device table of model_refresh
   int n_cast_jobs = 0, cast_blocks = 0, cast_tables = 0;      // blocks from cast_tables on are the embedding tables
   int *tok0 = nullptr, *tgt0 = nullptr, *pos = nullptr, *doc_start = nullptr, *raw_tok = nullptr, *raw_tgt = nullptr,

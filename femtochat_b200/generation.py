@@ -40,7 +40,8 @@ class KVCache:
 
 
 def prefill(model, cache: KVCache, tokens, positions=None):
-    """Runs the prompt [B][Tp] and returns the soft-capped logits of each column's last position, fp32 [B][V]."""
+    """Runs the prompt [B][Tp] and returns the soft-capped logits of each column's last position, fp32 [B][V].  The model's weights
+    are brought up to date first; the tokens that follow read those, and of a Θ that is written meanwhile its gates and scalars."""
     import torch
     tok, pos = _dev_i32(tokens), _dev_i32(positions)
     B, Tp = tok.shape

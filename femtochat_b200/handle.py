@@ -14,7 +14,8 @@ class Handle:
         _lib.check(_lib.lib().femto_refresh_weights(self.h, _lib.ptr(theta), _lib.stream_ptr()))
 
     def refresh_for(self, theta) -> None:
-        """For the library call with this Θ that follows: it makes the compute-type weights that it needs from it."""
+        """For the library call with this Θ that follows: it makes the compute-type weights that it needs from it.  (The GPT's handles
+        only; DecoderState, whose library call does not exist, refreshes at once.)"""
         _lib.check(_lib.lib().femto_weights_changed(self.h))
 
     def status_word(self) -> int:

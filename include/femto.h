@@ -94,8 +94,11 @@ int32_t femto_window_sizes(const femto_config* h_cfg, int32_t* h_left, int32_t* 
  * Call after any external write to Theta; femto_optimizer_step does it itself. */
 int32_t femto_refresh_weights(femto_handle* h, const float* theta, void* stream);
 /* Says that Theta was written: the next call that needs the copies makes them from the Theta it is given, as if femto_refresh_weights had
- * been called with it just before.  Calls that do not train need none of the embedding tables: until one that does, or
- * femto_refresh_weights, they read the rows of their tokens from the Theta they are given, as they read gates and scalars. */
+ * been called with it just before.  A loss or logits, on a handle without key/value caches, needs no copy of the embedding tables: it
+ * reads the rows of its tokens from the Theta it is given, and the next call that needs the tables copies them.  Tokens that follow a
+ * prompt read the copies that the prompt (or a later call with weights of its own) left, whatever is written to Theta meanwhile; gates and
+ * scalars are read from the Theta of each call.  For handles of femto_create: a decoder that lists its layers refuses it and takes
+ * femto_refresh_weights. */
 int32_t femto_weights_changed(femto_handle* h);
 
 /* loss_and_gradient! (ext/FemtoChatEnzymeExt.jl:38-44) with the training script's accumulation

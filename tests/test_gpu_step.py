@@ -500,9 +500,9 @@ def _bf16_server(B, H, G, L, T, doc_mask, vocab=1000):
 @pytest.mark.gpu
 @pytest.mark.parametrize("ctype,d,heads,kv", [("bfloat16", 256, 2, 1), ("bfloat16", 96, 3, 3), ("float32", 256, 2, 1), ("float32", 64, 4, 2)])
 def test_calls_that_do_not_train_read_embedding_rows_from_theta(ctype, d, heads, kv):
-    """After Theta was written, a loss, a prompt and the tokens after it leave the compute-type copies of the embedding tables as they were
-    and read rows of Theta instead: the same bits as a handle whose copies were all made.  A training step on that handle makes
-    them first.  Heads of 128 and of other sizes (both kernels behind the projections, the resident and the other decode step)."""
+    """After Theta was written, a loss leaves the compute-type copies of the embedding tables as they were and reads rows of Theta instead: the
+    same bits as a handle whose copies were all made.  A prompt, or a training step, on that handle makes them first.  Heads of 128 and of
+    other sizes (both kernels behind the projections, the resident and the other decode step)."""
     cfg = fb.GPTConfig(sequence_len=40, max_document_tokens=64, vocab_size=300, n_layer=3, n_head=heads, n_kv_head=kv, n_embed=d, window_pattern="SL")
     lay = fb.parameter_layout(cfg)
     theta = torch.zeros(lay.nparams, device="cuda")
@@ -543,6 +543,70 @@ def test_calls_that_do_not_train_read_embedding_rows_from_theta(ctype, d, heads,
         fb.loss_and_gradient_(params, m.state(2), lay, tok, tgt)
         deltas.append(params.delta.clone())
     assert torch.equal(deltas[0], deltas[1]) and float(deltas[0].abs().max()) > 0
+
+
+def _conversation(ctype, d, heads, kv):
+    """A GPT with value embeddings, tokens, and what overwrites its tables."""
+    cfg = fb.GPTConfig(sequence_len=40, max_document_tokens=64, vocab_size=300, n_layer=3, n_head=heads, n_kv_head=kv, n_embed=d, window_pattern="SL")
+    lay = fb.parameter_layout(cfg)
+    theta = torch.zeros(lay.nparams, device="cuda")
+    fb.initialize_(theta, lay, seed=5, all_nonzero=True)
+    g = torch.Generator(device="cuda").manual_seed(9)
+    tok, tgt = (torch.randint(1, 301, (2, 40), generator=g, device="cuda", dtype=torch.int32) for _ in range(2))
+    tables = [lay.embedding] + [b["ve_table"] for b in lay.blocks if b["ve_table"] is not None]
+
+    def write():
+        for t in tables:
+            theta[t.offset:t.offset + t.size].mul_(-0.5).add_(0.3)
+    return fb.GPT(fb.Params(theta), cfg, lay, compute_type=ctype), tok, tgt, write
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("evaluation", [False, True])
+@pytest.mark.parametrize("ctype,d,heads,kv", [("bfloat16", 256, 2, 1), ("bfloat16", 96, 3, 3), ("float32", 256, 2, 1)])
+def test_tokens_read_the_weights_of_their_prompt(ctype, d, heads, kv, evaluation):
+    """Tables written between a prompt and its tokens change nothing about those tokens, as matrices do not: the bits of a
+    conversation without the write.  Also with an evaluation on the same handle before the write."""
+    got = []
+    for written in (False, True):
+        model, tok, tgt, write = _conversation(ctype, d, heads, kv)
+        kc = fb.KVCache(model.state(2), 2, 40)
+        out = [fb.prefill(model, kc, tok[:, :20]).clone()]
+        if evaluation:
+            out.append(model(tok, tgt, reduction="none"))
+        if written:
+            write()
+        got.append(out + [fb.decode_step(model, kc, tok[:, t]) for t in range(20, 24)])
+        kc.close()
+    assert all(torch.equal(a, b) for a, b in zip(*got))
+    # the next prompt reads what was written
+    kc = fb.KVCache(model.state(2), 2, 40)
+    assert not torch.equal(fb.prefill(model, kc, tok[:, :20]), got[1][0])
+    kc.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("ctype,d,heads,kv", [("bfloat16", 256, 2, 1), ("bfloat16", 96, 3, 3), ("float32", 64, 4, 2)])
+def test_tokens_take_a_theta_of_any_alignment(ctype, d, heads, kv):
+    """femto_decode_step reads single values of Theta: a copy at an address that is no multiple of 8 gives the same bits, also where it is
+    the call that makes the weights."""
+    model, tok, _, _ = _conversation(ctype, d, heads, kv)
+    st, theta = model.state(2), model.params.theta
+    odd = torch.empty(theta.numel() + 1, device="cuda")[1:]
+    odd.copy_(theta)
+    assert _lib.ptr(odd).value % 8 == 4
+    out = []
+    for th in (theta, odd):
+        kc = fb.KVCache(st, 2, 40)
+        fb.prefill(model, kc, tok[:, :20])
+        for t in range(20, 24):
+            if t == 22:
+                st.refresh_for(th)
+            z = torch.empty(2, 300, device="cuda")
+            _lib.check(_lib.lib().femto_decode_step(st.h, kc.c, _lib.ptr(th), _lib.ptr(tok[:, t].contiguous()), None, 2, _lib.ptr(z), None))
+            out.append(z)
+        kc.close()
+    assert all(torch.equal(a, b) for a, b in zip(out[:4], out[4:])) and float(out[0].abs().max()) > 0
 
 
 @pytest.mark.gpu
