@@ -117,6 +117,8 @@ struct PerDevice {
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // Dependent side of a kernel launched with launch_dependent(): nothing an earlier kernel wrote may be read, and nothing an
 // earlier kernel reads may be written, before this.  Returns at once in a kernel that was launched in the ordinary way.
+// What earlier kernels write is not __restrict__ in such a kernel, and not read by __ldg: the compiler may move a load of what it holds for
+// constant to before the wait, and did.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Lines of memory on their way to L2 before pdl_wait(): weights, states and cached rows whose addresses a kernel knows from its
 // arguments.  L2 is coherent, so a line that an earlier kernel has yet to write is no harm.  In a decode step, whose weights push

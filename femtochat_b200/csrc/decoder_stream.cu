@@ -25,8 +25,8 @@ constexpr int FEW = 4;    // blocks that ask for the norms' weights ahead (one i
                           // and any of k_parallel_resid's a prompt of 7108 rows 1.2 %)
 
 template <typename T>
-__global__ void __launch_bounds__(RT) k_dec_embed(const T* __restrict__ table, const int* __restrict__ tokens, int ld_tok, int T_,
-                                                  int base, int vocab, float scale, float* __restrict__ x, const NextNorms<T> nn, int d,
+__global__ void __launch_bounds__(RT) k_dec_embed(const T* __restrict__ table, const int* tokens, int ld_tok, int T_,
+                                                  int base, int vocab, float scale, float* x, const NextNorms<T> nn, int d,
                                                   float eps, unsigned int* status) {
   pdl_trigger();
   pdl_wait();
@@ -70,10 +70,9 @@ template <typename T> __device__ __forceinline__ void store4(T* p, float a, floa
 
 // NV 4-element vectors per thread stay in registers between the sum and the norms (NV = 0: any width, through memory).
 // AHEAD, up to a row a multiprocessor: the norms' weights are in registers before the wait, and x is on its way with y (a token of Zurevik d20,
-// 4 rows: 876 -> 860 us; a prompt of 7108 rows is 1.5 % slower so, its blocks have fewer registers to hide behind).  y is not __restrict__:
-// what the compiler holds for constant it may load before the wait.
+// 4 rows: 876 -> 860 us; a prompt of 7108 rows is 1.5 % slower so, its blocks have fewer registers to hide behind).
 template <typename T, int NV, bool AHEAD>
-__global__ void __launch_bounds__(RT) k_parallel_resid(float* __restrict__ x, const T* y, const T* y2, const MoeRows m,
+__global__ void __launch_bounds__(RT) k_parallel_resid(float* x, const T* y, const T* y2, const MoeRows m,
                                                        const NextNorms<T> nn, int d, float eps) {
   pdl_trigger();
   float4 ahead[NV > 0 ? NV : 1], ahead2[NV > 0 ? NV : 1];
@@ -167,10 +166,9 @@ __global__ void __launch_bounds__(RT) k_parallel_resid(float* __restrict__ x, co
 }
 
 // NV 4-element vectors per thread stay in registers between the two norms (NV = 0: any width, through memory).
-// y is not __restrict__: what the compiler holds for constant it may load before the wait.
 template <typename T, int NV>
-__global__ void __launch_bounds__(RT) k_resid_norm(float* __restrict__ x, const T* y, const float* __restrict__ w_post,
-                                                   float m, const float* __restrict__ w_pre, T* __restrict__ h, int d, float eps) {
+__global__ void __launch_bounds__(RT) k_resid_norm(float* x, const T* y, const float* __restrict__ w_post,
+                                                   float m, const float* __restrict__ w_pre, T* h, int d, float eps) {
   pdl_trigger();
   const long long base = (long long)blockIdx.x * d;
   if constexpr (NV > 0) {
@@ -256,8 +254,8 @@ __global__ void __launch_bounds__(RT) k_resid_norm(float* __restrict__ x, const 
 }
 
 template <typename T>
-__global__ void __launch_bounds__(RT) k_gather_norm(const float* __restrict__ x, const int* __restrict__ want, int stride,
-                                                    const float* __restrict__ w, T* __restrict__ h, int d, float eps) {
+__global__ void __launch_bounds__(RT) k_gather_norm(const float* x, const int* want, int stride,
+                                                    const float* __restrict__ w, T* h, int d, float eps) {
   pdl_trigger();
   if (blockIdx.x < FEW) prefetch_l2(w, 4ll * d, threadIdx.x, RT);
   pdl_wait();
@@ -271,8 +269,8 @@ __global__ void __launch_bounds__(RT) k_gather_norm(const float* __restrict__ x,
 
 // LG lanes per (row, group).
 template <typename T, int V, int LG>
-__global__ void __launch_bounds__(256) k_gated_norm(const T* __restrict__ in, const float* __restrict__ w, int w_all,
-                                                    const T* __restrict__ gate, long long ldg, T* __restrict__ out, long long n,
+__global__ void __launch_bounds__(256) k_gated_norm(const T* in, const float* __restrict__ w, int w_all,
+                                                    const T* gate, long long ldg, T* out, long long n,
                                                     int groups, int size, float eps) {
   pdl_trigger();
   if (blockIdx.x < FEW) prefetch_l2(w, 4ll * size * (w_all ? groups : 1), threadIdx.x, 256);
@@ -310,7 +308,7 @@ __global__ void __launch_bounds__(256) k_gated_norm(const T* __restrict__ in, co
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) k_gated_mlp(const T* __restrict__ gu, T* __restrict__ act, long long n, int ffp) {
+__global__ void __launch_bounds__(256) k_gated_mlp(const T* gu, T* act, long long n, int ffp) {
   pdl_trigger();
   pdl_wait();
   constexpr int V = VecN<T>::n;
@@ -350,8 +348,8 @@ __global__ void __launch_bounds__(256) k_pack_transposed(const float* __restrict
 // silu(row n of the gate weights) * row n of the up weights, which alternate in groups of 32 rows.
 constexpr int RL_ROWS = 8;
 template <typename T, bool GATED>
-__global__ void __launch_bounds__(256) k_rows_linear(const T* __restrict__ X, long long ldx, const T* __restrict__ W, long long ldw,
-                                                     void* __restrict__ C, long long ldc, int M, int N, int K, int f32_out, const RowsOut out) {
+__global__ void __launch_bounds__(256) k_rows_linear(const T* X, long long ldx, const T* __restrict__ W, long long ldw,
+                                                     void* C, long long ldc, int M, int N, int K, int f32_out, const RowsOut out) {
   pdl_trigger();
   pdl_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -391,8 +389,8 @@ __global__ void __launch_bounds__(256) k_rows_linear(const T* __restrict__ X, lo
 // before the kernel waits for its predecessor.  LISTS: the rows of a block are one list of k_moe_choose_few, its weights those
 // of the list's expert.
 template <int NT, bool GATED, bool LISTS>
-__global__ void __launch_bounds__(256) k_rows_mma(const bf16* __restrict__ X, long long ldx, const bf16* __restrict__ W, long long ldw,
-                                                  void* __restrict__ C, long long ldc, int M, int N, int K, int epi, const RowsBatch bt) {
+__global__ void __launch_bounds__(256) k_rows_mma(const bf16* X, long long ldx, const bf16* __restrict__ W, long long ldw,
+                                                  void* C, long long ldc, int M, int N, int K, int epi, const RowsBatch bt) {
   const int* list = nullptr;
   // The first product over lists waits for them before it lets its dependents start; the second starts its weights with the lists
   // that are there then, while the first one's last blocks run.

@@ -275,7 +275,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       if (below_diagonal(g, mt, nt, TILE_M)) continue;
       const int m0 = mt * TILE_M + rank * BM;           // first row of A this CTA loads
       const int n0 = nt * BN + rank * G::BN_LOCAL;      // first column of B this CTA loads (its half, in a pair)
-      const int bb = g.groups ? __ldg(g.groups + 1 + mt * TILE_M / g.group_rows) : g.strideB ? bz : 0;   // which matrix of B
+      const int bb = g.groups ? g.groups[1 + mt * TILE_M / g.group_rows] : g.strideB ? bz : 0;   // which matrix of B
       for (int kb = kb0; kb < kb1; kb++) {
         if (!mbar_wait_warp(&empty[stage], phase ^ 1, abort_flag, g.status)) { ok = false; break; }
         uint8_t* sa = smem + stage * STAGE_BYTES;

@@ -12,7 +12,7 @@ namespace {
 // ---- new rows ---------------------------------------------------------------------------------------------------------
 // out[0 .. ldo) = rms_norm(in[0 .. size)) w, then zeros; by one warp
 template <typename T, int V>
-__device__ __forceinline__ void warp_norm(const T* __restrict__ in, const float* __restrict__ w, T* __restrict__ out, int ldo, int size,
+__device__ __forceinline__ void warp_norm(const T* in, const float* __restrict__ w, T* out, int ldo, int size,
                                           float eps, int lane) {
   float ss = 0.f;
 #pragma unroll 4

@@ -16,7 +16,7 @@ constexpr int MAX_EXPERTS = 1024, MAX_TOP = 32;
 
 // By one warp: the k-th largest logit of a row (ties: the lower index) ends up in lane k, as index and softmax weight.
 template <int PER>
-__device__ __forceinline__ void choose(const float* __restrict__ z, const float* __restrict__ bias, int experts, int top, int lane, int& id,
+__device__ __forceinline__ void choose(const float* z, const float* __restrict__ bias, int experts, int top, int lane, int& id,
                                        float& weight) {
   float v[PER];
 #pragma unroll
@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(1024) k_moe_choose_few(const MoeArgs a) {
 
 // y[row] = sum over its choices of weight * result
 template <typename T>
-__global__ void __launch_bounds__(256) k_moe_combine(const MoeRows m, T* __restrict__ y, int d) {
+__global__ void __launch_bounds__(256) k_moe_combine(const MoeRows m, T* y, int d) {
   pdl_trigger();
   pdl_wait();
   const long long row = blockIdx.x;

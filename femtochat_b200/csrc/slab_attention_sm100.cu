@@ -396,7 +396,7 @@ slab_attn_kernel(const __grid_constant__ CUtensorMap tmQu, const __grid_constant
           const uint4* g = reinterpret_cast<const uint4*>(p.gate + row * p.ld_gate + (long long)it.h * p.vdim + p.col0 + col);
 #pragma unroll
           for (int j = 0; j < 8; j++)
-            if (col + j * 8 < p.cols) gate[j] = __ldg(g + j);
+            if (col + j * 8 < p.cols) gate[j] = g[j];
         }
       }
       xl[X * 128 + r] = l;

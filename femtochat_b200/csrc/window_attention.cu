@@ -25,7 +25,7 @@ struct Visible {
 // ---- norms of q and k, in place ---------------------------------------------------------------------------------------
 // LG lanes per vector of `dim` entries: the heads * maps vectors of a row of q, then the kv_heads * maps of its new cache row.
 template <typename T, int V, int LG>
-__global__ void __launch_bounds__(256) k_qk_norm(T* __restrict__ q, long long ldq, T* __restrict__ kv, long long ld, int maxT, int first, int Tn,
+__global__ void __launch_bounds__(256) k_qk_norm(T* q, long long ldq, T* kv, long long ld, int maxT, int first, int Tn,
                                                  int nq, int nk, int dim, const float* __restrict__ wq, const float* __restrict__ wk, float eps,
                                                  long long n) {
   pdl_trigger();

@@ -255,3 +255,22 @@ def test_shard_plan_tiles_the_parameter_vector(world):
         if t.size >= fb.optim.SHARD_MIN_TABLE and t.size % (4 * world) == 0:
             for r in range(world):
                 assert (t.offset + r * (t.size // world), t.size // world, r) in plan
+
+
+def test_kernels_that_wait_for_their_predecessor_read_its_results_by_plain_loads():
+    """The compiler may move a load through a __restrict__ pointer, or __ldg, to before griddepcontrol.wait: in kernels with that wait only weights and
+    tables, which no kernel of a chain writes, are marked so."""
+    weights, seen = {"table", "w", "w_post", "w_pre", "W", "wq", "wk"}, 0
+    csrc = os.path.join(os.path.dirname(fb.__file__), "csrc")
+    for name in sorted(f for f in os.listdir(csrc) if f.endswith(".cu")):
+        src = open(os.path.join(csrc, name)).read()
+        for m in re.finditer(r"__global__ .*?(k_\w+|\w+_kernel)\(([^{;]*?)\)\s*\{\n(.*?)\n\}\n", src, re.S):
+            kernel, args, body = m.groups()
+            if "pdl_wait()" not in body and "grid_dependency_wait()" not in body:
+                continue
+            seen += 1
+            marked = set(re.findall(r"__restrict__ (\w+)", args))
+            assert marked <= weights, (name, kernel, marked - weights)
+            read = set(re.findall(r"__ldg\((?:reinterpret_cast<[^>]*>\()?([\w.]+)", body))
+            assert read <= {"w", "wp", "g.bias", "p.sink", "p.lambda"}, (name, kernel, read)
+    assert seen >= 30
