@@ -217,7 +217,8 @@ struct GemmArgs {
   const float* bias = nullptr;   // [N] added to the columns before the store (EPI_STORE)
   bool any_size = false;   // no later step repeats this product bit for bit (no training step): results smaller than a tile take the
                            // tensor cores as well, and K may be cut into ranges that are added at the end
-  bool whole_k = false;    // K is never cut: in a model with experts a sum in another order can choose between two nearly equal ones
+  bool whole_k = false;    // K is not cut, whatever the number of rows: in a model with experts a sum in another order can choose between two
+                           // nearly equal ones.  (Products of more than ROWS_STREAM rows, that is: up to there k_rows_mma adds eight ranges of K.)
   int ring = 0;   // depth of the operand ring of the tensor-core kernel; 0 = the deepest that fits (fewer stages leave
                   // shared memory free for kernels of another stream to run on the same SMs)
   // cross-entropy statistics epilogue

@@ -889,7 +889,7 @@ int gemm_tc_bf16(const GemmArgs& g, cudaStream_t s) {
   p.kblocks = cdiv(g.K, BK);
   const int tiles = p.tiles_m * p.tiles_n * g.batch;
   int splits = 1;
-  if (g.epi == EPI_F32 && tiles < 4 * workers) {
+  if (g.epi == EPI_F32 && !g.whole_k && tiles < 4 * workers) {
     // Pick the split count that minimises waves x k-blocks per unit PLUS what the partials cost: every split writes
     // and re-reads one fp32 copy of the result (8 bytes per element through HBM, the reduce pass not overlapped with
     // anything).  Both terms in units of one k-block of one worker, with round figures for the two rates.

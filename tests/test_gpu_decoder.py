@@ -150,6 +150,20 @@ def test_models_with_experts_sum_in_one_order():
     ok(model)
 
 
+def test_fp32_products_of_models_with_experts_sum_in_one_order():
+    """The same for products with fp32 results, which the persistent kernel cuts by their number of rows: the decays of a delta rule beside
+    experts, 5120 columns from a rank of 520.  44 rows take narrow tiles and 143 the persistent kernel, with three ranges of K if it may cut it."""
+    cfg = dc.config(*[dc.delta(heads=40, kv_heads=1, dim=128, vdim=64, ff=0) for _ in range(2)], vocab=512, width=256)
+    for layer in cfg["layers"]:
+        layer["mlp"] = dc.moe(ff=256, experts=4)
+    model, _ = dc.model_and_weights(cfg, (520, 8), "bfloat16", seed=16)
+    t = torch.stack([dc.tokens(11, cfg["vocab"], 80 + b) for b in range(13)])
+    few = fb.extend(model, cache_for(model, 11, 4), t[:4], want=[], residuals=True)[1]
+    many = fb.extend(model, cache_for(model, 11, 13), t, want=[], residuals=True)[1]
+    assert torch.equal(many[:, :44], few)
+    ok(model)
+
+
 @BOTH
 @pytest.mark.parametrize("name", ["mixed", "large"])
 def test_steps_as_one_launch_equal_plain_launches(name, dtype):
