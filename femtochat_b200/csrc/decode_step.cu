@@ -731,8 +731,9 @@ int resident(int nt, int gmax, int ks, size_t smem, int& ring) {
 
 }  // namespace
 
-// bf16, heads of 128 channels (so every width is a multiple of 128), at most 8 query heads a key head, and as many columns as
-// leave room for the ring (16 up to d = 2000 or so, 8 up to 3000); anything else takes the chain of kernels of decode.cu.
+// bf16, heads of 128 channels (so every width is a multiple of 128), at most 8 query heads a key head, d up to 4096, and as many columns as
+// leave room for MIN_RING slots of the ring: 8, or 16 up to d = 2816 (2560 with more than two query heads a key head; odd multiples of 128
+// have slots of half the size and go up to 3456 and 3200).  Anything else takes the chain of kernels of decode.cu.
 void decode_step_plan(const femto_handle* h, int max_batch, DecodeStepState& st) {
   st.blocks_n = st.columns = 0;
   if (!h->bf || h->hd != HD || (h->d & 127) || (h->Vp & (TILE - 1)) || h->H % h->Hkv || h->H / h->Hkv > 8 || h->d > 128 * 32) return;
