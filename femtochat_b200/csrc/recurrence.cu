@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(256) k_conv_tail(const DeltaPrepArgs a) {
 // q, k and its own v, decays and gates; the decays reach the others through distributed shared memory, the state's rows are
 // on their way to registers meanwhile, and the squares for the norm meet the same way.  A warp has whole rows of the state.  Clocks of
 // one block's thread (10 heads, 128 x 128) found what to mend: four rows a warp where it has one, and 4-way bank conflicts, were 5.5 us of 14.
-// From the projections' end, one column: 14.4 us with those, 8.3 without; 10.2 since the norms before the projections end earlier.
+// From the projections' end, one column: 14.4 us with those, 8.3 without (10.2 in the chain as it is now).
 __device__ __forceinline__ float sigmoid_f(float z) { return 1.f / (1.f + expf(-z)); }
 
 __device__ __forceinline__ void store_peer(const float* p, uint32_t rank, float v) {

@@ -150,6 +150,17 @@ def test_models_with_experts_sum_in_one_order():
     ok(model)
 
 
+@pytest.mark.parametrize("layer", [dc.sinks(heads=2, kv_heads=1, dim=72, vdim=24, size=40), dc.sinks(heads=4, kv_heads=2, dim=64, vdim=128, size=40),
+                                   dc.differential(heads=2, kv_heads=1, dim=64, vdim=64, size=40)])
+def test_one_token_whose_key_tiles_fill_48_kilobytes(layer):
+    """Keys and values padded to 128 + 64 channels take 48 KB of dynamic shared memory, beside the kernel's own."""
+    cfg = dc.zurevik(layer, width=64)
+    model, w = dc.model_and_weights(cfg, (8, 8), "bfloat16", seed=17)
+    t = dc.tokens(20, cfg["vocab"], 90)
+    assert dc.rel_error(dc.feed(model, cache_for(model, 20), t, (12,) + (1,) * 8), lo.Sequence(cfg, w).feed(t)) < TOL["bfloat16"]
+    ok(model)
+
+
 def test_fp32_products_of_models_with_experts_sum_in_one_order():
     """The same for products with fp32 results, which the persistent kernel cuts by their number of rows: the decays of a delta rule beside
     experts, 5120 columns from a rank of 520.  44 rows take narrow tiles and 143 the persistent kernel, with three ranges of K if it may cut it."""
