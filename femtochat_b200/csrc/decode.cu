@@ -432,7 +432,7 @@ extern "C" int32_t femto_kv_cache_create(femto_handle* h, int32_t max_batch, int
     decode_step_carve(h, p, c->step);
     if (const int r = decode_step_setup(h, c->step, c->K, c->V)) { cudaFree(c->mem); delete c; return r; }
   }
-  h->decodes = true;
+  c->share = h->caches;
   *out = c;
   return 0;
 }

@@ -20,6 +20,7 @@ struct LayerState {
 
 struct femto_kv_cache {
   femto_handle* h = nullptr;
+  std::shared_ptr<int> share;                 // GPT: of h->caches
   int maxB = 0, maxT = 0, B = 0, len = 0;     // len: tokens cached per column (all columns alike)
   char* mem = nullptr;
   std::vector<void*> K, V;                    // GPT, per block: [maxB][maxT][kv] of the compute type

@@ -644,7 +644,7 @@ int model_step(femto_handle* h, const float* theta, float* delta, const int* tok
   const bool two = backward && h->hi && h->lo && !gemm_profiling();
   // The tokens behind a prompt, or behind an evaluation between them, read the copies, whatever is written to Theta meanwhile: where there is
   // a cache, those of the tables are made too.
-  FEMTO_TRY(model_ensure_weights(h, theta, backward || h->decodes, s));
+  FEMTO_TRY(model_ensure_weights(h, theta, backward || h->decodes(), s));
   cudaStream_t chain = two ? h->hi : s;
   if (two) {
     cudaEvent_t e = h->ev_fork[h->ev_next++ % femto_handle::N_FORK];

@@ -1,6 +1,7 @@
 // The handle behind the C ABI: configuration, flat layout, workspace arena and the
 // forward / reverse schedule of the GPT step.
 #pragma once
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -42,7 +43,10 @@ struct femto_handle {
   bool weights_valid = false;
   bool weights_changed = false;   // Theta was written since: the next call that reads the copies makes them from the Theta it is given
   bool tables_live = false;       // ... all but those of the embedding tables, whose rows calls that do not train read from their Theta
-  bool decodes = false;           // a cache was made: its tokens read the copies that the call before them left, those of the tables too
+  // Every cache of the handle has a share of this (and may outlive the handle).  Where there is one, its tokens read the copies that the call
+  // before them left, those of the tables too.
+  std::shared_ptr<int> caches = std::make_shared<int>(0);
+  bool decodes() const { return caches.use_count() > 1; }
   struct CastJob* cast_jobs = nullptr;   // device table of model_refresh
   int n_cast_jobs = 0, cast_blocks = 0, cast_tables = 0;      // blocks from cast_tables on are the embedding tables
   int *tok0 = nullptr, *tgt0 = nullptr, *pos = nullptr, *doc_start = nullptr, *raw_tok = nullptr, *raw_tgt = nullptr,

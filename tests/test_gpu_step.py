@@ -579,10 +579,13 @@ def test_tokens_read_the_weights_of_their_prompt(ctype, d, heads, kv, evaluation
         got.append(out + [fb.decode_step(model, kc, tok[:, t]) for t in range(20, 24)])
         kc.close()
     assert all(torch.equal(a, b) for a, b in zip(*got))
-    # the next prompt reads what was written
-    kc = fb.KVCache(model.state(2), 2, 40)
-    assert not torch.equal(fb.prefill(model, kc, tok[:, :20]), got[1][0])
-    kc.close()
+    # the next prompt reads what was written, and so does one behind an evaluation that no cache made copy the tables
+    for _ in range(2):
+        kc = fb.KVCache(model.state(2), 2, 40)
+        got.append([fb.prefill(model, kc, tok[:, :20])] + [fb.decode_step(model, kc, tok[:, t]) for t in range(20, 24)])
+        kc.close()
+        model(tok, tgt, reduction="none")
+    assert not torch.equal(got[2][0], got[1][0]) and all(torch.equal(a, b) for a, b in zip(*got[2:]))
 
 
 @pytest.mark.gpu
